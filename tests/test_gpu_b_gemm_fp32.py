@@ -67,3 +67,23 @@ def test_fp32_class_bias_relu_and_4096_sampled_rows(gpu):
     rows = g.choice(4096, size=32, replace=False)
     err = so.rel_frobenius(dc.numpy()[rows], so.matmul(False, True, 1.0, a[rows], b, 0.0, None))
     assert err <= TOL_F32
+
+
+@pytest.mark.parametrize("at,bt,shift_a,shift_b", [(False, True, 1, 0), (True, False, 0, 3), (False, False, 2, 1)])
+def test_fp32_class_takes_operands_off_the_16_byte_grid(gpu, at, bt, shift_a, shift_b):
+    """The split kernel reads an operand that is only 4-byte aligned element by element: the same bits as the
+    aligned operand gives (same arithmetic), including the sums' order when there is no split along K."""
+    m, n, k = 132, 68, 36
+    a, b, _ = _operands(5, at, bt, m, n, k, "normal")
+
+    def place(x, shift):
+        flat = gpu.DeviceArray.from_numpy(np.concatenate([np.zeros(shift, np.float32), x.ravel()]))
+        return flat.view(x.shape, "f32", 4 * shift)
+
+    out = []
+    for sa, sb in ((0, 0), (shift_a, shift_b)):
+        dc = gpu.DeviceArray((m, n), "f32")
+        gpu.matmul(at, bt, 1.0, place(a, sa), place(b, sb), 0.0, dc, in_dtype="f32")
+        out.append(dc.numpy())
+    np.testing.assert_array_equal(out[0], out[1])
+    assert so.rel_frobenius(out[0], so.matmul(at, bt, 1.0, a, b, 0.0, None)) <= TOL_F32
