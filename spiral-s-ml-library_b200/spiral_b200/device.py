@@ -7,6 +7,7 @@ This package accepts anything that can name a device address -- a
 integer -- and passes the raw pointer through the C ABI.
 """
 import ctypes
+import math
 
 import numpy as np
 
@@ -68,7 +69,7 @@ class DeviceArray:
             raise ValueError("unknown dtype %r" % (dtype,))
         self.shape = tuple(int(s) for s in (shape if isinstance(shape, (tuple, list)) else (shape,)))
         self.dtype = dtype
-        self.size = int(np.prod(self.shape)) if self.shape else 1
+        self.size = math.prod(self.shape)
         self.nbytes = self.size * _ITEMSIZE[dtype]
         self._owner = owner
         self._owned = ptr is None

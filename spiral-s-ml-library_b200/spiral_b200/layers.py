@@ -14,6 +14,8 @@ global-memory pass for every activation and head; here ``graph_run_host`` fuses
 only nodes that cannot be fused run as stand-alone kernels.  Tensors are 3-D in
 the reference (blocks, rows, features); the leading dimensions are the batch.
 """
+import math
+
 import numpy as np
 
 from . import primitives
@@ -35,7 +37,7 @@ class Node:
 
     @property
     def rows(self):
-        return int(np.prod(self.dims[:-1]))
+        return int(math.prod(self.dims[:-1]))
 
     @property
     def cols(self):
