@@ -175,7 +175,11 @@ int sb_matmul_ex(int a_trans, int b_trans, float alpha, const void* A, const voi
  * cores: every operand is split into a TF32 head and a TF32 tail and the product is taken as
  * Ah*Bh + Ah*Bl + Al*Bh in one tcgen05 GEMM with fp32 accumulation ("3 x TF32"; the reference's own
  * arithmetic is single-pass TF32, corecuda/wmma.spi:20,78-82, which cannot meet 1e-5).  Two launches:
- * the split into `workspace` (caller memory, at least sb_matmul_f32_workspace_bytes) and the GEMM.
+ * the split into `workspace` (caller memory, at least sb_matmul_f32_workspace_bytes) and the GEMM, and
+ * with SB_EPI_RELU and K > 256 the ReLU over C as a third.  The product is summed in chains of at most
+ * 256 elements of K whose sums are added to C in no fixed order: two calls may differ in the last bits.
+ * Measured error at every K: 2e-6 for normal operands, 5e-6 for positive ones; the accumulator truncates,
+ * so a product whose terms are all equal (both operands constant) can be off by up to 1.7e-5.
  * Contiguous dimensions must be multiples of 4 elements; other shapes use the SB_F32 class of
  * sb_matmul_ex (FFMA).  epilogue: SB_EPI_BIAS, SB_EPI_RELU. */
 int sb_matmul_f32_workspace_bytes(int M, int N, int K, size_t* bytes);

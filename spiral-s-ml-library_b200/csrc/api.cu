@@ -92,8 +92,8 @@ struct SplitJob {
   int part[3];
 };
 
-// c_init: when non-null the same launch also brings C to beta * C (zero for beta == 0), the state the
-// split-K tiles are then added to.
+// c_init: when non-null the same launch also brings C [c_count / c_cols, c_cols] to beta * C + bias (C is not read
+// for beta == 0; bias: only with BIAS), the state the split-K tiles are then added to.
 //
 // Bound by what it moves (4 bytes read, 12 written per operand element; the workspace mostly stays in L2), so a
 // thread takes four elements at a time: every contiguous dimension is a multiple of 4 (the caller's check), so a
@@ -123,20 +123,26 @@ __device__ __forceinline__ void split_quad(const SplitJob& j, bool vec, long lon
   for (int p = 0; p < 3; ++p) *reinterpret_cast<float4*>(j.dst + base + p * pitch) = j.part[p] ? lo : hi;
 }
 
+template <bool BIAS>
 __global__ void __launch_bounds__(256)
-split3_kernel(SplitJob ja, SplitJob jb, float* c_init, long long c_count, float beta, int vec_a, int vec_b) {
+split3_kernel(SplitJob ja, SplitJob jb, float* c_init, long long c_count, int c_cols, float beta, const float* bias,
+              int vec_a, int vec_b) {
   sb_grid_dependency_wait();
   sb_grid_dependents_launch();
   const long long na = ja.rows * ja.cols / 4, total = na + jb.rows * jb.cols / 4;
   const long long step = (long long)gridDim.x * blockDim.x;
   const long long first = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c_init) {                      // C is 16-byte aligned and N a multiple of 32 wherever it is initialised here
+  if (c_init) {                      // C is 16-byte aligned and its rows are whole quads (the caller's check)
     float4* c4 = reinterpret_cast<float4*>(c_init);
     for (long long t = first; t < c_count / 4; t += step) {
       float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
       if (beta != 0.0f) {
         v = c4[t];
         v = make_float4(beta * v.x, beta * v.y, beta * v.z, beta * v.w);
+      }
+      if (BIAS) {                    // only 4-byte aligned
+        const float* b = bias + 4 * (t % (c_cols / 4));
+        v = make_float4(v.x + b[0], v.y + b[1], v.z + b[2], v.w + b[3]);
       }
       c4[t] = v;
     }
@@ -190,14 +196,21 @@ int sb_matmul_f32x3(int a_trans, int b_trans, float alpha, const float* A, const
   const long long cap = (long long)sb_sm_count() * 16;
   if (blocks > cap) blocks = cap;
   cudaStream_t s = (cudaStream_t)stream;
-  // Split-K with the tiles ADDED to C (TMA reduce-add) serves two ends.  Accuracy: the tensor core's
-  // fp32 accumulator does not round to nearest, so a long chain of accumulations drifts (4e-5 at
-  // K = 4096 in one pass); chains of at most 256 elements of K per part stay far below 1e-5 and the
-  // additions between chains are ordinary fp32 additions.  Parallelism: a 512 x 512 output is four
-  // tiles; with the splits it is spread over the whole GPU.  Needs a plain product (no bias / ReLU)
-  // and whole 32-column chunks; C is first brought to beta * C (zero for beta == 0).
+  // Split-K with the tiles ADDED to C (TMA reduce-add) serves two ends.  Accuracy: the tensor core's fp32
+  // accumulator does not round to nearest, so a chain of accumulations drifts in proportion to its length.  Relative
+  // Frobenius error of ONE chain, 1024 x 1020, normal / positive / positive operands constant along K: 2.7e-6 /
+  // 3.7e-6 / 4.6e-6 at K = 256, 5.3e-6 / 7.5e-6 / 9.3e-6 at 512, 1.1e-5 / 1.5e-5 / - at 1024, 4.2e-5 / 6.2e-5 / - at
+  // 4096: over the 1e-5 of this class from K = 600 on.  Chains of at most 256 elements of K keep 1.9e-6 / 5.1e-6 at
+  // K = 4096 and 2.0e-6 / 5.3e-6 at 262144, for every width and epilogue; the additions between chains are ordinary
+  // fp32 additions.  Parallelism: a 512 x 512 output is four tiles; with the splits it is spread over the whole GPU.
+  // Against one chain: 500 x 500 x 1024 37 -> 17 us, 1024 x 1020 x 2048 68 -> 44, 2048 x 2044 x 260 24 -> 30,
+  // 2048 x 2044 x 2048 94 -> 103.
+  // C is first brought to beta * C + bias by the split kernel.  A ReLU needs the complete sum and becomes a pass over
+  // C, so such a product is split only where its accuracy needs it (512 x 512 x 1024 36 -> 19 us,
+  // 2048 x 2048 x 2048 94 -> 108, 2048 x 2048 x 260 24 -> 38).  Below 3 * K = 512 there is nothing to gain for either end.
+  const bool relu = (epilogue & SB_EPI_RELU) != 0;
   int splits = 1;
-  if (epilogue == 0 && N % 32 == 0 && 3 * K >= 512) {
+  if (3LL * K >= 512 && !(relu && K <= 256)) {
     const int by_accuracy = (K + 255) / 256;
     const long long tiles = (long long)((M + 255) / 256) * ((N + 255) / 256);
     long long by_fill = tiles > 0 ? (sb_sm_count() / 2) / tiles : 1;                // one wave of CTA pairs
@@ -205,24 +218,25 @@ int sb_matmul_f32x3(int a_trans, int b_trans, float alpha, const float* A, const
     const int by_k = (3 * K) / 128 > 0 ? (3 * K) / 128 : 1;                          // at least two k-blocks of 64 per split
     long long want = by_accuracy > by_fill ? by_accuracy : by_fill;
     if (want > by_k) want = by_k;
-    if (want > 128) want = 128;
     splits = (int)(want < 1 ? 1 : want);
   }
-  const bool init_c = splits > 1 && beta != 1.0f;
-  SB_CUDA(sb_launch(split3_kernel, dim3((int)blocks), dim3(256), 0, s, 1, ja, jb, init_c ? C : (float*)nullptr,
-                    (long long)M * N, beta, (reinterpret_cast<uintptr_t>(A) & 15) == 0 ? 1 : 0,
+  const float* init_bias = splits > 1 && (epilogue & SB_EPI_BIAS) ? bias : nullptr;
+  const bool init_c = splits > 1 && (beta != 1.0f || init_bias);
+  SB_CUDA(sb_launch(init_bias ? split3_kernel<true> : split3_kernel<false>, dim3((int)blocks), dim3(256), 0, s, 1, ja, jb, init_c ? C : (float*)nullptr,
+                    (long long)M * N, N, beta, init_bias, (reinterpret_cast<uintptr_t>(A) & 15) == 0 ? 1 : 0,
                     (reinterpret_cast<uintptr_t>(B) & 15) == 0 ? 1 : 0));
   SB_COUNT_LAUNCH();
   SB_CUDA(cudaGetLastError());
   if (splits > 1) {
     int used = 0;
     // `C` doubles as the partials pointer: every condition for adding into C holds here by construction
-    // (fp32 output, no epilogue, aligned rows, whole chunks), so no partial is ever written.
+    // (fp32 output, no epilogue in the GEMM, aligned rows; the plan takes whole 32-column chunks per tile and
+    // the boxes are clipped at N), so no partial is ever written.
     int rc = sb_umma_gemm_launch(a_trans, b_trans, alpha, a3, b3, 0.0f, C, M, N, 3 * K, SB_TF32, SB_F32, 0, nullptr, nullptr,
                                  nullptr, nullptr, s, splits, &used, nullptr, C);
     if (rc != SB_OK) return rc;
     if (used != 1) return sb_fail(SB_ERR_UNSUPPORTED, "internal: sb_matmul_f32x3 expected its splits to be added into C");
-    return SB_OK;
+    return relu ? sb_relu(C, C, (size_t)M * N, stream) : SB_OK;
   }
   return sb_umma_gemm_launch(a_trans, b_trans, alpha, a3, b3, beta, C, M, N, 3 * K, SB_TF32, SB_F32, epilogue, bias, nullptr,
                              nullptr, nullptr, s);

@@ -87,3 +87,47 @@ def test_fp32_class_takes_operands_off_the_16_byte_grid(gpu, at, bt, shift_a, sh
         out.append(dc.numpy())
     np.testing.assert_array_equal(out[0], out[1])
     assert so.rel_frobenius(out[0], so.matmul(at, bt, 1.0, a, b, 0.0, None)) <= TOL_F32
+
+
+@pytest.mark.parametrize("at,bt,m,n,k,epilogue,beta", [
+    (False, True, 129, 20, 2048, (), 0.0), (False, True, 300, 252, 2048, (), -0.5), (True, False, 128, 1020, 2048, (), 0.0),
+    (False, False, 260, 36, 4096, (), 1.0), (True, True, 64, 4, 4096, (), 0.0), (False, True, 1, 36, 2048, (), -0.5),
+    (False, True, 300, 128, 2048, ("bias",), 1.0), (False, False, 129, 100, 2048, ("bias",), -0.5),
+    (False, True, 300, 128, 2048, ("relu",), 0.0), (True, False, 132, 252, 2048, ("bias", "relu"), 0.0),
+    (False, True, 70, 256, 4096, ("bias", "relu"), -0.5), (False, True, 257, 68, 260, ("bias", "relu"), 0.0),
+    (False, True, 64, 96, 256, ("bias", "relu"), 0.0), (False, True, 64, 68, 176, ("bias",), 1.0)])
+@pytest.mark.parametrize("dist", ["normal", "positive"])
+def test_fp32_class_holds_for_long_k_ragged_n_and_epilogues(gpu, at, bt, m, n, k, epilogue, beta, dist):
+    """The chains of accumulations that the tensor core makes are cut whatever the width of C and the epilogue: a
+    single chain is off by 1.1e-5 (normal) and 1.5e-5 (positive operands) at K = 1024, more in proportion beyond."""
+    g = so.rng(m + n + k)
+    draw = (lambda s: g.uniform(0, 1, size=s)) if dist == "positive" else (lambda s: g.normal(size=s))
+    a, b = draw((k, m) if at else (m, k)).astype(np.float32), draw((n, k) if bt else (k, n)).astype(np.float32)
+    c, bias = g.normal(size=(m, n)).astype(np.float32), g.normal(size=n).astype(np.float32)
+    want = so.matmul(at, bt, 1.5, a, b, beta, c)
+    if beta == 0:
+        c[:] = np.nan                                        # not read
+    if "bias" in epilogue:
+        want = want + bias
+    if "relu" in epilogue:
+        want = so.relu(want)
+    dc = gpu.DeviceArray.from_numpy(c)
+    gpu.matmul(at, bt, 1.5, gpu.DeviceArray.from_numpy(a), gpu.DeviceArray.from_numpy(b), beta, dc, in_dtype="f32",
+               epilogue=epilogue, bias=gpu.DeviceArray.from_numpy(bias) if "bias" in epilogue else None)
+    assert so.rel_frobenius(dc.numpy(), want) <= TOL_F32
+
+
+@pytest.mark.parametrize("n,epilogue", [(64, ()), (36, ("bias", "relu"))])
+def test_fp32_class_holds_for_very_long_k(gpu, n, epilogue):
+    """K = 200000: 782 parts."""
+    m, k = 64, 200000
+    g = so.rng(8)
+    a, b = g.uniform(0, 1, size=(m, k)).astype(np.float32), g.uniform(0, 1, size=(n, k)).astype(np.float32)
+    bias = g.normal(size=n).astype(np.float32)
+    want = so.matmul(False, True, 1.0, a, b, 0.0, None)
+    if epilogue:
+        want = so.relu(want + bias)
+    dc = gpu.DeviceArray((m, n), "f32")
+    gpu.matmul(False, True, 1.0, gpu.DeviceArray.from_numpy(a), gpu.DeviceArray.from_numpy(b), 0.0, dc, in_dtype="f32",
+               epilogue=epilogue, bias=gpu.DeviceArray.from_numpy(bias) if epilogue else None)
+    assert so.rel_frobenius(dc.numpy(), want) <= TOL_F32
