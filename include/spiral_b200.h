@@ -386,11 +386,13 @@ int sb_policy_decide(const sb_decide_args* args, void* stream);
  * SB_STATIC_WORKSPACE_BYTES (32 MiB, held by every GPU that loads the library
  * until the process exits); larger requests return SB_ERR_TOO_LARGE.  It calls
  * no cudaMalloc / cudaFree.  The first call on a device looks up the array's
- * device address and sets kernel attributes; make that call before starting any
- * stream capture.  All calls share the one array and it keeps the last call's
- * contents (every byte used is rewritten before it is read, so nothing needs
- * clearing): two calls that overlap on the GPU -- different streams, or
- * different host threads -- race on it. */
+ * device address, creates one event and sets kernel attributes; make that call
+ * before starting any stream capture.  All calls share the one array and it
+ * keeps the last call's contents (every byte used is rewritten before it is
+ * read, so nothing needs clearing).  A call waits on the GPU for the one before
+ * it, whatever streams and host threads they come from.  Launches captured into
+ * a graph are not part of that order: whoever launches such a graph keeps it
+ * from overlapping with other users of the array. */
 #define SB_STATIC_WORKSPACE_BYTES (32u * 1024u * 1024u)
 int sb_mlp_forward_static(int n_layers, const int* sizes, int batch, int in_dtype, const void* x,
                           const void* w_compute, const float* params, int head, const uint8_t* mask,

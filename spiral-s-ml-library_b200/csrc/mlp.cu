@@ -18,6 +18,7 @@
 // all-reduce), per-layer activation buffers and one scratch buffer.
 #include "common.cuh"
 
+#include <mutex>
 
 namespace {
 
@@ -589,25 +590,31 @@ int sb_mlp_forward(int n_layers, const int* sizes, int batch, int in_dtype, cons
 // In host code the name `g_static_workspace` is only a host-side stand-in for
 // the symbol, not a device address; the real address is looked up once per
 // device with cudaGetSymbolAddress and that pointer is what the kernels get.
+//
+// All calls on a device use the one array, so a call waits on the GPU for the
+// call before it, whatever streams and host threads the two come from: its
+// stream waits for the event that the call before recorded behind its last
+// launch.  A stream under capture takes no part in this (its launches run when
+// the graph does, and an event of a capture may not be waited for outside it).
 // ---------------------------------------------------------------------------
 static __device__ __align__(256) unsigned char g_static_workspace[SB_STATIC_WORKSPACE_BYTES];
 
 namespace {
-unsigned char* g_static_workspace_addr[64] = {nullptr};
+struct StaticWorkspace {
+  std::mutex lock;                 // held while a call is issued: wait, launches, record
+  unsigned char* addr = nullptr;   // device address, looked up on the device's first call
+  cudaEvent_t done = nullptr;      // behind the last launch of the last call that was not captured
+};
+StaticWorkspace g_static_ws[64];
 
-// Device address of the static workspace on the current device (looked up on
-// the first call per device, with that device current).
-int static_workspace_address(unsigned char** out) {
-  int dev = 0;
-  SB_CUDA(cudaGetDevice(&dev));
-  if (dev < 0 || dev >= 64) return sb_fail(SB_ERR_UNSUPPORTED, "sb_mlp_forward_static: device index %d out of range", dev);
-  if (!g_static_workspace_addr[dev]) {
-    void* p = nullptr;
-    SB_CUDA(cudaGetSymbolAddress(&p, g_static_workspace));
-    if (!p) return sb_fail(SB_ERR_CUDA, "sb_mlp_forward_static: cudaGetSymbolAddress returned a null address");
-    g_static_workspace_addr[dev] = reinterpret_cast<unsigned char*>(p);
-  }
-  *out = g_static_workspace_addr[dev];
+// Looks up what the current device's first call needs; `ws->lock` is held.
+int static_workspace_init(StaticWorkspace* ws) {
+  if (ws->addr) return SB_OK;
+  if (!ws->done) SB_CUDA(cudaEventCreateWithFlags(&ws->done, cudaEventDisableTiming));
+  void* p = nullptr;
+  SB_CUDA(cudaGetSymbolAddress(&p, g_static_workspace));
+  if (!p) return sb_fail(SB_ERR_CUDA, "sb_mlp_forward_static: cudaGetSymbolAddress returned a null address");
+  ws->addr = reinterpret_cast<unsigned char*>(p);
   return SB_OK;
 }
 }  // namespace
@@ -630,14 +637,26 @@ int sb_mlp_forward_static(int n_layers, const int* sizes, int batch, int in_dtyp
     return sb_fail(SB_ERR_TOO_LARGE,
                    "sb_mlp_forward_static: hidden activations need %zu bytes, the built-in workspace holds %zu; "
                    "use sb_mlp_forward with caller memory for this batch", offset, (size_t)SB_STATIC_WORKSPACE_BYTES);
-  unsigned char* base = nullptr;
-  rc = static_workspace_address(&base);
+  int dev = 0;
+  SB_CUDA(cudaGetDevice(&dev));
+  if (dev < 0 || dev >= 64) return sb_fail(SB_ERR_UNSUPPORTED, "sb_mlp_forward_static: device index %d out of range", dev);
+  StaticWorkspace& ws = g_static_ws[dev];
+  std::lock_guard<std::mutex> guard(ws.lock);
+  rc = static_workspace_init(&ws);
   if (rc != SB_OK) return rc;
-  for (int i = 0; i + 1 < n_layers; ++i) acts[i] = base + offsets[i];
+  for (int i = 0; i + 1 < n_layers; ++i) acts[i] = ws.addr + offsets[i];
+  cudaStream_t s = (cudaStream_t)stream;
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  SB_CUDA(cudaStreamIsCapturing(s, &capture));
+  const bool ordered = n_layers > 1 && capture == cudaStreamCaptureStatusNone;
+  if (ordered) SB_CUDA(cudaStreamWaitEvent(s, ws.done, 0));     // returns at once for an event never recorded
   // Every slab is completely overwritten by its layer before the next layer
   // reads it, so nothing left behind by an earlier call needs clearing.
-  return sb_mlp_forward(n_layers, sizes, batch, in_dtype, x, w_compute, params, n_layers > 1 ? acts : nullptr,
-                        nullptr, head, mask, out, actions, stream);
+  rc = sb_mlp_forward(n_layers, sizes, batch, in_dtype, x, w_compute, params, n_layers > 1 ? acts : nullptr,
+                      nullptr, head, mask, out, actions, stream);
+  // Also behind a call that failed: some of its layers may have been launched.
+  if (ordered) SB_CUDA(cudaEventRecord(ws.done, s));
+  return rc;
 }
 
 int sb_mlp_backward_scratch_bytes(int n_layers, const int* sizes, int batch, int in_dtype, size_t* bytes) {

@@ -170,8 +170,9 @@ class PolicyMLP:
         For callers that may not allocate device memory (no allocator of their own, a context where
         allocation is forbidden, inside a stream capture).  `out` (fp32 [batch, actions]) and
         `actions` (int32 [batch], for argmax heads) are caller buffers.  Raises SpiralError
-        (SB_ERR_TOO_LARGE) when batch x hidden widths does not fit.  Calls share the one workspace:
-        do not overlap two of them on the GPU.
+        (SB_ERR_TOO_LARGE) when batch x hidden widths does not fit.  Calls share the one workspace and
+        run one after the other on the GPU, whatever streams and threads they come from; only a graph
+        that captured such a call must be kept from overlapping with others.
         """
         flags = self.head_flags if head_flags is None else head_flags
         _lib.call("sb_mlp_forward_static", self.n_layers, self._sizes_c, self.batch,

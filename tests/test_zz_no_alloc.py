@@ -8,6 +8,7 @@ tolerance the other MLP tests use (2e-3 relative Frobenius error); both paths ru
 kernels, so the results are normally identical.
 """
 import ctypes
+import threading
 
 import numpy as np
 import pytest
@@ -53,3 +54,44 @@ def test_no_alloc_forward_rejects_what_does_not_fit(gpu):
         _lib.call("sb_mlp_forward_static", 2, sizes, 65536, _lib.BF16, 16, 16, None, 8, None, 16, None, None)
     assert err.value.code == -6          # SB_ERR_TOO_LARGE
     assert "workspace" in str(err.value)
+
+
+def test_no_alloc_forwards_of_two_streams_and_threads_do_not_share_the_workspace_at_once(gpu):
+    """Calls with nothing between them but the library, on two streams, first from one host thread and then from
+    two: every result equals, bit for bit, what the net with a workspace of its own gives."""
+    calls = 24
+    jobs = []
+    for seed, sizes, batch in ((5, [32, 256, 256, 256, 3], 8192), (6, [64, 512, 512, 10], 4096)):
+        ws, bs = so.mlp_weights(seed, sizes)
+        net = gpu.PolicyMLP(sizes, batch, in_dtype="f16", head=("masked_softmax",))
+        net.load_weights(ws, bs)
+        xs = [gpu.to_storage(so.rng(10 * seed + i).random((batch, sizes[0]), dtype=np.float32), "f16") for i in range(2)]
+        want = [net.forward(x).numpy() for x in xs]
+        outs = [gpu.DeviceArray((batch, sizes[-1]), "f32") for _ in range(calls)]
+        jobs.append((net, xs, want, outs, gpu.Stream()))
+
+    def issue(job, i):
+        net, xs, _, outs, stream = job
+        net.forward_no_alloc(xs[i % 2], outs[i], stream=stream.ptr)
+
+    def check():
+        for net, xs, want, outs, stream in jobs:
+            stream.synchronize()
+            for i, out in enumerate(outs):
+                np.testing.assert_array_equal(out.numpy(), want[i % 2])
+                out.fill_zero()
+        gpu.synchronize()
+
+    for out in jobs[0][3] + jobs[1][3]:
+        out.fill_zero()
+    gpu.synchronize()
+    for i in range(calls):
+        for job in jobs:
+            issue(job, i)
+    check()
+    threads = [threading.Thread(target=lambda j=job: [issue(j, i) for i in range(calls)]) for job in jobs]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    check()
