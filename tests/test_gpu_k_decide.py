@@ -148,3 +148,58 @@ def test_holdem_cem_shape_512_to_64(gpu):
     with pytest.raises(gpu.SpiralError) as err:
         gpu.EnsemblePolicyMLP([512, 256, 64], 128, 2, in_dtype="bf16").forward_head(gpu.DeviceArray((128, 512), "bf16"), prefix=3)
     assert err.value.code == -3
+
+
+@pytest.mark.parametrize("path", ["fused", "layerwise", "decide"])
+@pytest.mark.parametrize("rows", [256, "limit - 1", "limit", "limit + 1"])
+def test_encoder_and_net_queued_without_synchronisation(gpu, path, rows):
+    """encode -> net -> encode -> net on one stream, all through ONE input matrix, the records replaced on the
+    stream between rounds: the encoder moves up beside the kernel before it and lets the net move up beside itself
+    (up to one piece of 16 bytes per thread), and nothing may be read early or overwritten while it is read.  The
+    same bits as with a synchronisation after every call."""
+    from spiral_b200 import _lib
+    limit = gpu.sm_count() * 16 * 256 // 4             # the encoder's threads; 32 features in f16 are 4 pieces
+    rows = {"limit - 1": limit - 1, "limit": limit, "limit + 1": limit + 1}.get(rows, rows)
+    rounds, sizes = 4, [32, 64, 64, 3]
+    src = [gpu.DeviceArray.from_numpy(so.leduc_states(80 + i, rows)[0]) for i in range(3)]
+    records = [gpu.DeviceArray((rows, len(so.LEDUC_WIDTHS)), "u8") for _ in range(2)]
+    x = gpu.DeviceArray((rows, 32), "f16")
+    nets = []
+    for j in range(2):
+        if path == "decide":
+            nets.append(gpu.EnsemblePolicyMLP(sizes, rows, 2, in_dtype="f16", with_bias=False))
+            nets[j].load_weights(member_weights(760 + 10 * j, sizes, 2))
+        else:
+            nets.append(gpu.PolicyMLP(sizes, rows, in_dtype="f16"))
+            nets[j].load_weights(*so.mlp_weights(760 + j, sizes))
+    copies = [[gpu.DeviceArray(net.probs.shape, "f32") for net in nets] for _ in range(rounds)]
+
+    def copy(dst, a):
+        _lib.call("sb_memcpy_d2d", dst.ptr, a.ptr, a.nbytes, None)
+
+    def run(after_each):
+        for out in copies[0] + copies[1] + copies[2] + copies[3]:
+            out.fill_zero()
+        for r in range(rounds):
+            for j in range(2):
+                copy(records[j], src[(r + j) % 3])
+            after_each()
+            for j, net in enumerate(nets):
+                if path == "decide":
+                    net.decide(r, fields=records[j], widths=so.LEDUC_WIDTHS)
+                else:
+                    gpu.primitives.encode_states(records[j], so.LEDUC_WIDTHS, None, x)
+                    after_each()
+                    (net.forward_fused if path == "fused" else net.forward)(x)
+                after_each()
+            for j, net in enumerate(nets):
+                copy(copies[r][j], net.probs)
+            after_each()
+        return [[out.numpy() for out in pair] for pair in copies]
+
+    want = run(gpu.synchronize)
+    got = run(lambda: None)
+    for r in range(rounds):
+        for j in range(2):
+            np.testing.assert_array_equal(got[r][j], want[r][j])
+    assert not np.array_equal(want[0][0], want[1][0])
