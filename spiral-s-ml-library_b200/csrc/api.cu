@@ -98,9 +98,9 @@ struct SplitJob {
 // Bound by what it moves (4 bytes read, 12 written per operand element; the workspace mostly stays in L2), so a
 // thread takes four elements at a time: every contiguous dimension is a multiple of 4 (the caller's check), so a
 // quad never crosses a row and its three destinations are 16-byte aligned.  The operands themselves need only be
-// 4-byte aligned: VEC_A / VEC_B say which of them can be read as quads.  One element per thread with a 64-bit
-// division each was bound by issue instead: for a 2048^3 product 52 -> 23 us for this kernel (134 MB moved, most of
-// it in L2), 137 -> 113 us for the call; at 512^3 6.9 -> 4.9 us and 14.8 -> 13.3 us.
+// 4-byte aligned: vec_a / vec_b say which of them can be read as quads.  One element per thread with a 64-bit
+// division each was bound by issue instead: for a 2048^3 product 52 -> 23 us for this kernel (151 MB moved, 17 of them
+// C brought to zero, most of it in L2), 137 -> 113 us for the call; at 512^3 6.9 -> 4.9 us and 14.8 -> 13.3 us.
 __device__ __forceinline__ float4 load_quad(const float* p, bool vec) {
   return vec ? *reinterpret_cast<const float4*>(p) : make_float4(p[0], p[1], p[2], p[3]);
 }
@@ -111,7 +111,7 @@ __device__ __forceinline__ void split_quad(const SplitJob& j, bool vec, long lon
   const float4 lo = make_float4(tf32_rn(x.x - hi.x), tf32_rn(x.y - hi.y), tf32_rn(x.z - hi.z), tf32_rn(x.w - hi.w));
   long long base, pitch;             // where part 0 of this quad goes, and from one part to the next
   if (j.k_is_col) {
-    const uint32_t cq = (uint32_t)(j.cols >> 2);
+    const uint32_t cq = (uint32_t)(j.cols >> 2);      // the 64-bit form: operands from 69 GB on, with a workspace in managed memory
     const long long r = quad <= 0xffffffffLL ? (long long)((uint32_t)quad / cq) : quad / cq;
     base = 4 * quad + 2 * r * j.cols;
     pitch = j.cols;

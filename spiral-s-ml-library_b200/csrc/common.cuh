@@ -110,9 +110,13 @@ constexpr int SB_NUM_SMS_FALLBACK = 148;
 // its CTAs set themselves up (barriers, tensor memory, descriptor prefetch) and
 // then block in sb_grid_dependency_wait() until the earlier grid has completed
 // and its writes are visible.  Every kernel launched this way must call
-// sb_grid_dependency_wait() before its first access to global memory, and
-// calls sb_grid_dependents_launch() right after it so that its own successor
-// can move up the same way.  SB_NO_PDL=1 in the environment turns the
+// sb_grid_dependency_wait() before its first access to global memory, in every
+// thread, and may call sb_grid_dependents_launch() only after it, so that its
+// own successor can move up the same way without running ahead of the kernel
+// before both.  All do so right after the wait, except encode_states_kernel,
+// which does so only when a thread has at most one piece to write (beside
+// several passes the successor's resident CTAs cost more than they save).
+// A kernel that does not call it releases its successor by ending.  SB_NO_PDL=1 in the environment turns the
 // attribute off (plain stream order); the device calls are then no-ops.
 __device__ __forceinline__ void sb_grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void sb_grid_dependents_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
