@@ -61,8 +61,9 @@ def matmul(a_trans, b_trans, alpha, a, b, beta, c, in_dtype=None, epilogue=(), b
            aux_in=None, aux_out=None, stream=None):
     """``c <- alpha * op(a) @ op(b) + beta * c`` with an optional fused epilogue.
 
-    ``in_dtype``: 'f32' (FFMA, 1e-5 class), 'tf32' (fp32 storage, TF32 multiply),
-    'bf16', 'f16'; by default fp32 storage runs as 'tf32', the reference's own
+    ``in_dtype``: 'f32' (1e-5 class: 3 x TF32 on the tensor cores where the contiguous
+    dimensions are multiples of 4 and the epilogue is bias / ReLU, FFMA otherwise), 'tf32'
+    (fp32 storage, TF32 multiply), 'bf16', 'f16'; by default fp32 storage runs as 'tf32', the reference's own
     arithmetic.  ``epilogue``: iterable of names from EPILOGUE_FLAGS.
     """
     m, n, k = _dims(bool(a_trans), bool(b_trans), a, b, c)
