@@ -373,8 +373,17 @@ __device__ __forceinline__ void umma_issue(uint32_t tmem_d, uint32_t a_lo, uint3
   }
 }
 
-// 32 lanes x 32-bit, 16 / 32 consecutive columns: thread t of the warp gets
+// 32 lanes x 32-bit, 4 / 8 / 16 / 32 consecutive columns: thread t of the warp gets
 // TMEM lane (lane_base + t), columns [col, col + n).
+__device__ __forceinline__ void tmem_ld4(uint32_t taddr, uint32_t* r) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(taddr) : "memory");
+}
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t* r) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr) : "memory");
+}
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t* r) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
@@ -400,6 +409,22 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t* r) {
 }
 __device__ __forceinline__ void tmem_ld_wait() {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+// The first W columns of a row, for a row head.
+template <int W>
+__device__ __forceinline__ void tmem_ld_head(uint32_t taddr, uint32_t* r) {
+  if constexpr (W == 64) {
+    tmem_ld32(taddr, r);
+    tmem_ld32(taddr + 32u, r + 32);
+  } else if constexpr (W == 32) {
+    tmem_ld32(taddr, r);
+  } else if constexpr (W == 16) {
+    tmem_ld16(taddr, r);
+  } else if constexpr (W == 8) {
+    tmem_ld8(taddr, r);
+  } else {
+    tmem_ld4(taddr, r);
+  }
 }
 
 // ------------------ CTA pairs (cluster of 2, cta_group::2) ------------------

@@ -104,6 +104,7 @@ struct UmmaGemmParams {
   int wide;            // 1: 16-bit output boxes span two chunks (64 columns, 128-byte rows)
   uint32_t epi_offset; // byte offset of the epilogue staging area from the stage base
   SbRowHead head;      // the row head, when epi holds a head flag
+  int head_width;      // columns of a row that the head holds in registers (sb_row_head_width)
   int epi_warps;       // 8 or 16 epilogue warps (the kernel instance launched)
   int reduce_add;      // 1: tiles are added to C through TMA reduce-add stores (split-K into one matrix, peer copies)
   int peer_rows;       // > 0: rows [r * peer_rows, (r + 1) * peer_rows) of C are added to rank r's copy (out map r)
@@ -788,21 +789,19 @@ struct HeadShared {
 __shared__ HeadShared g_head;
 
 // One warp finishes the head rows of its TMEM lane quadrant: a thread holds the first W values of
-// its row (the whole row when N <= W), applies scale / old C / bias / ReLU and hands over to the
-// shared row head.  Out of line for the same reason as epilogue_tile.
+// its row (all that the head needs, sb_row_head_columns), applies scale / old C / bias / ReLU and hands over to the
+// shared row head.  The mask bytes are requested before the wait for the accumulator.  Out of line for the same
+// reason as epilogue_tile; false when the wait expired.
 template <int W>
-__device__ __noinline__ void epilogue_head(uint32_t t_row, long long row, int M) {
+__device__ __noinline__ bool epilogue_head(uint32_t t_row, long long row, int M, uint32_t bar_full, uint32_t parity) {
+  typename SbLegalWord<W>::type legal = 0;
+  if (row < M) legal = sb_row_head_legal<W>(g_head.rh, row);
+  if (!mbar_wait(bar_full, parity, &g_abort_flag, SB_SITE_EPI_TMEM_FULL)) return false;
+  tc_fence_after_sync();
   uint32_t raw[W];
-  if constexpr (W == 64) {
-    tmem_ld32(t_row, raw);
-    tmem_ld32(t_row + 32u, raw + 32);
-  } else if constexpr (W == 32) {
-    tmem_ld32(t_row, raw);
-  } else {
-    tmem_ld16(t_row, raw);
-  }
+  tmem_ld_head<W>(t_row, raw);
   tmem_ld_wait();
-  if (row >= M) return;
+  if (row >= M) return true;
   float* v = reinterpret_cast<float*>(raw);
   const int n = g_head.rh.n;
   float* crow = g_head.C + row * g_head.ldc;
@@ -819,7 +818,8 @@ __device__ __noinline__ void epilogue_head(uint32_t t_row, long long row, int M)
       v[j] = x;
     }
   }
-  sb_row_head_finish<W>(g_head.rh, v, row, crow);
+  sb_row_head_finish<W>(g_head.rh, v, legal, row, crow);
+  return true;
 }
 
 constexpr int EPI_HEAD_MASK = SB_EPI_MASKED_SOFTMAX | SB_EPI_REGRET_MATCHING | SB_EPI_ARGMAX | SB_EPI_SAMPLE | SB_EPI_BINARIZE;
@@ -1090,13 +1090,20 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
       const uint32_t full_bar = smem_u32(&bar_tmem_full[acc]);
       if (EW == 8 && head) {           // row heads always run on the eight-warp instance
         if constexpr (EW == 8) {
-          if (!mbar_wait(full_bar, acc_phase, abortp, SB_SITE_EPI_TMEM_FULL)) break;
-          tc_fence_after_sync();
-          if (half == 0) {               // a thread finishes a whole head row: the second warp of the quadrant idles
-            if (p.block_n > 32) epilogue_head<64>(t_row, (long long)row0_warp + lane, p.M);
-            else if (p.block_n > 16) epilogue_head<32>(t_row, (long long)row0_warp + lane, p.M);
-            else epilogue_head<16>(t_row, (long long)row0_warp + lane, p.M);
+          bool ok;
+          const long long row = (long long)row0_warp + lane;
+          if (half != 0) {               // a thread finishes a whole head row: the second warp of the quadrant idles
+            ok = mbar_wait(full_bar, acc_phase, abortp, SB_SITE_EPI_TMEM_FULL);
+          } else {
+            switch (p.head_width) {
+              case 4: ok = epilogue_head<4>(t_row, row, p.M, full_bar, acc_phase); break;
+              case 8: ok = epilogue_head<8>(t_row, row, p.M, full_bar, acc_phase); break;
+              case 16: ok = epilogue_head<16>(t_row, row, p.M, full_bar, acc_phase); break;
+              case 32: ok = epilogue_head<32>(t_row, row, p.M, full_bar, acc_phase); break;
+              default: ok = epilogue_head<64>(t_row, row, p.M, full_bar, acc_phase); break;
+            }
           }
+          if (!ok) break;
         }
       } else {
         const int n0 = n_blk * p.block_n + (half_tile > 0 ? item_n : 0);
@@ -1389,13 +1396,6 @@ int sb_umma_gemm_launch(int a_trans, int b_trans, float alpha, const void* A, co
   p.M = M; p.N = N; p.K = K;
   p.a_mn = a_trans ? 1 : 0;   // A stored [K,M]: M contiguous
   p.b_mn = b_trans ? 0 : 1;   // B stored [K,N]: N contiguous
-  // Whole 32-column chunks per tile where every chunk must leave as a box: sign words, column sums, and
-  // tiles that are added to C (split-K accumulation, peer copies).
-  plan_umma(p, in_dtype, cached_sm_count(), !(epi & EPI_HEAD_MASK) && sb_pair_mode_enabled(),
-            (epi & (EPI_GATE_MASK | SB_EPI_COLSUM_OUT)) != 0 || (split_partials && splits > 1) || to_peers);
-  p.alpha = alpha; p.beta = beta;
-  p.C = C; p.ldc = N; p.out_dtype = out_dtype;
-  p.epi = epi; p.bias = bias; p.mask = mask; p.aux_in = aux_in; p.aux_out = aux_out;
   if (epi & EPI_HEAD_MASK) {
     if (head) {
       p.head = *head;
@@ -1409,7 +1409,18 @@ int sb_umma_gemm_launch(int a_trans, int b_trans, float alpha, const void* A, co
     if (!sb_umma_head_fits(N, p.head.prefix))
       return sb_fail(SB_ERR_UNSUPPORTED, "a fused row head holds %d columns (%d under a prefix mask of at most %d)",
                      UG_HEAD_MAX_N, UG_HEAD_MAX_TILE_N, UG_HEAD_MAX_N);
+    p.head_width = sb_row_head_width(p.head);
+    // Columns that the head turns into zeros are not multiplied: the tile spans those that it holds in registers.
+    p.N = sb_row_head_columns(p.head) < N ? sb_row_head_columns(p.head) : N;
   }
+  // Whole 32-column chunks per tile where every chunk must leave as a box: sign words, column sums, and
+  // tiles that are added to C (split-K accumulation, peer copies).
+  plan_umma(p, in_dtype, cached_sm_count(), !(epi & EPI_HEAD_MASK) && sb_pair_mode_enabled(),
+            (epi & (EPI_GATE_MASK | SB_EPI_COLSUM_OUT)) != 0 || (split_partials && splits > 1) || to_peers);
+  p.N = N;
+  p.alpha = alpha; p.beta = beta;
+  p.C = C; p.ldc = N; p.out_dtype = out_dtype;
+  p.epi = epi; p.bias = bias; p.mask = mask; p.aux_in = aux_in; p.aux_out = aux_out;
 
   // TMA needs 16-byte aligned bases and row pitches.
   const long long lda = a_trans ? M : K;

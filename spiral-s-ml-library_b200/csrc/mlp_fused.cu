@@ -67,6 +67,7 @@ struct FusedParams {
   // head
   float* out;
   SbRowHead head;                     // n, flags, prefix, mask, seed, ...; argmax_out / sample_out are [members, batch]
+  int head_width;                     // columns of a row that the head holds in registers (sb_row_head_width)
   int hidden_norm;                    // 1: x / sum(x^2) over the row before every ReLU
   // training forward: the hidden activations and their ReLU sign words are also written to global
   // memory for the backward pass (single net only)
@@ -81,29 +82,30 @@ struct FusedParams {
   float* prob_ensemble;               // [batch, members]
 };
 
-// The last layer: a thread takes the first W values of its row out of tensor memory, adds the bias and
-// hands over to the shared row head.
+// The last layer: a thread takes the first W values of its row out of tensor memory (all that the head needs,
+// sb_row_head_columns), adds the bias and hands over to the shared row head.  Bias and mask bytes are requested
+// before the wait for the accumulator.  False when that wait expired.
 template <int W>
-__device__ __noinline__ void fused_head(const SbRowHead& h, const float* bias, float* out, uint32_t t_row, long long row,
-                                        int batch) {
+__device__ __noinline__ bool fused_head(const SbRowHead& h, const float* bias, float* out, uint32_t t_row, long long row,
+                                        int batch, uint32_t bar_full, uint32_t parity, volatile int* abortp) {
+  typename SbLegalWord<W>::type legal = 0;
+  float b[W];
+  if (row < batch) legal = sb_row_head_legal<W>(h, row);
+#pragma unroll
+  for (int j = 0; j < W; ++j) b[j] = bias && j < h.n ? __ldg(bias + j) : 0.f;
+  if (!mbar_wait(bar_full, parity, abortp, SB_SITE_MLP_ACC)) return false;
+  tc_fence_after_sync();
   uint32_t raw[W];
-  if constexpr (W == 64) {
-    tmem_ld32(t_row, raw);
-    tmem_ld32(t_row + 32u, raw + 32);
-  } else if constexpr (W == 32) {
-    tmem_ld32(t_row, raw);
-  } else {
-    tmem_ld16(t_row, raw);
-  }
+  tmem_ld_head<W>(t_row, raw);
   tmem_ld_wait();
-  if (row >= batch) return;
+  if (row >= batch) return true;
   float* v = reinterpret_cast<float*>(raw);
   if (bias) {
 #pragma unroll
-    for (int j = 0; j < W; ++j)
-      if (j < h.n) v[j] += __ldg(bias + j);
+    for (int j = 0; j < W; ++j) v[j] += b[j];
   }
-  sb_row_head_finish<W>(h, v, row, out + row * h.n);
+  sb_row_head_finish<W>(h, v, legal, row, out + row * h.n);
+  return true;
 }
 
 // One warp's share of a hidden layer: chunks `half`, half+2, ... of 32 columns.
@@ -378,26 +380,33 @@ mlp_fused_kernel(const __grid_constant__ FusedMaps maps, const __grid_constant__
       __syncwarp();
       const float* head_bias = p.bias[L - 1] ? p.bias[L - 1] + pofs : nullptr;
       for (int l = 0; l < L; ++l) {
-        if (!mbar_wait(smem_u32(&bar_acc_full), acc_phase, abortp, SB_SITE_MLP_ACC)) { ok = false; break; }
-        acc_phase ^= 1u;
-        tc_fence_after_sync();
         const uint32_t t_acc = t_row + (uint32_t)((l & 1) * p.acc_stride);
+        const long long grow = (long long)tile * 128 + row_in_tile;
+        if (l < L - 1 || half != 0) {
+          if (!mbar_wait(smem_u32(&bar_acc_full), acc_phase, abortp, SB_SITE_MLP_ACC)) { ok = false; break; }
+          tc_fence_after_sync();
+        }
         if (l < L - 1) {
           const float* bias_l = p.bias[l] ? p.bias[l] + pofs : nullptr;
-          const long long grow = (long long)tile * 128 + row_in_tile;
           if (p.is_bf16) fused_hidden<true>(t_acc, p.n_pad[l], bias_l, act_base, bias_smem, row_in_tile, lane, half, p.hidden_norm, smem_u32(&bar_chunk[0]), p.bits[l], grow, p.batch);
           else fused_hidden<false>(t_acc, p.n_pad[l], bias_l, act_base, bias_smem, row_in_tile, lane, half, p.hidden_norm, smem_u32(&bar_chunk[0]), p.bits[l], grow, p.batch);
         } else {
           if (half == 0) {
-            const long long row = (long long)tile * 128 + row_in_tile;
-            if (p.n_pad[l] > 32) fused_head<64>(h, head_bias, out_m, t_acc, row, p.batch);
-            else if (p.n_pad[l] > 16) fused_head<32>(h, head_bias, out_m, t_acc, row, p.batch);
-            else fused_head<16>(h, head_bias, out_m, t_acc, row, p.batch);
+            const uint32_t full = smem_u32(&bar_acc_full);
+            switch (p.head_width) {
+              case 4: ok = fused_head<4>(h, head_bias, out_m, t_acc, grow, p.batch, full, acc_phase, abortp); break;
+              case 8: ok = fused_head<8>(h, head_bias, out_m, t_acc, grow, p.batch, full, acc_phase, abortp); break;
+              case 16: ok = fused_head<16>(h, head_bias, out_m, t_acc, grow, p.batch, full, acc_phase, abortp); break;
+              case 32: ok = fused_head<32>(h, head_bias, out_m, t_acc, grow, p.batch, full, acc_phase, abortp); break;
+              default: ok = fused_head<64>(h, head_bias, out_m, t_acc, grow, p.batch, full, acc_phase, abortp); break;
+            }
+            if (!ok) break;
           }
           tc_fence_before_sync();
           __syncwarp();
           if (lane == 0) mbar_arrive(smem_u32(&bar_item_done));
         }
+        acc_phase ^= 1u;
       }
       if (ok && p.tile_counters && half == 0) {
         // Decision tail (ml/models.spi:51-76).  The four head warps publish their rows of this member, count
@@ -513,6 +522,8 @@ static int fused_launch(const char* who, int n_layers, const int* sizes, int bat
   FusedMaps maps;
   FusedParams p;
   memset(&p, 0, sizeof(p));
+  head.n = n_out;
+  const int head_cols = sb_row_head_columns(head);      // columns that the head turns into zeros are not multiplied
   p.n_layers = n_layers;
   p.batch = batch;
   p.is_bf16 = in_dtype == SB_BF16;
@@ -525,7 +536,7 @@ static int fused_launch(const char* who, int n_layers, const int* sizes, int bat
   for (int l = 0; l <= n_layers; ++l) p.width[l] = sizes[l];
   for (int l = 0; l < n_layers; ++l) {
     const bool last = l == n_layers - 1;
-    p.n_pad[l] = last ? (sizes[l + 1] + 15) / 16 * 16 : sizes[l + 1];
+    p.n_pad[l] = last ? (head_cols + 15) / 16 * 16 : sizes[l + 1];
     p.k_chunks[l] = (sizes[l] + 63) / 64;
     p.idesc[l] = sb_umma_idesc(in_dtype, 0, 0, 128, p.n_pad[l]);
     p.w_bytes[l] = (uint32_t)p.n_pad[l] * 128u;
@@ -557,8 +568,7 @@ static int fused_launch(const char* who, int n_layers, const int* sizes, int bat
   p.acc_stride = 32;
   while (p.acc_stride < max_n) p.acc_stride <<= 1;
   p.tmem_cols = 2 * p.acc_stride;            // two accumulators (at most 2 x 256 columns)
-  head.n = n_out;
-  p.out = out; p.head = head; p.hidden_norm = hidden_norm ? 1 : 0;
+  p.out = out; p.head = head; p.head_width = sb_row_head_width(head); p.hidden_norm = hidden_norm ? 1 : 0;
   p.members = members;
   if (decide) {
     p.tile_counters = decide->tile_counters; p.ensemble_id = decide->ensemble_id; p.action = decide->action;
@@ -566,6 +576,9 @@ static int fused_launch(const char* who, int n_layers, const int* sizes, int bat
   }
   p.stage_bytes = ((uint32_t)max_n * 128u + 1023u) / 1024u * 1024u;     // stages stay 1024-byte aligned (swizzle atoms)
   const size_t smem = (size_t)p.w_offset + (size_t)FM_W_STAGES * p.stage_bytes + 1024;
+  // Which nets are taken depends on the widths alone, not on how few columns the head of a call needs.
+  const uint32_t full_n = (uint32_t)((n_out + 15) / 16 * 16 > max_n ? (n_out + 15) / 16 * 16 : max_n);
+  const size_t smem_limit_case = (size_t)p.w_offset + (size_t)FM_W_STAGES * (full_n * 128u) + 1024;
 
   static std::atomic<bool> attr_set[64];
   int dev = 0;
@@ -574,9 +587,9 @@ static int fused_launch(const char* who, int n_layers, const int* sizes, int bat
     SB_CUDA(cudaFuncSetAttribute(mlp_fused_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 225 * 1024));
     attr_set[dev].store(true, std::memory_order_release);
   }
-  if (smem > 225 * 1024)
+  if (smem_limit_case > 225 * 1024)
     return sb_fail(SB_ERR_UNSUPPORTED, "%s: the input tile, the widest hidden tile and the weight ring need %zu bytes of "
-                                       "shared memory (inputs wider than 256 fit with hidden layers of at most 128)", who, smem);
+                                       "shared memory (inputs wider than 256 fit with hidden layers of at most 128)", who, smem_limit_case);
   const int sms = sb_sm_count();
   const int grid = p.num_items < sms ? p.num_items : sms;
   double flops = 0.0;

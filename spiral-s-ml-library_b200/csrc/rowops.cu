@@ -96,7 +96,7 @@ __global__ void __launch_bounds__(128) row_head_kernel(const float* x, float* ou
     const float* xr = x + r * h.n;
 #pragma unroll
     for (int j = 0; j < W; ++j) v[j] = j < h.n ? xr[j] : 0.f;
-    sb_row_head_finish<W>(h, v, r, out + r * h.n);
+    sb_row_head_finish<W>(h, v, sb_row_head_legal<W>(h, r), r, out + r * h.n);
   }
 }
 
@@ -355,9 +355,13 @@ static int launch_narrow_head(const float* x, float* out, int rows, int cols, co
   h.n = cols; h.flags = flag; h.prefix = prefix < 0 ? -1 : (prefix > cols ? cols : prefix); h.mask = mask;
   const int grid = grid_for(rows, 128);
   cudaStream_t s = (cudaStream_t)stream;
-  if (cols <= 16) row_head_kernel<16><<<grid, 128, 0, s>>>(x, out, rows, h);
-  else if (cols <= 32) row_head_kernel<32><<<grid, 128, 0, s>>>(x, out, rows, h);
-  else row_head_kernel<64><<<grid, 128, 0, s>>>(x, out, rows, h);
+  switch (sb_row_head_width(h)) {
+    case 4: row_head_kernel<4><<<grid, 128, 0, s>>>(x, out, rows, h); break;
+    case 8: row_head_kernel<8><<<grid, 128, 0, s>>>(x, out, rows, h); break;
+    case 16: row_head_kernel<16><<<grid, 128, 0, s>>>(x, out, rows, h); break;
+    case 32: row_head_kernel<32><<<grid, 128, 0, s>>>(x, out, rows, h); break;
+    default: row_head_kernel<64><<<grid, 128, 0, s>>>(x, out, rows, h); break;
+  }
   SB_COUNT_LAUNCH();
   SB_CUDA(cudaGetLastError());
   return SB_OK;

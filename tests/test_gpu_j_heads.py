@@ -70,6 +70,43 @@ def test_wide_and_prefix_heads_with_sampling(gpu, n, prefix, heads):
     assert np.all(mask_host[np.arange(m), picked])                            # only legal actions are drawn
 
 
+@pytest.mark.parametrize("n,prefix", [(1, -1), (3, -1), (4, -1), (5, -1), (8, -1), (9, -1), (16, -1), (17, -1), (32, -1), (33, -1),
+                                      (64, 0), (64, 4), (64, 5), (64, 8), (64, 9), (64, 16), (64, 17), (64, 32), (64, 33), (6, 4)])
+def test_head_register_widths(gpu, n, prefix):
+    """Every width of registers a head may take (4, 8, 16, 32, 64) at its edges, with a byte mask (some rows without
+    a legal action) and with a prefix: in the GEMM, in the fused net and as a kernel of its own."""
+    m, k = 333, 64
+    a, b = operands(800 + 70 * n + prefix, m, n, k)
+    mask_host = so.prefix_mask((m, n), prefix) if prefix >= 0 else so.rng(24).random((m, n)) < 0.6
+    mask_dev = None if prefix >= 0 else gpu.DeviceArray.from_numpy(mask_host.astype(np.uint8))
+    logits = so.matmul(False, True, 1.0, a, b, 0.0, None)
+    want = so.masked_regret_matching(so.masked_softmax(logits, mask_host), mask_host)
+    heads = ("masked_softmax", "regret_matching", "argmax", "sample")
+    u = so.philox_uniform(7, np.arange(m), 0)
+
+    def check(got, idx, smp, tol):
+        np.testing.assert_allclose(got, want, atol=tol)
+        assert np.all(got[~mask_host] == 0)
+        np.testing.assert_array_equal(idx, np.argmax(got, axis=1))
+        np.testing.assert_array_equal(smp, so.discrete_sampling(got, u))
+
+    idx, smp, c = gpu.DeviceArray((m,), "i32"), gpu.DeviceArray((m,), "i32"), gpu.DeviceArray((m, n), "f32")
+    spec = gpu.head_spec(heads, prefix=prefix, mask=mask_dev, argmax_out=idx, sample_out=smp, seed=7)
+    gpu.matmul_head(False, True, 1.0, gpu.DeviceArray.from_numpy(a), gpu.DeviceArray.from_numpy(b), 0.0, c, spec, in_dtype="tf32")
+    check(c.numpy(), idx.numpy(), smp.numpy(), 2e-5)
+
+    y = gpu.DeviceArray.from_numpy(logits.astype(np.float32))
+    gpu.primitives.softmax(y, y, mask=mask_dev, prefix=prefix)
+    np.testing.assert_allclose(y.numpy(), so.masked_softmax(logits, mask_host), atol=2e-6)
+    gpu.primitives.regret_matching(y, y, mask=mask_dev, prefix=prefix)
+    np.testing.assert_allclose(y.numpy(), want, atol=2e-6)
+
+    ens = gpu.EnsemblePolicyMLP([k, n], m, 1, in_dtype="f16", with_bias=False)
+    ens.load_weights([[b]])
+    probs = ens.forward_head(gpu.to_storage(a, "f16"), head=heads, prefix=prefix, mask=mask_dev, seed=7).numpy()[0]
+    check(probs, ens.actions.numpy()[0], ens.indices.numpy()[0], TOL)
+
+
 def test_sampling_frequencies_follow_the_probabilities(gpu):
     """Many rows with the same logits: the sampled indices follow the row's probabilities."""
     m, n, k = 65536, 64, 32
