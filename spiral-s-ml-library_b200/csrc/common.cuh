@@ -231,15 +231,48 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   return mbar_wait_slow(bar, parity, abort_flag, site);
 }
 
+// The same for a whole warp that stays together: every lane has seen the phase complete when it returns true, and all
+// lanes return the same.  In line to the end, and decided by votes alone: around a call, or a branch that might
+// diverge, the compiler keeps nothing of the caller's loop in uniform registers (see umma_issue).
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag, int site) {
+  unsigned long long t0 = 0;
+#pragma unroll 1
+  for (uint32_t i = 0; !__all_sync(0xffffffffu, mbar_try_wait(bar, parity)); ++i) {
+    if (i < 2048u) continue;
+    const unsigned long long now = global_timer_ns();
+    if (i == 2048u) t0 = now;
+    if (__any_sync(0xffffffffu, *abort_flag != 0)) return false;
+    if (__any_sync(0xffffffffu, now - t0 > SB_WAIT_LIMIT_NS)) {
+      if ((threadIdx.x & 31) == 0) {
+        *abort_flag = 1;
+        atomicCAS(&g_sb_status[0], 0, site);
+        atomicAdd(&g_sb_status[1], 1);
+      }
+      return false;
+    }
+    if (i == 0xffffffffu) i = 2048u;
+  }
+  return true;
+}
+
+// True in one lane of a warp that stays together.  Chosen by elect.sync and not as `lane == 0`: the compiler then knows
+// that a single lane issues what is predicated on it.
+__device__ __forceinline__ bool elect_one_lane() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(p));
+  return p != 0;
+}
+
 // --------------------------------- TMA --------------------------------------
 // Plain (non-multicast) 2-D tiled bulk-tensor load into this CTA's shared
-// memory; completion is reported to `bar` as transaction bytes.
+// memory; completion is reported to `bar` as transaction bytes.  Issued by the lanes with `issue` (one of a warp).
 __device__ __forceinline__ void tma_load_2d(uint32_t dst_smem, const CUtensorMap* tmap, int x, int y,
-                                            uint32_t bar) {
+                                            uint32_t bar, bool issue) {
   asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%2, %3}], [%4];"
-      ::"r"(dst_smem), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(x), "r"(y), "r"(bar)
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+      "@q cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+      " [%0], [%1, {%2, %3}], [%4];\n\t}"
+      ::"r"(dst_smem), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(x), "r"(y), "r"(bar), "r"((uint32_t)issue)
       : "memory");
 }
 // 16 bytes from global to shared memory without passing through registers (cp.async); the copies
@@ -251,11 +284,12 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 // The same for a 3-D tensor (x innermost).
 __device__ __forceinline__ void tma_load_3d(uint32_t dst_smem, const CUtensorMap* tmap, int x, int y, int z,
-                                            uint32_t bar) {
+                                            uint32_t bar, bool issue) {
   asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%2, %3, %4}], [%5];"
-      ::"r"(dst_smem), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(x), "r"(y), "r"(z), "r"(bar)
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %6, 0;\n\t"
+      "@q cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+      " [%0], [%1, {%2, %3, %4}], [%5];\n\t}"
+      ::"r"(dst_smem), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(x), "r"(y), "r"(z), "r"(bar), "r"((uint32_t)issue)
       : "memory");
 }
 // 2-D tiled bulk-tensor store from this CTA's shared memory; elements outside
@@ -313,64 +347,39 @@ __device__ __forceinline__ void tc_fence_after_sync() {
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
 // Arrives once on `bar` when every tcgen05.mma issued so far by this thread
-// has finished reading shared memory and writing tensor memory.
-__device__ __forceinline__ void tc_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
-               : "memory");
+// has finished reading shared memory and writing tensor memory.  By the lanes with `issue` (one of a warp).
+__device__ __forceinline__ void tc_commit(uint32_t bar, bool issue) {
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
+               "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}"
+               ::"r"(bar), "r"((uint32_t)issue) : "memory");
 }
-// D[tmem] (+)= A[smem desc] * B[smem desc]; `accumulate == 0` overwrites D.
-__device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b,
-                                         uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
-      "}"
-      ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-__device__ __forceinline__ void umma_tf32(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b,
-                                          uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t"
-      "}"
-      ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-
-// Variants taking each 64-bit shared-memory descriptor as (lo, hi) words: the
-// hi word is constant per operand and the lo word (start address) is the only
-// part that moves, so the issuing thread does 32-bit adds only.
+// D[tmem] (+)= A[smem desc] * B[smem desc]; `accumulate == 0` overwrites D.  Each 64-bit shared-memory descriptor comes
+// as (lo, hi) words: the hi word is constant per operand and the lo word (start address) is the only part that moves.
+//
+// Issued by the lane with `issue` (elect_one_lane, always the same).  The warp runs its loop together and only the
+// instruction is predicated, because the operands of these instructions are uniform registers: in code that one lane
+// runs alone (`if (lane == 0) { ... }`) every operand is first moved there.  Cost to the issuing warp of four MMAs of
+// N = 16 with one wait, nothing else running: 355 clocks for the branch, 483 for a loop with run-time layer tables
+// predicated on `lane == 0`, 244 for the same loop predicated on elect.sync.  In the GEMM: 4096^3 121.4 -> 118.9 us,
+// 32768 x 1024 x 1024 with bias, ReLU and sign words 66.6 -> 64.1, TF32 4000 x 3000 x 1000 53.0 -> 51.5.
 template <bool PAIR, bool TF32>
 __device__ __forceinline__ void umma_issue(uint32_t tmem_d, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo,
-                                           uint32_t b_hi, uint32_t idesc, uint32_t accumulate) {
+                                           uint32_t b_hi, uint32_t idesc, uint32_t accumulate, bool issue) {
+#define SB_UMMA_ASM(GROUP, KIND)                                                                                       \
+  "{\n\t.reg .pred p, q;\n\t.reg .b64 da, db;\n\tmov.b64 da, {%1, %2};\n\tmov.b64 db, {%3, %4};\n\t"             \
+  "setp.ne.b32 p, %6, 0;\n\tsetp.ne.b32 q, %7, 0;\n\t@q tcgen05.mma.cta_group::" GROUP ".kind::" KIND               \
+  " [%0], da, db, %5, p;\n\t}"
+#define SB_UMMA_ARGS                                                                                                   \
+  ::"r"(tmem_d), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate), "r"((uint32_t)issue) : "memory"
   if (PAIR) {
-    if (TF32)
-      asm volatile(
-          "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\tmov.b64 da, {%1, %2};\n\tmov.b64 db, {%3, %4};\n\t"
-          "setp.ne.b32 p, %6, 0;\n\ttcgen05.mma.cta_group::2.kind::tf32 [%0], da, db, %5, p;\n\t}"
-          ::"r"(tmem_d), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate) : "memory");
-    else
-      asm volatile(
-          "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\tmov.b64 da, {%1, %2};\n\tmov.b64 db, {%3, %4};\n\t"
-          "setp.ne.b32 p, %6, 0;\n\ttcgen05.mma.cta_group::2.kind::f16 [%0], da, db, %5, p;\n\t}"
-          ::"r"(tmem_d), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate) : "memory");
+    if (TF32) asm volatile(SB_UMMA_ASM("2", "tf32") SB_UMMA_ARGS);
+    else asm volatile(SB_UMMA_ASM("2", "f16") SB_UMMA_ARGS);
   } else {
-    if (TF32)
-      asm volatile(
-          "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\tmov.b64 da, {%1, %2};\n\tmov.b64 db, {%3, %4};\n\t"
-          "setp.ne.b32 p, %6, 0;\n\ttcgen05.mma.cta_group::1.kind::tf32 [%0], da, db, %5, p;\n\t}"
-          ::"r"(tmem_d), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate) : "memory");
-    else
-      asm volatile(
-          "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\tmov.b64 da, {%1, %2};\n\tmov.b64 db, {%3, %4};\n\t"
-          "setp.ne.b32 p, %6, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n\t}"
-          ::"r"(tmem_d), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate) : "memory");
+    if (TF32) asm volatile(SB_UMMA_ASM("1", "tf32") SB_UMMA_ARGS);
+    else asm volatile(SB_UMMA_ASM("1", "f16") SB_UMMA_ARGS);
   }
+#undef SB_UMMA_ASM
+#undef SB_UMMA_ARGS
 }
 
 // 32 lanes x 32-bit, 4 / 8 / 16 / 32 consecutive columns: thread t of the warp gets
@@ -410,6 +419,16 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t* r) {
 __device__ __forceinline__ void tmem_ld_wait() {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
+// The same, tied to 32 registers of an earlier load: nothing that reads them can move above the wait, also when
+// another load is issued between the wait and their use.
+__device__ __forceinline__ void tmem_ld_wait32(uint32_t* r) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
+                 "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]),
+                 "+r"(r[16]), "+r"(r[17]), "+r"(r[18]), "+r"(r[19]), "+r"(r[20]), "+r"(r[21]), "+r"(r[22]), "+r"(r[23]),
+                 "+r"(r[24]), "+r"(r[25]), "+r"(r[26]), "+r"(r[27]), "+r"(r[28]), "+r"(r[29]), "+r"(r[30]), "+r"(r[31])
+               :: "memory");
+}
 // The first W columns of a row, for a row head.
 template <int W>
 __device__ __forceinline__ void tmem_ld_head(uint32_t taddr, uint32_t* r) {
@@ -425,6 +444,51 @@ __device__ __forceinline__ void tmem_ld_head(uint32_t taddr, uint32_t* r) {
   } else {
     tmem_ld4(taddr, r);
   }
+}
+
+// --------------------------- packed arithmetic ------------------------------
+// Two fp32 operations in one instruction (the packed forms that sm_100 adds); each half rounds as the scalar form.
+__device__ __forceinline__ unsigned long long pack_f32x2(float lo, float hi) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void unpack_f32x2(unsigned long long v, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ void fma_f32x2(unsigned long long& c, unsigned long long a, unsigned long long b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ unsigned long long add_f32x2(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ unsigned long long sub_f32x2(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+// max(0, x) of two values rounded to 16 bits, lo in the low half.  Rounding keeps the order, so this is the rounded
+// ReLU; a NaN gives 0, as fmaxf does.
+template <bool BF16>
+__device__ __forceinline__ uint32_t relu_pack2(float lo, float hi) {
+  uint32_t d;
+  if (BF16) asm("{\n\t.reg .b32 t;\n\tcvt.rn.bf16x2.f32 t, %1, %2;\n\tmax.bf16x2 %0, t, %3;\n\t}" : "=r"(d) : "f"(hi), "f"(lo), "r"(0));
+  else asm("{\n\t.reg .b32 t;\n\tcvt.rn.f16x2.f32 t, %1, %2;\n\tmax.f16x2 %0, t, %3;\n\t}" : "=r"(d) : "f"(hi), "f"(lo), "r"(0));
+  return d;
+}
+// Bit j = (v[j] > 0): the sign of 0 - v, which is +0 for both zeros and positive for a NaN, shifted in from the top.
+__device__ __forceinline__ uint32_t positive_bits32(const float* v) {
+  uint32_t w = 0u;
+#pragma unroll
+  for (int j = 30; j >= 0; j -= 2) {
+    float lo, hi;
+    unpack_f32x2(sub_f32x2(0ull, pack_f32x2(v[j], v[j + 1])), lo, hi);
+    w = __funnelshift_l(__float_as_uint(hi), w, 1);
+    w = __funnelshift_l(__float_as_uint(lo), w, 1);
+  }
+  return w;
 }
 
 // ------------------ CTA pairs (cluster of 2, cta_group::2) ------------------
@@ -451,11 +515,12 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
 // memory, the transaction bytes are reported to `bar`, which may live in the
 // pair's leader CTA (a shared::cluster address).  No multicast.
 __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst_smem, const CUtensorMap* tmap, int x, int y,
-                                                 uint32_t bar_cluster_addr) {
+                                                 uint32_t bar_cluster_addr, bool issue) {
   asm volatile(
-      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%2, %3}], [%4];"
-      ::"r"(dst_smem), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(x), "r"(y), "r"(bar_cluster_addr)
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+      "@q cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
+      " [%0], [%1, {%2, %3}], [%4];\n\t}"
+      ::"r"(dst_smem), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(x), "r"(y), "r"(bar_cluster_addr), "r"((uint32_t)issue)
       : "memory");
 }
 __device__ __forceinline__ void tmem_alloc_pair(uint32_t dst_smem, uint32_t ncols) {
@@ -472,37 +537,13 @@ __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols
 }
 // Commit of the pair's MMAs: arrives on the barrier at this shared-memory offset
 // in every CTA named by `cta_mask` (bit r = CTA rank r of the cluster).
-__device__ __forceinline__ void tc_commit_pair(uint32_t bar, uint16_t cta_mask) {
+__device__ __forceinline__ void tc_commit_pair(uint32_t bar, uint16_t cta_mask, bool issue) {
   asm volatile(
-      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-      ::"r"(bar), "h"(cta_mask)
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t"
+      "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}"
+      ::"r"(bar), "h"(cta_mask), "r"((uint32_t)issue)
       : "memory");
 }
-// M = 256 MMA of a CTA pair: each CTA supplies its 128 rows of A and half of the
-// N columns of B from the same shared-memory offsets, and keeps its 128 rows of D.
-__device__ __forceinline__ void umma_f16_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b,
-                                              uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t"
-      "}"
-      ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-__device__ __forceinline__ void umma_tf32_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b,
-                                               uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::tf32 [%0], %1, %2, %3, p;\n\t"
-      "}"
-      ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-
 // ---------------------- UMMA descriptors (sm_100) ---------------------------
 // Shared-memory matrix descriptor, 128-byte swizzle.  Fields (bit ranges):
 //   [0,14)  start address >> 4       [16,30) leading byte offset >> 4

@@ -912,87 +912,88 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
   sb_grid_dependency_wait();
   sb_grid_dependents_launch();
 
+  // Producers and issuer are whole warps that run their loops together; single instructions are predicated on `one`
+  // (see umma_issue).
+  const bool one = elect_one_lane();
   if (warp == 0 || warp == 2 + EW) {
-    // Two producer threads: warp 0 arms the stage's barrier and loads A, the last warp loads B.  One thread
+    // Two producer warps: warp 0 arms the stage's barrier and loads A, the last warp loads B.  One thread
     // issuing all four loads of a stage measured 3 % slower on main-loop-bound GEMMs (4096^3: 1307 ->
     // 1346 TFLOP/s): a TMA instruction occupies its thread for long enough to matter.  A load whose
     // bytes land before the barrier is armed is in order: the transaction count may run negative.
     const bool do_a = warp == 0, do_b = !do_a;
-    if (lane == 0) {
-      // The issue loop of a single thread: keep it to a handful of instructions
-      // per k-block (addresses advance by adds, nothing is recomputed).
-      int stage = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      const int b_cols = PAIR ? p.block_n / 2 : p.block_n;   // half of the B columns per CTA in a pair
-      const uint32_t full0_local = smem_u32(&bar_full[0]);
-      const uint32_t full0 = PAIR ? map_to_cta(full0_local, 0u) : full0_local;
-      const uint32_t empty0 = smem_u32(&bar_empty[0]);
-      const bool a_mn = p.a_mn != 0, b_mn = p.b_mn != 0;
-      const int a_boxes = p.a_boxes, mn_box_elems = p.mn_box_elems, block_k = p.block_k;
-      const uint32_t mn_box_bytes = p.mn_box_bytes, a_stage_bytes = p.a_stage_bytes;
-      const int subs = p.subs;
-      const uint32_t a_sub_bytes = p.a_sub_bytes, b_sub_bytes = p.b_sub_bytes;
-      const int stages = p.stages;
-      uint32_t a_dst = stage_base;
-      WorkIter it(p, worker, num_workers);
-      int tile, split, kb_begin, kb_end, half;
-      while (ok && it.next(p, tile, split, kb_begin, kb_end, half)) {
-        int m_blk, n_blk;
-        tile_coords(p, tile, m_blk, n_blk);
-        const int m0 = m_blk * TILE_M + (int)cta_rank * UG_BLOCK_M;
-        // A half tile: half as many B columns per CTA (half the boxes, or a tensor map with half-height boxes).
-        const int item_cols = half < 0 ? b_cols : b_cols / 2;
-        const int n0 = n_blk * p.block_n + (half > 0 ? p.block_n / 2 : 0) + (int)cta_rank * item_cols;
-        const CUtensorMap* map_b = half < 0 ? &tmap_b : &out_maps.b_tail;
-        const int b_boxes = half < 0 ? p.b_boxes : p.b_boxes / 2;
-        const uint32_t item_b_bytes = half < 0 ? p.b_stage_bytes : p.b_stage_bytes / 2u;
-        const uint32_t tx_bytes = PAIR ? 2u * (a_stage_bytes + item_b_bytes) : a_stage_bytes + item_b_bytes;
-        int k0 = kb_begin * block_k;
-        for (int kb = kb_begin; kb < kb_end; ++kb, k0 += block_k) {
-          if (!mbar_wait(empty0 + 8u * (uint32_t)stage, phase ^ 1u, abortp, SB_SITE_PRODUCER_EMPTY)) {
-            ok = false;
-            break;
+    // Keep the issue loop to a handful of instructions
+    // per k-block (addresses advance by adds, nothing is recomputed).
+    int stage = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    const int b_cols = PAIR ? p.block_n / 2 : p.block_n;   // half of the B columns per CTA in a pair
+    const uint32_t full0_local = smem_u32(&bar_full[0]);
+    const uint32_t full0 = PAIR ? map_to_cta(full0_local, 0u) : full0_local;
+    const uint32_t empty0 = smem_u32(&bar_empty[0]);
+    const bool a_mn = p.a_mn != 0, b_mn = p.b_mn != 0;
+    const int a_boxes = p.a_boxes, mn_box_elems = p.mn_box_elems, block_k = p.block_k;
+    const uint32_t mn_box_bytes = p.mn_box_bytes, a_stage_bytes = p.a_stage_bytes;
+    const int subs = p.subs;
+    const uint32_t a_sub_bytes = p.a_sub_bytes, b_sub_bytes = p.b_sub_bytes;
+    const int stages = p.stages;
+    uint32_t a_dst = stage_base;
+    WorkIter it(p, worker, num_workers);
+    int tile, split, kb_begin, kb_end, half;
+    while (ok && it.next(p, tile, split, kb_begin, kb_end, half)) {
+      int m_blk, n_blk;
+      tile_coords(p, tile, m_blk, n_blk);
+      const int m0 = m_blk * TILE_M + (int)cta_rank * UG_BLOCK_M;
+      // A half tile: half as many B columns per CTA (half the boxes, or a tensor map with half-height boxes).
+      const int item_cols = half < 0 ? b_cols : b_cols / 2;
+      const int n0 = n_blk * p.block_n + (half > 0 ? p.block_n / 2 : 0) + (int)cta_rank * item_cols;
+      const CUtensorMap* map_b = half < 0 ? &tmap_b : &out_maps.b_tail;
+      const int b_boxes = half < 0 ? p.b_boxes : p.b_boxes / 2;
+      const uint32_t item_b_bytes = half < 0 ? p.b_stage_bytes : p.b_stage_bytes / 2u;
+      const uint32_t tx_bytes = PAIR ? 2u * (a_stage_bytes + item_b_bytes) : a_stage_bytes + item_b_bytes;
+      int k0 = kb_begin * block_k;
+      for (int kb = kb_begin; kb < kb_end; ++kb, k0 += block_k) {
+        if (!mbar_wait_warp(empty0 + 8u * (uint32_t)stage, phase ^ 1u, abortp, SB_SITE_PRODUCER_EMPTY)) {
+          ok = false;
+          break;
+        }
+        // In a pair only the leader arms its full barrier, with the bytes of both CTAs.
+        if (one && do_a && (!PAIR || leader)) mbar_arrive_expect_tx(full0_local + 8u * (uint32_t)stage, tx_bytes);
+        const uint32_t full = full0 + 8u * (uint32_t)stage;
+        const uint32_t b_dst = a_dst + a_stage_bytes;
+        if (!do_a) {
+        } else if (!a_mn) {
+          for (int s = 0; s < subs; ++s) {
+            if (PAIR) tma_load_2d_pair(a_dst + (uint32_t)s * a_sub_bytes, &tmap_a, k0 + s * mn_box_elems, m0, full, one);
+            else tma_load_2d(a_dst + (uint32_t)s * a_sub_bytes, &tmap_a, k0 + s * mn_box_elems, m0, full, one);
           }
-          // In a pair only the leader arms its full barrier, with the bytes of both CTAs.
-          if (do_a && (!PAIR || leader)) mbar_arrive_expect_tx(full0_local + 8u * (uint32_t)stage, tx_bytes);
-          const uint32_t full = full0 + 8u * (uint32_t)stage;
-          const uint32_t b_dst = a_dst + a_stage_bytes;
-          if (!do_a) {
-          } else if (!a_mn) {
-            for (int s = 0; s < subs; ++s) {
-              if (PAIR) tma_load_2d_pair(a_dst + (uint32_t)s * a_sub_bytes, &tmap_a, k0 + s * mn_box_elems, m0, full);
-              else tma_load_2d(a_dst + (uint32_t)s * a_sub_bytes, &tmap_a, k0 + s * mn_box_elems, m0, full);
-            }
-          } else {
-            for (int i = 0; i < a_boxes; ++i) {
-              if (PAIR) tma_load_2d_pair(a_dst + (uint32_t)i * mn_box_bytes, &tmap_a, m0 + i * mn_box_elems, k0, full);
-              else tma_load_2d(a_dst + (uint32_t)i * mn_box_bytes, &tmap_a, m0 + i * mn_box_elems, k0, full);
-            }
+        } else {
+          for (int i = 0; i < a_boxes; ++i) {
+            if (PAIR) tma_load_2d_pair(a_dst + (uint32_t)i * mn_box_bytes, &tmap_a, m0 + i * mn_box_elems, k0, full, one);
+            else tma_load_2d(a_dst + (uint32_t)i * mn_box_bytes, &tmap_a, m0 + i * mn_box_elems, k0, full, one);
           }
-          if (!do_b) {
-          } else if (!b_mn) {
-            for (int s = 0; s < subs; ++s) {
-              if (PAIR) tma_load_2d_pair(b_dst + (uint32_t)s * b_sub_bytes, map_b, k0 + s * mn_box_elems, n0, full);
-              else tma_load_2d(b_dst + (uint32_t)s * b_sub_bytes, map_b, k0 + s * mn_box_elems, n0, full);
-            }
-          } else {
-            for (int i = 0; i < b_boxes; ++i) {
-              if (PAIR) tma_load_2d_pair(b_dst + (uint32_t)i * mn_box_bytes, &tmap_b, n0 + i * mn_box_elems, k0, full);
-              else tma_load_2d(b_dst + (uint32_t)i * mn_box_bytes, &tmap_b, n0 + i * mn_box_elems, k0, full);
-            }
+        }
+        if (!do_b) {
+        } else if (!b_mn) {
+          for (int s = 0; s < subs; ++s) {
+            if (PAIR) tma_load_2d_pair(b_dst + (uint32_t)s * b_sub_bytes, map_b, k0 + s * mn_box_elems, n0, full, one);
+            else tma_load_2d(b_dst + (uint32_t)s * b_sub_bytes, map_b, k0 + s * mn_box_elems, n0, full, one);
           }
-          a_dst += stage_bytes;
-          if (++stage == stages) {
-            stage = 0;
-            phase ^= 1u;
-            a_dst = stage_base;
+        } else {
+          for (int i = 0; i < b_boxes; ++i) {
+            if (PAIR) tma_load_2d_pair(b_dst + (uint32_t)i * mn_box_bytes, &tmap_b, n0 + i * mn_box_elems, k0, full, one);
+            else tma_load_2d(b_dst + (uint32_t)i * mn_box_bytes, &tmap_b, n0 + i * mn_box_elems, k0, full, one);
           }
+        }
+        a_dst += stage_bytes;
+        if (++stage == stages) {
+          stage = 0;
+          phase ^= 1u;
+          a_dst = stage_base;
         }
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && leader) {
+    if (leader) {
       // tcgen05.mma issue blocks while the tensor pipe's short queue is full, so
       // every other instruction of this thread is time the pipe may run dry:
       // descriptors are kept as (lo, hi) words, the lo word advances by adds.
@@ -1020,7 +1021,7 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
       int tile, split, kb_begin, kb_end, half;
       while (ok && it.next(p, tile, split, kb_begin, kb_end, half)) {
         const uint32_t idesc = half < 0 ? p.idesc : p.idesc_tail;
-        if (!mbar_wait(smem_u32(&bar_tmem_empty[acc]), acc_phase ^ 1u, abortp, SB_SITE_MMA_TMEM_EMPTY)) {
+        if (!mbar_wait_warp(smem_u32(&bar_tmem_empty[acc]), acc_phase ^ 1u, abortp, SB_SITE_MMA_TMEM_EMPTY)) {
           ok = false;
           break;
         }
@@ -1028,25 +1029,25 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
         const uint32_t d_tmem = tmem_base + (uint32_t)(acc * p.acc_stride);
         uint32_t accumulate = 0u;
         for (int kb = kb_begin; kb < kb_end; ++kb) {
-          if (!mbar_wait(full0 + 8u * (uint32_t)stage, phase, abortp, SB_SITE_MMA_FULL)) {
+          if (!mbar_wait_warp(full0 + 8u * (uint32_t)stage, phase, abortp, SB_SITE_MMA_FULL)) {
             ok = false;
             break;
           }
           tc_fence_after_sync();
-          umma_issue<PAIR, TF32>(d_tmem, a_lo, a_hi, b_lo, b_hi, idesc, accumulate);
-          umma_issue<PAIR, TF32>(d_tmem, a_lo + a_kstep, a_hi, b_lo + b_kstep, b_hi, idesc, 1u);
-          umma_issue<PAIR, TF32>(d_tmem, a_lo + 2u * a_kstep, a_hi, b_lo + 2u * b_kstep, b_hi, idesc, 1u);
-          umma_issue<PAIR, TF32>(d_tmem, a_lo + 3u * a_kstep, a_hi, b_lo + 3u * b_kstep, b_hi, idesc, 1u);
+          umma_issue<PAIR, TF32>(d_tmem, a_lo, a_hi, b_lo, b_hi, idesc, accumulate, one);
+          umma_issue<PAIR, TF32>(d_tmem, a_lo + a_kstep, a_hi, b_lo + b_kstep, b_hi, idesc, 1u, one);
+          umma_issue<PAIR, TF32>(d_tmem, a_lo + 2u * a_kstep, a_hi, b_lo + 2u * b_kstep, b_hi, idesc, 1u, one);
+          umma_issue<PAIR, TF32>(d_tmem, a_lo + 3u * a_kstep, a_hi, b_lo + 3u * b_kstep, b_hi, idesc, 1u, one);
           if (two_subs) {
             const uint32_t a2 = a_lo + a_sub_step, b2 = b_lo + b_sub_step;
-            umma_issue<PAIR, TF32>(d_tmem, a2, a_hi, b2, b_hi, idesc, 1u);
-            umma_issue<PAIR, TF32>(d_tmem, a2 + a_kstep, a_hi, b2 + b_kstep, b_hi, idesc, 1u);
-            umma_issue<PAIR, TF32>(d_tmem, a2 + 2u * a_kstep, a_hi, b2 + 2u * b_kstep, b_hi, idesc, 1u);
-            umma_issue<PAIR, TF32>(d_tmem, a2 + 3u * a_kstep, a_hi, b2 + 3u * b_kstep, b_hi, idesc, 1u);
+            umma_issue<PAIR, TF32>(d_tmem, a2, a_hi, b2, b_hi, idesc, 1u, one);
+            umma_issue<PAIR, TF32>(d_tmem, a2 + a_kstep, a_hi, b2 + b_kstep, b_hi, idesc, 1u, one);
+            umma_issue<PAIR, TF32>(d_tmem, a2 + 2u * a_kstep, a_hi, b2 + 2u * b_kstep, b_hi, idesc, 1u, one);
+            umma_issue<PAIR, TF32>(d_tmem, a2 + 3u * a_kstep, a_hi, b2 + 3u * b_kstep, b_hi, idesc, 1u, one);
           }
           accumulate = 1u;
-          if (PAIR) tc_commit_pair(empty0 + 8u * (uint32_t)stage, (uint16_t)3);
-          else tc_commit(empty0 + 8u * (uint32_t)stage);
+          if (PAIR) tc_commit_pair(empty0 + 8u * (uint32_t)stage, (uint16_t)3, one);
+          else tc_commit(empty0 + 8u * (uint32_t)stage, one);
           a_lo += stage_step;
           b_lo += stage_step;
           if (++stage == stages) {
@@ -1057,8 +1058,8 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
           }
         }
         if (!ok) break;
-        if (PAIR) tc_commit_pair(smem_u32(&bar_tmem_full[acc]), (uint16_t)3);
-        else tc_commit(smem_u32(&bar_tmem_full[acc]));
+        if (PAIR) tc_commit_pair(smem_u32(&bar_tmem_full[acc]), (uint16_t)3, one);
+        else tc_commit(smem_u32(&bar_tmem_full[acc]), one);
         acc ^= 1;
         if (acc == 0) acc_phase ^= 1u;
       }

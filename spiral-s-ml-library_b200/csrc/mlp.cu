@@ -230,19 +230,6 @@ colsum_kernel(const DyT* __restrict__ dy, float* __restrict__ db, int rows, int 
 // with the multiply-adds on warp-level MMAs, m16n8k16, was built and measured: 4 us faster at
 // 32768 x 1024 with 10 outputs, 28 us slower for a 3-output head -- gating, packing, column sums
 // and stores cost the same either way and the MMA does 16 multiply-adds whatever K is.)
-// Two fp32 fused multiply-adds in one instruction (the packed form sm_100 adds): c += a * b on register pairs.
-__device__ __forceinline__ unsigned long long pack_f32x2(float lo, float hi) {
-  unsigned long long r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ void unpack_f32x2(unsigned long long v, float& lo, float& hi) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-__device__ __forceinline__ void fma_f32x2(unsigned long long& c, unsigned long long a, unsigned long long b) {
-  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b));
-}
-
 constexpr int ND_THREADS = 384;
 constexpr int ND_MAX_SLOTS = ND_THREADS / 32;
 template <typename T, int KV>

@@ -34,8 +34,11 @@ namespace {
 
 constexpr int FM_MAX_LAYERS = 8;
 constexpr int FM_THREADS = 320;
+constexpr size_t FM_SMEM_LIMIT = 225 * 1024;            // dynamic shared memory; the static part stays below 2 KB
 constexpr int FM_EPI_WARPS = 8;
-constexpr int FM_W_STAGES = 4;
+constexpr int FM_W_STAGES = 4;                         // stages of the weight ring that decide which nets fit
+constexpr int FM_W_STAGES_MAX = 8;                     // stages taken where shared memory is left
+constexpr uint32_t FM_BIAS_BYTES = FM_EPI_WARPS * 512u; // a layer's biases, one copy of its own columns per epilogue warp
 constexpr uint32_t FM_CHUNK_BYTES = 128u * 128u;       // activation chunk: 128 rows x 64 elements x 2 B
 // A weight stage holds one 64-column K-chunk of a layer: (widest layer's rows) x 128 bytes, at most 256 rows.
 
@@ -51,10 +54,10 @@ struct FusedParams {
   int width[FM_MAX_LAYERS + 1];       // width[0] = input features
   int n_pad[FM_MAX_LAYERS];           // MMA N of layer l (hidden: width; last: padded to 16 or 32)
   int k_chunks[FM_MAX_LAYERS];        // ceil(in_l / 64)
+  int k_steps[FM_MAX_LAYERS];         // ceil(in_l / 16): MMAs of the layer
   uint32_t idesc[FM_MAX_LAYERS];
   uint32_t w_bytes[FM_MAX_LAYERS];    // bytes of one weight chunk of layer l
   const float* bias[FM_MAX_LAYERS];   // may be null
-  int is_bf16;
   int tmem_cols;
   int acc_stride;                     // TMEM columns between the two accumulators (layers alternate between them)
   int num_tiles;                      // 128-row tiles of the batch
@@ -64,6 +67,8 @@ struct FusedParams {
   uint32_t x_chunks;                  // chunks of the input tile
   uint32_t stage_bytes;               // bytes of one weight stage
   uint32_t act_offset, w_offset;      // byte offsets of the activation tile and the weight ring
+  int w_stages;                       // stages of the weight ring
+  uint32_t bias_offset;               // byte offset of the epilogue warps' bias buffers
   // head
   float* out;
   SbRowHead head;                     // n, flags, prefix, mask, seed, ...; argmax_out / sample_out are [members, batch]
@@ -83,117 +88,135 @@ struct FusedParams {
 };
 
 // The last layer: a thread takes the first W values of its row out of tensor memory (all that the head needs,
-// sb_row_head_columns), adds the bias and hands over to the shared row head.  Bias and mask bytes are requested
-// before the wait for the accumulator.  False when that wait expired.
+// sb_row_head_columns), adds the bias (from the warp's buffer) and hands over to the shared row head.  The accumulator
+// is handed back (`bar_done`) as soon as the row is in registers.
 template <int W>
-__device__ __noinline__ bool fused_head(const SbRowHead& h, const float* bias, float* out, uint32_t t_row, long long row,
-                                        int batch, uint32_t bar_full, uint32_t parity, volatile int* abortp) {
-  typename SbLegalWord<W>::type legal = 0;
-  float b[W];
-  if (row < batch) legal = sb_row_head_legal<W>(h, row);
-#pragma unroll
-  for (int j = 0; j < W; ++j) b[j] = bias && j < h.n ? __ldg(bias + j) : 0.f;
-  if (!mbar_wait(bar_full, parity, abortp, SB_SITE_MLP_ACC)) return false;
-  tc_fence_after_sync();
+__device__ __noinline__ void fused_head(const SbRowHead& h, unsigned long long legal, bool has_bias, uint32_t bias_smem,
+                                        float* out, uint32_t t_row, long long row, int batch, uint32_t bar_done) {
   uint32_t raw[W];
   tmem_ld_head<W>(t_row, raw);
   tmem_ld_wait();
-  if (row >= batch) return true;
+  tc_fence_before_sync();
+  __syncwarp();
+  if ((threadIdx.x & 31) == 0) mbar_arrive(bar_done);
+  if (row >= batch) return;
   float* v = reinterpret_cast<float*>(raw);
-  if (bias) {
+  if (has_bias) {
 #pragma unroll
-    for (int j = 0; j < W; ++j) v[j] += b[j];
+    for (int j = 0; j < W; j += 4) {
+      float4 b;
+      asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+                   : "r"(bias_smem + 4u * (uint32_t)j) : "memory");
+      v[j] += b.x; v[j + 1] += b.y; v[j + 2] += b.z; v[j + 3] += b.w;
+    }
   }
-  sb_row_head_finish<W>(h, v, legal, row, out + row * h.n);
-  return true;
+  sb_row_head_finish<W>(h, v, (typename SbLegalWord<W>::type)legal, row, out + row * h.n);
 }
 
-// One warp's share of a hidden layer: chunks `half`, half+2, ... of 32 columns.
+// Finishes 32 columns of a row: bias, ReLU, rounding to the storage type, and the swizzled store into the activation
+// tile (`dst` = the row's 128 bytes of the 64-column chunk, `piece0` = first of its four 16-byte pieces, `key` the row's
+// swizzle).  `word` (or null) takes the sign word of the row and chunk.
+template <bool BF16>
+__device__ __forceinline__ void hidden_chunk(uint32_t* raw, bool norm, float sumsq, bool has_bias, uint32_t bias_addr,
+                                             uint32_t* word, uint32_t dst, uint32_t piece0, uint32_t key) {
+  float* v = reinterpret_cast<float*>(raw);
+  if (norm) {
+#pragma unroll
+    for (int j = 0; j < 32; ++j) v[j] = sumsq != 0.f ? v[j] / sumsq : 0.f;
+  }
+  if (has_bias) {
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      unsigned long long b0, b1;       // the same address for the whole warp
+      asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(b0), "=l"(b1) : "r"(bias_addr + 16u * (uint32_t)q) : "memory");
+      unpack_f32x2(add_f32x2(pack_f32x2(v[4 * q], v[4 * q + 1]), b0), v[4 * q], v[4 * q + 1]);
+      unpack_f32x2(add_f32x2(pack_f32x2(v[4 * q + 2], v[4 * q + 3]), b1), v[4 * q + 2], v[4 * q + 3]);
+    }
+  }
+  if (word) *word = positive_bits32(v);
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const uint4 out = make_uint4(relu_pack2<BF16>(v[8 * q], v[8 * q + 1]), relu_pack2<BF16>(v[8 * q + 2], v[8 * q + 3]),
+                                 relu_pack2<BF16>(v[8 * q + 4], v[8 * q + 5]), relu_pack2<BF16>(v[8 * q + 6], v[8 * q + 7]));
+    st_shared_v4(dst + (((piece0 + (uint32_t)q) ^ key) << 4), out);
+  }
+}
+
+// One warp's share of a hidden layer: chunks `half`, half + 2, ... of 32 columns (at most four).
 // Writes relu(acc + bias) in the storage type into the activation tile, in the
 // 128-byte-swizzled K-major layout the next layer's A descriptors expect:
 // element (row, j) -> chunk j / 64, byte row * 128 + (((j % 64) / 8) ^ (row % 8)) * 16 + (j % 8) * 2.
 // After each 32-column chunk the warp arrives on the barrier of the 64-column activation chunk it
 // belongs to (`chunk_bar0` + 8 bytes per chunk): the next layer's MMAs on that K-chunk start as soon as
 // all eight warps have delivered it, while the later chunks of this layer are still being finished.
+//
+// A tile's time is the chain of these chunks, so what a chunk waits for is asked for early: the layer's biases go to
+// the warp's own buffer before the accumulator is awaited, and the next chunk is on its way out of tensor memory
+// while this one is finished.  Per chunk that leaves about 85 instructions (packed adds, rounding before the ReLU).
+// What bounds a 256-wide layer then (4200 clocks per 128 rows) is shared memory at 128 bytes a clock: the MMAs read
+// 64 KB of activations and 128 KB of weights, the weights are written once per tile (128 KB), the activations
+// (64 KB), and the biases are read as 16-byte broadcasts that each move 512 bytes (128 KB): 4096 clocks.  Sixteen
+// warps of two chunks each were slower for that reason (126.6 -> 136 us for 265216 rows).
+// Measured with the issue loops of this kernel and the GEMM predicated instead of branched (see umma_issue):
+// 262144 rows 156 -> 127 us, 16384 rows 14.9 -> 12.8, Leduc training step of 65536 rows 207 -> 191.
+// False when a wait expired.
 template <bool BF16>
-__device__ __noinline__ void fused_hidden(uint32_t t_row, int n_cols, const float* bias, uint32_t act_base,
-                                          uint32_t bias_smem, int row_in_tile, int lane, int half, int norm,
-                                          uint32_t chunk_bar0, uint32_t* bits_out, long long row, int batch) {
-  const int nchunks = n_cols >> 5;
+__device__ __forceinline__ bool fused_hidden(uint32_t t_row, int n_cols, const float* bias, uint32_t act_base,
+                                          uint32_t bias_smem, int row_in_tile, int half, bool norm,
+                                          uint32_t chunk_bar0, uint32_t* bits_out, long long row, int batch,
+                                          uint32_t bar_full, uint32_t parity, uint32_t bar_act_free, uint32_t act_parity,
+                                          volatile int* abortp) {
+  const int lane = (int)(threadIdx.x & 31);
+  const int mine = n_cols >> 6;                  // chunks of this warp
+  if (bias) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (i < mine) {
+        const float b = __ldg(bias + (half + 2 * i) * 32 + lane);
+        asm volatile("st.shared.f32 [%0], %1;" ::"r"(bias_smem + 4u * (uint32_t)(i * 32 + lane)), "f"(b) : "memory");
+      }
+    __syncwarp();
+  }
+  if (!mbar_wait(bar_full, parity, abortp, SB_SITE_MLP_ACC)) return false;
+  tc_fence_after_sync();
   // Row normalisation (local_ln_l2, ml/primitives.spi:701-703; no bias in this mode): a first pass
   // over the whole accumulator row sums the squares; both warps of a quadrant do it for themselves.
   float sumsq = 0.f;
+  uint32_t raw_a[32], raw_b[32];
   if (norm) {
-    for (int c = 0; c < nchunks; ++c) {
-      uint32_t raw[32];
-      tmem_ld32(t_row + (uint32_t)(c * 32), raw);
-      tmem_ld_wait();
+    for (int c = 0; c < 2 * mine; ++c) {
+      tmem_ld32(t_row + (uint32_t)(c * 32), raw_a);
+      tmem_ld_wait32(raw_a);
 #pragma unroll
-      for (int j = 0; j < 32; ++j) sumsq = fmaf(__uint_as_float(raw[j]), __uint_as_float(raw[j]), sumsq);
+      for (int j = 0; j < 32; ++j) sumsq = fmaf(__uint_as_float(raw_a[j]), __uint_as_float(raw_a[j]), sumsq);
     }
   }
-  float bias_cur = 0.f, bias_nxt = 0.f;
-  if (bias && half < nchunks) bias_cur = __ldg(bias + half * 32 + lane);
-  for (int c = half; c < nchunks; c += 2) {
-    uint32_t raw[32];
-    tmem_ld32(t_row + (uint32_t)(c * 32), raw);
-    if (bias && c + 2 < nchunks) bias_nxt = __ldg(bias + (c + 2) * 32 + lane);
-    tmem_ld_wait();
-    float* v = reinterpret_cast<float*>(raw);
-    if (norm) {
-#pragma unroll
-      for (int j = 0; j < 32; ++j) v[j] = sumsq != 0.f ? v[j] / sumsq : 0.f;
-    }
-    if (bias) {
-      asm volatile("st.shared.f32 [%0], %1;" ::"r"(bias_smem + 4u * (uint32_t)lane), "f"(bias_cur) : "memory");
-      __syncwarp();
-#pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        uint4 b;
-        asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(b.x), "=r"(b.y), "=r"(b.z), "=r"(b.w)
-                     : "r"(bias_smem + 16u * (uint32_t)q) : "memory");
-        v[4 * q + 0] += __uint_as_float(b.x);
-        v[4 * q + 1] += __uint_as_float(b.y);
-        v[4 * q + 2] += __uint_as_float(b.z);
-        v[4 * q + 3] += __uint_as_float(b.w);
-      }
-      __syncwarp();
-    }
-    if (bits_out) {
-      // ReLU sign word of this row and chunk (bit j = value j > 0), stored [chunk, row]: the 32 rows of
-      // the warp are 32 consecutive words.  The backward pass gates its gradients by these words.
-      uint32_t signs = 0u;
-#pragma unroll
-      for (int j = 0; j < 32; ++j) signs |= (v[j] > 0.f ? 1u : 0u) << j;
-      if (row < batch) bits_out[(long long)c * batch + row] = signs;
-    }
-    const int col0 = c * 32;
-    const uint32_t chunk_base = act_base + (uint32_t)(col0 >> 6) * FM_CHUNK_BYTES + (uint32_t)row_in_tile * 128u;
-    const uint32_t piece0 = (uint32_t)((col0 & 63) >> 3);
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      uint32_t packed[4];
-#pragma unroll
-      for (int t = 0; t < 4; ++t) {
-        const float lo = fmaxf(v[q * 8 + 2 * t], 0.f), hi = fmaxf(v[q * 8 + 2 * t + 1], 0.f);
-        if (BF16) {
-          __nv_bfloat162 h2 = __floats2bfloat162_rn(lo, hi);
-          packed[t] = *reinterpret_cast<uint32_t*>(&h2);
-        } else {
-          __half2 h2 = __floats2half2_rn(lo, hi);
-          packed[t] = *reinterpret_cast<uint32_t*>(&h2);
-        }
-      }
-      const uint32_t addr = chunk_base + (((piece0 + (uint32_t)q) ^ ((uint32_t)row_in_tile & 7u)) << 4);
-      st_shared_v4(addr, make_uint4(packed[0], packed[1], packed[2], packed[3]));
-    }
-    bias_cur = bias_nxt;
+  // Training forward: the stores of the previous layer's activations must have read the tile before it is overwritten.
+  if (bar_act_free && !mbar_wait(bar_act_free, act_parity, abortp, SB_SITE_MLP_ACT)) return false;
+  const uint32_t key = (uint32_t)row_in_tile & 7u;
+  const uint32_t dst0 = act_base + (uint32_t)row_in_tile * 128u;
+  uint32_t* word = bits_out && row < batch ? bits_out + (long long)half * batch + row : nullptr;
+  tmem_ld32(t_row + (uint32_t)(half * 32), raw_a);
+  auto finish = [&](uint32_t* raw, int i) {      // chunk half + 2 i: the left or right half of activation chunk i
+    hidden_chunk<BF16>(raw, norm, sumsq, bias != nullptr, bias_smem + 128u * (uint32_t)i,
+                       word ? word + 2LL * i * batch : nullptr, dst0 + (uint32_t)i * FM_CHUNK_BYTES, 4u * (uint32_t)half, key);
     // generic-proxy writes of the activation tile must be visible to the MMA's async-proxy reads
     fence_proxy_async_smem();
     tc_fence_before_sync();
     __syncwarp();
-    if (lane == 0) mbar_arrive(chunk_bar0 + 8u * (uint32_t)(c >> 1));
+    if (lane == 0) mbar_arrive(chunk_bar0 + 8u * (uint32_t)i);
+  };
+#pragma unroll 1
+  for (int i = 0; i < mine; i += 2) {
+    tmem_ld_wait32(raw_a);
+    if (i + 1 < mine) tmem_ld32(t_row + (uint32_t)((half + 2 * i + 2) * 32), raw_b);
+    finish(raw_a, i);
+    if (i + 1 >= mine) break;
+    tmem_ld_wait32(raw_b);
+    if (i + 2 < mine) tmem_ld32(t_row + (uint32_t)((half + 2 * i + 4) * 32), raw_a);
+    finish(raw_b, i + 1);
   }
+  return true;
 }
 
 // The per-decision tail for one state, once every member's probabilities and sampled index are in
@@ -215,17 +238,18 @@ __device__ __noinline__ void decide_row(const FusedParams& p, long long row) {
     p.prob_ensemble[row * p.members + e] = a >= 0 ? __ldcg(prow + (long long)e * p.out_stride + a) : 0.f;
 }
 
+template <bool BF16>
 __global__ void __launch_bounds__(FM_THREADS, 1)
 mlp_fused_kernel(const __grid_constant__ FusedMaps maps, const __grid_constant__ FusedParams p) {
   extern __shared__ uint8_t fm_smem_raw[];
-  __shared__ __align__(8) uint64_t bar_x_full, bar_x_empty, bar_acc_full, bar_item_done, bar_tail_in, bar_tail_out;
+  __shared__ __align__(8) uint64_t bar_x_full, bar_x_empty, bar_act_free, bar_tail_in, bar_tail_out;
+  __shared__ __align__(8) uint64_t bar_acc_full[2], bar_head_done[2];      // per accumulator
   __shared__ __align__(8) uint64_t bar_chunk[4];       // 64-column chunk k of the activation tile is written (8 warps each)
-  __shared__ __align__(8) uint64_t bar_w_full[FM_W_STAGES], bar_w_empty[FM_W_STAGES];
+  __shared__ __align__(8) uint64_t bar_w_full[FM_W_STAGES_MAX], bar_w_empty[FM_W_STAGES_MAX];
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
   __shared__ int tile_is_complete;
   __shared__ SbRowHead head_slot[FM_EPI_WARPS];
-  __shared__ __align__(16) float bias_spread[FM_EPI_WARPS][32];
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t base = (smem_u32(fm_smem_raw) + 1023u) & ~1023u;
@@ -236,12 +260,15 @@ mlp_fused_kernel(const __grid_constant__ FusedMaps maps, const __grid_constant__
   if (tid == 0) {
     mbar_init(smem_u32(&bar_x_full), 1);
     mbar_init(smem_u32(&bar_x_empty), 1);
-    mbar_init(smem_u32(&bar_acc_full), 1);
-    mbar_init(smem_u32(&bar_item_done), FM_EPI_WARPS);
+    mbar_init(smem_u32(&bar_act_free), 1);
+    for (int a = 0; a < 2; ++a) {
+      mbar_init(smem_u32(&bar_acc_full[a]), 1);
+      mbar_init(smem_u32(&bar_head_done[a]), 4);    // the four warps that finish head rows
+    }
     for (int k = 0; k < 4; ++k) mbar_init(smem_u32(&bar_chunk[k]), FM_EPI_WARPS);
     mbar_init(smem_u32(&bar_tail_in), 4);       // the four warps that finish head rows
     mbar_init(smem_u32(&bar_tail_out), 1);
-    for (int s = 0; s < FM_W_STAGES; ++s) {
+    for (int s = 0; s < p.w_stages; ++s) {
       mbar_init(smem_u32(&bar_w_full[s]), 1);
       mbar_init(smem_u32(&bar_w_empty[s]), 1);
     }
@@ -263,96 +290,101 @@ mlp_fused_kernel(const __grid_constant__ FusedMaps maps, const __grid_constant__
   sb_grid_dependency_wait();
   sb_grid_dependents_launch();
 
+  // The producer and the issuer are whole warps that run their loops together; single instructions are predicated on
+  // `one` (see umma_issue).
+  const bool one = elect_one_lane();
   if (warp == 0) {
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t w_phase = 0, x_phase = 0;
-      bool ok = true;
-      for (int item = blockIdx.x; ok && item < p.num_items; item += gridDim.x) {
-        const int member = item / p.num_tiles, tile = item - member * p.num_tiles;
-        if (!mbar_wait(smem_u32(&bar_x_empty), x_phase ^ 1u, abortp, SB_SITE_MLP_ACT)) break;
-        x_phase ^= 1u;
-        mbar_arrive_expect_tx(smem_u32(&bar_x_full), p.x_chunks * FM_CHUNK_BYTES);
-        for (uint32_t c = 0; c < p.x_chunks; ++c)
-          tma_load_2d(x_base + c * FM_CHUNK_BYTES, &maps.x, (int)(c * 64), tile * 128, smem_u32(&bar_x_full));
-        for (int l = 0; ok && l < L; ++l) {
-          for (int c = 0; c < p.k_chunks[l]; ++c) {
-            if (!mbar_wait(smem_u32(&bar_w_empty[stage]), w_phase ^ 1u, abortp, SB_SITE_MLP_WEIGHTS)) {
-              ok = false;
-              break;
-            }
-            mbar_arrive_expect_tx(smem_u32(&bar_w_full[stage]), p.w_bytes[l]);
-            tma_load_3d(w_base + (uint32_t)stage * p.stage_bytes, &maps.w[l], c * 64, 0, member, smem_u32(&bar_w_full[stage]));
-            if (++stage == FM_W_STAGES) {
-              stage = 0;
-              w_phase ^= 1u;
-            }
+    int stage = 0;
+    uint32_t w_phase = 0, x_phase = 0;
+    bool ok = true;
+    for (int item = blockIdx.x; ok && item < p.num_items; item += gridDim.x) {
+      const int member = item / p.num_tiles, tile = item - member * p.num_tiles;
+      if (!mbar_wait_warp(smem_u32(&bar_x_empty), x_phase ^ 1u, abortp, SB_SITE_MLP_ACT)) break;
+      x_phase ^= 1u;
+      if (one) mbar_arrive_expect_tx(smem_u32(&bar_x_full), p.x_chunks * FM_CHUNK_BYTES);
+      for (uint32_t c = 0; c < p.x_chunks; ++c)
+        tma_load_2d(x_base + c * FM_CHUNK_BYTES, &maps.x, (int)(c * 64), tile * 128, smem_u32(&bar_x_full), one);
+      for (int l = 0; ok && l < L; ++l) {
+        for (int c = 0; c < p.k_chunks[l]; ++c) {
+          if (!mbar_wait_warp(smem_u32(&bar_w_empty[stage]), w_phase ^ 1u, abortp, SB_SITE_MLP_WEIGHTS)) {
+            ok = false;
+            break;
+          }
+          if (one) mbar_arrive_expect_tx(smem_u32(&bar_w_full[stage]), p.w_bytes[l]);
+          tma_load_3d(w_base + (uint32_t)stage * p.stage_bytes, &maps.w[l], c * 64, 0, member, smem_u32(&bar_w_full[stage]), one);
+          if (++stage == p.w_stages) {
+            stage = 0;
+            w_phase ^= 1u;
           }
         }
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t w_phase = 0, x_phase = 0, item_phase = 0, chunk_phase = 0;     // chunk_phase: one parity bit per chunk barrier
-      bool ok = true;
-      const uint32_t hi = (uint32_t)(umma_smem_desc(0u, 16u, 1024u, 2u) >> 32);
-      for (int item = blockIdx.x; ok && item < p.num_items; item += gridDim.x) {
-        const int tile = item % p.num_tiles;
-        for (int l = 0; ok && l < L; ++l) {
-          uint32_t a_base;
-          if (l == 0) {
-            if (!mbar_wait(smem_u32(&bar_x_full), x_phase, abortp, SB_SITE_MLP_ACT)) { ok = false; break; }
-            x_phase ^= 1u;
-            a_base = x_base;
-          } else {
-            a_base = act_base;
-          }
-          tc_fence_after_sync();
-          // Layers alternate between two accumulators: the epilogue of layer l-1 still reads its own while
-          // this layer's first MMAs run.  (Layer l+1 reuses the accumulator of layer l-1 only after every
-          // chunk of this layer's input -- the whole of layer l-1's epilogue -- has been delivered.)
-          const uint32_t d_tmem = tmem_base + (uint32_t)((l & 1) * p.acc_stride);
-          uint32_t accumulate = 0u;
-          for (int c = 0; c < p.k_chunks[l]; ++c) {
-            if (l > 0) {
-              // K-chunk c of this layer's input = 64-column chunk c of the previous layer's output
-              if (!mbar_wait(smem_u32(&bar_chunk[c]), (chunk_phase >> c) & 1u, abortp, SB_SITE_MLP_ACT)) { ok = false; break; }
-              chunk_phase ^= 1u << c;
-              tc_fence_after_sync();
-              // Training forward: the delivered chunk of the previous layer's output also leaves for global
-              // memory; the tile in shared memory already has the layout of a TMA box.
-              if (p.store_acts) {
-                tma_store_2d(&maps.act[l - 1], a_base + (uint32_t)c * FM_CHUNK_BYTES, c * 64, tile * 128);
-                bulk_commit_group();
-              }
-            }
-            if (!mbar_wait(smem_u32(&bar_w_full[stage]), w_phase, abortp, SB_SITE_MLP_WEIGHTS)) { ok = false; break; }
+    int stage = 0;
+    uint32_t w_phase = 0, x_phase = 0, chunk_phase = 0, head_phase = 0;     // chunk_phase, head_phase: one parity bit per barrier
+    uint32_t acc = 0;
+    bool ok = true;
+    const uint32_t hi = (uint32_t)(umma_smem_desc(0u, 16u, 1024u, 2u) >> 32);
+    int done = 0;                               // items before this one
+    for (int item = blockIdx.x; ok && item < p.num_items; item += gridDim.x, ++done) {
+      const int tile = item % p.num_tiles;
+      for (int l = 0; ok && l < L; ++l, acc ^= 1u) {
+        uint32_t a_base;
+        if (l == 0) {
+          if (!mbar_wait_warp(smem_u32(&bar_x_full), x_phase, abortp, SB_SITE_MLP_ACT)) { ok = false; break; }
+          x_phase ^= 1u;
+          a_base = x_base;
+        } else {
+          a_base = act_base;
+        }
+        // Layers alternate between two accumulators, across items too: the epilogue of layer l-1 still reads its
+        // own while this layer's first MMAs run, and the next item's first layer runs beside the head of this one.
+        // The accumulator of two layers ago is free: a hidden layer's because all of its chunks were delivered
+        // before the layer after it began, a head's when its four warps have said so.
+        if (L > 1 ? (l == 1 && done > 0) : done > 1) {
+          if (!mbar_wait_warp(smem_u32(&bar_head_done[acc]), (head_phase >> acc) & 1u, abortp, SB_SITE_MLP_ACT)) { ok = false; break; }
+          head_phase ^= 1u << acc;
+        }
+        tc_fence_after_sync();
+        const uint32_t d_tmem = tmem_base + acc * (uint32_t)p.acc_stride;
+        uint32_t accumulate = 0u;
+        for (int c = 0; c < p.k_chunks[l]; ++c) {
+          if (l > 0) {
+            // K-chunk c of this layer's input = 64-column chunk c of the previous layer's output
+            if (!mbar_wait_warp(smem_u32(&bar_chunk[c]), (chunk_phase >> c) & 1u, abortp, SB_SITE_MLP_ACT)) { ok = false; break; }
+            chunk_phase ^= 1u << c;
             tc_fence_after_sync();
-            const uint32_t a_lo = (uint32_t)umma_smem_desc(a_base + (uint32_t)c * FM_CHUNK_BYTES, 16u, 1024u, 2u);
-            const uint32_t b_lo = (uint32_t)umma_smem_desc(w_base + (uint32_t)stage * p.stage_bytes, 16u, 1024u, 2u);
+            // Training forward: the delivered chunk of the previous layer's output also leaves for global
+            // memory; the tile in shared memory already has the layout of a TMA box.
+            if (p.store_acts && one) {
+              tma_store_2d(&maps.act[l - 1], a_base + (uint32_t)c * FM_CHUNK_BYTES, c * 64, tile * 128);
+              bulk_commit_group();
+            }
+          }
+          if (!mbar_wait_warp(smem_u32(&bar_w_full[stage]), w_phase, abortp, SB_SITE_MLP_WEIGHTS)) { ok = false; break; }
+          tc_fence_after_sync();
+          const uint32_t a_lo = (uint32_t)umma_smem_desc(a_base + (uint32_t)c * FM_CHUNK_BYTES, 16u, 1024u, 2u);
+          const uint32_t b_lo = (uint32_t)umma_smem_desc(w_base + (uint32_t)stage * p.stage_bytes, 16u, 1024u, 2u);
+          const uint32_t steps = (uint32_t)(p.k_steps[l] - 4 * c);      // beyond the layer's inputs both tiles are zero
 #pragma unroll
-            for (uint32_t ks = 0; ks < 4; ++ks) {
-              umma_issue<false, false>(d_tmem, a_lo + 2u * ks, hi, b_lo + 2u * ks, hi, p.idesc[l], accumulate);
+          for (uint32_t ks = 0; ks < 4; ++ks) {
+            if (ks < steps) {
+              umma_issue<false, false>(d_tmem, a_lo + 2u * ks, hi, b_lo + 2u * ks, hi, p.idesc[l], accumulate, one);
               accumulate = 1u;
             }
-            tc_commit(smem_u32(&bar_w_empty[stage]));
-            if (++stage == FM_W_STAGES) {
-              stage = 0;
-              w_phase ^= 1u;
-            }
           }
-          if (!ok) break;
-          if (l == 0) tc_commit(smem_u32(&bar_x_empty));     // the input tile may be refilled
-          // This layer's epilogue overwrites the activation tile: the stores of its chunks must have read it.
-          if (p.store_acts && l > 0) bulk_wait_group_read<0>();
-          tc_commit(smem_u32(&bar_acc_full));
+          tc_commit(smem_u32(&bar_w_empty[stage]), one);
+          if (++stage == p.w_stages) {
+            stage = 0;
+            w_phase ^= 1u;
+          }
         }
-        // The next tile's layers overwrite the accumulators and the activation tile: wait until the head
-        // has read the last accumulator.
-        if (ok && item + (int)gridDim.x < p.num_items) {
-          if (!mbar_wait(smem_u32(&bar_item_done), item_phase, abortp, SB_SITE_MLP_ACT)) break;
-          item_phase ^= 1u;
+        if (!ok) break;
+        if (l == 0) tc_commit(smem_u32(&bar_x_empty), one);     // the input tile may be refilled
+        tc_commit(smem_u32(&bar_acc_full[acc]), one);
+        if (p.store_acts && l > 0 && one) {    // the stores of this layer's input have read the activation tile
+          bulk_wait_group_read<0>();
+          mbar_arrive(smem_u32(&bar_act_free));
         }
       }
     }
@@ -360,8 +392,9 @@ mlp_fused_kernel(const __grid_constant__ FusedMaps maps, const __grid_constant__
     const int quad = warp & 3, half = (warp - 2) >> 2;
     const int row_in_tile = quad * 32 + lane;
     const uint32_t t_row = tmem_base + ((uint32_t)(quad * 32) << 16);
-    const uint32_t bias_smem = smem_u32(&bias_spread[warp - 2][0]);
-    uint32_t acc_phase = 0, tail_phase = 0;
+    const uint32_t bias_smem = base + p.bias_offset + (uint32_t)(warp - 2) * 512u;
+    uint32_t layer = 0, tail_phase = 0;           // layer: counts layers across items; its last two bits are accumulator and phase
+    uint32_t act_phase = 1;                       // the first tile finds the activation tile free
     // This warp's copy of the head description (in shared memory: the head code reads a field where it
     // needs it instead of holding the whole structure in registers); member-specific fields are set per item.
     SbRowHead& h = head_slot[warp - 2];
@@ -380,33 +413,47 @@ mlp_fused_kernel(const __grid_constant__ FusedMaps maps, const __grid_constant__
       __syncwarp();
       const float* head_bias = p.bias[L - 1] ? p.bias[L - 1] + pofs : nullptr;
       for (int l = 0; l < L; ++l) {
-        const uint32_t t_acc = t_row + (uint32_t)((l & 1) * p.acc_stride);
+        const uint32_t acc = layer & 1u, acc_phase = (layer >> 1) & 1u;
+        ++layer;
+        const uint32_t t_acc = t_row + acc * (uint32_t)p.acc_stride;
+        const uint32_t full = smem_u32(&bar_acc_full[acc]);
         const long long grow = (long long)tile * 128 + row_in_tile;
-        if (l < L - 1 || half != 0) {
-          if (!mbar_wait(smem_u32(&bar_acc_full), acc_phase, abortp, SB_SITE_MLP_ACC)) { ok = false; break; }
-          tc_fence_after_sync();
-        }
         if (l < L - 1) {
           const float* bias_l = p.bias[l] ? p.bias[l] + pofs : nullptr;
-          if (p.is_bf16) fused_hidden<true>(t_acc, p.n_pad[l], bias_l, act_base, bias_smem, row_in_tile, lane, half, p.hidden_norm, smem_u32(&bar_chunk[0]), p.bits[l], grow, p.batch);
-          else fused_hidden<false>(t_acc, p.n_pad[l], bias_l, act_base, bias_smem, row_in_tile, lane, half, p.hidden_norm, smem_u32(&bar_chunk[0]), p.bits[l], grow, p.batch);
-        } else {
-          if (half == 0) {
-            const uint32_t full = smem_u32(&bar_acc_full);
-            switch (p.head_width) {
-              case 4: ok = fused_head<4>(h, head_bias, out_m, t_acc, grow, p.batch, full, acc_phase, abortp); break;
-              case 8: ok = fused_head<8>(h, head_bias, out_m, t_acc, grow, p.batch, full, acc_phase, abortp); break;
-              case 16: ok = fused_head<16>(h, head_bias, out_m, t_acc, grow, p.batch, full, acc_phase, abortp); break;
-              case 32: ok = fused_head<32>(h, head_bias, out_m, t_acc, grow, p.batch, full, acc_phase, abortp); break;
-              default: ok = fused_head<64>(h, head_bias, out_m, t_acc, grow, p.batch, full, acc_phase, abortp); break;
+          const uint32_t act_free = p.store_acts ? smem_u32(&bar_act_free) : 0u;
+          ok = fused_hidden<BF16>(t_acc, p.n_pad[l], bias_l, act_base, bias_smem, row_in_tile, half, p.hidden_norm != 0,
+                                  smem_u32(&bar_chunk[0]), p.bits[l], grow, p.batch, full, acc_phase, act_free, act_phase, abortp);
+          act_phase ^= 1u;
+        } else if (half == 0) {
+          // What the head needs beside the accumulator is asked for before the wait: its biases (into the warp's
+          // buffer) and the row's mask bytes.
+          if (head_bias) {
+#pragma unroll
+            for (int j = lane; j < 64; j += 32) {
+              const float b = j < h.n ? __ldg(head_bias + j) : 0.f;
+              asm volatile("st.shared.f32 [%0], %1;" ::"r"(bias_smem + 4u * (uint32_t)j), "f"(b) : "memory");
             }
-            if (!ok) break;
           }
-          tc_fence_before_sync();
+          unsigned long long legal = 0ull;
+          if (grow < p.batch) {
+            if (p.head_width <= 4) legal = sb_row_head_legal<4>(h, grow);
+            else if (p.head_width <= 16) legal = sb_row_head_legal<16>(h, grow);
+            else legal = sb_row_head_legal<64>(h, grow);
+          }
           __syncwarp();
-          if (lane == 0) mbar_arrive(smem_u32(&bar_item_done));
+          if (!mbar_wait(full, acc_phase, abortp, SB_SITE_MLP_ACC)) { ok = false; break; }
+          tc_fence_after_sync();
+          const uint32_t head_done = smem_u32(&bar_head_done[acc]);
+          const bool hb = head_bias != nullptr;
+          switch (p.head_width) {
+            case 4: fused_head<4>(h, legal, hb, bias_smem, out_m, t_acc, grow, p.batch, head_done); break;
+            case 8: fused_head<8>(h, legal, hb, bias_smem, out_m, t_acc, grow, p.batch, head_done); break;
+            case 16: fused_head<16>(h, legal, hb, bias_smem, out_m, t_acc, grow, p.batch, head_done); break;
+            case 32: fused_head<32>(h, legal, hb, bias_smem, out_m, t_acc, grow, p.batch, head_done); break;
+            default: fused_head<64>(h, legal, hb, bias_smem, out_m, t_acc, grow, p.batch, head_done); break;
+          }
         }
-        acc_phase ^= 1u;
+        if (!ok) break;
       }
       if (ok && p.tile_counters && half == 0) {
         // Decision tail (ml/models.spi:51-76).  The four head warps publish their rows of this member, count
@@ -526,7 +573,6 @@ static int fused_launch(const char* who, int n_layers, const int* sizes, int bat
   const int head_cols = sb_row_head_columns(head);      // columns that the head turns into zeros are not multiplied
   p.n_layers = n_layers;
   p.batch = batch;
-  p.is_bf16 = in_dtype == SB_BF16;
   p.num_tiles = (batch + 127) / 128;
   p.num_items = p.num_tiles * members;
   p.member_stride = off[2 * n_layers];
@@ -538,6 +584,7 @@ static int fused_launch(const char* who, int n_layers, const int* sizes, int bat
     const bool last = l == n_layers - 1;
     p.n_pad[l] = last ? (head_cols + 15) / 16 * 16 : sizes[l + 1];
     p.k_chunks[l] = (sizes[l] + 63) / 64;
+    p.k_steps[l] = (sizes[l] + 15) / 16;
     p.idesc[l] = sb_umma_idesc(in_dtype, 0, 0, 128, p.n_pad[l]);
     p.w_bytes[l] = (uint32_t)p.n_pad[l] * 128u;
     p.bias[l] = params ? params + off[2 * l + 1] : nullptr;
@@ -575,27 +622,34 @@ static int fused_launch(const char* who, int n_layers, const int* sizes, int bat
     p.prob_selected = decide->prob_selected; p.prob_ensemble = decide->prob_ensemble;
   }
   p.stage_bytes = ((uint32_t)max_n * 128u + 1023u) / 1024u * 1024u;     // stages stay 1024-byte aligned (swizzle atoms)
-  const size_t smem = (size_t)p.w_offset + (size_t)FM_W_STAGES * p.stage_bytes + 1024;
   // Which nets are taken depends on the widths alone, not on how few columns the head of a call needs.
   const uint32_t full_n = (uint32_t)((n_out + 15) / 16 * 16 > max_n ? (n_out + 15) / 16 * 16 : max_n);
-  const size_t smem_limit_case = (size_t)p.w_offset + (size_t)FM_W_STAGES * (full_n * 128u) + 1024;
+  const size_t smem_needed = (size_t)p.w_offset + (size_t)FM_W_STAGES * (full_n * 128u) + 1024;
+  if (smem_needed > FM_SMEM_LIMIT)
+    return sb_fail(SB_ERR_UNSUPPORTED, "%s: the input tile, the widest hidden tile and the weight ring need %zu bytes of "
+                                       "shared memory (inputs wider than 256 fit with hidden layers of at most 128)", who, smem_needed);
+  // The ring takes what is left beside the bias buffers: more than the four stages of the rule above for narrow
+  // layers, three for the widest nets with biases.
+  const uint32_t bias_bytes = params ? FM_BIAS_BYTES : 0u;
+  p.w_stages = (int)((FM_SMEM_LIMIT - 1024 - p.w_offset - bias_bytes) / p.stage_bytes);
+  if (p.w_stages > FM_W_STAGES_MAX) p.w_stages = FM_W_STAGES_MAX;
+  p.bias_offset = p.w_offset + (uint32_t)p.w_stages * p.stage_bytes;
+  const size_t smem = (size_t)p.bias_offset + bias_bytes + 1024;
 
   static std::atomic<bool> attr_set[64];
   int dev = 0;
   SB_CUDA(cudaGetDevice(&dev));
   if (dev >= 0 && dev < 64 && !attr_set[dev].load(std::memory_order_acquire)) {
-    SB_CUDA(cudaFuncSetAttribute(mlp_fused_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 225 * 1024));
+    SB_CUDA(cudaFuncSetAttribute(mlp_fused_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FM_SMEM_LIMIT));
+    SB_CUDA(cudaFuncSetAttribute(mlp_fused_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FM_SMEM_LIMIT));
     attr_set[dev].store(true, std::memory_order_release);
   }
-  if (smem_limit_case > 225 * 1024)
-    return sb_fail(SB_ERR_UNSUPPORTED, "%s: the input tile, the widest hidden tile and the weight ring need %zu bytes of "
-                                       "shared memory (inputs wider than 256 fit with hidden layers of at most 128)", who, smem_limit_case);
   const int sms = sb_sm_count();
   const int grid = p.num_items < sms ? p.num_items : sms;
   double flops = 0.0;
   for (int l = 0; l < n_layers; ++l) flops += 2.0 * batch * (double)sizes[l] * sizes[l + 1] * members;
   sb_prof_before((cudaStream_t)stream);
-  SB_CUDA(sb_launch(mlp_fused_kernel, dim3(grid), dim3(FM_THREADS), smem, (cudaStream_t)stream, 1, maps, p));
+  SB_CUDA(sb_launch(in_dtype == SB_BF16 ? mlp_fused_kernel<true> : mlp_fused_kernel<false>, dim3(grid), dim3(FM_THREADS), smem, (cudaStream_t)stream, 1, maps, p));
   sb_prof_after((cudaStream_t)stream, flops);
   SB_COUNT_LAUNCH();
   SB_CUDA(cudaGetLastError());
@@ -689,7 +743,7 @@ static bool fused_shape_ok(int n_layers, const int* sizes, int in_dtype) {
   if ((n_out + 15) / 16 * 16 > max_n) max_n = (n_out + 15) / 16 * 16;
   const size_t stage = ((size_t)max_n * 128 + 1023) / 1024 * 1024;
   const size_t smem = (size_t)((sizes[0] + 63) / 64 + max_act_chunks) * FM_CHUNK_BYTES + FM_W_STAGES * stage + 1024;
-  return smem <= 225 * 1024;
+  return smem <= FM_SMEM_LIMIT;
 }
 
 extern "C" int sb_mlp_fused_supported(int n_layers, const int* sizes, int in_dtype) {

@@ -200,6 +200,44 @@ def test_fused_persistent_forward_matches_layerwise_and_oracle(gpu, in_dtype, ba
     assert agree.mean() > 0.999
 
 
+@pytest.mark.parametrize("with_bias", [True, False])
+@pytest.mark.parametrize("sizes", [[8, 3], [512, 64], [24, 64, 5], [40, 192, 33], [32, 256, 256, 256, 3], [72, 64, 64, 128, 10],
+                                   [128, 256, 256, 17], [504, 128, 64, 4]])
+def test_fused_forward_over_many_tiles_per_cta(gpu, sizes, with_bias):
+    """Tiles that follow each other on one SM (the next tile's first layer runs beside this one's head): the same
+    bits as rows that find the SM idle, for one to four layers, every hidden width, inputs that end inside an MMA's
+    16 columns, and the widest shapes that fit in shared memory; the training forward's activations and sign words too."""
+    tile_rows = 128 * gpu.sm_count()
+    batch = 3 * tile_rows + 77
+    net, ws, bs = build(gpu, sizes, batch, "f16", 14, head=("masked_softmax", "argmax"), bias_scale=0.1)
+    train = gpu.PolicyMLP(sizes, batch, in_dtype="f16", with_bias=with_bias, training=True)
+    net = gpu.PolicyMLP(sizes, batch, in_dtype="f16", head=("masked_softmax", "argmax"), with_bias=with_bias)
+    g = so.rng(14)
+    x = (g.random((batch, sizes[0])) < 0.3).astype(np.float32)
+    dx = gpu.to_storage(x, "f16")
+    for n in (net, train):
+        n.load_weights(ws, bs if with_bias else None)
+    got = net.forward_fused(dx).numpy().copy()
+    actions = net.actions.numpy().copy()
+    np.testing.assert_array_equal(train.forward(dx).numpy(), got)
+    np.testing.assert_array_equal(actions, np.argmax(got, axis=1))
+    acts = [a.numpy() for a in train.activations]
+    for first in range(0, batch, tile_rows):
+        rows = min(tile_rows, batch - first)
+        part = gpu.PolicyMLP(sizes, rows, in_dtype="f16", with_bias=with_bias, training=True)
+        part.load_weights(ws, bs if with_bias else None)
+        view = dx.view((rows, sizes[0]), offset_bytes=first * sizes[0] * 2)
+        np.testing.assert_array_equal(part.forward(view).numpy(), got[first:first + rows])
+        for i, a in enumerate(part.activations):
+            np.testing.assert_array_equal(a.numpy(), acts[i][first:first + rows])
+            words = train.relu_bits[i].numpy().reshape(sizes[i + 1] // 32, batch)
+            np.testing.assert_array_equal(part.relu_bits[i].numpy().reshape(-1, rows), words[:, first:first + rows])
+    rows = slice(batch - 500, batch)
+    want = so.mlp_forward(x[rows], ws, bs if with_bias else [np.zeros_like(b) for b in bs], np.ones((500, sizes[-1]), np.uint8),
+                          in_dtype="f16", act_dtype="f16")
+    assert so.rel_frobenius(got[rows], want) <= TOL
+
+
 def test_fused_forward_other_shapes_and_limits(gpu):
     from spiral_b200 import SpiralError
     sizes, batch = [64, 128, 64, 10], 777
