@@ -232,10 +232,19 @@ __device__ __noinline__ void decide_row(const FusedParams& p, long long row) {
   const int a = __ldcg(p.head.sample_out + (long long)e_id * p.batch + row);
   p.ensemble_id[row] = e_id;
   p.action[row] = a;
-  const float* prow = p.out + row * n;
-  p.prob_selected[row] = a >= 0 ? __ldcg(prow + (long long)e_id * p.out_stride + a) : 0.f;
-  for (int e = 0; e < p.members; ++e)
-    p.prob_ensemble[row * p.members + e] = a >= 0 ? __ldcg(prow + (long long)e * p.out_stride + a) : 0.f;
+  const float* prow = p.out + row * n + (a >= 0 ? a : 0);
+  p.prob_selected[row] = a >= 0 ? __ldcg(prow + (long long)e_id * p.out_stride) : 0.f;
+  float* by_member = p.prob_ensemble + row * p.members;
+  // The members' probabilities lie a whole output apart: eight are on their way at a time (a load and a store in turn
+  // took a memory round trip per member; 16 members, 256 states: 19.8 -> 19.1 us).
+  for (int e0 = 0; e0 < p.members; e0 += 8) {
+    float v[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = a >= 0 && e0 + j < p.members ? __ldcg(prow + (long long)(e0 + j) * p.out_stride) : 0.f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (e0 + j < p.members) by_member[e0 + j] = v[j];
+  }
 }
 
 template <bool BF16>
