@@ -603,10 +603,7 @@ __device__ __noinline__ bool epilogue_tile(uint32_t t_row, int row0_warp, int n0
     tmem_ld32(t_row + (uint32_t)(c * 32), raw_a);
     fetch(c + STRIDE, bias_nxt, gate_nxt);    // in flight while this chunk is finished
     tmem_ld_wait();
-    if (ln_l2) {
-#pragma unroll
-      for (int j = 0; j < 32; ++j) raw_a[j] = __float_as_uint(sumsq != 0.f ? __uint_as_float(raw_a[j]) / sumsq : 0.f);
-    }
+    if (ln_l2) divide_row32(reinterpret_cast<float*>(raw_a), sumsq);
     const int col0 = n0 + c * 32;
     if (rows_live && col0 < N) {
       const uint32_t box = sbuf + ((EW == 8 && MODE != -2 && sizeof(OutT) == 2 && g_epi.tma_c) ? box_sel : 0u);

@@ -120,10 +120,7 @@ template <bool BF16>
 __device__ __forceinline__ void hidden_chunk(uint32_t* raw, bool norm, float sumsq, bool has_bias, uint32_t bias_addr,
                                              uint32_t* word, uint32_t dst, uint32_t piece0, uint32_t key) {
   float* v = reinterpret_cast<float*>(raw);
-  if (norm) {
-#pragma unroll
-    for (int j = 0; j < 32; ++j) v[j] = sumsq != 0.f ? v[j] / sumsq : 0.f;
-  }
+  if (norm) divide_row32(v, sumsq);
   if (has_bias) {
 #pragma unroll
     for (int q = 0; q < 8; ++q) {

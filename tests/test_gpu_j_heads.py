@@ -162,6 +162,32 @@ def test_row_normalisation_epilogue(gpu, n, out_dtype, in_dtype):
                    gpu.DeviceArray((8, 512), out_dtype), in_dtype=in_dtype, epilogue=("ln_l2",))
 
 
+def test_row_normalisation_over_the_whole_range(gpu):
+    """x / sum(x^2) where the sum is zero, subnormal, small, ordinary, large and infinite, in one tile: every row is
+    the IEEE quotient by the fp32 sum of squares.  The rows come through a product with the identity, so they are
+    exact; the sum's order is the kernel's own: 64 roundings of positive terms, 64 * 2^-24 = 3.9e-6 relative."""
+    n = 64
+    g = so.rng(77)
+    x = so.round_tf32(g.normal(size=(256, n)).astype(np.float32))
+    scales = np.array([0.0, 1e-30, 1e-22, 1e-19, 1e-12, 3e-7, 1.0, 1e5, 3e7, 1e15, 1e18, 1e20, 1e30], np.float32)
+    with np.errstate(over="ignore", under="ignore"):
+        x = so.round_tf32(x * scales[np.arange(256) % len(scales)][:, None])
+        want = so.ln_l2(x)
+    for rows in (slice(0, 256), slice(6, 7)):          # mixed with the others, and alone
+        a = np.ascontiguousarray(x[rows])
+        c = gpu.DeviceArray((a.shape[0], n), "f32")
+        gpu.matmul(False, True, 1.0, gpu.DeviceArray.from_numpy(a), gpu.DeviceArray.from_numpy(np.eye(n, dtype=np.float32)),
+                   0.0, c, in_dtype="tf32", epilogue=("ln_l2",))
+        got = c.numpy()
+        ok = np.isfinite(want[rows]) & (np.abs(want[rows]) > 1e-37)
+        s = np.sum(np.square(a.astype(np.float64)), axis=1)
+        ordinary = ((s > 1e-36) & (s < 3e38))[:, None] & ok
+        with np.errstate(divide="ignore", invalid="ignore"):
+            quotient = a / s[:, None]
+        np.testing.assert_allclose(got[ordinary], quotient[ordinary], rtol=5e-6)
+        assert np.all(got[s == 0] == 0) and np.all(got[s > 3.5e38] == 0)
+
+
 def test_reference_test_net_runs_in_three_launches(gpu):
     """The reference's test net (ml/layers.spi:594-608; game/leduc/tests/train.spi:88-101): three dense layers
     with ln_l2 + relu between them and a prefix-masked softmax + sampling head, every member of an ensemble:
