@@ -66,11 +66,13 @@ int check_head(const char* who, const SbRowHead& h, int N) {
 // fp32 class on the tensor cores: the "3 x TF32" split.
 //
 // An fp32 value x is written hi + lo with hi = tf32(x) and lo = tf32(x - hi) (both rounded to
-// nearest); then A * B = Ah*Bh + Ah*Bl + Al*Bh up to terms of relative size 2^-22.  The three products
-// are ONE tensor-core GEMM over operands concatenated along K:
-//     [Ah | Ah | Al] (M x 3K)   times   [Bh ; Bl ; Bh] (3K x N),
-// accumulated in fp32 in tensor memory.  A pre-pass kernel writes the concatenated operands (in the
-// same storage order as the originals, so every layout flag carries over) into a caller workspace.
+// nearest); then A * B = Ah*Bh + Ah*Bl + Al*Bh up to terms of relative size 2^-22.  A pre-pass kernel
+// writes both parts of both operands (in the storage order of the originals, so every layout flag
+// carries over) into a caller workspace; ONE tensor-core GEMM brings the four tiles of a K range into a
+// pipeline stage and issues the three products from them, accumulated in fp32 in tensor memory.
+// (The three products as one GEMM over operands concatenated to 3K read six tiles where these are four,
+// and a main loop of TF32 is bound by the operand bytes that reach an SM: 2048^3 98 -> 80 us, 4096 x
+// 4096 x 512 103 -> 85, 256 x 256 x 16384 46 -> 35, 512^3 unchanged, bound by the host.)
 // ---------------------------------------------------------------------------
 namespace {
 
@@ -81,26 +83,22 @@ __device__ __forceinline__ float tf32_rn(float v) {
   return __uint_as_float(u & 0xffffe000u);
 }
 
-// `src` is [rows, cols] row-major.  k_is_col: K runs along the columns (dst [rows, 3 * cols], the three
-// parts side by side in every row); otherwise K runs along the rows (dst [3 * rows, cols], the parts
-// stacked).  Part order p0, p1, p2 with 0 = hi, 1 = lo.  Two matrices per launch (A then B).
+// `src` is a matrix of `count` elements; dst takes its high part and, behind it, its low part in the same order.  Two
+// matrices per launch (A then B).
 struct SplitJob {
   const float* src;
   float* dst;
-  long long rows, cols;
-  int k_is_col;
-  int part[3];
+  long long count;
 };
 
 // c_init: when non-null the same launch also brings C [c_count / c_cols, c_cols] to beta * C + bias (C is not read
 // for beta == 0; bias: only with BIAS), the state the split-K tiles are then added to.
 //
-// Bound by what it moves (4 bytes read, 12 written per operand element; the workspace mostly stays in L2), so a
-// thread takes four elements at a time: every contiguous dimension is a multiple of 4 (the caller's check), so a
-// quad never crosses a row and its three destinations are 16-byte aligned.  The operands themselves need only be
-// 4-byte aligned: vec_a / vec_b say which of them can be read as quads.  One element per thread with a 64-bit
-// division each was bound by issue instead: for a 2048^3 product 52 -> 23 us for this kernel (151 MB moved, 17 of them
-// C brought to zero, most of it in L2), 137 -> 113 us for the call; at 512^3 6.9 -> 4.9 us and 14.8 -> 13.3 us.
+// Bound by what it moves (4 bytes read, 8 written per operand element; the workspace mostly stays in L2), so a
+// thread takes four elements at a time: every contiguous dimension is a multiple of 4 (the caller's check), so the two
+// destinations of a quad are 16-byte aligned.  The operands themselves need only be 4-byte aligned: vec_a / vec_b say
+// which of them can be read as quads.  One element per thread was bound by issue instead: 137 -> 113 us for a 2048^3
+// product with it.
 __device__ __forceinline__ float4 load_quad(const float* p, bool vec) {
   return vec ? *reinterpret_cast<const float4*>(p) : make_float4(p[0], p[1], p[2], p[3]);
 }
@@ -109,27 +107,17 @@ __device__ __forceinline__ void split_quad(const SplitJob& j, bool vec, long lon
   const float4 x = load_quad(j.src + 4 * quad, vec);
   const float4 hi = make_float4(tf32_rn(x.x), tf32_rn(x.y), tf32_rn(x.z), tf32_rn(x.w));
   const float4 lo = make_float4(tf32_rn(x.x - hi.x), tf32_rn(x.y - hi.y), tf32_rn(x.z - hi.z), tf32_rn(x.w - hi.w));
-  long long base, pitch;             // where part 0 of this quad goes, and from one part to the next
-  if (j.k_is_col) {
-    const uint32_t cq = (uint32_t)(j.cols >> 2);      // the 64-bit form: operands from 69 GB on, with a workspace in managed memory
-    const long long r = quad <= 0xffffffffLL ? (long long)((uint32_t)quad / cq) : quad / cq;
-    base = 4 * quad + 2 * r * j.cols;
-    pitch = j.cols;
-  } else {
-    base = 4 * quad;
-    pitch = j.rows * j.cols;
-  }
-#pragma unroll
-  for (int p = 0; p < 3; ++p) *reinterpret_cast<float4*>(j.dst + base + p * pitch) = j.part[p] ? lo : hi;
+  *reinterpret_cast<float4*>(j.dst + 4 * quad) = hi;
+  *reinterpret_cast<float4*>(j.dst + j.count + 4 * quad) = lo;
 }
 
 template <bool BIAS>
 __global__ void __launch_bounds__(256)
-split3_kernel(SplitJob ja, SplitJob jb, float* c_init, long long c_count, int c_cols, float beta, const float* bias,
+split_kernel(SplitJob ja, SplitJob jb, float* c_init, long long c_count, int c_cols, float beta, const float* bias,
               int vec_a, int vec_b) {
   sb_grid_dependency_wait();
   sb_grid_dependents_launch();
-  const long long na = ja.rows * ja.cols / 4, total = na + jb.rows * jb.cols / 4;
+  const long long na = ja.count / 4, total = na + jb.count / 4;
   const long long step = (long long)gridDim.x * blockDim.x;
   const long long first = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (c_init) {                      // C is 16-byte aligned and its rows are whole quads (the caller's check)
@@ -184,13 +172,11 @@ int sb_matmul_f32x3(int a_trans, int b_trans, float alpha, const float* A, const
     return sb_fail(SB_ERR_MISALIGNED, "sb_matmul_f32x3: contiguous dimensions must be multiples of 4 elements and C 16-byte "
                                       "aligned (use the SB_F32 class of sb_matmul_ex for other shapes)");
   char* ws = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(workspace) + 255) & ~(uintptr_t)255);
-  float* a3 = reinterpret_cast<float*>(ws);
-  float* b3 = reinterpret_cast<float*>(ws + ((size_t)3 * M * K * 4 + 255) / 256 * 256);
+  float* a2 = reinterpret_cast<float*>(ws);
+  float* b2 = reinterpret_cast<float*>(ws + ((size_t)3 * M * K * 4 + 255) / 256 * 256);
   SplitJob ja, jb;
-  ja.src = A; ja.dst = a3; ja.rows = a_trans ? K : M; ja.cols = a_trans ? M : K; ja.k_is_col = a_trans ? 0 : 1;
-  ja.part[0] = 0; ja.part[1] = 0; ja.part[2] = 1;                     // Ah | Ah | Al
-  jb.src = B; jb.dst = b3; jb.rows = b_trans ? N : K; jb.cols = b_trans ? K : N; jb.k_is_col = b_trans ? 1 : 0;
-  jb.part[0] = 0; jb.part[1] = 1; jb.part[2] = 0;                     // Bh ; Bl ; Bh
+  ja.src = A; ja.dst = a2; ja.count = (long long)M * K;
+  jb.src = B; jb.dst = b2; jb.count = (long long)N * K;
   const long long total = ((long long)M * K + (long long)N * K) / 4;       // quads: contiguous dimensions are multiples of 4
   long long blocks = (total + 255) / 256;
   const long long cap = (long long)sb_sm_count() * 16;
@@ -203,11 +189,9 @@ int sb_matmul_f32x3(int a_trans, int b_trans, float alpha, const float* A, const
   // 4096: over the 1e-5 of this class from K = 600 on.  Chains of at most 256 elements of K keep 1.9e-6 / 5.1e-6 at
   // K = 4096 and 2.0e-6 / 5.3e-6 at 262144, for every width and epilogue; the additions between chains are ordinary
   // fp32 additions.  Parallelism: a 512 x 512 output is four tiles; with the splits it is spread over the whole GPU.
-  // Against one chain: 500 x 500 x 1024 37 -> 17 us, 1024 x 1020 x 2048 68 -> 44, 2048 x 2044 x 260 24 -> 30,
-  // 2048 x 2044 x 2048 94 -> 103.
   // C is first brought to beta * C + bias by the split kernel.  A ReLU needs the complete sum and becomes a pass over
-  // C, so such a product is split only where its accuracy needs it (512 x 512 x 1024 36 -> 19 us,
-  // 2048 x 2048 x 2048 94 -> 108, 2048 x 2048 x 260 24 -> 38).  Below 3 * K = 512 there is nothing to gain for either end.
+  // C, so such a product is split only where its accuracy needs it.  Below 3 * K = 512 there is nothing to gain for
+  // either end.
   const bool relu = (epilogue & SB_EPI_RELU) != 0;
   int splits = 1;
   if (3LL * K >= 512 && !(relu && K <= 256)) {
@@ -215,14 +199,14 @@ int sb_matmul_f32x3(int a_trans, int b_trans, float alpha, const float* A, const
     const long long tiles = (long long)((M + 255) / 256) * ((N + 255) / 256);
     long long by_fill = tiles > 0 ? (sb_sm_count() / 2) / tiles : 1;                // one wave of CTA pairs
     if (by_fill > 8) by_fill = 8;             // every split adds a whole tile to C: more than a few cost more than they spread
-    const int by_k = (3 * K) / 128 > 0 ? (3 * K) / 128 : 1;                          // at least two k-blocks of 64 per split
+    const int by_k = K / 64 > 0 ? K / 64 : 1;                                        // at least two k-blocks of 32 per split
     long long want = by_accuracy > by_fill ? by_accuracy : by_fill;
     if (want > by_k) want = by_k;
     splits = (int)(want < 1 ? 1 : want);
   }
   const float* init_bias = splits > 1 && (epilogue & SB_EPI_BIAS) ? bias : nullptr;
   const bool init_c = splits > 1 && (beta != 1.0f || init_bias);
-  SB_CUDA(sb_launch(init_bias ? split3_kernel<true> : split3_kernel<false>, dim3((int)blocks), dim3(256), 0, s, 1, ja, jb, init_c ? C : (float*)nullptr,
+  SB_CUDA(sb_launch(init_bias ? split_kernel<true> : split_kernel<false>, dim3((int)blocks), dim3(256), 0, s, 1, ja, jb, init_c ? C : (float*)nullptr,
                     (long long)M * N, N, beta, init_bias, (reinterpret_cast<uintptr_t>(A) & 15) == 0 ? 1 : 0,
                     (reinterpret_cast<uintptr_t>(B) & 15) == 0 ? 1 : 0));
   SB_COUNT_LAUNCH();
@@ -232,14 +216,14 @@ int sb_matmul_f32x3(int a_trans, int b_trans, float alpha, const float* A, const
     // `C` doubles as the partials pointer: every condition for adding into C holds here by construction
     // (fp32 output, no epilogue in the GEMM, aligned rows; the plan takes whole 32-column chunks per tile and
     // the boxes are clipped at N), so no partial is ever written.
-    int rc = sb_umma_gemm_launch(a_trans, b_trans, alpha, a3, b3, 0.0f, C, M, N, 3 * K, SB_TF32, SB_F32, 0, nullptr, nullptr,
-                                 nullptr, nullptr, s, splits, &used, nullptr, C);
+    int rc = sb_umma_gemm_launch(a_trans, b_trans, alpha, a2, b2, 0.0f, C, M, N, K, SB_TF32, SB_F32, 0, nullptr, nullptr,
+                                 nullptr, nullptr, s, splits, &used, nullptr, C, nullptr, true);
     if (rc != SB_OK) return rc;
     if (used != 1) return sb_fail(SB_ERR_UNSUPPORTED, "internal: sb_matmul_f32x3 expected its splits to be added into C");
     return relu ? sb_relu(C, C, (size_t)M * N, stream) : SB_OK;
   }
-  return sb_umma_gemm_launch(a_trans, b_trans, alpha, a3, b3, beta, C, M, N, 3 * K, SB_TF32, SB_F32, epilogue, bias, nullptr,
-                             nullptr, nullptr, s);
+  return sb_umma_gemm_launch(a_trans, b_trans, alpha, a2, b2, beta, C, M, N, K, SB_TF32, SB_F32, epilogue, bias, nullptr,
+                             nullptr, nullptr, s, 1, nullptr, nullptr, nullptr, nullptr, true);
 }
 
 int sb_matmul_ex(int a_trans, int b_trans, float alpha, const void* A, const void* B, float beta,

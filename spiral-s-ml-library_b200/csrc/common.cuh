@@ -89,7 +89,9 @@ int sb_umma_gemm_launch(int a_trans, int b_trans, float alpha, const void* A, co
                         int epi, const float* bias, const uint8_t* mask, const void* aux_in,
                         void* aux_out, cudaStream_t stream, int splits = 1, int* splits_used = nullptr,
                         const SbRowHead* head = nullptr, void* split_partials = nullptr,
-                        const SbPeerOut* peer_out = nullptr);
+                        const SbPeerOut* peer_out = nullptr, bool three_products = false);
+// `three_products` (SB_TF32 only): A and B are [2, ...] stacks of two matrices each, a high and a low part, and the
+// product is Ah Bh + Ah Bl + Al Bh.
 // True when a row head over N columns (legal columns j < prefix when prefix >= 0) runs inside the GEMM.
 bool sb_umma_head_fits(int N, int prefix);
 
@@ -549,6 +551,15 @@ __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst_smem, const CUtens
       "@q cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
       " [%0], [%1, {%2, %3}], [%4];\n\t}"
       ::"r"(dst_smem), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(x), "r"(y), "r"(bar_cluster_addr), "r"((uint32_t)issue)
+      : "memory");
+}
+__device__ __forceinline__ void tma_load_3d_pair(uint32_t dst_smem, const CUtensorMap* tmap, int x, int y, int z,
+                                                 uint32_t bar_cluster_addr, bool issue) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %6, 0;\n\t"
+      "@q cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
+      " [%0], [%1, {%2, %3, %4}], [%5];\n\t}"
+      ::"r"(dst_smem), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(x), "r"(y), "r"(z), "r"(bar_cluster_addr), "r"((uint32_t)issue)
       : "memory");
 }
 __device__ __forceinline__ void tmem_alloc_pair(uint32_t dst_smem, uint32_t ncols) {

@@ -110,6 +110,7 @@ struct UmmaGemmParams {
   int peer_rows;       // > 0: rows [r * peer_rows, (r + 1) * peer_rows) of C are added to rank r's copy (out map r)
   int tail_first;      // work items from this one on are HALF tiles (block_n / 2 columns); == num_work: none
   uint32_t idesc_tail; // instruction descriptor of a half tile
+  int three;           // 1: the two sub-blocks of a stage are the high and low parts of the same K range, three products
 };
 
 // Walks the work of one worker (a CTA, or a CTA pair): work items (split, tile) strided over the
@@ -933,6 +934,7 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
     const int subs = p.subs;
     const uint32_t a_sub_bytes = p.a_sub_bytes, b_sub_bytes = p.b_sub_bytes;
     const int stages = p.stages;
+    const bool three = p.three != 0;
     uint32_t a_dst = stage_base;
     WorkIter it(p, worker, num_workers);
     int tile, split, kb_begin, kb_end, half;
@@ -957,7 +959,31 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
         if (one && do_a && (!PAIR || leader)) mbar_arrive_expect_tx(full0_local + 8u * (uint32_t)stage, tx_bytes);
         const uint32_t full = full0 + 8u * (uint32_t)stage;
         const uint32_t b_dst = a_dst + a_stage_bytes;
-        if (!do_a) {
+        if (TF32 && three) {
+          // Sub-block s of both operands is part s of the same K range: K-major slabs one behind the other, MN-major
+          // boxes in two halves (the part is the third coordinate of the map).
+          if (do_a) {
+            const uint32_t sub = a_mn ? mn_box_bytes / 2u : a_sub_bytes;
+            for (int i = 0; i < a_boxes; ++i)
+              for (int s = 0; s < 2; ++s) {
+                const uint32_t dst = a_dst + (uint32_t)i * mn_box_bytes + (uint32_t)s * sub;
+                const int x = a_mn ? m0 + i * mn_box_elems : k0, y = a_mn ? k0 : m0;
+                if (PAIR) tma_load_3d_pair(dst, &tmap_a, x, y, s, full, one);
+                else tma_load_3d(dst, &tmap_a, x, y, s, full, one);
+              }
+          } else {
+            const uint32_t sub = b_mn ? mn_box_bytes / 2u : b_sub_bytes;
+            const int boxes = b_mn ? b_boxes : 1;
+            for (int i = 0; i < boxes; ++i)
+              for (int s = 0; s < 2; ++s) {
+                const uint32_t dst = b_dst + (uint32_t)i * mn_box_bytes + (uint32_t)s * sub;
+                const int x = b_mn ? n0 + i * mn_box_elems : k0, y = b_mn ? k0 : n0;
+                const CUtensorMap* map = b_mn ? &tmap_b : map_b;
+                if (PAIR) tma_load_3d_pair(dst, map, x, y, s, full, one);
+                else tma_load_3d(dst, map, x, y, s, full, one);
+              }
+          }
+        } else if (!do_a) {
         } else if (!a_mn) {
           for (int s = 0; s < subs; ++s) {
             if (PAIR) tma_load_2d_pair(a_dst + (uint32_t)s * a_sub_bytes, &tmap_a, k0 + s * mn_box_elems, m0, full, one);
@@ -969,7 +995,7 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
             else tma_load_2d(a_dst + (uint32_t)i * mn_box_bytes, &tmap_a, m0 + i * mn_box_elems, k0, full, one);
           }
         }
-        if (!do_b) {
+        if (!do_b || (TF32 && three)) {
         } else if (!b_mn) {
           for (int s = 0; s < subs; ++s) {
             if (PAIR) tma_load_2d_pair(b_dst + (uint32_t)s * b_sub_bytes, map_b, k0 + s * mn_box_elems, n0, full, one);
@@ -1010,10 +1036,32 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
       const uint32_t stage_step = stage_bytes >> 4;
       const uint32_t a_kstep = p.a_kstep, b_kstep = p.b_kstep;
       const uint32_t a_sub_step = p.a_sub_step, b_sub_step = p.b_sub_step;
-      const bool two_subs = p.subs == 2;
+      const bool two_subs = p.subs == 2, three = p.three != 0;
       const uint32_t full0 = smem_u32(&bar_full[0]), empty0 = smem_u32(&bar_empty[0]);
       const int stages = p.stages;
       uint32_t a_lo = a_lo0, b_lo = b_lo0;
+      auto issue_four = [&](uint32_t d, uint32_t a, uint32_t b, uint32_t id, uint32_t accumulate) {   // one 128-byte K sub-block
+        umma_issue<PAIR, TF32>(d, a, a_hi, b, b_hi, id, accumulate, one);
+        umma_issue<PAIR, TF32>(d, a + a_kstep, a_hi, b + b_kstep, b_hi, id, 1u, one);
+        umma_issue<PAIR, TF32>(d, a + 2u * a_kstep, a_hi, b + 2u * b_kstep, b_hi, id, 1u, one);
+        umma_issue<PAIR, TF32>(d, a + 3u * a_kstep, a_hi, b + 3u * b_kstep, b_hi, id, 1u, one);
+      };
+      auto issue_cross = [&](uint32_t d, uint32_t a, uint32_t b, uint32_t id, uint32_t accumulate) {  // Ah Bl + Al Bh of a stage
+        issue_four(d, a, b + b_sub_step, id, accumulate);
+        issue_four(d, a + a_sub_step, b, id, 1u);
+      };
+      auto release_stage = [&]() {
+        if (PAIR) tc_commit_pair(empty0 + 8u * (uint32_t)stage, (uint16_t)3, one);
+        else tc_commit(empty0 + 8u * (uint32_t)stage, one);
+        a_lo += stage_step;
+        b_lo += stage_step;
+        if (++stage == stages) {
+          stage = 0;
+          phase ^= 1u;
+          a_lo = a_lo0;
+          b_lo = b_lo0;
+        }
+      };
       WorkIter it(p, worker, num_workers);
       int tile, split, kb_begin, kb_end, half;
       while (ok && it.next(p, tile, split, kb_begin, kb_end, half)) {
@@ -1025,34 +1073,49 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
         tc_fence_after_sync();
         const uint32_t d_tmem = tmem_base + (uint32_t)(acc * p.acc_stride);
         uint32_t accumulate = 0u;
-        for (int kb = kb_begin; kb < kb_end; ++kb) {
+        int kb = kb_begin;
+        if (TF32 && three) {
+          // A stage is the high and low parts of one K range.  The accumulator truncates at every MMA, by its own size:
+          // the chain starts with the small products Ah Bl + Al Bh of its first two stages, whose sums are 2^-11 of the
+          // rest, and only then takes their Ah Bh.  (All three products stage by stage: 18 % more error at 512^3.)
+          const int lead = min(2, kb_end - kb_begin);
+          int st = stage;
+          uint32_t ph = phase, al = a_lo, bl = b_lo;
+          for (int i = 0; i < lead; ++i) {
+            if (!mbar_wait_warp(full0 + 8u * (uint32_t)st, ph, abortp, SB_SITE_MMA_FULL)) {
+              ok = false;
+              break;
+            }
+            tc_fence_after_sync();
+            issue_cross(d_tmem, al, bl, idesc, accumulate);
+            accumulate = 1u;
+            al += stage_step;
+            bl += stage_step;
+            if (++st == stages) {
+              st = 0;
+              ph ^= 1u;
+              al = a_lo0;
+              bl = b_lo0;
+            }
+          }
+          if (!ok) break;
+          for (int i = 0; i < lead; ++i) {
+            issue_four(d_tmem, a_lo, b_lo, idesc, 1u);
+            release_stage();
+          }
+          kb += lead;
+        }
+        for (; kb < kb_end; ++kb) {
           if (!mbar_wait_warp(full0 + 8u * (uint32_t)stage, phase, abortp, SB_SITE_MMA_FULL)) {
             ok = false;
             break;
           }
           tc_fence_after_sync();
-          umma_issue<PAIR, TF32>(d_tmem, a_lo, a_hi, b_lo, b_hi, idesc, accumulate, one);
-          umma_issue<PAIR, TF32>(d_tmem, a_lo + a_kstep, a_hi, b_lo + b_kstep, b_hi, idesc, 1u, one);
-          umma_issue<PAIR, TF32>(d_tmem, a_lo + 2u * a_kstep, a_hi, b_lo + 2u * b_kstep, b_hi, idesc, 1u, one);
-          umma_issue<PAIR, TF32>(d_tmem, a_lo + 3u * a_kstep, a_hi, b_lo + 3u * b_kstep, b_hi, idesc, 1u, one);
-          if (two_subs) {
-            const uint32_t a2 = a_lo + a_sub_step, b2 = b_lo + b_sub_step;
-            umma_issue<PAIR, TF32>(d_tmem, a2, a_hi, b2, b_hi, idesc, 1u, one);
-            umma_issue<PAIR, TF32>(d_tmem, a2 + a_kstep, a_hi, b2 + b_kstep, b_hi, idesc, 1u, one);
-            umma_issue<PAIR, TF32>(d_tmem, a2 + 2u * a_kstep, a_hi, b2 + 2u * b_kstep, b_hi, idesc, 1u, one);
-            umma_issue<PAIR, TF32>(d_tmem, a2 + 3u * a_kstep, a_hi, b2 + 3u * b_kstep, b_hi, idesc, 1u, one);
-          }
+          issue_four(d_tmem, a_lo, b_lo, idesc, accumulate);
+          if (TF32 && three) issue_cross(d_tmem, a_lo, b_lo, idesc, 1u);
+          else if (two_subs) issue_four(d_tmem, a_lo + a_sub_step, b_lo + b_sub_step, idesc, 1u);
           accumulate = 1u;
-          if (PAIR) tc_commit_pair(empty0 + 8u * (uint32_t)stage, (uint16_t)3, one);
-          else tc_commit(empty0 + 8u * (uint32_t)stage, one);
-          a_lo += stage_step;
-          b_lo += stage_step;
-          if (++stage == stages) {
-            stage = 0;
-            phase ^= 1u;
-            a_lo = a_lo0;
-            b_lo = b_lo0;
-          }
+          release_stage();
         }
         if (!ok) break;
         if (PAIR) tc_commit_pair(smem_u32(&bar_tmem_full[acc]), (uint16_t)3, one);
@@ -1190,22 +1253,23 @@ EncodeTiledFn get_encode_tiled() {
 // 2-D row-major tensor [rows, cols] -> tensor map with box [box_rows, box_cols],
 // 128-byte swizzle (box_cols * elem size must be 128 bytes), zero fill outside.
 // `swz`: SWZ_128 (16-byte chunks), SWZ_128_CHUNK32 (32-byte chunks, MN-major
-// TF32 operands) or SWZ_64 (64-byte rows, 16-bit output boxes).
+// TF32 operands) or SWZ_64 (64-byte rows, 16-bit output boxes).  `parts` > 1: that many such tensors one behind the
+// other, the part as a third coordinate of the map.
 enum TmapSwizzle { SWZ_128 = 0, SWZ_128_CHUNK32 = 1, SWZ_64 = 2 };
 
 int make_tmap_2d(CUtensorMap* map, const void* base, int in_dtype, long long rows, long long cols,
-                 int box_rows, int box_cols, int swz) {
+                 int box_rows, int box_cols, int swz, int parts = 1) {
   EncodeTiledFn enc = get_encode_tiled();
   if (!enc) return sb_fail(SB_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
   const int es = sb_dtype_size(in_dtype);
   CUtensorMapDataType dt = in_dtype == SB_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16
                            : in_dtype == SB_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16
                                                 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
-  cuuint64_t gdim[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-  cuuint64_t gstride[1] = {(cuuint64_t)cols * (cuuint64_t)es};
-  cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows};
-  cuuint32_t estr[2] = {1, 1};
-  CUresult r = enc(map, dt, 2, const_cast<void*>(base), gdim, gstride, box, estr,
+  cuuint64_t gdim[3] = {(cuuint64_t)cols, (cuuint64_t)rows, (cuuint64_t)parts};
+  cuuint64_t gstride[2] = {(cuuint64_t)cols * (cuuint64_t)es, (cuuint64_t)cols * (cuuint64_t)es * (cuuint64_t)rows};
+  cuuint32_t box[3] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows, 1u};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = enc(map, dt, parts > 1 ? 3 : 2, const_cast<void*>(base), gdim, gstride, box, estr,
                    CU_TENSOR_MAP_INTERLEAVE_NONE,
                    swz == SWZ_128_CHUNK32 ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B
                    : swz == SWZ_64      ? CU_TENSOR_MAP_SWIZZLE_64B
@@ -1312,11 +1376,11 @@ void plan_umma(UmmaGemmParams& p, int in_dtype, int sms, bool allow_pair, bool c
   const int sub_bytes = (UG_BLOCK_M + b_cols) * 128;
   const int budget = UG_SMEM_LIMIT - 2048 - UG_EPI_STAGING - g_gemm_smem_reserve.load(std::memory_order_relaxed);
   const int sub_k = 128 / es;
-  p.subs = (budget / (2 * sub_bytes) >= 3 && p.K >= 6 * sub_k) ? 2 : 1;
-  p.block_k = p.subs * sub_k;
+  p.subs = (p.three || (budget / (2 * sub_bytes) >= 3 && p.K >= 6 * sub_k)) ? 2 : 1;
+  p.block_k = p.three ? sub_k : p.subs * sub_k;
   p.k_blocks = (p.K + p.block_k - 1) / p.block_k;
   p.kb_per_split = p.k_blocks;
-  p.mn_box_bytes = (uint32_t)p.block_k * 128u;
+  p.mn_box_bytes = (uint32_t)(p.subs * sub_k) * 128u;
   p.a_sub_bytes = UG_BLOCK_M * 128u;
   p.b_sub_bytes = (uint32_t)b_cols * 128u;
   p.a_stage_bytes = (uint32_t)p.subs * p.a_sub_bytes;
@@ -1378,7 +1442,7 @@ int sb_umma_gemm_launch(int a_trans, int b_trans, float alpha, const void* A, co
                         float beta, void* C, int M, int N, int K, int in_dtype, int out_dtype,
                         int epi, const float* bias, const uint8_t* mask, const void* aux_in,
                         void* aux_out, cudaStream_t stream, int splits, int* splits_used, const SbRowHead* head,
-                        void* split_partials, const SbPeerOut* peer_out) {
+                        void* split_partials, const SbPeerOut* peer_out, bool three_products) {
   const bool to_peers = peer_out && peer_out->n > 1;
   if (to_peers) {
     if (!sb_umma_peer_out_ok(M, N, peer_out->n) || out_dtype != SB_F32 || epi != 0 || beta != 0.0f || alpha != 1.0f)
@@ -1392,6 +1456,7 @@ int sb_umma_gemm_launch(int a_trans, int b_trans, float alpha, const void* A, co
   UmmaGemmParams p;
   memset(&p, 0, sizeof(p));
   p.M = M; p.N = N; p.K = K;
+  p.three = three_products ? 1 : 0;
   p.a_mn = a_trans ? 1 : 0;   // A stored [K,M]: M contiguous
   p.b_mn = b_trans ? 0 : 1;   // B stored [K,N]: N contiguous
   if (epi & EPI_HEAD_MASK) {
@@ -1432,11 +1497,12 @@ int sb_umma_gemm_launch(int a_trans, int b_trans, float alpha, const void* A, co
 
   CUtensorMap ta, tb;
   int rc;
-  if (!p.a_mn) rc = make_tmap_2d(&ta, A, in_dtype, M, K, UG_BLOCK_M, p.mn_box_elems, SWZ_128);
-  else rc = make_tmap_2d(&ta, A, in_dtype, K, M, p.block_k, p.mn_box_elems, p.a_layout == 1u ? SWZ_128_CHUNK32 : SWZ_128);
+  const int parts = p.three ? 2 : 1;
+  if (!p.a_mn) rc = make_tmap_2d(&ta, A, in_dtype, M, K, UG_BLOCK_M, p.mn_box_elems, SWZ_128, parts);
+  else rc = make_tmap_2d(&ta, A, in_dtype, K, M, p.block_k, p.mn_box_elems, p.a_layout == 1u ? SWZ_128_CHUNK32 : SWZ_128, parts);
   if (rc != SB_OK) return rc;
-  if (!p.b_mn) rc = make_tmap_2d(&tb, B, in_dtype, N, K, p.pair ? p.block_n / 2 : p.block_n, p.mn_box_elems, SWZ_128);
-  else rc = make_tmap_2d(&tb, B, in_dtype, K, N, p.block_k, p.mn_box_elems, p.b_layout == 1u ? SWZ_128_CHUNK32 : SWZ_128);
+  if (!p.b_mn) rc = make_tmap_2d(&tb, B, in_dtype, N, K, p.pair ? p.block_n / 2 : p.block_n, p.mn_box_elems, SWZ_128, parts);
+  else rc = make_tmap_2d(&tb, B, in_dtype, K, N, p.block_k, p.mn_box_elems, p.b_layout == 1u ? SWZ_128_CHUNK32 : SWZ_128, parts);
   if (rc != SB_OK) return rc;
 
   if (splits > 1) {
@@ -1515,7 +1581,7 @@ int sb_umma_gemm_launch(int a_trans, int b_trans, float alpha, const void* A, co
       p.num_work = p.num_tiles + rem;
       p.idesc_tail = sb_umma_idesc(in_dtype, p.a_mn, p.b_mn, 2 * UG_BLOCK_M, p.block_n / 2);
       if (!p.b_mn) {
-        rc = make_tmap_2d(&tc.b_tail, B, in_dtype, N, K, p.block_n / 4, p.mn_box_elems, SWZ_128);
+        rc = make_tmap_2d(&tc.b_tail, B, in_dtype, N, K, p.block_n / 4, p.mn_box_elems, SWZ_128, parts);
         if (rc != SB_OK) return rc;
       }
     }
@@ -1546,7 +1612,7 @@ int sb_umma_gemm_launch(int a_trans, int b_trans, float alpha, const void* A, co
     else if (p.epi_warps == 16) SB_CUDA(sb_launch(umma_gemm_kernel<true, false, 16>, dim3(2 * workers), dim3(ug_threads(16)), smem, stream, 2, ta, tb, tc, p));
     else SB_CUDA(sb_launch(umma_gemm_kernel<true, false>, dim3(2 * workers), dim3(ug_threads(8)), smem, stream, 2, ta, tb, tc, p));
   }
-  sb_prof_after(stream, 2.0 * M * N * K);
+  sb_prof_after(stream, (p.three ? 6.0 : 2.0) * M * N * K);
   SB_COUNT_LAUNCH();
   SB_CUDA(cudaGetLastError());
   return SB_OK;

@@ -41,7 +41,7 @@ def test_layouts_and_ragged_shapes(gpu, at, bt, m, n, k):
 @pytest.mark.parametrize("m,n,k", [(256, 192, 320), (512, 512, 512), (1000, 520, 260), (4, 4, 4)])
 def test_fp32_class_on_tensor_cores_all_layouts(gpu, at, bt, m, n, k):
     """Shapes whose contiguous dimensions are multiples of 4 take the 3 x TF32 tensor-core path (operands split
-    into TF32 head and tail, one GEMM over the K-concatenated parts): still within 1e-5 of the float64 product."""
+    into TF32 head and tail, one GEMM of their three products): still within 1e-5 of the float64 product."""
     a, b, c = _operands(900 + m + n + k, at, bt, m, n, k, "normal")
     dc = gpu.DeviceArray.from_numpy(c)
     l0 = gpu.launch_count()
@@ -67,6 +67,18 @@ def test_fp32_class_bias_relu_and_4096_sampled_rows(gpu):
     rows = g.choice(4096, size=32, replace=False)
     err = so.rel_frobenius(dc.numpy()[rows], so.matmul(False, True, 1.0, a[rows], b, 0.0, None))
     assert err <= TOL_F32
+
+
+@pytest.mark.parametrize("at,bt", [(False, True), (False, False), (True, False), (True, True)])
+@pytest.mark.parametrize("m,n,k", [(132, 68, 4), (260, 300, 28), (260, 256, 32), (516, 260, 36), (128, 64, 64), (300, 192, 68),
+                                   (260, 68, 100), (5120, 1024, 160), (5000, 1020, 96)])
+def test_fp32_class_short_chains(gpu, at, bt, m, n, k):
+    """One, two and more stages of 32 elements of K with their three products, the last one ragged; single tiles and,
+    with 80 tiles for 74 pairs, half-width ones in the last wave.  A chain this short is off by 1.1e-6 (160 elements)."""
+    a, b, c = _operands(40 + m + n + k, at, bt, m, n, k, "normal")
+    dc = gpu.DeviceArray.from_numpy(c)
+    gpu.matmul(at, bt, 1.5, gpu.DeviceArray.from_numpy(a), gpu.DeviceArray.from_numpy(b), -0.5, dc, in_dtype="f32")
+    assert so.rel_frobenius(dc.numpy(), so.matmul(at, bt, 1.5, a, b, -0.5, c)) <= 3e-6
 
 
 @pytest.mark.parametrize("at,bt,shift_a,shift_b", [(False, True, 1, 0), (True, False, 0, 3), (False, False, 2, 1)])
