@@ -170,4 +170,5 @@ def check(rc):
 
 def call(name, *args):
     """Calls an int-returning entry point and raises SpiralError on failure."""
-    return check(getattr(load(), name)(*args))
+    rc = getattr(_lib or load(), name)(*args)
+    return check(rc) if rc != SB_OK else rc

@@ -174,13 +174,22 @@ def device_ptr(obj):
     raise TypeError("cannot take a device pointer from %r" % type(obj))
 
 
+_TAG_OF = {}
+
+
 def dtype_tag(obj):
     """Storage dtype tag of a device array-like ('f32', 'bf16', 'f16', ...)."""
     if isinstance(obj, DeviceArray):
         return obj.dtype
-    name = str(getattr(obj, "dtype", "")).replace("torch.", "")
-    return {"float32": "f32", "bfloat16": "bf16", "float16": "f16", "int32": "i32", "uint8": "u8",
-            "bool": "u8"}.get(name, None)
+    dtype = getattr(obj, "dtype", "")
+    try:
+        return _TAG_OF[dtype]
+    except (KeyError, TypeError):
+        name = str(dtype).replace("torch.", "")
+        tag = {"float32": "f32", "bfloat16": "bf16", "float16": "f16", "int32": "i32", "uint8": "u8", "bool": "u8"}.get(name, None)
+        if tag is not None and type(dtype).__hash__ is not None:
+            _TAG_OF[dtype] = tag                   # keyed by the dtype (torch, numpy, ...), of which there are a handful
+        return tag
 
 
 def stream_ptr(stream):

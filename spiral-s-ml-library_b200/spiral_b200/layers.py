@@ -14,12 +14,14 @@ global-memory pass for every activation and head; here ``graph_run_host`` fuses
 only nodes that cannot be fused run as stand-alone kernels.  Tensors are 3-D in
 the reference (blocks, rows, features); the leading dimensions are the batch.
 """
+import ctypes
 import math
 
 import numpy as np
 
-from . import primitives
-from .device import DeviceArray
+from . import _lib, primitives
+from .device import DeviceArray, stream_ptr
+from .matmul import EPILOGUE_FLAGS, _dims, head_spec
 from .matmul import matmul as _matmul
 
 WEIGHT_ID, WORKSPACE_ID, WEIGHT_ADJOINT_ID = 0, 1, 2     # ml/layers.spi:6-12
@@ -145,11 +147,21 @@ class Model:
                 sizes[WORKSPACE_ID] += _round_up(n.rows * 4, _ALIGN)
         self.partition_bytes = tuple(sizes)
         self.arenas = None
+        self._plans = {}
 
     def allocate(self):
         if self.arenas is None:
             self.arenas = [DeviceArray.zeros((max(b, 16),), "u8") for b in self.partition_bytes]
         return self
+
+    def plan(self, ensemble, draw):
+        """The launches of a run (``_Plan``) for one member, ``draw``: sample nodes draw on the device."""
+        plan = self._plans.get((ensemble, draw))
+        if plan is None or plan.arenas != model_to_model_ptrs(self):
+            if len(self._plans) >= 256:            # more than any ensemble's members: run with ever new indices
+                self._plans = {}
+            plan = self._plans[(ensemble, draw)] = _Plan(self, ensemble, draw)
+        return plan
 
     def tensor(self, node, rounded=False):
         """Typed view of a node's output inside the workspace arena.  ``rounded``: tagged 'tf32' so that the
@@ -232,81 +244,118 @@ def graph_run_host(model, stream=None, ensemble=0, seed=None, row_offset=0):
     Fusion: ``matmul [-> ln_l2] -> relu`` is one GEMM launch, and so is ``matmul -> softmax /
     regret_matching [-> sample] | argmax | binarize`` (a prefix mask is an argument of the head: no mask
     matrix, no allocation, no synchronisation); everything else runs as a stand-alone kernel."""
-    nodes = model.nodes
-    tc = model.in_dtype == "tf32"
-    i = 1
-    while i < len(nodes):
-        n = nodes[i]
-        src = model.tensor(n.src)
-        if n.op == "matmul":
-            j = i + 1
-            w = model.weight(n, ensemble)
-            # hidden layer: [ln_l2 ->] relu
-            k, epilogue = j, []
-            if tc and k + 1 < len(nodes) and nodes[k].op == "ln_l2" and nodes[k + 1].op == "relu" \
-                    and n.cols % 32 == 0 and n.cols <= 256:
-                epilogue, k = ["ln_l2", "relu"], k + 2
-            elif k < len(nodes) and nodes[k].op == "relu":
-                epilogue, k = ["relu"], k + 1
-            if epilogue:
-                feeds_matmul = k < len(nodes) and nodes[k].op == "matmul"
-                _matmul(False, True, 1.0, src, w, 0.0, model.tensor(nodes[k - 1], rounded=feeds_matmul),
-                        in_dtype=model.in_dtype, epilogue=tuple(epilogue), stream=stream)
-                i = k
+    plan = model.plan(ensemble, seed is not None)
+    stream = stream_ptr(stream)
+    for step in plan.steps:
+        step(stream, seed, row_offset)
+    return model.tensor(model.nodes[-1])
+
+
+class _Plan:
+    """The launches of a graph for one ensemble member: what ``graph_run_host`` decides from the graph alone (which
+    nodes fuse, shapes, arguments), so that a run passes ready arguments.  Its addresses are those of the model's
+    arenas, which the model owns; ``Model.plan`` makes a new plan when an arena is another.  Nothing in a plan changes
+    after it is made: threads and streams may share it.  (Deciding anew took the host 35 us for the test graph of three
+    layers, longer than its kernels.)"""
+
+    def __init__(self, model, ensemble, draw):
+        self.steps = []
+        self.arenas = model_to_model_ptrs(model)
+        nodes = model.nodes
+        i = 1
+        while i < len(nodes):
+            n = nodes[i]
+            if n.op == "matmul":
+                i = self._matmul(model, ensemble, draw, i)
                 continue
-            # row head: softmax and regret matching fuse (in that order) when they share one prefix,
-            # then one of sample / argmax; or the sign hash by itself
-            head, size, last, k = [], None, n, j
-            while k < len(nodes) and nodes[k].op in ("softmax", "regret_matching"):
-                want = "masked_softmax" if nodes[k].op == "softmax" else "regret_matching"
-                if want in head or (want == "masked_softmax" and "regret_matching" in head):
-                    break
-                if size is not None and nodes[k].attrs["size"] != size:
-                    break
-                size = nodes[k].attrs["size"]
-                head.append(want)
-                last, k = nodes[k], k + 1
-            kw = {}
-            if head and k < len(nodes) and nodes[k].op == "sample" and seed is not None:
-                head.append("sample")
-                kw = dict(sample_out=model.tensor(nodes[k]), seed=int(seed), row_offset=int(row_offset), position=int(ensemble))
-                k += 1
-            elif head and k < len(nodes) and nodes[k].op == "argmax":
-                head.append("argmax")
-                kw = dict(argmax_out=model.tensor(nodes[k]))
-                k += 1
-            elif not head and k < len(nodes) and nodes[k].op == "binarize" and n.cols <= 32:
-                head.append("binarize")
-                kw = dict(hash_out=model.tensor(nodes[k]), modulo=nodes[k].attrs["modulo"])
-                k += 1
-            if head:
-                from .matmul import head_spec, matmul_head
-                spec = head_spec(tuple(head), prefix=-1 if size is None else size, **kw)
-                matmul_head(False, True, 1.0, src, w, 0.0, model.tensor(last), spec, in_dtype=model.in_dtype, stream=stream)
-                i = k
-                continue
-            _matmul(False, True, 1.0, src, w, 0.0, model.tensor(n), in_dtype=model.in_dtype, stream=stream)
-            i = j
-            continue
-        out = model.tensor(n)
-        if n.op == "relu":
-            primitives.relu(src, out, stream=stream)
-        elif n.op == "softmax":
-            primitives.softmax(src, out, prefix=n.attrs["size"], stream=stream)
-        elif n.op == "regret_matching":
-            primitives.regret_matching(src, out, prefix=n.attrs["size"], stream=stream)
-        elif n.op == "ln_l2":
-            primitives.ln_l2(src, out, stream=stream)
-        elif n.op == "argmax":
-            primitives.argmax(src, out, stream=stream)
-        elif n.op == "binarize":
-            primitives.binarize(n.attrs["modulo"], src, out, stream=stream)
-        elif n.op == "sample":
-            if seed is not None:
-                primitives.sample_seeded(src, out, seed, row_offset=row_offset, position=ensemble, stream=stream)
+            src, out = model.tensor(n.src), model.tensor(n)
+            if n.op == "relu":
+                self._add(primitives.relu, src, out)
+            elif n.op == "softmax":
+                self._add(primitives.softmax, src, out, prefix=n.attrs["size"])
+            elif n.op == "regret_matching":
+                self._add(primitives.regret_matching, src, out, prefix=n.attrs["size"])
+            elif n.op == "ln_l2":
+                self._add(primitives.ln_l2, src, out)
+            elif n.op == "argmax":
+                self._add(primitives.argmax, src, out)
+            elif n.op == "binarize":
+                self._add(primitives.binarize, n.attrs["modulo"], src, out)
+            elif n.op == "sample" and draw:
+                self.steps.append(lambda stream, seed, row_offset, src=src, out=out: primitives.sample_seeded(
+                    src, out, seed, row_offset=row_offset, position=ensemble, stream=stream))
+            elif n.op == "sample":
+                self._add(primitives.sample, src, model.uniforms(n), out)
             else:
-                primitives.sample(src, model.uniforms(n), out, stream=stream)
-        else:
-            raise ValueError("unknown node %r" % n.op)
-        i += 1
-    return model.tensor(nodes[-1])
+                raise ValueError("unknown node %r" % n.op)
+            i += 1
+
+    def _add(self, function, *args, **kw):
+        self.steps.append(lambda stream, seed, row_offset: function(*args, stream=stream, **kw))
+
+    def _gemm(self, model, src, w, out, epilogue=()):
+        if model.in_dtype != "tf32":               # the fp32 class: its workspace is the stream's
+            self._add(_matmul, False, True, 1.0, src, w, 0.0, out, in_dtype=model.in_dtype, epilogue=epilogue)
+            return
+        m, n, k = _dims(False, True, src, w, out)
+        flags = 0
+        for name in epilogue:
+            flags |= EPILOGUE_FLAGS[name]
+        args = ("sb_matmul_ex", 0, 1, 1.0, src.ptr, w.ptr, 0.0, out.ptr, m, n, k, _lib.DTYPE_CODES["tf32"],
+                _lib.DTYPE_CODES[out.dtype], flags, None, None, None, None)
+        self.steps.append(lambda stream, seed, row_offset: _lib.call(*args, stream))
+
+    def _matmul(self, model, ensemble, draw, i):
+        """The launch that starts with the matmul node ``i``; returns the node after the last one it covers."""
+        nodes, n, j = model.nodes, model.nodes[i], i + 1
+        src, w = model.tensor(n.src), model.weight(n, ensemble)
+        # hidden layer: [ln_l2 ->] relu
+        k, epilogue = j, ()
+        if model.in_dtype == "tf32" and k + 1 < len(nodes) and nodes[k].op == "ln_l2" and nodes[k + 1].op == "relu" \
+                and n.cols % 32 == 0 and n.cols <= 256:
+            epilogue, k = ("ln_l2", "relu"), k + 2
+        elif k < len(nodes) and nodes[k].op == "relu":
+            epilogue, k = ("relu",), k + 1
+        if epilogue:
+            feeds_matmul = k < len(nodes) and nodes[k].op == "matmul"
+            self._gemm(model, src, w, model.tensor(nodes[k - 1], rounded=feeds_matmul), epilogue)
+            return k
+        # row head: softmax and regret matching fuse (in that order) when they share one prefix,
+        # then one of sample / argmax; or the sign hash by itself
+        head, size, last, k = [], None, n, j
+        while k < len(nodes) and nodes[k].op in ("softmax", "regret_matching"):
+            want = "masked_softmax" if nodes[k].op == "softmax" else "regret_matching"
+            if want in head or (want == "masked_softmax" and "regret_matching" in head):
+                break
+            if size is not None and nodes[k].attrs["size"] != size:
+                break
+            size = nodes[k].attrs["size"]
+            head.append(want)
+            last, k = nodes[k], k + 1
+        kw, drawn = {}, False
+        if head and k < len(nodes) and nodes[k].op == "sample" and draw:
+            head.append("sample")
+            kw, drawn = dict(sample_out=model.tensor(nodes[k]), position=int(ensemble)), True
+            k += 1
+        elif head and k < len(nodes) and nodes[k].op == "argmax":
+            head.append("argmax")
+            kw = dict(argmax_out=model.tensor(nodes[k]))
+            k += 1
+        elif not head and k < len(nodes) and nodes[k].op == "binarize" and n.cols <= 32:
+            head.append("binarize")
+            kw = dict(hash_out=model.tensor(nodes[k]), modulo=nodes[k].attrs["modulo"])
+            k += 1
+        if not head:
+            self._gemm(model, src, w, model.tensor(n))
+            return j
+        out, prefix, head = model.tensor(last), -1 if size is None else size, tuple(head)
+        m, n_cols, depth = _dims(False, True, src, w, out)
+        args = ("sb_matmul_head", 0, 1, 1.0, src.ptr, w.ptr, 0.0, out.ptr, m, n_cols, depth,
+                _lib.DTYPE_CODES[model.in_dtype], 0, None)
+
+        def run(stream, seed, row_offset):         # a head description of its own per run: the seed is in it
+            spec = head_spec(head, prefix=prefix, seed=int(seed) if drawn else 0, row_offset=int(row_offset) if drawn else 0, **kw)
+            _lib.call(*args, ctypes.byref(spec), stream)
+
+        self.steps.append(run)
+        return k

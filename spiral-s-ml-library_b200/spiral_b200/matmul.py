@@ -7,7 +7,7 @@ updated in place: ``c <- alpha * op(a) @ op(b) + beta * c``.
 import ctypes
 
 from . import _lib
-from .device import device_ptr, dtype_tag, stream_ptr
+from .device import DeviceArray, device_ptr, dtype_tag, stream_ptr
 
 EPILOGUE_FLAGS = {
     "bias": _lib.EPI_BIAS, "relu": _lib.EPI_RELU, "relu_grad": _lib.EPI_RELU_GRAD,
@@ -44,11 +44,12 @@ def _f32x3_aligned(a_trans, b_trans, m, n, k):
 
 
 def _f32x3_workspace(m, n, k, stream):
-    from .device import DeviceArray
-    need = ctypes.c_size_t(0)
-    _lib.call("sb_matmul_f32_workspace_bytes", m, n, k, ctypes.byref(need))
     key = stream_ptr(stream) or 0
     ws = _F32X3_WORKSPACES.get(key)
+    if ws is not None and ws.nbytes >= 12 * (m + n) * k + 1024:      # no more than this is ever asked for
+        return ws
+    need = ctypes.c_size_t(0)
+    _lib.call("sb_matmul_f32_workspace_bytes", m, n, k, ctypes.byref(need))
     if ws is None or ws.nbytes < need.value:
         if ws is not None:
             _lib.call("sb_stream_sync", stream_ptr(stream))      # the old buffer may still be in use
@@ -67,10 +68,10 @@ def matmul(a_trans, b_trans, alpha, a, b, beta, c, in_dtype=None, epilogue=(), b
     arithmetic.  ``epilogue``: iterable of names from EPILOGUE_FLAGS.
     """
     m, n, k = _dims(bool(a_trans), bool(b_trans), a, b, c)
-    storage = dtype_tag(a)
+    storage, storage_b = dtype_tag(a), dtype_tag(b)
     fp32_storage = ("f32", "tf32")                 # 'tf32' tags fp32 storage whose values are TF32-rounded
-    if storage != dtype_tag(b) and not (storage in fp32_storage and dtype_tag(b) in fp32_storage):
-        raise TypeError("a and b must share a storage dtype (%s vs %s)" % (storage, dtype_tag(b)))
+    if storage != storage_b and not (storage in fp32_storage and storage_b in fp32_storage):
+        raise TypeError("a and b must share a storage dtype (%s vs %s)" % (storage, storage_b))
     if in_dtype is None:
         in_dtype = "tf32" if storage in ("f32", "tf32") else storage
     if (in_dtype in ("f32", "tf32")) != (storage in ("f32", "tf32")) or \

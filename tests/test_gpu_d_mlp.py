@@ -349,6 +349,38 @@ def test_checkpoint_round_trip(gpu, tmp_path):
         gpu.PolicyMLP([32, 128, 3], batch, in_dtype="bf16").load(path)
 
 
+def test_layer_graph_runs_again_with_other_inputs_seeds_members_and_arenas(gpu):
+    """A run passes arguments that were made ready by an earlier one: nothing of that run's input, seed, row offset,
+    member or stream may come back, nor an arena that has been exchanged for another."""
+    L = gpu.layers
+    g = L.masked_softmax_and_discrete_sample(5, L.matmul_ensemble((3, 64, 32), L.relu(L.ln_l2(L.matmul((32, 64), L.input("x", (1, 200, 32)))))))
+    model, fresh = (L.pass_init(L.create_model(g)) for _ in range(2))
+    xs = [so.round_tf32(so.rng(90 + i).normal(size=(200, 32)).astype(np.float32)) for i in range(2)]
+
+    def run(m, i, e, seed, offset, stream=None):
+        L.key_extract(m, "x").upload(xs[i])
+        gpu.synchronize()
+        idx = L.graph_run_host(m, ensemble=e, seed=seed, row_offset=offset, stream=stream)
+        gpu.synchronize()
+        return idx.numpy().copy(), m.tensor(m.nodes[-2]).numpy().copy()
+
+    stream = gpu.Stream()
+    cases = [(0, 0, 5, 0, None), (1, 2, 6, 10 ** 6, stream), (0, 0, 7, 3, None), (1, 1, 5, 0, stream), (0, 2, 6, 1, None)]
+    for case in cases:
+        fresh._plans.clear()
+        for a, b in zip(run(model, *case), run(fresh, *case)):
+            np.testing.assert_array_equal(a, b)
+    old = list(model.arenas)
+    model.arenas = None
+    L.pass_init(model.allocate(), seed=1)
+    other, same = run(model, 0, 0, 5, 0), run(fresh, 0, 0, 5, 0)
+    assert old[1].ptr != model.arenas[1].ptr and not np.array_equal(other[1], same[1])
+    w = [so.round_tf32(w) for w in L.get_weights(model, 0)]
+    h = so.round_tf32(so.relu(so.ln_l2(so.matmul(False, True, 1.0, xs[0], w[0], 0.0, None))))
+    want = so.masked_softmax(so.matmul(False, True, 1.0, h, w[1], 0.0, None), so.prefix_mask((200, 32), 5))
+    assert so.rel_frobenius(other[1], want) <= TOL
+
+
 def test_layer_graph_sampling_head(gpu):
     """masked_softmax_and_discrete_sample (ml/layers.spi:422-431): indices are legal (below the prefix
     size), follow the oracle for the uniforms in use, and change with the seed."""
