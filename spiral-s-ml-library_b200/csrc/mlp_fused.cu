@@ -5,10 +5,10 @@
 // The reference runs such a net as block_matmul -> block_map -> block_row_map device
 // functions with a global-memory round trip per node (ml/layers.spi:181-252,
 // generated ml/layers.py:4500-4546).  Here a CTA owns 128 batch rows at a time:
-//   warp 0, lane 0 : TMA producer -- the input tile, then every layer's weights in
+//   warp 0         : TMA producer -- the input tile, then every layer's weights in
 //                    64-column K-chunks through a ring of shared-memory stages
 //                    (weights come from L2: the whole net is a few hundred KB).
-//   warp 1, lane 0 : tcgen05.mma issuer -- layer l multiplies the activation tile in
+//   warp 1         : tcgen05.mma issuer -- layer l multiplies the activation tile in
 //                    shared memory (A, K-major, 128-byte swizzle) by the weight chunk
 //                    (B) into one TMEM accumulator of up to 256 fp32 columns.
 //   warps 2..9     : epilogue -- read the accumulator (one row per thread), add bias,
