@@ -1601,10 +1601,11 @@ int sb_umma_gemm_launch(int a_trans, int b_trans, float alpha, const void* A, co
   if (p.epi_warps == 0) p.epi_warps = 8;
   // A last wave that would fill at most half of the pairs is cut into half-width tiles (twice as many
   // items, each about half as long): 4096^3 is 256 tiles on 74 pairs, three full waves and 34 tiles.
+  // An MN-major B is halved by boxes: a CTA's columns have to be an even number of them (16 bits: 256-column tiles only).
   p.tail_first = p.num_work;
   p.idesc_tail = p.idesc;
   if (p.pair && p.splits == 1 && !to_peers && !(epi & (EPI_HEAD_MASK | SB_EPI_LN_L2)) && p.block_n % 128 == 0 &&
-      tail_split_enabled()) {
+      (!p.b_mn || p.b_boxes % 2 == 0) && tail_split_enabled()) {
     const int workers = cached_sm_count() / 2;
     const int rem = workers > 0 ? p.num_tiles % workers : 0;
     if (p.num_tiles > workers && rem > 0 && 2 * rem <= workers) {
