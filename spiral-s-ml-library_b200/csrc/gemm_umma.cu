@@ -110,6 +110,7 @@ struct UmmaGemmParams {
   int peer_rows;       // > 0: rows [r * peer_rows, (r + 1) * peer_rows) of C are added to rank r's copy (out map r)
   int tail_first;      // work items from this one on are HALF tiles (block_n / 2 columns); == num_work: none
   uint32_t idesc_tail; // instruction descriptor of a half tile
+  int hold_colsum;     // 1: an epilogue warp meets the same four 32-column chunks of C in all its tiles and adds their sums once
   int three;           // 1: the two sub-blocks of a stage are the high and low parts of the same K range, three products
 };
 
@@ -741,7 +742,7 @@ __device__ __noinline__ bool epilogue_tile_wide(uint32_t t_row, int row0_warp, i
   if constexpr (MODE >= 0 && (MODE & 16) != 0) {
     if (held) sums = *held;
   }
-  // Chunk a of the row: half 0 has chunks 0 1 4 5 in x y z w, half 1 chunks 2 3 6 7.
+  // Half 0 has chunks 0 1 4 5 of C in x y z w, half 1 chunks 2 3 6 7 (p.hold_colsum: in every item of the launch).
   auto take_sums = [&](float sum, int col0, int second) {
     if (!held) add_colsum(sum, col0, lane);
     else if (col0 & 128) (second ? sums.w : sums.z) += sum;
@@ -1163,7 +1164,7 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
     }
     // Column sums of a launch with one column tile are held back until the last tile.
     float4 held_sums = make_float4(0.f, 0.f, 0.f, 0.f);
-    float4* held = EW == 8 && p.wide && p.tiles_n == 1 && epi_mode >= 16 ? &held_sums : nullptr;
+    float4* held = EW == 8 && p.hold_colsum && epi_mode >= 16 ? &held_sums : nullptr;
     WorkIter it(p, worker, num_workers);
     int tile, split, kb_begin, kb_end, half_tile;
     while (it.next(p, tile, split, kb_begin, kb_end, half_tile)) {
@@ -1618,6 +1619,9 @@ int sb_umma_gemm_launch(int a_trans, int b_trans, float alpha, const void* A, co
       }
     }
   }
+  // One column tile, all of whose items are whole tiles or the 128-column halves of a 256-column one.  (The right half of
+  // a 128-column tile gives columns 64 and 96 to the warps that hold 0 and 32 of a whole one.)
+  p.hold_colsum = p.wide && p.tiles_n == 1 && (p.tail_first == p.num_work || p.block_n == 256) ? 1 : 0;
   if (p.reduce_add && !p.tma_store)
     return sb_fail(SB_ERR_UNSUPPORTED, "internal: split-K accumulation was chosen for a C that cannot take TMA stores");
   const size_t smem = umma_dyn_smem(p);

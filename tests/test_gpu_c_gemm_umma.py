@@ -239,6 +239,34 @@ def test_column_sums_epilogue(gpu, m, n, k, out_dtype, gated):
     np.testing.assert_allclose(sums.numpy(), want, rtol=0, atol=2e-4 * np.sqrt(m * k))
 
 
+@pytest.mark.parametrize("n,k,in_dtype", [(32, 256, "bf16"), (64, 128, "f16"), (96, 192, "bf16"), (128, 192, "bf16"), (128, 512, "f16"),
+                                          (160, 256, "f16"), (192, 192, "bf16"), (256, 128, "bf16"), (256, 256, "f16")])
+@pytest.mark.parametrize("bt", [False, True])
+@pytest.mark.parametrize("waves,tiles,rows", [(1, 0, 1), (1, 37, -9), (1, 38, 0), (3, 34, 0)])
+def test_column_sums_over_many_tiles(gpu, n, k, in_dtype, bt, waves, tiles, rows):
+    """Rows for several tiles per worker (a dgrad of a large batch; 65536 rows with 148 SMs): last waves that may be cut
+    into half-width tiles (up to half of the pairs) and one that may not.  Every column holds the sum of all its rows:
+    with positive operands a tile is 1/256 or more of it, the roundings of its rows / 32 + k additions far less."""
+    pairs = gpu.sm_count() // 2
+    m = 256 * (waves * pairs + tiles) + rows
+    rtol = (m / 32 + k) * 2.0 ** -23
+    assert rtol < 0.1 / 256
+    g = so.rng(45 + n + k)
+    a = so.round_input(g.random((m, k), np.float32), in_dtype)
+    b = so.round_input(g.random((n, k) if bt else (k, n), np.float32) / np.float32(k), in_dtype)
+    da, db = gpu.DeviceArray.from_numpy(a, in_dtype), gpu.DeviceArray.from_numpy(b, in_dtype)
+    w = b.T.astype(np.float64) if bt else b.astype(np.float64)
+    for gate in (None, g.integers(0, 2 ** 32, size=(n // 32, m), dtype=np.uint64).astype(np.uint32)):
+        sums, c = gpu.DeviceArray.zeros((n,), "f32"), gpu.DeviceArray((m, n), in_dtype)
+        if gate is None:
+            kw, want = dict(epilogue=("colsum_out",)), a.sum(axis=0, dtype=np.float64) @ w
+        else:
+            kw = dict(epilogue=("relu_grad_mask", "colsum_out"), aux_in=gpu.DeviceArray.from_numpy(gate.view(np.int32), "i32"))
+            want = np.where(bits_to_bool(gate, m, n), a @ w.astype(np.float32), 0).sum(axis=0, dtype=np.float64)
+        gpu.matmul(False, bt, 1.0, da, db, 0.0, c, in_dtype=in_dtype, aux_out=sums, **kw)
+        np.testing.assert_allclose(sums.numpy(), want, rtol=rtol)
+
+
 def test_column_sums_rejects_unsupported_combinations(gpu):
     a, b, c = operands(44, False, True, 64, 64, 64, "bf16")
     sums = gpu.DeviceArray.zeros((64,), "f32")

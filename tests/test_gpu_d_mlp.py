@@ -93,6 +93,8 @@ def test_backward_gradients(gpu, in_dtype, sizes, batch):
     ("f16", [64, 96, 12], 777),          # 12 outputs, a row of three warps' worth of 16-byte groups
     ("bf16", [32, 160, 16], 520),        # 16 outputs: the widest head the CUDA-core dgrad takes
     ("bf16", [32, 128, 8], 4096),
+    ("bf16", [32, 128, 256, 3], 65536),  # and the tensor-core dgrad of a layer with 128 inputs over more tiles than workers
+    ("bf16", [64, 96, 256, 10], 65536),
 ])
 def test_backward_gradients_head_widths(gpu, in_dtype, sizes, batch):
     """The dgrad of a head with at most 16 outputs runs on the CUDA cores (one instance per width class,
