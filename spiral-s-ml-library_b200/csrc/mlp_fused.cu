@@ -411,6 +411,7 @@ mlp_fused_kernel(const __grid_constant__ FusedMaps maps, const __grid_constant__
       const int member = item / p.num_tiles, tile = item - member * p.num_tiles;
       const long long pofs = (long long)member * p.member_stride;
       float* out_m = p.out + (long long)member * p.out_stride;
+      __syncwarp();                 // every lane is done with its row of the item before: with `h` and the biases it read
       if (lane == 0) {
         h.argmax_out = p.head.argmax_out ? p.head.argmax_out + (long long)member * p.batch : nullptr;
         h.sample_out = p.head.sample_out ? p.head.sample_out + (long long)member * p.batch : nullptr;

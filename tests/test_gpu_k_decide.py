@@ -53,6 +53,35 @@ def test_leduc_cem_shape_64_columns_three_legal(gpu):
         np.testing.assert_array_equal(single.forward_head(dx, head=("regret_matching",), prefix=3).numpy()[0], probs[e])
 
 
+@pytest.mark.parametrize("with_bias", [False, True])
+@pytest.mark.parametrize("sizes,prefix", [([32, 64, 3], -1), ([64, 40], 5), ([32, 128, 64], -1)])
+def test_sampling_head_with_the_members_of_several_items_on_one_sm(gpu, sizes, prefix, with_bias):
+    """A warp goes from one member's head to another's: actions, indices and probabilities land with the member that
+    they belong to, drawn from its own output of the stream, as when the member runs alone.  A last tile of 3 rows
+    leaves most lanes of a warp with nothing to do."""
+    members, batch = 7, 128 * 61 + 3
+    assert members * 62 > gpu.sm_count()
+    g = so.rng(73)
+    ws = member_weights(720, sizes, members)
+    bs = [[g.normal(0.0, 0.3, size=n).astype(np.float32) for n in sizes[1:]] for _ in range(members)] if with_bias else None
+    dx = gpu.to_storage((g.random((batch, sizes[0])) < 0.2).astype(np.float32), "bf16")
+    mask = None
+    if prefix < 0:
+        mask = (g.random((batch, sizes[-1])) < 0.6).astype(np.uint8)
+        mask[:, 0] = 1
+        mask = gpu.DeviceArray.from_numpy(mask)
+    kw = dict(head=("masked_softmax", "regret_matching", "argmax", "sample"), prefix=prefix, mask=mask, seed=9, row_offset=77)
+    ens = gpu.EnsemblePolicyMLP(sizes, batch, members, in_dtype="bf16", with_bias=with_bias)
+    ens.load_weights(ws, bs)
+    probs = ens.forward_head(dx, position=2, **kw).numpy()
+    single = gpu.EnsemblePolicyMLP(sizes, batch, 1, in_dtype="bf16", with_bias=with_bias)
+    for e in range(members):
+        single.load_weights([ws[e]], [bs[e]] if with_bias else None)
+        np.testing.assert_array_equal(single.forward_head(dx, position=2 + e, **kw).numpy()[0], probs[e])
+        np.testing.assert_array_equal(single.actions.numpy()[0], ens.actions.numpy()[e])
+        np.testing.assert_array_equal(single.indices.numpy()[0], ens.indices.numpy()[e])
+
+
 def test_row_normalised_net_with_sampling_head_over_128_columns(gpu):
     """128 -> 128 -> 128 -> 128, ln_l2 + relu between the layers, `masked_softmax_and_discrete_sample' 3`
     (game/leduc/tests/train.spi:88-101), weights N(0, 0.1) as the reference initialises them."""
