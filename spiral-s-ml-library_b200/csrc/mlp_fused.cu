@@ -492,7 +492,7 @@ mlp_fused_kernel(const __grid_constant__ FusedMaps maps, const __grid_constant__
     }
   }
 
-  if (warp == 1 && lane == 0 && p.store_acts) bulk_wait_group<0>();
+  if (warp == 1 && one && p.store_acts) bulk_wait_group<0>();      // bulk groups belong to the lane that issued the stores
   __syncwarp();
   tc_fence_before_sync();
   __syncthreads();
