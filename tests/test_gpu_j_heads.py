@@ -188,6 +188,37 @@ def test_row_normalisation_over_the_whole_range(gpu):
         assert np.all(got[s == 0] == 0) and np.all(got[s > 3.5e38] == 0)
 
 
+def test_row_normalisation_is_the_ieee_quotient(gpu):
+    """Bit for bit x / s with s the kernel's own chain of fused multiply-adds (float64 holds a TF32 square and an fp32
+    sum), 0 where s is 0: warps of one kind each, so that both ways to divide are met and their limits (s around 1e-12
+    and 1e12, elements around 2^-86 beside ordinary ones), and warps that mix kinds."""
+    n = 64
+    g = so.rng(78)
+
+    def rows(low, high):                                        # 32 rows with sums of squares between the two
+        x = g.normal(size=(32, n))
+        return x * np.sqrt(g.uniform(low, high, 32) / np.sum(x * x, axis=1))[:, None]
+
+    kinds = [rows(0.5, 2.0), rows(1e3, 1e5), rows(1.02e-12, 2e-12), rows(0.5e-12, 0.98e-12), rows(0.5e12, 0.98e12),
+             rows(1.02e12, 2e12), rows(0.5, 2.0), rows(0.5, 2.0), rows(1e-10, 1e10), rows(0.5, 2.0), rows(0.5, 2.0)]
+    kinds[6][:, 5::7] *= 0.5 ** g.integers(75, 95, size=kinds[6][:, 5::7].shape)
+    kinds[7][:, 3::5] *= 0.5 ** g.integers(95, 108, size=kinds[7][:, 3::5].shape)
+    kinds[8][::3] = 0
+    kinds[9][::4] *= 1e-30                                      # squares that are 0 in fp32
+    kinds[10] *= 10.0 ** g.uniform(-18, 18, 32)[:, None]
+    kinds[10][5] = g.normal(size=n) * 1e30                      # a sum beyond fp32
+    x = so.round_tf32(np.concatenate(kinds).astype(np.float32))
+    s = np.zeros(len(x), np.float32)
+    with np.errstate(over="ignore", under="ignore", divide="ignore", invalid="ignore"):
+        for j in range(n):
+            s = (x[:, j].astype(np.float64) ** 2 + s).astype(np.float32)
+        want = np.where(s[:, None] != 0, x / s[:, None], np.float32(0))
+    c = gpu.DeviceArray((len(x), n), "f32")
+    gpu.matmul(False, True, 1.0, gpu.DeviceArray.from_numpy(x), gpu.DeviceArray.from_numpy(np.eye(n, dtype=np.float32)), 0.0, c,
+               in_dtype="tf32", epilogue=("ln_l2",))
+    np.testing.assert_array_equal(c.numpy(), want)
+
+
 def test_reference_test_net_runs_in_three_launches(gpu):
     """The reference's test net (ml/layers.spi:594-608; game/leduc/tests/train.spi:88-101): three dense layers
     with ln_l2 + relu between them and a prefix-masked softmax + sampling head, every member of an ensemble:
