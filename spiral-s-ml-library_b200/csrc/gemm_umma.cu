@@ -695,7 +695,8 @@ __device__ __forceinline__ uint32_t wide_prepare(float* v, float bias_lane, uint
 //
 // `held` (modes with column sums, a single column tile): the sums of this warp's four chunks over all its tiles, for one
 // reduction per kernel instead of one per tile.  A 65536 x 256 dgrad sends 16384 reductions to eight 128-byte lines:
-// 28.1 us, 20.7 without any, 24.7 held back; the Leduc training step 191 -> 187.5 us.
+// 28.1 us, 20.7 without any, 24.7 held back; the Leduc training step 191 -> 187.5 us.  With one tile per worker it
+// costs more than it saves (11.9 -> 13.6 us for 18944 rows): p.hold_colsum says where the line lies.
 template <typename OutT, int MODE>
 __device__ __noinline__ bool epilogue_tile_wide(uint32_t t_row, int row0_warp, int n0, int block_n, int split,
                                                 uint32_t bar_full, uint32_t parity, float4* held) {
@@ -1620,8 +1621,12 @@ int sb_umma_gemm_launch(int a_trans, int b_trans, float alpha, const void* A, co
     }
   }
   // One column tile, all of whose items are whole tiles or the 128-column halves of a 256-column one.  (The right half of
-  // a 128-column tile gives columns 64 and 96 to the warps that hold 0 and 32 of a whole one.)
-  p.hold_colsum = p.wide && p.tiles_n == 1 && (p.tail_first == p.num_work || p.block_n == 256) ? 1 : 0;
+  // a 128-column tile gives columns 64 and 96 to the warps that hold 0 and 32 of a whole one.)  And enough tiles per
+  // worker: adding at the end costs 4 us (in local memory, and nothing left to hide it) and saves 2.4 (256 columns) or
+  // 1.4 (128) a tile.
+  const int sum_workers = p.pair ? cached_sm_count() / 2 : cached_sm_count();
+  p.hold_colsum = p.wide && p.tiles_n == 1 && (p.tail_first == p.num_work || p.block_n == 256) &&
+                  2LL * p.num_tiles > (p.block_n >= 192 ? 3LL : 4LL) * sum_workers ? 1 : 0;
   if (p.reduce_add && !p.tma_store)
     return sb_fail(SB_ERR_UNSUPPORTED, "internal: split-K accumulation was chosen for a C that cannot take TMA stores");
   const size_t smem = umma_dyn_smem(p);
