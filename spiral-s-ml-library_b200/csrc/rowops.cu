@@ -94,9 +94,11 @@ __global__ void __launch_bounds__(128) row_head_kernel(const float* x, float* ou
   for (long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x; r < rows; r += (long long)gridDim.x * blockDim.x) {
     float v[W];
     const float* xr = x + r * h.n;
+    // The mask bytes first (behind the values: 65536 x 40 softmax 16.4 -> 18.5 us, 16384 x 64 12.3 -> 13.5).
+    const typename SbLegalWord<W>::type legal = sb_row_head_legal<W>(h, r);
 #pragma unroll
     for (int j = 0; j < W; ++j) v[j] = j < h.n ? xr[j] : 0.f;
-    sb_row_head_finish<W>(h, v, sb_row_head_legal<W>(h, r), r, out + r * h.n);
+    sb_row_head_finish<W>(h, v, legal, r, out + r * h.n);
   }
 }
 
