@@ -596,7 +596,7 @@ __device__ __noinline__ bool epilogue_tile(uint32_t t_row, int row0_warp, int n0
   // accumulator row sums the squares (both warps of a quadrant do it, each for itself); the tile
   // spans the row (one column tile, N a multiple of 32), columns beyond N are zero.
   float sumsq = 0.f;
-  const bool ln_l2 = MODE == -1 && g_epi.ln_l2 != 0;
+  const bool ln_l2 = EW == 8 && MODE == -1 && g_epi.ln_l2 != 0;
   if (ln_l2) {
     for (int cc = 0; cc < nfull; ++cc) {
       tmem_ld32(t_row + (uint32_t)(cc * 32), raw_a);
@@ -1589,8 +1589,11 @@ int sb_umma_gemm_launch(int a_trans, int b_trans, float alpha, const void* A, co
   if (p.coalesced && beta == 0.0f && !(epi & SB_EPI_RELU_GRAD) && (p.splits == 1 || p.reduce_add || M % 32 == 0)) {
     const int cdt = es_out == 4 ? SB_F32 : out_dtype;
     // Sixteen epilogue warps: CTA-pair tiles with a 16-bit output and next to no main loop; one 32 x 32
-    // box per chunk, no 64-column boxes.
-    p.epi_warps = (p.pair && es_out == 2 && !(epi & EPI_HEAD_MASK) && p.block_n % 32 == 0 && p.k_blocks <= 2 &&
+    // box per chunk, no 64-column boxes.  Not with the row normalisation: its divisions do not fit beside the rest in 96
+    // registers, and the spills cost every other launch of that instance 1 to 2 % (65536 x 256 x 128 with bias, ReLU
+    // and sign words 18.2 -> 18.0 us without it, 65536 x 1024 x 64 gated with column sums 66.0 -> 64.2; the
+    // normalisation itself, 65536 x 256 x 128: 24.0 there, 27.6 here, 34.8 with plain divisions there).
+    p.epi_warps = (p.pair && es_out == 2 && !(epi & (EPI_HEAD_MASK | SB_EPI_LN_L2)) && p.block_n % 32 == 0 && p.k_blocks <= 2 &&
                    epi16_enabled()) ? 16 : 8;
     p.wide = (es_out == 2 && p.block_n % 64 == 0 && !(epi & SB_EPI_LN_L2) && p.epi_warps == 8) ? 1 : 0;
     for (int r = 0; r < (to_peers ? peer_out->n : 1); ++r) {
