@@ -147,7 +147,15 @@ class Model:
                 sizes[WORKSPACE_ID] += _round_up(n.rows * 4, _ALIGN)
         self.partition_bytes = tuple(sizes)
         self.arenas = None
-        self._plans = {}
+
+    @property
+    def arenas(self):
+        """The three device buffers (weights, workspace, weight adjoint), or None before ``allocate``."""
+        return self._arenas
+
+    @arenas.setter
+    def arenas(self, arenas):
+        self._arenas, self._plans, self._planned_for = arenas, {}, None     # plans hold views of the old ones
 
     def allocate(self):
         if self.arenas is None:
@@ -156,8 +164,11 @@ class Model:
 
     def plan(self, ensemble, draw):
         """The launches of a run (``_Plan``) for one member, ``draw``: sample nodes draw on the device."""
+        now = (self.in_dtype, model_to_model_ptrs(self))
+        if now != self._planned_for:
+            self._plans, self._planned_for = {}, now
         plan = self._plans.get((ensemble, draw))
-        if plan is None or plan.arenas != model_to_model_ptrs(self):
+        if plan is None:
             if len(self._plans) >= 256:            # more than any ensemble's members: run with ever new indices
                 self._plans = {}
             plan = self._plans[(ensemble, draw)] = _Plan(self, ensemble, draw)
@@ -254,13 +265,12 @@ def graph_run_host(model, stream=None, ensemble=0, seed=None, row_offset=0):
 class _Plan:
     """The launches of a graph for one ensemble member: what ``graph_run_host`` decides from the graph alone (which
     nodes fuse, shapes, arguments), so that a run passes ready arguments.  Its addresses are those of the model's
-    arenas, which the model owns; ``Model.plan`` makes a new plan when an arena is another.  Nothing in a plan changes
+    arenas, which the model owns; ``Model.plan`` drops all plans when an arena is another.  Nothing in a plan changes
     after it is made: threads and streams may share it.  (Deciding anew took the host 35 us for the test graph of three
     layers, longer than its kernels.)"""
 
     def __init__(self, model, ensemble, draw):
         self.steps = []
-        self.arenas = model_to_model_ptrs(model)
         nodes = model.nodes
         i = 1
         while i < len(nodes):

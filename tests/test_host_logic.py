@@ -50,6 +50,40 @@ def test_layer_graph_planner_mirrors_reference_shapes(sb):
         L.matmul((31, 8), L.input("input", (1, 8, 32)))
 
 
+def test_layer_graph_plans_follow_the_arenas_and_the_arithmetic(sb):
+    """A plan is kept per member and kind of run, never beyond the arenas that its arguments point into: once one is
+    exchanged, by assignment or in place, nothing keeps the old buffers.  (Made-up addresses; nothing is launched.)"""
+    import weakref
+    L = sb.layers
+    g = L.masked_softmax_and_discrete_sample(3, L.matmul_ensemble((4, 64, 32), L.relu(L.matmul((32, 64), L.input("x", (1, 8, 32))))))
+    model = L.create_model(g, allocate=False)
+
+    def arenas(base):
+        return [sb.DeviceArray((max(n, 16),), "u8", ptr=base + (i << 24)) for i, n in enumerate(model.partition_bytes)]
+
+    model.arenas = arenas(1 << 32)
+    plans = [model.plan(e, draw) for e in range(4) for draw in (False, True)]
+    assert len(set(map(id, plans))) == 8
+    assert plans == [model.plan(e, draw) for e in range(4) for draw in (False, True)]
+    old = [weakref.ref(a) for a in model.arenas]
+    model.in_dtype = "f32"
+    assert model.plan(0, False) is not plans[0]
+    del plans
+    model.arenas = arenas(1 << 33)
+    assert all(r() is None for r in old)
+    plans = [model.plan(e, True) for e in range(4)]
+    old = weakref.ref(model.arenas[1])
+    model.arenas[1] = arenas(1 << 34)[1]
+    assert model.plan(2, True) is not plans[2]
+    del plans
+    assert old() is None
+    for e in range(4):
+        for _ in range(300):
+            model.plan(e, True)
+    with pytest.raises(IndexError):
+        model.plan(4, True)
+
+
 RANK_SCRIPT = textwrap.dedent('''
     import os, sys
     sys.path.insert(0, os.environ["SB_ROOT"]); sys.path.insert(0, os.path.join(os.environ["SB_ROOT"], "spiral-s-ml-library_b200"))
