@@ -148,7 +148,7 @@ extern "C" {
 int sb_matmul_f32_workspace_bytes(int M, int N, int K, size_t* bytes) {
   if (!bytes) return sb_fail(SB_ERR_BAD_ARG, "sb_matmul_f32_workspace_bytes: null output");
   if (M < 0 || N < 0 || K < 0) return sb_fail(SB_ERR_BAD_ARG, "sb_matmul_f32_workspace_bytes: negative dimension");
-  const size_t a = ((size_t)3 * M * K * 4 + 255) / 256 * 256, b = ((size_t)3 * N * K * 4 + 255) / 256 * 256;
+  const size_t a = ((size_t)2 * M * K * 4 + 255) / 256 * 256, b = ((size_t)2 * N * K * 4 + 255) / 256 * 256;     // high and low parts
   *bytes = a + b + 256;
   return SB_OK;
 }
@@ -164,16 +164,16 @@ int sb_matmul_f32x3(int a_trans, int b_trans, float alpha, const float* A, const
   size_t need = 0;
   sb_matmul_f32_workspace_bytes(M, N, K, &need);
   if (workspace_bytes < need) return sb_fail(SB_ERR_BAD_ARG, "sb_matmul_f32x3: workspace of %zu bytes, %zu needed", workspace_bytes, need);
-  if ((long long)3 * K > 0x7fffffffLL) return sb_fail(SB_ERR_TOO_LARGE, "sb_matmul_f32x3: 3 * K exceeds the index range");
-  // Row pitches of the concatenated operands must be multiples of 16 bytes (TMA): K % 4 == 0 where K is
+  if (3LL * K > 0x7fffffffLL) return sb_fail(SB_ERR_TOO_LARGE, "sb_matmul_f32x3: K exceeds the index range");
+  // Row pitches of the split operands must be multiples of 16 bytes (TMA): K % 4 == 0 where K is
   // contiguous, M (N) % 4 == 0 where M (N) is.
-  const long long lda = a_trans ? M : 3LL * K, ldb = b_trans ? 3LL * K : N;
+  const long long lda = a_trans ? M : K, ldb = b_trans ? K : N;
   if ((lda * 4) % 16 != 0 || (ldb * 4) % 16 != 0 || ((long long)N * 4) % 16 != 0 || (reinterpret_cast<uintptr_t>(C) & 15))
     return sb_fail(SB_ERR_MISALIGNED, "sb_matmul_f32x3: contiguous dimensions must be multiples of 4 elements and C 16-byte "
                                       "aligned (use the SB_F32 class of sb_matmul_ex for other shapes)");
   char* ws = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(workspace) + 255) & ~(uintptr_t)255);
   float* a2 = reinterpret_cast<float*>(ws);
-  float* b2 = reinterpret_cast<float*>(ws + ((size_t)3 * M * K * 4 + 255) / 256 * 256);
+  float* b2 = reinterpret_cast<float*>(ws + ((size_t)2 * M * K * 4 + 255) / 256 * 256);
   SplitJob ja, jb;
   ja.src = A; ja.dst = a2; ja.count = (long long)M * K;
   jb.src = B; jb.dst = b2; jb.count = (long long)N * K;

@@ -46,7 +46,7 @@ def _f32x3_aligned(a_trans, b_trans, m, n, k):
 def _f32x3_workspace(m, n, k, stream):
     key = stream_ptr(stream) or 0
     ws = _F32X3_WORKSPACES.get(key)
-    if ws is not None and ws.nbytes >= 12 * (m + n) * k + 1024:      # no more than this is ever asked for
+    if ws is not None and ws.nbytes >= 8 * (m + n) * k + 1024:      # no more than this is ever asked for
         return ws
     need = ctypes.c_size_t(0)
     _lib.call("sb_matmul_f32_workspace_bytes", m, n, k, ctypes.byref(need))

@@ -143,3 +143,23 @@ def test_fp32_class_holds_for_very_long_k(gpu, n, epilogue):
     gpu.matmul(False, True, 1.0, gpu.DeviceArray.from_numpy(a), gpu.DeviceArray.from_numpy(b), 0.0, dc, in_dtype="f32",
                epilogue=epilogue, bias=gpu.DeviceArray.from_numpy(bias) if epilogue else None)
     assert so.rel_frobenius(dc.numpy(), want) <= TOL_F32
+
+
+@pytest.mark.parametrize("shift", [0, 16, 200])
+@pytest.mark.parametrize("m,n,k", [(4, 4, 4), (132, 68, 20), (260, 300, 1028)])
+def test_fp32_class_stays_inside_the_workspace_that_it_asks_for(gpu, m, n, k, shift):
+    """Two parts per operand and the slack of their alignment, wherever the workspace starts; what lies around a
+    workspace of exactly that size stays as it was."""
+    import ctypes
+    from spiral_b200 import _lib
+    need = ctypes.c_size_t()
+    _lib.call("sb_matmul_f32_workspace_bytes", m, n, k, ctypes.byref(need))
+    assert need.value <= 8 * (m + n) * k + 1024
+    a, b, c = _operands(60 + m, False, True, m, n, k, "normal")
+    da, db, dc = (gpu.DeviceArray.from_numpy(v) for v in (a, b, c))
+    guard = np.full(shift + need.value + 512, 0xA5, np.uint8)
+    ws = gpu.DeviceArray.from_numpy(guard)
+    _lib.call("sb_matmul_f32x3", 0, 1, 1.0, da.ptr, db.ptr, 0.0, dc.ptr, m, n, k, 0, None, ws.ptr + shift, need.value, None)
+    assert so.rel_frobenius(dc.numpy(), so.matmul(False, True, 1.0, a, b, 0.0, None)) <= TOL_F32
+    after = ws.numpy()
+    assert np.all(after[:shift] == 0xA5) and np.all(after[shift + need.value:] == 0xA5)
