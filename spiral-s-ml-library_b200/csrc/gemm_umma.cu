@@ -1391,6 +1391,10 @@ void plan_umma(UmmaGemmParams& p, int in_dtype, int sms, bool allow_pair, bool c
       }
     }
   }
+  // Pipeline bytes.  The three products of the fp32 class keep both parts of a K range in one stage and need two
+  // stages: on a single CTA a tile is no wider than what a reserve leaves room for (without one 256 columns fit).
+  const int budget = UG_SMEM_LIMIT - 2048 - UG_EPI_STAGING - g_gemm_smem_reserve.load(std::memory_order_relaxed);
+  if (p.three && !p.pair) best_bn = min(best_bn, (budget / (4 * 128) - UG_BLOCK_M) / gran * gran);
   p.block_n = best_bn;
   p.tiles_n = (p.N + p.block_n - 1) / p.block_n;
   p.num_tiles = p.tiles_m * p.tiles_n;
@@ -1407,7 +1411,6 @@ void plan_umma(UmmaGemmParams& p, int in_dtype, int sms, bool allow_pair, bool c
   // tensor pipe from running back to back); they are used when at least three
   // such stages still fit and K is long enough to fill them.
   const int sub_bytes = (UG_BLOCK_M + b_cols) * 128;
-  const int budget = UG_SMEM_LIMIT - 2048 - UG_EPI_STAGING - g_gemm_smem_reserve.load(std::memory_order_relaxed);
   const int sub_k = 128 / es;
   p.subs = (p.three || (budget / (2 * sub_bytes) >= 3 && p.K >= 6 * sub_k)) ? 2 : 1;
   p.block_k = p.three ? sub_k : p.subs * sub_k;

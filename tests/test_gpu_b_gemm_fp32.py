@@ -163,3 +163,19 @@ def test_fp32_class_stays_inside_the_workspace_that_it_asks_for(gpu, m, n, k, sh
     assert so.rel_frobenius(dc.numpy(), so.matmul(False, True, 1.0, a, b, 0.0, None)) <= TOL_F32
     after = ws.numpy()
     assert np.all(after[:shift] == 0xA5) and np.all(after[shift + need.value:] == 0xA5)
+
+
+@pytest.mark.parametrize("at,bt", [(False, True), (False, False), (True, False)])
+@pytest.mark.parametrize("m,n,k", [(100, 252, 300), (128, 256, 64), (64, 1000, 512), (300, 256, 300)])
+def test_fp32_class_beside_a_shared_memory_reserve(gpu, at, bt, m, n, k):
+    """Two stages of a single CTA's 256-column tile take all of the pipeline's memory: with 64 KB reserved its tiles are
+    narrower (pairs keep theirs), and the product is the same within the class."""
+    from spiral_b200 import _lib
+    a, b, c = _operands(70 + n, at, bt, m, n, k, "normal")
+    da, db, dc = (gpu.DeviceArray.from_numpy(v) for v in (a, b, c))
+    _lib.call("sb_gemm_reserve_smem", 65536)
+    try:
+        gpu.matmul(at, bt, 1.0, da, db, 0.5, dc, in_dtype="f32")
+    finally:
+        _lib.call("sb_gemm_reserve_smem", 0)
+    assert so.rel_frobenius(dc.numpy(), so.matmul(at, bt, 1.0, a, b, 0.5, c)) <= TOL_F32
