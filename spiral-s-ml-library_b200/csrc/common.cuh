@@ -361,8 +361,8 @@ __device__ __forceinline__ void tc_commit(uint32_t bar, bool issue) {
 // Issued by the lane with `issue` (elect_one_lane, always the same).  The warp runs its loop together and only the
 // instruction is predicated, because the operands of these instructions are uniform registers: in code that one lane
 // runs alone (`if (lane == 0) { ... }`) every operand is first moved there.  Cost to the issuing warp of four MMAs of
-// N = 16 with one wait, nothing else running: 355 clocks for the branch, 483 for a loop with run-time layer tables
-// predicated on `lane == 0`, 244 for the same loop predicated on elect.sync.  In the GEMM: 4096^3 121.4 -> 118.9 us,
+// N = 16 with one wait, nothing else running: 355 clocks for the branch and 182 for this form; with run-time layer tables
+// in the loop 483 predicated on `lane == 0` and 244 predicated on elect.sync.  In the GEMM: 4096^3 121.4 -> 118.9 us,
 // 32768 x 1024 x 1024 with bias, ReLU and sign words 66.6 -> 64.1, TF32 4000 x 3000 x 1000 53.0 -> 51.5.
 template <bool PAIR, bool TF32>
 __device__ __forceinline__ void umma_issue(uint32_t tmem_d, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo,
@@ -476,21 +476,20 @@ __device__ __forceinline__ unsigned long long sub_f32x2(unsigned long long a, un
   asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
   return r;
 }
-// v[j] /= s for 32 values of a row, 0 for s == 0.  One IEEE reciprocal r for all of them, q = v r, and the correction
+// v[j] /= s for 32 values of a row, 0 for s == 0.  One IEEE reciprocal r (row_reciprocal) for the whole row, q = v r, and the correction
 // q + r (v - q s) with fused multiply-adds, which rounds the quotient correctly (P. Markstein, "Computation of
 // elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34(1), 1990) as long as nothing on
 // the way leaves the normal range: with s below 2^40 that holds for values of 0 and from 2^-86 on.  A warp in which
 // some s or some value is beyond these ranges divides one by one.  Three packed instructions per pair and three for the
 // least value instead of 32 divisions: a row-normalised layer of 65536 x 128 x 128 31.3 -> 20.9 us, of 8192 rows
 // 11.4 -> 9.0 (20.0 and 8.9 without the least value).
-__device__ __forceinline__ void divide_row32(float* v, float s) {
-  const bool plain = s > 1e-12f && s < 1e12f;
+__device__ __forceinline__ float row_reciprocal(float s) { return s > 1e-12f && s < 1e12f ? 1.f / s : 0.f; }   // 0: no short way
+__device__ __forceinline__ void divide_row32(float* v, float s, float r) {
   uint32_t least = 0xffffffffu;                    // of the doubled bits less one: no sign, and a zero comes out largest
 #pragma unroll
   for (int j = 0; j < 32; ++j) least = min(least, 2u * __float_as_uint(v[j]) - 1u);
-  const bool in_range = (plain || s == 0.f) && least >= (2u * (127u - 86u) << 23) - 1u;
+  const bool in_range = (r != 0.f || s == 0.f) && least >= (2u * (127u - 86u) << 23) - 1u;
   if (__all_sync(0xffffffffu, in_range)) {
-    const float r = plain ? 1.f / s : 0.f;         // s == 0: every v is 0 too
     const unsigned long long r2 = pack_f32x2(r, r), ns2 = pack_f32x2(-s, -s);
 #pragma unroll
     for (int j = 0; j < 32; j += 2) {

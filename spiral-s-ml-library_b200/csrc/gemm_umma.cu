@@ -605,11 +605,12 @@ __device__ __noinline__ bool epilogue_tile(uint32_t t_row, int row0_warp, int n0
       for (int j = 0; j < 32; ++j) sumsq = fmaf(__uint_as_float(raw_a[j]), __uint_as_float(raw_a[j]), sumsq);
     }
   }
+  const float inv = ln_l2 ? row_reciprocal(sumsq) : 0.f;
   for (; c < nfull; c += STRIDE) {
     tmem_ld32(t_row + (uint32_t)(c * 32), raw_a);
     fetch(c + STRIDE, bias_nxt, gate_nxt);    // in flight while this chunk is finished
     tmem_ld_wait();
-    if (ln_l2) divide_row32(reinterpret_cast<float*>(raw_a), sumsq);
+    if (ln_l2) divide_row32(reinterpret_cast<float*>(raw_a), sumsq, inv);
     const int col0 = n0 + c * 32;
     if (rows_live && col0 < N) {
       const uint32_t box = sbuf + ((EW == 8 && MODE != -2 && sizeof(OutT) == 2 && g_epi.tma_c) ? box_sel : 0u);
@@ -1100,7 +1101,8 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
         if (TF32 && three) {
           // A stage is the high and low parts of one K range.  The accumulator truncates at every MMA, by its own size:
           // the chain starts with the small products Ah Bl + Al Bh of its first two stages, whose sums are 2^-11 of the
-          // rest, and only then takes their Ah Bh.  (All three products stage by stage: 18 % more error at 512^3.)
+          // rest, and only then takes their Ah Bh.  (All three products stage by stage: 6.1e-7 instead
+          // of 2.0e-7 at 512^3, 1.95e-6 instead of 1.81e-6 at 2048^3.)
           const int lead = min(2, kb_end - kb_begin);
           int st = stage;
           uint32_t ph = phase, al = a_lo, bl = b_lo;

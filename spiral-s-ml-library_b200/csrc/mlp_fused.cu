@@ -33,6 +33,7 @@
 namespace {
 
 constexpr int FM_MAX_LAYERS = 8;
+constexpr int FM_HIDDEN_NONE = 0, FM_HIDDEN_RELU = 1, FM_HIDDEN_NORM = 2;
 constexpr int FM_THREADS = 320;
 constexpr size_t FM_SMEM_LIMIT = 225 * 1024;            // dynamic shared memory; the static part stays below 2 KB
 constexpr int FM_EPI_WARPS = 8;
@@ -52,7 +53,7 @@ struct FusedParams {
   int n_layers;
   int batch;
   int width[FM_MAX_LAYERS + 1];       // width[0] = input features
-  int n_pad[FM_MAX_LAYERS];           // MMA N of layer l (hidden: width; last: padded to 16 or 32)
+  int n_pad[FM_MAX_LAYERS];           // MMA N of layer l (hidden: width; last: what the head needs, a multiple of 16)
   int k_chunks[FM_MAX_LAYERS];        // ceil(in_l / 64)
   int k_steps[FM_MAX_LAYERS];         // ceil(in_l / 16): MMAs of the layer
   uint32_t idesc[FM_MAX_LAYERS];
@@ -73,7 +74,6 @@ struct FusedParams {
   float* out;
   SbRowHead head;                     // n, flags, prefix, mask, seed, ...; argmax_out / sample_out are [members, batch]
   int head_width;                     // columns of a row that the head holds in registers (sb_row_head_width)
-  int hidden_norm;                    // 1: x / sum(x^2) over the row before every ReLU
   // training forward: the hidden activations and their ReLU sign words are also written to global
   // memory for the backward pass (single net only)
   int store_acts;
@@ -116,11 +116,11 @@ __device__ __noinline__ void fused_head(const SbRowHead& h, unsigned long long l
 // Finishes 32 columns of a row: bias, ReLU, rounding to the storage type, and the swizzled store into the activation
 // tile (`dst` = the row's 128 bytes of the 64-column chunk, `piece0` = first of its four 16-byte pieces, `key` the row's
 // swizzle).  `word` (or null) takes the sign word of the row and chunk.
-template <bool BF16>
-__device__ __forceinline__ void hidden_chunk(uint32_t* raw, bool norm, float sumsq, bool has_bias, uint32_t bias_addr,
+template <bool BF16, bool NORM>
+__device__ __forceinline__ void hidden_chunk(uint32_t* raw, float sumsq, float inv, bool has_bias, uint32_t bias_addr,
                                              uint32_t* word, uint32_t dst, uint32_t piece0, uint32_t key) {
   float* v = reinterpret_cast<float*>(raw);
-  if (norm) divide_row32(v, sumsq);
+  if (NORM) divide_row32(v, sumsq, inv);
   if (has_bias) {
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
@@ -150,16 +150,16 @@ __device__ __forceinline__ void hidden_chunk(uint32_t* raw, bool norm, float sum
 // A tile's time is the chain of these chunks, so what a chunk waits for is asked for early: the layer's biases go to
 // the warp's own buffer before the accumulator is awaited, and the next chunk is on its way out of tensor memory
 // while this one is finished.  Per chunk that leaves about 85 instructions (packed adds, rounding before the ReLU).
-// What bounds a 256-wide layer then (4200 clocks per 128 rows) is shared memory at 128 bytes a clock: the MMAs read
-// 64 KB of activations and 128 KB of weights, the weights are written once per tile (128 KB), the activations
-// (64 KB), and the biases are read as 16-byte broadcasts that each move 512 bytes (128 KB): 4096 clocks.  Sixteen
-// warps of two chunks each were slower for that reason (126.6 -> 136 us for 265216 rows).
-// Measured with the issue loops of this kernel and the GEMM predicated instead of branched (see umma_issue):
-// 262144 rows 156 -> 127 us, 16384 rows 14.9 -> 12.8, Leduc training step of 65536 rows 207 -> 191.
+// No unit is full then: of the 20200 clocks of a 128-row tile of the Leduc net (262144 rows) the shared-memory pipe is
+// busy for 5560 with loads and stores and for 3840 with the MMAs' operands, the tensor pipe for 24 %, and 28 % of the
+// issue slots are used.  What is left is the chain: MMAs of a chunk, accumulator out of tensor memory, activations
+// back.  Sixteen warps of two chunks each did not shorten it (126.6 -> 136 us for 265216 rows).
+// Measured with the issue loops of this kernel and the GEMM predicated instead of branched (see umma_issue) and with
+// the narrow heads (row_head.cuh): 262144 rows 202 -> 135 us, 16384 rows 18.2 -> 13.5.
 // False when a wait expired.
-template <bool BF16>
+template <bool BF16, bool NORM>
 __device__ __forceinline__ bool fused_hidden(uint32_t t_row, int n_cols, const float* bias, uint32_t act_base,
-                                          uint32_t bias_smem, int row_in_tile, int half, bool norm,
+                                          uint32_t bias_smem, int row_in_tile, int half,
                                           uint32_t chunk_bar0, uint32_t* bits_out, long long row, int batch,
                                           uint32_t bar_full, uint32_t parity, uint32_t bar_act_free, uint32_t act_parity,
                                           volatile int* abortp) {
@@ -180,7 +180,7 @@ __device__ __forceinline__ bool fused_hidden(uint32_t t_row, int n_cols, const f
   // over the whole accumulator row sums the squares; both warps of a quadrant do it for themselves.
   float sumsq = 0.f;
   uint32_t raw_a[32], raw_b[32];
-  if (norm) {
+  if (NORM) {
     for (int c = 0; c < 2 * mine; ++c) {
       tmem_ld32(t_row + (uint32_t)(c * 32), raw_a);
       tmem_ld_wait32(raw_a);
@@ -188,6 +188,7 @@ __device__ __forceinline__ bool fused_hidden(uint32_t t_row, int n_cols, const f
       for (int j = 0; j < 32; ++j) sumsq = fmaf(__uint_as_float(raw_a[j]), __uint_as_float(raw_a[j]), sumsq);
     }
   }
+  const float inv = NORM ? row_reciprocal(sumsq) : 0.f;
   // Training forward: the stores of the previous layer's activations must have read the tile before it is overwritten.
   if (bar_act_free && !mbar_wait(bar_act_free, act_parity, abortp, SB_SITE_MLP_ACT)) return false;
   const uint32_t key = (uint32_t)row_in_tile & 7u;
@@ -195,7 +196,7 @@ __device__ __forceinline__ bool fused_hidden(uint32_t t_row, int n_cols, const f
   uint32_t* word = bits_out && row < batch ? bits_out + (long long)half * batch + row : nullptr;
   tmem_ld32(t_row + (uint32_t)(half * 32), raw_a);
   auto finish = [&](uint32_t* raw, int i) {      // chunk half + 2 i: the left or right half of activation chunk i
-    hidden_chunk<BF16>(raw, norm, sumsq, bias != nullptr, bias_smem + 128u * (uint32_t)i,
+    hidden_chunk<BF16, NORM>(raw, sumsq, inv, bias != nullptr, bias_smem + 128u * (uint32_t)i,
                        word ? word + 2LL * i * batch : nullptr, dst0 + (uint32_t)i * FM_CHUNK_BYTES, 4u * (uint32_t)half, key);
     // generic-proxy writes of the activation tile must be visible to the MMA's async-proxy reads
     fence_proxy_async_smem();
@@ -244,7 +245,11 @@ __device__ __noinline__ void decide_row(const FusedParams& p, long long row) {
   }
 }
 
-template <bool BF16>
+// HIDDEN: what the hidden layers are, FM_HIDDEN_NONE (a single layer), FM_HIDDEN_RELU or FM_HIDDEN_NORM (x / sum(x^2) over
+// the row before every ReLU, no bias).  Instances of their own: with the divisions of
+// the one and the chunk loop of the other in every kernel, registers went short where they are not used.  Leduc net,
+// 262144 rows 137 -> 129 us, 16384 rows 13.9 -> 13.3; one layer of 512-64, 16 members, 512 states 23 -> 18.5.
+template <bool BF16, int HIDDEN>
 __global__ void __launch_bounds__(FM_THREADS, 1)
 mlp_fused_kernel(const __grid_constant__ FusedMaps maps, const __grid_constant__ FusedParams p) {
   extern __shared__ uint8_t fm_smem_raw[];
@@ -290,7 +295,7 @@ mlp_fused_kernel(const __grid_constant__ FusedMaps maps, const __grid_constant__
   tc_fence_after_sync();
   const uint32_t tmem_base = tmem_slot;
   volatile int* abortp = &abort_flag;
-  const int L = p.n_layers;
+  const int L = HIDDEN == FM_HIDDEN_NONE ? 1 : p.n_layers;
   // Set-up above touched only this CTA's shared and tensor memory; everything below reads or writes
   // global memory and therefore waits for the kernel before it on the stream.
   sb_grid_dependency_wait();
@@ -425,10 +430,10 @@ mlp_fused_kernel(const __grid_constant__ FusedMaps maps, const __grid_constant__
         const uint32_t t_acc = t_row + acc * (uint32_t)p.acc_stride;
         const uint32_t full = smem_u32(&bar_acc_full[acc]);
         const long long grow = (long long)tile * 128 + row_in_tile;
-        if (l < L - 1) {
+        if (HIDDEN != FM_HIDDEN_NONE && l < L - 1) {
           const float* bias_l = p.bias[l] ? p.bias[l] + pofs : nullptr;
           const uint32_t act_free = p.store_acts ? smem_u32(&bar_act_free) : 0u;
-          ok = fused_hidden<BF16>(t_acc, p.n_pad[l], bias_l, act_base, bias_smem, row_in_tile, half, p.hidden_norm != 0,
+          ok = fused_hidden<BF16, HIDDEN == FM_HIDDEN_NORM>(t_acc, p.n_pad[l], bias_l, act_base, bias_smem, row_in_tile, half,
                                   smem_u32(&bar_chunk[0]), p.bits[l], grow, p.batch, full, acc_phase, act_free, act_phase, abortp);
           act_phase ^= 1u;
         } else if (half == 0) {
@@ -622,7 +627,7 @@ static int fused_launch(const char* who, int n_layers, const int* sizes, int bat
   p.acc_stride = 32;
   while (p.acc_stride < max_n) p.acc_stride <<= 1;
   p.tmem_cols = 2 * p.acc_stride;            // two accumulators (at most 2 x 256 columns)
-  p.out = out; p.head = head; p.head_width = sb_row_head_width(head); p.hidden_norm = hidden_norm ? 1 : 0;
+  p.out = out; p.head = head; p.head_width = sb_row_head_width(head);
   p.members = members;
   if (decide) {
     p.tile_counters = decide->tile_counters; p.ensemble_id = decide->ensemble_id; p.action = decide->action;
@@ -636,19 +641,23 @@ static int fused_launch(const char* who, int n_layers, const int* sizes, int bat
     return sb_fail(SB_ERR_UNSUPPORTED, "%s: the input tile, the widest hidden tile and the weight ring need %zu bytes of "
                                        "shared memory (inputs wider than 256 fit with hidden layers of at most 128)", who, smem_needed);
   // The ring takes what is left beside the bias buffers: more than the four stages of the rule above for narrow
-  // layers, three for the widest nets with biases.
+  // layers, three for the widest nets with biases (65 to 128 inputs, 256-wide layers: 128-256-256-17, 262144 rows,
+  // 194 -> 165 us with them; without biases, four stages, 184 -> 160).
   const uint32_t bias_bytes = params ? FM_BIAS_BYTES : 0u;
   p.w_stages = (int)((FM_SMEM_LIMIT - 1024 - p.w_offset - bias_bytes) / p.stage_bytes);
   if (p.w_stages > FM_W_STAGES_MAX) p.w_stages = FM_W_STAGES_MAX;
   p.bias_offset = p.w_offset + (uint32_t)p.w_stages * p.stage_bytes;
   const size_t smem = (size_t)p.bias_offset + bias_bytes + 1024;
 
+  static void (*const kernels[2][3])(FusedMaps, FusedParams) = {
+      {mlp_fused_kernel<false, FM_HIDDEN_NONE>, mlp_fused_kernel<false, FM_HIDDEN_RELU>, mlp_fused_kernel<false, FM_HIDDEN_NORM>},
+      {mlp_fused_kernel<true, FM_HIDDEN_NONE>, mlp_fused_kernel<true, FM_HIDDEN_RELU>, mlp_fused_kernel<true, FM_HIDDEN_NORM>}};
   static std::atomic<bool> attr_set[64];
   int dev = 0;
   SB_CUDA(cudaGetDevice(&dev));
   if (dev >= 0 && dev < 64 && !attr_set[dev].load(std::memory_order_acquire)) {
-    SB_CUDA(cudaFuncSetAttribute(mlp_fused_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FM_SMEM_LIMIT));
-    SB_CUDA(cudaFuncSetAttribute(mlp_fused_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FM_SMEM_LIMIT));
+    for (int b = 0; b < 2; ++b)
+      for (int k = 0; k < 3; ++k) SB_CUDA(cudaFuncSetAttribute(kernels[b][k], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FM_SMEM_LIMIT));
     attr_set[dev].store(true, std::memory_order_release);
   }
   const int sms = sb_sm_count();
@@ -656,7 +665,7 @@ static int fused_launch(const char* who, int n_layers, const int* sizes, int bat
   double flops = 0.0;
   for (int l = 0; l < n_layers; ++l) flops += 2.0 * batch * (double)sizes[l] * sizes[l + 1] * members;
   sb_prof_before((cudaStream_t)stream);
-  SB_CUDA(sb_launch(in_dtype == SB_BF16 ? mlp_fused_kernel<true> : mlp_fused_kernel<false>, dim3(grid), dim3(FM_THREADS), smem, (cudaStream_t)stream, 1, maps, p));
+  SB_CUDA(sb_launch(kernels[in_dtype == SB_BF16][n_layers == 1 ? FM_HIDDEN_NONE : hidden_norm ? FM_HIDDEN_NORM : FM_HIDDEN_RELU], dim3(grid), dim3(FM_THREADS), smem, (cudaStream_t)stream, 1, maps, p));
   sb_prof_after((cudaStream_t)stream, flops);
   SB_COUNT_LAUNCH();
   SB_CUDA(cudaGetLastError());
