@@ -71,8 +71,8 @@ int check_head(const char* who, const SbRowHead& h, int N) {
 // carries over) into a caller workspace; ONE tensor-core GEMM brings the four tiles of a K range into a
 // pipeline stage and issues the three products from them, accumulated in fp32 in tensor memory.
 // (The three products as one GEMM over operands concatenated to 3K read six tiles where these are four,
-// and a main loop of TF32 is bound by the operand bytes that reach an SM: 2048^3 98 -> 80 us, 4096 x
-// 4096 x 512 103 -> 85, 256 x 256 x 16384 46 -> 35, 512^3 unchanged, bound by the host.)
+// and a main loop of TF32 is bound by the operand bytes that reach an SM: 2048^3 117 -> 99 us (other inputs
+// every call; 106 -> 89 with the same), 4096 x 4096 x 512 102 -> 86, 256 x 256 x 16384 44 -> 34, 512^3 bound by the host.)
 // ---------------------------------------------------------------------------
 namespace {
 
@@ -184,11 +184,11 @@ int sb_matmul_f32x3(int a_trans, int b_trans, float alpha, const float* A, const
   cudaStream_t s = (cudaStream_t)stream;
   // Split-K with the tiles ADDED to C (TMA reduce-add) serves two ends.  Accuracy: the tensor core's fp32
   // accumulator does not round to nearest, so a chain of accumulations drifts in proportion to its length.  Relative
-  // Frobenius error of ONE chain, 1024 x 1020, normal / positive / positive operands constant along K: 2.7e-6 /
-  // 3.7e-6 / 4.6e-6 at K = 256, 5.3e-6 / 7.5e-6 / 9.3e-6 at 512, 1.1e-5 / 1.5e-5 / - at 1024, 4.2e-5 / 6.2e-5 / - at
-  // 4096: over the 1e-5 of this class from K = 600 on.  Chains of at most 256 elements of K keep 1.9e-6 / 5.1e-6 at
-  // K = 4096 and 2.0e-6 / 5.3e-6 at 262144, for every width and epilogue; the additions between chains are ordinary
-  // fp32 additions.  Parallelism: a 512 x 512 output is four tiles; with the splits it is spread over the whole GPU.
+  // Frobenius error of ONE chain, 1024 x 1020, normal / positive / positive operands constant along K, measured on the
+  // form with operands concatenated to 3K: 2.7e-6 / 3.7e-6 / 4.6e-6 at K = 256, 5.3e-6 / 7.5e-6 / 9.3e-6 at 512,
+  // 1.1e-5 / 1.5e-5 / - at 1024, 4.2e-5 / 6.2e-5 / - at 4096: over the 1e-5 of this class from K = 600 on.  Chains of
+  // at most 256 elements of K in the present form keep 1.8e-6 / 2.6e-6 / 2.4e-6 at K = 4096 and 1.9e-6 / 2.7e-6 /
+  // 7.9e-6 at 262144, for every width and epilogue; the additions between chains are ordinary fp32 additions.  Parallelism: a 512 x 512 output is four tiles; with the splits it is spread over the whole GPU.
   // C is first brought to beta * C + bias by the split kernel.  A ReLU needs the complete sum and becomes a pass over
   // C, so such a product is split only where its accuracy needs it.  Below 3 * K = 512 there is nothing to gain for
   // either end.

@@ -211,7 +211,8 @@ def test_fused_forward_over_many_tiles_per_cta(gpu, sizes, with_bias):
     16 columns, and the widest shapes that fit in shared memory; the training forward's activations and sign words too."""
     tile_rows = 128 * gpu.sm_count()
     batch = 3 * tile_rows + 77
-    net, ws, bs = build(gpu, sizes, batch, "f16", 14, head=("masked_softmax", "argmax"), bias_scale=0.1)
+    ws, bs = so.mlp_weights(14, sizes)
+    bs = [(so.rng(114 + i).normal(size=b.shape) * 0.1).astype(np.float32) for i, b in enumerate(bs)]
     train = gpu.PolicyMLP(sizes, batch, in_dtype="f16", with_bias=with_bias, training=True)
     net = gpu.PolicyMLP(sizes, batch, in_dtype="f16", head=("masked_softmax", "argmax"), with_bias=with_bias)
     g = so.rng(14)
