@@ -11,11 +11,15 @@
 //   warp 1         : tcgen05.mma issuer -- layer l multiplies the activation tile in
 //                    shared memory (A, K-major, 128-byte swizzle) by the weight chunk
 //                    (B) into one TMEM accumulator of up to 256 fp32 columns.
-//   warps 2..9     : epilogue -- read the accumulator (one row per thread), add bias,
+//   warp 2         : training forward -- stores the delivered activation chunks (TMA).
+//   warp 3         : biases to shared memory.
+//   warps 4..11    : epilogue -- read the accumulator (one row per thread), add bias,
 //                    ReLU, round to the 16-bit storage type and write the result back
 //                    into the activation tile in exactly the swizzled K-major layout
-//                    the next layer's MMAs read; the last layer ends in the row head
-//                    (masked softmax / regret matching / argmax) written to global.
+//                    the next layer's MMAs read.
+//   warps 12..15   : the last layer's row head (masked softmax / regret matching /
+//                    argmax) written to global, beside the next tile's first layers.
+//                    A single-layer net has no epilogue warps and two such groups.
 // 16-bit arithmetic classes only (SB_F16, SB_BF16); widths: input <= 512 and a
 // multiple of 8 (inputs beyond 256 as far as shared memory allows: the reference's Hold'em
 // policy net is 512 -> 64, game/nl_hu_holdem/model_cem.spi:71-98), hidden layers multiples of 64 up to 256, output <= 64 (<= 256 when a
@@ -34,12 +38,15 @@ namespace {
 
 constexpr int FM_MAX_LAYERS = 8;
 constexpr int FM_HIDDEN_NONE = 0, FM_HIDDEN_RELU = 1, FM_HIDDEN_NORM = 2;
-constexpr int FM_THREADS = 320;
+constexpr int FM_HEAD_BIAS = 64;                        // floats kept for the head's biases, zero beyond the outputs
+// Warps of an instance: four with a job each (producer, issuer, activation stores, biases), eight for the epilogue of the
+// hidden layers, and groups of four that finish head rows (a single-layer net is nothing but heads: two groups take turns).
+__host__ __device__ constexpr int fm_epi_warps(int hidden) { return hidden == FM_HIDDEN_NONE ? 0 : 8; }
+__host__ __device__ constexpr int fm_head_groups(int hidden) { return hidden == FM_HIDDEN_NONE ? 2 : 1; }
+__host__ __device__ constexpr int fm_threads(int hidden) { return 32 * (4 + fm_epi_warps(hidden) + 4 * fm_head_groups(hidden)); }
 constexpr size_t FM_SMEM_LIMIT = 225 * 1024;            // dynamic shared memory; the static part stays below 2 KB
-constexpr int FM_EPI_WARPS = 8;
 constexpr int FM_W_STAGES = 4;                         // stages of the weight ring that decide which nets fit
 constexpr int FM_W_STAGES_MAX = 8;                     // stages taken where shared memory is left
-constexpr uint32_t FM_BIAS_BYTES = FM_EPI_WARPS * 512u; // a layer's biases, one copy of its own columns per epilogue warp
 constexpr uint32_t FM_CHUNK_BYTES = 128u * 128u;       // activation chunk: 128 rows x 64 elements x 2 B
 // A weight stage holds one 64-column K-chunk of a layer: (widest layer's rows) x 128 bytes, at most 256 rows.
 
@@ -69,7 +76,9 @@ struct FusedParams {
   uint32_t stage_bytes;               // bytes of one weight stage
   uint32_t act_offset, w_offset;      // byte offsets of the activation tile and the weight ring
   int w_stages;                       // stages of the weight ring
-  uint32_t bias_offset;               // byte offset of the epilogue warps' bias buffers
+  uint32_t bias_offset;               // byte offset of the biases: all layers of a member one behind the other
+  uint32_t bias_bytes;                // bytes of one member's biases; two such buffers take turns when there are several members
+  uint32_t bias_pos[FM_MAX_LAYERS];   // byte offset of a layer's biases in a buffer
   // head
   float* out;
   SbRowHead head;                     // n, flags, prefix, mask, seed, ...; argmax_out / sample_out are [members, batch]
@@ -147,41 +156,31 @@ __device__ __forceinline__ void hidden_chunk(uint32_t* raw, float sumsq, float i
 // belongs to (`chunk_bar0` + 8 bytes per chunk): the next layer's MMAs on that K-chunk start as soon as
 // all eight warps have delivered it, while the later chunks of this layer are still being finished.
 //
-// A tile's time is the chain of these chunks, so what a chunk waits for is asked for early: the layer's biases go to
-// the warp's own buffer before the accumulator is awaited, and the next chunk is on its way out of tensor memory
-// while this one is finished.  Per chunk that leaves about 85 instructions (packed adds, rounding before the ReLU).
-// No unit is full then: of the 20200 clocks of a 128-row tile of the Leduc net (262144 rows) the shared-memory pipe is
-// busy for 5560 with loads and stores and for 3840 with the MMAs' operands, the tensor pipe for 24 %, and 28 % of the
-// issue slots are used.  What is left is the chain: MMAs of a chunk, accumulator out of tensor memory, activations
-// back.  Sixteen warps of two chunks each did not shorten it (126.6 -> 136 us for 265216 rows).
-// Measured with the issue loops of this kernel and the GEMM predicated instead of branched (see umma_issue) and with
-// the narrow heads (row_head.cuh): 262144 rows 202 -> 135 us, 16384 rows 18.2 -> 13.5.
+// A tile's time is the chain of these chunks.  Clock stamps of a tile of the Leduc net (262144 rows): 3860 clocks a hidden
+// layer, of which a chunk takes 640 (85 instructions 460, proxy fence 110, the next chunk's wait 70) and the way from the
+// last chunk over its MMAs to the next accumulator 920 + 210.  What kept other warps waiting before: the head, finished by
+// half of these warps (2300 for the mask bytes, 2200 for the rows), and the biases, 1200 to 2000 per layer from global
+// memory.  Heads and biases now have warps of their own: 262144 rows 129.1 -> 91.7 us, 16384 rows 13.3 -> 12.3, training
+// forward of 65536 rows 47.8 -> 38.9, 128-256-256-17 155 -> 113; 16 members of 512-64, 4096 states 59 -> 48.
+// Tried: sixteen warps of two chunks each (80 registers: 106 us); the last K-chunk by halves of the columns, so that the
+// epilogue starts on the left one (101: MMAs of 128 columns read A twice).
 // False when a wait expired.
 template <bool BF16, bool NORM>
-__device__ __forceinline__ bool fused_hidden(uint32_t t_row, int n_cols, const float* bias, uint32_t act_base,
-                                          uint32_t bias_smem, int row_in_tile, int half,
+__device__ __forceinline__ bool fused_hidden(uint32_t t_row, int n_cols, bool has_bias, uint32_t bias_smem, uint32_t act_base,
+                                          int row_in_tile, int half,
                                           uint32_t chunk_bar0, uint32_t* bits_out, long long row, int batch,
                                           uint32_t bar_full, uint32_t parity, uint32_t bar_act_free, uint32_t act_parity,
                                           volatile int* abortp) {
   const int lane = (int)(threadIdx.x & 31);
-  const int mine = n_cols >> 6;                  // chunks of this warp
-  if (bias) {
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-      if (i < mine) {
-        const float b = __ldg(bias + (half + 2 * i) * 32 + lane);
-        asm volatile("st.shared.f32 [%0], %1;" ::"r"(bias_smem + 4u * (uint32_t)(i * 32 + lane)), "f"(b) : "memory");
-      }
-    __syncwarp();
-  }
-  if (!mbar_wait(bar_full, parity, abortp, SB_SITE_MLP_ACC)) return false;
+  const int chunks = n_cols >> 5;
+  if (!mbar_wait_warp(bar_full, parity, abortp, SB_SITE_MLP_ACC)) return false;
   tc_fence_after_sync();
   // Row normalisation (local_ln_l2, ml/primitives.spi:701-703; no bias in this mode): a first pass
   // over the whole accumulator row sums the squares; both warps of a quadrant do it for themselves.
   float sumsq = 0.f;
   uint32_t raw_a[32], raw_b[32];
   if (NORM) {
-    for (int c = 0; c < 2 * mine; ++c) {
+    for (int c = 0; c < chunks; ++c) {
       tmem_ld32(t_row + (uint32_t)(c * 32), raw_a);
       tmem_ld_wait32(raw_a);
 #pragma unroll
@@ -189,30 +188,31 @@ __device__ __forceinline__ bool fused_hidden(uint32_t t_row, int n_cols, const f
     }
   }
   const float inv = NORM ? row_reciprocal(sumsq) : 0.f;
+  tmem_ld32(t_row + (uint32_t)(half * 32), raw_a);
   // Training forward: the stores of the previous layer's activations must have read the tile before it is overwritten.
-  if (bar_act_free && !mbar_wait(bar_act_free, act_parity, abortp, SB_SITE_MLP_ACT)) return false;
+  if (bar_act_free && !mbar_wait_warp(bar_act_free, act_parity, abortp, SB_SITE_MLP_ACT)) return false;
   const uint32_t key = (uint32_t)row_in_tile & 7u;
   const uint32_t dst0 = act_base + (uint32_t)row_in_tile * 128u;
-  uint32_t* word = bits_out && row < batch ? bits_out + (long long)half * batch + row : nullptr;
-  tmem_ld32(t_row + (uint32_t)(half * 32), raw_a);
-  auto finish = [&](uint32_t* raw, int i) {      // chunk half + 2 i: the left or right half of activation chunk i
-    hidden_chunk<BF16, NORM>(raw, sumsq, inv, bias != nullptr, bias_smem + 128u * (uint32_t)i,
-                       word ? word + 2LL * i * batch : nullptr, dst0 + (uint32_t)i * FM_CHUNK_BYTES, 4u * (uint32_t)half, key);
+  uint32_t* word = bits_out && row < batch ? bits_out + row : nullptr;
+  auto finish = [&](uint32_t* raw, int c) {      // chunk c of 32 columns: the left or right half of activation chunk c / 2
+    hidden_chunk<BF16, NORM>(raw, sumsq, inv, has_bias, bias_smem + 128u * (uint32_t)c,
+                       word ? word + (long long)c * batch : nullptr, dst0 + (uint32_t)(c >> 1) * FM_CHUNK_BYTES, 4u * (uint32_t)(c & 1), key);
     // generic-proxy writes of the activation tile must be visible to the MMA's async-proxy reads
     fence_proxy_async_smem();
     tc_fence_before_sync();
     __syncwarp();
-    if (lane == 0) mbar_arrive(chunk_bar0 + 8u * (uint32_t)i);
+    if (lane == 0) mbar_arrive(chunk_bar0 + 8u * (uint32_t)(c >> 1));
   };
+  // The next chunk is on its way out of tensor memory while this one is finished.
 #pragma unroll 1
-  for (int i = 0; i < mine; i += 2) {
+  for (int c = half; c < chunks; c += 4) {
     tmem_ld_wait32(raw_a);
-    if (i + 1 < mine) tmem_ld32(t_row + (uint32_t)((half + 2 * i + 2) * 32), raw_b);
-    finish(raw_a, i);
-    if (i + 1 >= mine) break;
+    if (c + 2 < chunks) tmem_ld32(t_row + (uint32_t)((c + 2) * 32), raw_b);
+    finish(raw_a, c);
+    if (c + 2 >= chunks) break;
     tmem_ld_wait32(raw_b);
-    if (i + 2 < mine) tmem_ld32(t_row + (uint32_t)((half + 2 * i + 4) * 32), raw_a);
-    finish(raw_b, i + 1);
+    if (c + 4 < chunks) tmem_ld32(t_row + (uint32_t)((c + 4) * 32), raw_a);
+    finish(raw_b, c + 2);
   }
   return true;
 }
@@ -250,23 +250,26 @@ __device__ __noinline__ void decide_row(const FusedParams& p, long long row) {
 // the one and the chunk loop of the other in every kernel, registers went short where they are not used.  Leduc net,
 // 262144 rows 137 -> 129 us, 16384 rows 13.9 -> 13.3; one layer of 512-64, 16 members, 512 states 23 -> 18.5.
 template <bool BF16, int HIDDEN>
-__global__ void __launch_bounds__(FM_THREADS, 1)
+__global__ void __launch_bounds__(fm_threads(HIDDEN), 1)
 mlp_fused_kernel(const __grid_constant__ FusedMaps maps, const __grid_constant__ FusedParams p) {
+  constexpr int EW = fm_epi_warps(HIDDEN), HG = fm_head_groups(HIDDEN);
   extern __shared__ uint8_t fm_smem_raw[];
-  __shared__ __align__(8) uint64_t bar_x_full, bar_x_empty, bar_act_free, bar_tail_in, bar_tail_out;
-  __shared__ __align__(8) uint64_t bar_acc_full[2], bar_head_done[2];      // per accumulator
+  __shared__ __align__(8) uint64_t bar_x_full, bar_x_empty, bar_act_free, bar_tail_in[HG], bar_tail_out[HG];
+  __shared__ __align__(8) uint64_t bar_bias_full[2], bar_bias_empty[2];
+  __shared__ __align__(8) uint64_t bar_acc_full[2], bar_head_full[2], bar_head_done[2];      // per accumulator: a hidden layer's or a head's, and its rows read
   __shared__ __align__(8) uint64_t bar_chunk[4];       // 64-column chunk k of the activation tile is written (8 warps each)
   __shared__ __align__(8) uint64_t bar_w_full[FM_W_STAGES_MAX], bar_w_empty[FM_W_STAGES_MAX];
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
-  __shared__ int tile_is_complete;
-  __shared__ SbRowHead head_slot[FM_EPI_WARPS];
+  __shared__ int tile_is_complete[HG];
+  __shared__ SbRowHead head_slot[4 * HG];
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t base = (smem_u32(fm_smem_raw) + 1023u) & ~1023u;
   const uint32_t x_base = base;                      // input tile: x_chunks x 16 KB
   const uint32_t act_base = base + p.act_offset;     // activation tile: up to 4 chunks
   const uint32_t w_base = base + p.w_offset;         // weight ring
+  const uint32_t bias_base = base + p.bias_offset;
 
   if (tid == 0) {
     mbar_init(smem_u32(&bar_x_full), 1);
@@ -274,11 +277,16 @@ mlp_fused_kernel(const __grid_constant__ FusedMaps maps, const __grid_constant__
     mbar_init(smem_u32(&bar_act_free), 1);
     for (int a = 0; a < 2; ++a) {
       mbar_init(smem_u32(&bar_acc_full[a]), 1);
+      mbar_init(smem_u32(&bar_head_full[a]), 1);
       mbar_init(smem_u32(&bar_head_done[a]), 4);    // the four warps that finish head rows
+      mbar_init(smem_u32(&bar_bias_full[a]), 1);
+      mbar_init(smem_u32(&bar_bias_empty[a]), EW + 4);   // every warp that reads an item's biases
     }
-    for (int k = 0; k < 4; ++k) mbar_init(smem_u32(&bar_chunk[k]), FM_EPI_WARPS);
-    mbar_init(smem_u32(&bar_tail_in), 4);       // the four warps that finish head rows
-    mbar_init(smem_u32(&bar_tail_out), 1);
+    for (int k = 0; k < 4; ++k) mbar_init(smem_u32(&bar_chunk[k]), 8);
+    for (int g = 0; g < HG; ++g) {
+      mbar_init(smem_u32(&bar_tail_in[g]), 4);       // the four warps that finish head rows
+      mbar_init(smem_u32(&bar_tail_out[g]), 1);
+    }
     for (int s = 0; s < p.w_stages; ++s) {
       mbar_init(smem_u32(&bar_w_full[s]), 1);
       mbar_init(smem_u32(&bar_w_empty[s]), 1);
@@ -336,17 +344,23 @@ mlp_fused_kernel(const __grid_constant__ FusedMaps maps, const __grid_constant__
     uint32_t acc = 0;
     bool ok = true;
     const uint32_t hi = (uint32_t)(umma_smem_desc(0u, 16u, 1024u, 2u) >> 32);
+    const uint32_t x_lo = (uint32_t)umma_smem_desc(x_base, 16u, 1024u, 2u);
+    const uint32_t act_lo = (uint32_t)umma_smem_desc(act_base, 16u, 1024u, 2u);
+    const uint32_t w_lo0 = (uint32_t)umma_smem_desc(w_base, 16u, 1024u, 2u);
+    const uint32_t w_full0 = smem_u32(&bar_w_full[0]), w_empty0 = smem_u32(&bar_w_empty[0]), chunk0 = smem_u32(&bar_chunk[0]);
+    const uint32_t w_step = p.stage_bytes >> 4;
+    const int w_stages = p.w_stages;
+    uint32_t w_lo = w_lo0;
     int done = 0;                               // items before this one
     for (int item = blockIdx.x; ok && item < p.num_items; item += gridDim.x, ++done) {
-      const int tile = item % p.num_tiles;
       for (int l = 0; ok && l < L; ++l, acc ^= 1u) {
-        uint32_t a_base;
+        const uint32_t idesc = p.idesc[l];
+        const int chunks = p.k_chunks[l];
+        int steps = p.k_steps[l];
+        uint32_t a_lo = l == 0 ? x_lo : act_lo;
         if (l == 0) {
           if (!mbar_wait_warp(smem_u32(&bar_x_full), x_phase, abortp, SB_SITE_MLP_ACT)) { ok = false; break; }
           x_phase ^= 1u;
-          a_base = x_base;
-        } else {
-          a_base = act_base;
         }
         // Layers alternate between two accumulators, across items too: the epilogue of layer l-1 still reads its
         // own while this layer's first MMAs run, and the next item's first layer runs beside the head of this one.
@@ -356,148 +370,209 @@ mlp_fused_kernel(const __grid_constant__ FusedMaps maps, const __grid_constant__
           if (!mbar_wait_warp(smem_u32(&bar_head_done[acc]), (head_phase >> acc) & 1u, abortp, SB_SITE_MLP_ACT)) { ok = false; break; }
           head_phase ^= 1u << acc;
         }
-        tc_fence_after_sync();
         const uint32_t d_tmem = tmem_base + acc * (uint32_t)p.acc_stride;
         uint32_t accumulate = 0u;
-        for (int c = 0; c < p.k_chunks[l]; ++c) {
+        for (int c = 0; c < chunks; ++c, steps -= 4) {
+          // The weights first: they have usually been there for long when the activations come, and a wait for
+          // what is there already costs the issuer some 100 clocks all the same (the other order: 91.7 -> 95 us).
+          if (!mbar_wait_warp(w_full0 + 8u * (uint32_t)stage, w_phase, abortp, SB_SITE_MLP_WEIGHTS)) { ok = false; break; }
           if (l > 0) {
             // K-chunk c of this layer's input = 64-column chunk c of the previous layer's output
-            if (!mbar_wait_warp(smem_u32(&bar_chunk[c]), (chunk_phase >> c) & 1u, abortp, SB_SITE_MLP_ACT)) { ok = false; break; }
+            if (!mbar_wait_warp(chunk0 + 8u * (uint32_t)c, (chunk_phase >> c) & 1u, abortp, SB_SITE_MLP_ACT)) { ok = false; break; }
             chunk_phase ^= 1u << c;
-            tc_fence_after_sync();
-            // Training forward: the delivered chunk of the previous layer's output also leaves for global
-            // memory; the tile in shared memory already has the layout of a TMA box.
-            if (p.store_acts && one) {
-              tma_store_2d(&maps.act[l - 1], a_base + (uint32_t)c * FM_CHUNK_BYTES, c * 64, tile * 128);
-              bulk_commit_group();
-            }
           }
-          if (!mbar_wait_warp(smem_u32(&bar_w_full[stage]), w_phase, abortp, SB_SITE_MLP_WEIGHTS)) { ok = false; break; }
           tc_fence_after_sync();
-          const uint32_t a_lo = (uint32_t)umma_smem_desc(a_base + (uint32_t)c * FM_CHUNK_BYTES, 16u, 1024u, 2u);
-          const uint32_t b_lo = (uint32_t)umma_smem_desc(w_base + (uint32_t)stage * p.stage_bytes, 16u, 1024u, 2u);
-          const uint32_t steps = (uint32_t)(p.k_steps[l] - 4 * c);      // beyond the layer's inputs both tiles are zero
-#pragma unroll
-          for (uint32_t ks = 0; ks < 4; ++ks) {
-            if (ks < steps) {
-              umma_issue<false, false>(d_tmem, a_lo + 2u * ks, hi, b_lo + 2u * ks, hi, p.idesc[l], accumulate, one);
-              accumulate = 1u;
-            }
-          }
-          tc_commit(smem_u32(&bar_w_empty[stage]), one);
-          if (++stage == p.w_stages) {
+          umma_issue<false, false>(d_tmem, a_lo, hi, w_lo, hi, idesc, accumulate, one);
+          umma_issue<false, false>(d_tmem, a_lo + 2u, hi, w_lo + 2u, hi, idesc, 1u, one && steps > 1);   // beyond the layer's inputs both tiles are zero
+          umma_issue<false, false>(d_tmem, a_lo + 4u, hi, w_lo + 4u, hi, idesc, 1u, one && steps > 2);
+          umma_issue<false, false>(d_tmem, a_lo + 6u, hi, w_lo + 6u, hi, idesc, 1u, one && steps > 3);
+          accumulate = 1u;
+          a_lo += FM_CHUNK_BYTES >> 4;
+          tc_commit(w_empty0 + 8u * (uint32_t)stage, one);
+          w_lo += w_step;
+          if (++stage == w_stages) {
             stage = 0;
+            w_lo = w_lo0;
             w_phase ^= 1u;
           }
         }
         if (!ok) break;
+        tc_commit(l < L - 1 ? smem_u32(&bar_acc_full[acc]) : smem_u32(&bar_head_full[acc]), one);
         if (l == 0) tc_commit(smem_u32(&bar_x_empty), one);     // the input tile may be refilled
-        tc_commit(smem_u32(&bar_acc_full[acc]), one);
-        if (p.store_acts && l > 0 && one) {    // the stores of this layer's input have read the activation tile
-          bulk_wait_group_read<0>();
-          mbar_arrive(smem_u32(&bar_act_free));
+      }
+    }
+  } else if (warp == 2) {
+    // Training forward: every delivered chunk of a hidden layer's output also leaves for global memory; the tile in shared
+    // memory already has the layout of a TMA box.  The epilogue overwrites the tile once the layer's stores have read it,
+    // so the chunk barriers cannot move on before this warp has seen them.
+    if (HIDDEN != FM_HIDDEN_NONE && p.store_acts) {
+      uint32_t chunk_phase = 0;
+      bool ok = true;
+      for (int item = blockIdx.x; ok && item < p.num_items; item += gridDim.x) {
+        const int tile = item % p.num_tiles;
+        for (int l = 0; ok && l < L - 1; ++l) {
+          for (int c = 0; c < p.k_chunks[l + 1]; ++c) {
+            if (!mbar_wait_warp(smem_u32(&bar_chunk[c]), (chunk_phase >> c) & 1u, abortp, SB_SITE_MLP_ACT)) { ok = false; break; }
+            chunk_phase ^= 1u << c;
+            if (one) {
+              tma_store_2d(&maps.act[l], act_base + (uint32_t)c * FM_CHUNK_BYTES, c * 64, tile * 128);
+              bulk_commit_group();
+            }
+          }
+          if (!ok) break;
+          if (one) {
+            bulk_wait_group_read<0>();
+            mbar_arrive(smem_u32(&bar_act_free));
+          }
         }
+      }
+      if (one) bulk_wait_group<0>();      // bulk groups belong to the lane that issued the stores
+    }
+  } else if (warp == 3) {
+    // Biases: a member's go to shared memory as a whole, once for a single net, and per item (two buffers that take turns)
+    // for an ensemble.
+    if (p.bias_bytes) {
+      int n = 0;
+      for (int item = blockIdx.x; item < p.num_items; item += gridDim.x, ++n) {
+        if (n > 0 && p.members == 1) break;
+        const long long pofs = (long long)(item / p.num_tiles) * p.member_stride;
+        const uint32_t buf = (uint32_t)(n & 1);
+        if (n > 1 && !mbar_wait_warp(smem_u32(&bar_bias_empty[buf]), ((n >> 1) & 1) ^ 1u, abortp, SB_SITE_MLP_ACT)) break;
+        for (int l = 0; l < L; ++l) {
+          const float* src = p.bias[l] + pofs;
+          const uint32_t dst = bias_base + buf * p.bias_bytes + p.bias_pos[l];
+          const int live = p.width[l + 1], n_pad = l < L - 1 ? live : FM_HEAD_BIAS;
+#pragma unroll 8
+          for (int j = lane; j < n_pad; j += 32) {
+            const float b = j < live ? __ldg(src + j) : 0.f;
+            asm volatile("st.shared.f32 [%0], %1;" ::"r"(dst + 4u * (uint32_t)j), "f"(b) : "memory");
+          }
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_u32(&bar_bias_full[buf]));
       }
     }
   } else {
-    const int quad = warp & 3, half = (warp - 2) >> 2;
+    const int quad = warp & 3;
     const int row_in_tile = quad * 32 + lane;
     const uint32_t t_row = tmem_base + ((uint32_t)(quad * 32) << 16);
-    const uint32_t bias_smem = base + p.bias_offset + (uint32_t)(warp - 2) * 512u;
-    uint32_t layer = 0, tail_phase = 0;           // layer: counts layers across items; its last two bits are accumulator and phase
-    uint32_t act_phase = 1;                       // the first tile finds the activation tile free
-    // This warp's copy of the head description (in shared memory: the head code reads a field where it
-    // needs it instead of holding the whole structure in registers); member-specific fields are set per item.
-    SbRowHead& h = head_slot[warp - 2];
-    if (lane == 0) h = p.head;
-    __syncwarp();
+    const bool has_bias = p.bias_bytes != 0u, rebias = has_bias && p.members > 1;
     bool ok = true;
-    for (int item = blockIdx.x; ok && item < p.num_items; item += gridDim.x) {
-      const int member = item / p.num_tiles, tile = item - member * p.num_tiles;
-      const long long pofs = (long long)member * p.member_stride;
-      float* out_m = p.out + (long long)member * p.out_stride;
-      __syncwarp();                 // every lane is done with its row of the item before: with `h` and the biases it read
-      if (lane == 0) {
-        h.argmax_out = p.head.argmax_out ? p.head.argmax_out + (long long)member * p.batch : nullptr;
-        h.sample_out = p.head.sample_out ? p.head.sample_out + (long long)member * p.batch : nullptr;
-        h.position = p.head.position + (unsigned long long)member;      // one draw per member from the row's stream
+    int n = 0;                            // items of this CTA before this one
+    // The biases of the item: in place before the first read, and for an ensemble handed back after the last.
+    bool bias_seen = false;
+    auto bias_wait = [&]() -> uint32_t {
+      const uint32_t buf = rebias ? (uint32_t)(n & 1) : 0u;
+      if (has_bias && (rebias || !bias_seen)) {
+        if (!mbar_wait_warp(smem_u32(&bar_bias_full[buf]), rebias ? (uint32_t)(n >> 1) & 1u : 0u, abortp, SB_SITE_MLP_ACT)) ok = false;
+        bias_seen = true;
       }
-      __syncwarp();
-      const float* head_bias = p.bias[L - 1] ? p.bias[L - 1] + pofs : nullptr;
-      for (int l = 0; l < L; ++l) {
-        const uint32_t acc = layer & 1u, acc_phase = (layer >> 1) & 1u;
-        ++layer;
-        const uint32_t t_acc = t_row + acc * (uint32_t)p.acc_stride;
-        const uint32_t full = smem_u32(&bar_acc_full[acc]);
-        const long long grow = (long long)tile * 128 + row_in_tile;
-        if (HIDDEN != FM_HIDDEN_NONE && l < L - 1) {
-          const float* bias_l = p.bias[l] ? p.bias[l] + pofs : nullptr;
-          const uint32_t act_free = p.store_acts ? smem_u32(&bar_act_free) : 0u;
-          ok = fused_hidden<BF16, HIDDEN == FM_HIDDEN_NORM>(t_acc, p.n_pad[l], bias_l, act_base, bias_smem, row_in_tile, half,
-                                  smem_u32(&bar_chunk[0]), p.bits[l], grow, p.batch, full, acc_phase, act_free, act_phase, abortp);
-          act_phase ^= 1u;
-        } else if (half == 0) {
-          // What the head needs beside the accumulator is asked for before the wait: its biases (into the warp's
-          // buffer) and the row's mask bytes.
-          if (head_bias) {
-#pragma unroll
-            for (int j = lane; j < 64; j += 32) {
-              const float b = j < h.n ? __ldg(head_bias + j) : 0.f;
-              asm volatile("st.shared.f32 [%0], %1;" ::"r"(bias_smem + 4u * (uint32_t)j), "f"(b) : "memory");
-            }
-          }
-          unsigned long long legal = 0ull;
-          if (grow < p.batch) {
-            if (p.head_width <= 4) legal = sb_row_head_legal<4>(h, grow);
-            else if (p.head_width <= 16) legal = sb_row_head_legal<16>(h, grow);
-            else legal = sb_row_head_legal<64>(h, grow);
-          }
-          __syncwarp();
-          if (!mbar_wait(full, acc_phase, abortp, SB_SITE_MLP_ACC)) { ok = false; break; }
-          tc_fence_after_sync();
-          const uint32_t head_done = smem_u32(&bar_head_done[acc]);
-          const bool hb = head_bias != nullptr;
-          switch (p.head_width) {
-            case 4: fused_head<4>(h, legal, hb, bias_smem, out_m, t_acc, grow, p.batch, head_done); break;
-            case 8: fused_head<8>(h, legal, hb, bias_smem, out_m, t_acc, grow, p.batch, head_done); break;
-            case 16: fused_head<16>(h, legal, hb, bias_smem, out_m, t_acc, grow, p.batch, head_done); break;
-            case 32: fused_head<32>(h, legal, hb, bias_smem, out_m, t_acc, grow, p.batch, head_done); break;
-            default: fused_head<64>(h, legal, hb, bias_smem, out_m, t_acc, grow, p.batch, head_done); break;
-          }
-        }
-        if (!ok) break;
-      }
-      if (ok && p.tile_counters && half == 0) {
-        // Decision tail (ml/models.spi:51-76).  The four head warps publish their rows of this member, count
-        // the member in; the CTA that counts the last member of the tile in sees every member's results.
-        // The two meeting points are mbarriers with bounded waits, like every other wait of the kernel.
-        __threadfence();
+      return bias_base + buf * p.bias_bytes;
+    };
+    auto bias_done = [&]() {
+      if (rebias) {
         __syncwarp();
-        if (lane == 0) mbar_arrive(smem_u32(&bar_tail_in));
-        if (warp == 2 && lane == 0) {
-          if (mbar_wait(smem_u32(&bar_tail_in), tail_phase, abortp, SB_SITE_MLP_ACT)) {
-            __threadfence();
-            const int before = atomicAdd(p.tile_counters + tile, 1);
-            __threadfence();
-            tile_is_complete = before == p.members - 1 ? 1 : 0;
-          } else {
-            tile_is_complete = 0;
+        if (lane == 0) mbar_arrive(smem_u32(&bar_bias_empty[n & 1]));
+      }
+    };
+    if (EW > 0 && warp < 4 + EW) {
+      if constexpr (EW > 0) {
+        const int half = (warp - 4) >> 2;
+        uint32_t layer = 0, acc_phase = 0;   // layers across items (the last bit is the accumulator), a parity bit per accumulator
+        uint32_t act_phase = 1;              // the first tile finds the activation tile free
+        const uint32_t act_free = p.store_acts ? smem_u32(&bar_act_free) : 0u;
+        for (int item = blockIdx.x; ok && item < p.num_items; item += gridDim.x, ++n) {
+          const int tile = item % p.num_tiles;
+          const long long grow = (long long)tile * 128 + row_in_tile;
+          const uint32_t bias_smem = bias_wait();
+          if (!ok) break;
+          for (int l = 0; l < L - 1; ++l, ++layer) {
+            const uint32_t acc = layer & 1u;
+            ok = fused_hidden<BF16, HIDDEN == FM_HIDDEN_NORM>(t_row + acc * (uint32_t)p.acc_stride, p.n_pad[l], has_bias,
+                     bias_smem + p.bias_pos[l], act_base, row_in_tile, half, smem_u32(&bar_chunk[0]), p.bits[l], grow,
+                     p.batch, smem_u32(&bar_acc_full[acc]), (acc_phase >> acc) & 1u, act_free, act_phase, abortp);
+            acc_phase ^= 1u << acc;
+            act_phase ^= 1u;
+            if (!ok) break;
           }
-          mbar_arrive(smem_u32(&bar_tail_out));
+          ++layer;                        // the head's
+          bias_done();
         }
-        if (!mbar_wait(smem_u32(&bar_tail_out), tail_phase, abortp, SB_SITE_MLP_ACT)) break;
-        tail_phase ^= 1u;
-        if (tile_is_complete) {
+      }
+    } else {
+      const int hw = warp - 4 - EW, hg = hw >> 2;
+      // This warp's copy of the head description (in shared memory: the head code reads a field where it
+      // needs it instead of holding the whole structure in registers); member-specific fields are set per item.
+      SbRowHead& h = head_slot[hw];
+      if (lane == 0) h = p.head;
+      __syncwarp();
+      uint32_t layer = (uint32_t)(L - 1), acc_phase = 0, tail_phase = 0;
+      for (int item = blockIdx.x; ok && item < p.num_items; item += gridDim.x, ++n, layer += (uint32_t)L) {
+        if (HG == 2 && (n & 1) != hg) continue;
+        const int member = item / p.num_tiles, tile = item - member * p.num_tiles;
+        const long long grow = (long long)tile * 128 + row_in_tile;
+        float* out_m = p.out + (long long)member * p.out_stride;
+        __syncwarp();                 // every lane is done with its row of the item before: with `h`
+        if (lane == 0) {
+          h.argmax_out = p.head.argmax_out ? p.head.argmax_out + (long long)member * p.batch : nullptr;
+          h.sample_out = p.head.sample_out ? p.head.sample_out + (long long)member * p.batch : nullptr;
+          h.position = p.head.position + (unsigned long long)member;      // one draw per member from the row's stream
+        }
+        __syncwarp();
+        // What the head needs beside the accumulator is asked for before the wait.
+        unsigned long long legal = 0ull;
+        if (grow < p.batch) {
+          if (p.head_width <= 4) legal = sb_row_head_legal<4>(h, grow);
+          else if (p.head_width <= 16) legal = sb_row_head_legal<16>(h, grow);
+          else legal = sb_row_head_legal<64>(h, grow);
+        }
+        const uint32_t bias_smem = bias_wait() + p.bias_pos[L - 1];
+        if (!ok) break;
+        const uint32_t acc = layer & 1u;
+        if (!mbar_wait_warp(smem_u32(&bar_head_full[acc]), (acc_phase >> acc) & 1u, abortp, SB_SITE_MLP_ACC)) break;
+        acc_phase ^= 1u << acc;
+        tc_fence_after_sync();
+        const uint32_t head_done = smem_u32(&bar_head_done[acc]);
+        const uint32_t t_acc = t_row + acc * (uint32_t)p.acc_stride;
+        switch (p.head_width) {
+          case 4: fused_head<4>(h, legal, has_bias, bias_smem, out_m, t_acc, grow, p.batch, head_done); break;
+          case 8: fused_head<8>(h, legal, has_bias, bias_smem, out_m, t_acc, grow, p.batch, head_done); break;
+          case 16: fused_head<16>(h, legal, has_bias, bias_smem, out_m, t_acc, grow, p.batch, head_done); break;
+          case 32: fused_head<32>(h, legal, has_bias, bias_smem, out_m, t_acc, grow, p.batch, head_done); break;
+          default: fused_head<64>(h, legal, has_bias, bias_smem, out_m, t_acc, grow, p.batch, head_done); break;
+        }
+        bias_done();
+        if (p.tile_counters) {
+          // Decision tail (ml/models.spi:51-76).  The four head warps publish their rows of this member, count
+          // the member in; the CTA that counts the last member of the tile in sees every member's results.
+          // The two meeting points are mbarriers with bounded waits, like every other wait of the kernel.
           __threadfence();
-          decide_row(p, (long long)tile * 128 + row_in_tile);
-          if (warp == 2 && lane == 0) p.tile_counters[tile] = 0;        // ready for the next call
+          __syncwarp();
+          if (lane == 0) mbar_arrive(smem_u32(&bar_tail_in[hg]));
+          if ((hw & 3) == 0 && lane == 0) {
+            if (mbar_wait(smem_u32(&bar_tail_in[hg]), tail_phase, abortp, SB_SITE_MLP_ACT)) {
+              __threadfence();
+              const int before = atomicAdd(p.tile_counters + tile, 1);
+              __threadfence();
+              tile_is_complete[hg] = before == p.members - 1 ? 1 : 0;
+            } else {
+              tile_is_complete[hg] = 0;
+            }
+            mbar_arrive(smem_u32(&bar_tail_out[hg]));
+          }
+          if (!mbar_wait_warp(smem_u32(&bar_tail_out[hg]), tail_phase, abortp, SB_SITE_MLP_ACT)) break;
+          tail_phase ^= 1u;
+          if (tile_is_complete[hg]) {
+            __threadfence();
+            decide_row(p, grow);
+            if ((hw & 3) == 0 && lane == 0) p.tile_counters[tile] = 0;        // ready for the next call
+          }
+          // tile_is_complete is rewritten only after all four warps have arrived for the next item.
         }
-        // tile_is_complete is rewritten only after all four warps have arrived for the next item.
       }
     }
   }
 
-  if (warp == 1 && one && p.store_acts) bulk_wait_group<0>();      // bulk groups belong to the lane that issued the stores
   __syncwarp();
   tc_fence_before_sync();
   __syncthreads();
@@ -640,10 +715,15 @@ static int fused_launch(const char* who, int n_layers, const int* sizes, int bat
   if (smem_needed > FM_SMEM_LIMIT)
     return sb_fail(SB_ERR_UNSUPPORTED, "%s: the input tile, the widest hidden tile and the weight ring need %zu bytes of "
                                        "shared memory (inputs wider than 256 fit with hidden layers of at most 128)", who, smem_needed);
-  // The ring takes what is left beside the bias buffers: more than the four stages of the rule above for narrow
-  // layers, three for the widest nets with biases (65 to 128 inputs, 256-wide layers: 128-256-256-17, 262144 rows,
-  // 194 -> 165 us with them; without biases, four stages, 184 -> 160).
-  const uint32_t bias_bytes = params ? FM_BIAS_BYTES : 0u;
+  // The ring takes what is left beside the biases: more than the four stages of the rule above for narrow
+  // layers, three for the widest nets with biases (65 to 128 inputs and 256-wide layers, or the full 227 KB otherwise).
+  if (params) {
+    for (int l = 0; l < n_layers; ++l) {
+      p.bias_pos[l] = p.bias_bytes;
+      p.bias_bytes += 4u * (uint32_t)(l < n_layers - 1 ? sizes[l + 1] : FM_HEAD_BIAS);
+    }
+  }
+  const uint32_t bias_bytes = p.bias_bytes * (members > 1 ? 2u : 1u);
   p.w_stages = (int)((FM_SMEM_LIMIT - 1024 - p.w_offset - bias_bytes) / p.stage_bytes);
   if (p.w_stages > FM_W_STAGES_MAX) p.w_stages = FM_W_STAGES_MAX;
   p.bias_offset = p.w_offset + (uint32_t)p.w_stages * p.stage_bytes;
@@ -665,7 +745,8 @@ static int fused_launch(const char* who, int n_layers, const int* sizes, int bat
   double flops = 0.0;
   for (int l = 0; l < n_layers; ++l) flops += 2.0 * batch * (double)sizes[l] * sizes[l + 1] * members;
   sb_prof_before((cudaStream_t)stream);
-  SB_CUDA(sb_launch(kernels[in_dtype == SB_BF16][n_layers == 1 ? FM_HIDDEN_NONE : hidden_norm ? FM_HIDDEN_NORM : FM_HIDDEN_RELU], dim3(grid), dim3(FM_THREADS), smem, (cudaStream_t)stream, 1, maps, p));
+  const int hidden = n_layers == 1 ? FM_HIDDEN_NONE : hidden_norm ? FM_HIDDEN_NORM : FM_HIDDEN_RELU;
+  SB_CUDA(sb_launch(kernels[in_dtype == SB_BF16][hidden], dim3(grid), dim3(fm_threads(hidden)), smem, (cudaStream_t)stream, 1, maps, p));
   sb_prof_after((cudaStream_t)stream, flops);
   SB_COUNT_LAUNCH();
   SB_CUDA(cudaGetLastError());

@@ -82,6 +82,24 @@ def test_sampling_head_with_the_members_of_several_items_on_one_sm(gpu, sizes, p
         np.testing.assert_array_equal(single.indices.numpy()[0], ens.indices.numpy()[e])
 
 
+@pytest.mark.parametrize("sizes", [[64, 40], [32, 64, 64, 3], [8, 5]])
+def test_members_biases_take_turns_over_many_items_on_one_sm(gpu, sizes):
+    """Seven or eight items a CTA, a member's biases in either of two buffers: the same bits as the member alone."""
+    members, batch = 9, 128 * 121 + 5
+    g = so.rng(75)
+    ws = member_weights(760, sizes, members)
+    bs = [[g.normal(0.0, 0.3, size=n).astype(np.float32) for n in sizes[1:]] for _ in range(members)]
+    dx = gpu.to_storage((g.random((batch, sizes[0])) < 0.2).astype(np.float32), "f16")
+    ens = gpu.EnsemblePolicyMLP(sizes, batch, members, in_dtype="f16", head=("masked_softmax", "argmax"))
+    ens.load_weights(ws, bs)
+    probs, actions = ens.forward(dx).numpy(), ens.actions.numpy()
+    single = gpu.PolicyMLP(sizes, batch, in_dtype="f16", head=("masked_softmax", "argmax"))
+    for e in range(members):
+        single.load_weights(ws[e], bs[e])
+        np.testing.assert_array_equal(single.forward_fused(dx).numpy(), probs[e])
+        np.testing.assert_array_equal(single.actions.numpy(), actions[e])
+
+
 def test_row_normalised_net_with_sampling_head_over_128_columns(gpu):
     """128 -> 128 -> 128 -> 128, ln_l2 + relu between the layers, `masked_softmax_and_discrete_sample' 3`
     (game/leduc/tests/train.spi:88-101), weights N(0, 0.1) as the reference initialises them."""
