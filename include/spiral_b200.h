@@ -335,6 +335,17 @@ int sb_mlp_forward_fused_head(int n_layers, const int* sizes, int batch, int mem
                               const void* x, const void* w_compute, const float* params, int hidden_norm,
                               const sb_head_spec* head, float* out, void* stream);
 
+/* A layer graph of dense layers as one launch, in the TF32 class (fp32 storage): hidden layers
+ * matmul [-> ln_l2] -> relu (ml/layers.spi:562-568, hidden_norm = 1 with ln_l2 in every one) and a last layer with a row
+ * head.  x is fp32 [rows, sizes[0]], weights[l] the [sizes[l+1], sizes[l]] matrix of layer l (rounded to TF32 where it
+ * was made), hidden[l] the fp32 [rows, sizes[l+1]] output of hidden layer l (rounded to TF32, as the next layer reads it),
+ * out fp32 [rows, sizes[n_layers]].  Two to eight layers, inputs of up to 256 columns (a multiple of 4), hidden widths
+ * multiples of 64 up to 256, outputs up to 64, or up to 256 under a prefix of at most 64; no sign hash.  sb_layers_fused_supported tells
+ * (1 / 0) whether widths and prefix (-1: none) are within these limits. */
+int sb_layers_fused_supported(int n_layers, const int* sizes, int prefix);
+int sb_layers_forward_fused(int n_layers, const int* sizes, int rows, const float* x, const void* const* weights,
+                            int hidden_norm, void* const* hidden, const sb_head_spec* head, float* out, void* stream);
+
 /* One policy decision per game state, the whole of models.noinline_run (ml/models.spi:9-76): the states
  * are serialised into the input tensor on the device (sb_encode_states; fields == NULL: x already holds
  * the input), every ensemble member's net runs on them, each member samples an action per state from

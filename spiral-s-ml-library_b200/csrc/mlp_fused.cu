@@ -20,11 +20,15 @@
 //   warps 12..15   : the last layer's row head (masked softmax / regret matching /
 //                    argmax) written to global, beside the next tile's first layers.
 //                    A single-layer net has no epilogue warps and two such groups.
-// 16-bit arithmetic classes only (SB_F16, SB_BF16); widths: input <= 512 and a
+// 16-bit arithmetic classes (SB_F16, SB_BF16), and TF32 storage for layer graphs (below); widths: input <= 512 and a
 // multiple of 8 (inputs beyond 256 as far as shared memory allows: the reference's Hold'em
 // policy net is 512 -> 64, game/nl_hu_holdem/model_cem.spi:71-98), hidden layers multiples of 64 up to 256, output <= 64 (<= 256 when a
 // prefix mask confines the head to its first 64 columns, the shape of the reference's
 // own policy nets, game/leduc/model_cem.spi:37,52-60).
+//
+// Layer graphs (sb_layers_forward_fused) run in TF32 storage: K-chunks of 32 values, inputs and hidden layers up to 256,
+// hidden outputs stored as in the training forward.  8192 rows, 128-128-128-128 with ln_l2 and a sampling head: 29.6 us as
+// three launches (each waits for the last tile of the one before, loads one tile per SM, and stores it), 14.0 as one.
 //
 // Optional, for the reference's graphs: ln_l2 before every ReLU (ml/layers.spi:562-568), a
 // sampling head that draws from a Philox stream per row (ml/layers.spi:422-431), and the
@@ -37,6 +41,9 @@
 namespace {
 
 constexpr int FM_MAX_LAYERS = 8;
+// Storage of activations and weights: 16 bits, or TF32 in 32 bits (layer graphs).  A K-chunk is 128 bytes of a row.
+constexpr int FM_F16 = 0, FM_BF16 = 1, FM_TF32 = 2;
+__host__ __device__ constexpr int fm_chunk_cols(int cls) { return cls == FM_TF32 ? 32 : 64; }
 constexpr int FM_HIDDEN_NONE = 0, FM_HIDDEN_RELU = 1, FM_HIDDEN_NORM = 2;
 constexpr int FM_HEAD_BIAS = 64;                        // floats kept for the head's biases, zero beyond the outputs
 // Warps of an instance: four with a job each (producer, issuer, activation stores, biases), eight for the epilogue of the
@@ -47,13 +54,13 @@ __host__ __device__ constexpr int fm_threads(int hidden) { return 32 * (4 + fm_e
 constexpr size_t FM_SMEM_LIMIT = 225 * 1024;            // dynamic shared memory; the static part stays below 2 KB
 constexpr int FM_W_STAGES = 4;                         // stages of the weight ring that decide which nets fit
 constexpr int FM_W_STAGES_MAX = 8;                     // stages taken where shared memory is left
-constexpr uint32_t FM_CHUNK_BYTES = 128u * 128u;       // activation chunk: 128 rows x 64 elements x 2 B
-// A weight stage holds one 64-column K-chunk of a layer: (widest layer's rows) x 128 bytes, at most 256 rows.
+constexpr uint32_t FM_CHUNK_BYTES = 128u * 128u;       // activation chunk: 128 rows x 128 bytes
+// A weight stage holds one K-chunk of a layer: (widest layer's rows) x 128 bytes, at most 256 rows.
 
 struct FusedMaps {
-  CUtensorMap x;                      // [batch, in] box {64, 128}
-  CUtensorMap w[FM_MAX_LAYERS];       // W_l [members, out_l, in_l] box {64, rows_l, 1}
-  CUtensorMap act[FM_MAX_LAYERS];     // training forward: hidden activations of layer l, [batch, width_l] box {64, 128}
+  CUtensorMap x;                      // [batch, in] box {chunk, 128}
+  CUtensorMap w[FM_MAX_LAYERS];       // W_l [members, out_l, in_l] box {chunk, rows_l, 1}
+  CUtensorMap act[FM_MAX_LAYERS];     // training forward, layer graph: hidden activations of layer l, [batch, width_l] box {chunk, 128}
 };
 
 struct FusedParams {
@@ -61,8 +68,8 @@ struct FusedParams {
   int batch;
   int width[FM_MAX_LAYERS + 1];       // width[0] = input features
   int n_pad[FM_MAX_LAYERS];           // MMA N of layer l (hidden: width; last: what the head needs, a multiple of 16)
-  int k_chunks[FM_MAX_LAYERS];        // ceil(in_l / 64)
-  int k_steps[FM_MAX_LAYERS];         // ceil(in_l / 16): MMAs of the layer
+  int k_chunks[FM_MAX_LAYERS];        // ceil(in_l / chunk)
+  int k_steps[FM_MAX_LAYERS];         // MMAs of the layer, 32 bytes of K each
   uint32_t idesc[FM_MAX_LAYERS];
   uint32_t w_bytes[FM_MAX_LAYERS];    // bytes of one weight chunk of layer l
   const float* bias[FM_MAX_LAYERS];   // may be null
@@ -75,6 +82,7 @@ struct FusedParams {
   uint32_t x_chunks;                  // chunks of the input tile
   uint32_t stage_bytes;               // bytes of one weight stage
   uint32_t act_offset, w_offset;      // byte offsets of the activation tile and the weight ring
+  int x_shared;                       // 1: the input tile lies in the activation tile (act_offset = 0); layer graphs of wide layers
   int w_stages;                       // stages of the weight ring
   uint32_t bias_offset;               // byte offset of the biases: all layers of a member one behind the other
   uint32_t bias_bytes;                // bytes of one member's biases; two such buffers take turns when there are several members
@@ -123,9 +131,9 @@ __device__ __noinline__ void fused_head(const SbRowHead& h, unsigned long long l
 }
 
 // Finishes 32 columns of a row: bias, ReLU, rounding to the storage type, and the swizzled store into the activation
-// tile (`dst` = the row's 128 bytes of the 64-column chunk, `piece0` = first of its four 16-byte pieces, `key` the row's
-// swizzle).  `word` (or null) takes the sign word of the row and chunk.
-template <bool BF16, bool NORM>
+// tile (`dst` = the row's 128 bytes of the activation chunk, `piece0` = first of its four 16-byte pieces there, all eight
+// in 32-bit storage, `key` the row's swizzle).  `word` (or null) takes the sign word of the row and chunk.
+template <int CLS, bool NORM>
 __device__ __forceinline__ void hidden_chunk(uint32_t* raw, float sumsq, float inv, bool has_bias, uint32_t bias_addr,
                                              uint32_t* word, uint32_t dst, uint32_t piece0, uint32_t key) {
   float* v = reinterpret_cast<float*>(raw);
@@ -140,21 +148,30 @@ __device__ __forceinline__ void hidden_chunk(uint32_t* raw, float sumsq, float i
     }
   }
   if (word) *word = positive_bits32(v);
+  if constexpr (CLS == FM_TF32) {
+    auto one = [&](int j) { return __float_as_uint(round_tf32_rn(fmaxf(v[j], 0.f))); };
 #pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    const uint4 out = make_uint4(relu_pack2<BF16>(v[8 * q], v[8 * q + 1]), relu_pack2<BF16>(v[8 * q + 2], v[8 * q + 3]),
-                                 relu_pack2<BF16>(v[8 * q + 4], v[8 * q + 5]), relu_pack2<BF16>(v[8 * q + 6], v[8 * q + 7]));
-    st_shared_v4(dst + (((piece0 + (uint32_t)q) ^ key) << 4), out);
+    for (int q = 0; q < 8; ++q)
+      st_shared_v4(dst + (((uint32_t)q ^ key) << 4), make_uint4(one(4 * q), one(4 * q + 1), one(4 * q + 2), one(4 * q + 3)));
+  } else {
+    constexpr bool BF16 = CLS == FM_BF16;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const uint4 out = make_uint4(relu_pack2<BF16>(v[8 * q], v[8 * q + 1]), relu_pack2<BF16>(v[8 * q + 2], v[8 * q + 3]),
+                                   relu_pack2<BF16>(v[8 * q + 4], v[8 * q + 5]), relu_pack2<BF16>(v[8 * q + 6], v[8 * q + 7]));
+      st_shared_v4(dst + (((piece0 + (uint32_t)q) ^ key) << 4), out);
+    }
   }
 }
 
 // One warp's share of a hidden layer: chunks `half`, half + 2, ... of 32 columns (at most four).
 // Writes relu(acc + bias) in the storage type into the activation tile, in the
 // 128-byte-swizzled K-major layout the next layer's A descriptors expect:
-// element (row, j) -> chunk j / 64, byte row * 128 + (((j % 64) / 8) ^ (row % 8)) * 16 + (j % 8) * 2.
-// After each 32-column chunk the warp arrives on the barrier of the 64-column activation chunk it
-// belongs to (`chunk_bar0` + 8 bytes per chunk): the next layer's MMAs on that K-chunk start as soon as
-// all eight warps have delivered it, while the later chunks of this layer are still being finished.
+// element (row, j) -> chunk j / 64, byte row * 128 + (((j % 64) / 8) ^ (row % 8)) * 16 + (j % 8) * 2
+// (32-bit storage: chunk j / 32, byte row * 128 + (((j % 32) / 4) ^ (row % 8)) * 16 + (j % 4) * 4).
+// After each 32-column chunk the warp arrives on the barrier of the activation chunk it belongs to
+// (`chunk_bar0` + 8 bytes per chunk): the next layer's MMAs on that K-chunk start as soon as all its
+// warps (eight, four in 32-bit storage) have delivered it, while the later chunks are still being finished.
 //
 // A tile's time is the chain of these chunks.  Clock stamps of a tile of the Leduc net (262144 rows): 3860 clocks a hidden
 // layer, of which a chunk takes 640 (85 instructions 460, proxy fence 110, the next chunk's wait 70) and the way from the
@@ -165,7 +182,7 @@ __device__ __forceinline__ void hidden_chunk(uint32_t* raw, float sumsq, float i
 // Tried: sixteen warps of two chunks each (80 registers: 106 us); the last K-chunk by halves of the columns, so that the
 // epilogue starts on the left one (101: MMAs of 128 columns read A twice).
 // False when a wait expired.
-template <bool BF16, bool NORM>
+template <int CLS, bool NORM>
 __device__ __forceinline__ bool fused_hidden(uint32_t t_row, int n_cols, bool has_bias, uint32_t bias_smem, uint32_t act_base,
                                           int row_in_tile, int half,
                                           uint32_t chunk_bar0, uint32_t* bits_out, long long row, int batch,
@@ -194,14 +211,16 @@ __device__ __forceinline__ bool fused_hidden(uint32_t t_row, int n_cols, bool ha
   const uint32_t key = (uint32_t)row_in_tile & 7u;
   const uint32_t dst0 = act_base + (uint32_t)row_in_tile * 128u;
   uint32_t* word = bits_out && row < batch ? bits_out + row : nullptr;
-  auto finish = [&](uint32_t* raw, int c) {      // chunk c of 32 columns: the left or right half of activation chunk c / 2
-    hidden_chunk<BF16, NORM>(raw, sumsq, inv, has_bias, bias_smem + 128u * (uint32_t)c,
-                       word ? word + (long long)c * batch : nullptr, dst0 + (uint32_t)(c >> 1) * FM_CHUNK_BYTES, 4u * (uint32_t)(c & 1), key);
+  // Chunk c of 32 columns: the left or right half of activation chunk c / 2, all of chunk c in 32-bit storage.
+  auto finish = [&](uint32_t* raw, int c) {
+    const uint32_t chunk = (uint32_t)(CLS == FM_TF32 ? c : c >> 1);
+    hidden_chunk<CLS, NORM>(raw, sumsq, inv, has_bias, bias_smem + 128u * (uint32_t)c,
+                       word ? word + (long long)c * batch : nullptr, dst0 + chunk * FM_CHUNK_BYTES, 4u * (uint32_t)(c & 1), key);
     // generic-proxy writes of the activation tile must be visible to the MMA's async-proxy reads
     fence_proxy_async_smem();
     tc_fence_before_sync();
     __syncwarp();
-    if (lane == 0) mbar_arrive(chunk_bar0 + 8u * (uint32_t)(c >> 1));
+    if (lane == 0) mbar_arrive(chunk_bar0 + 8u * chunk);
   };
   // The next chunk is on its way out of tensor memory while this one is finished.
 #pragma unroll 1
@@ -249,15 +268,16 @@ __device__ __noinline__ void decide_row(const FusedParams& p, long long row) {
 // the row before every ReLU, no bias).  Instances of their own: with the divisions of
 // the one and the chunk loop of the other in every kernel, registers went short where they are not used.  Leduc net,
 // 262144 rows 137 -> 129 us, 16384 rows 13.9 -> 13.3; one layer of 512-64, 16 members, 512 states 23 -> 18.5.
-template <bool BF16, int HIDDEN>
+template <int CLS, int HIDDEN>
 __global__ void __launch_bounds__(fm_threads(HIDDEN), 1)
 mlp_fused_kernel(const __grid_constant__ FusedMaps maps, const __grid_constant__ FusedParams p) {
-  constexpr int EW = fm_epi_warps(HIDDEN), HG = fm_head_groups(HIDDEN);
+  constexpr int EW = fm_epi_warps(HIDDEN), HG = fm_head_groups(HIDDEN), CHUNK = fm_chunk_cols(CLS);
+  constexpr bool TF32 = CLS == FM_TF32;
   extern __shared__ uint8_t fm_smem_raw[];
   __shared__ __align__(8) uint64_t bar_x_full, bar_x_empty, bar_act_free, bar_tail_in[HG], bar_tail_out[HG];
   __shared__ __align__(8) uint64_t bar_bias_full[2], bar_bias_empty[2];
   __shared__ __align__(8) uint64_t bar_acc_full[2], bar_head_full[2], bar_head_done[2];      // per accumulator: a hidden layer's or a head's, and its rows read
-  __shared__ __align__(8) uint64_t bar_chunk[4];       // 64-column chunk k of the activation tile is written (8 warps each)
+  __shared__ __align__(8) uint64_t bar_chunk[8];       // chunk k of the activation tile is written (8 warps each, 4 in 32-bit storage)
   __shared__ __align__(8) uint64_t bar_w_full[FM_W_STAGES_MAX], bar_w_empty[FM_W_STAGES_MAX];
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
@@ -273,7 +293,7 @@ mlp_fused_kernel(const __grid_constant__ FusedMaps maps, const __grid_constant__
 
   if (tid == 0) {
     mbar_init(smem_u32(&bar_x_full), 1);
-    mbar_init(smem_u32(&bar_x_empty), 1);
+    mbar_init(smem_u32(&bar_x_empty), p.x_shared ? 2 : 1);   // the MMAs that read it last; shared: and the stores of the last hidden layer
     mbar_init(smem_u32(&bar_act_free), 1);
     for (int a = 0; a < 2; ++a) {
       mbar_init(smem_u32(&bar_acc_full[a]), 1);
@@ -282,7 +302,7 @@ mlp_fused_kernel(const __grid_constant__ FusedMaps maps, const __grid_constant__
       mbar_init(smem_u32(&bar_bias_full[a]), 1);
       mbar_init(smem_u32(&bar_bias_empty[a]), EW + 4);   // every warp that reads an item's biases
     }
-    for (int k = 0; k < 4; ++k) mbar_init(smem_u32(&bar_chunk[k]), 8);
+    for (int k = 0; k < 8; ++k) mbar_init(smem_u32(&bar_chunk[k]), TF32 ? 4 : 8);
     for (int g = 0; g < HG; ++g) {
       mbar_init(smem_u32(&bar_tail_in[g]), 4);       // the four warps that finish head rows
       mbar_init(smem_u32(&bar_tail_out[g]), 1);
@@ -322,7 +342,7 @@ mlp_fused_kernel(const __grid_constant__ FusedMaps maps, const __grid_constant__
       x_phase ^= 1u;
       if (one) mbar_arrive_expect_tx(smem_u32(&bar_x_full), p.x_chunks * FM_CHUNK_BYTES);
       for (uint32_t c = 0; c < p.x_chunks; ++c)
-        tma_load_2d(x_base + c * FM_CHUNK_BYTES, &maps.x, (int)(c * 64), tile * 128, smem_u32(&bar_x_full), one);
+        tma_load_2d(x_base + c * FM_CHUNK_BYTES, &maps.x, (int)c * CHUNK, tile * 128, smem_u32(&bar_x_full), one);
       for (int l = 0; ok && l < L; ++l) {
         for (int c = 0; c < p.k_chunks[l]; ++c) {
           if (!mbar_wait_warp(smem_u32(&bar_w_empty[stage]), w_phase ^ 1u, abortp, SB_SITE_MLP_WEIGHTS)) {
@@ -330,7 +350,7 @@ mlp_fused_kernel(const __grid_constant__ FusedMaps maps, const __grid_constant__
             break;
           }
           if (one) mbar_arrive_expect_tx(smem_u32(&bar_w_full[stage]), p.w_bytes[l]);
-          tma_load_3d(w_base + (uint32_t)stage * p.stage_bytes, &maps.w[l], c * 64, 0, member, smem_u32(&bar_w_full[stage]), one);
+          tma_load_3d(w_base + (uint32_t)stage * p.stage_bytes, &maps.w[l], c * CHUNK, 0, member, smem_u32(&bar_w_full[stage]), one);
           if (++stage == p.w_stages) {
             stage = 0;
             w_phase ^= 1u;
@@ -377,15 +397,15 @@ mlp_fused_kernel(const __grid_constant__ FusedMaps maps, const __grid_constant__
           // what is there already costs the issuer some 100 clocks all the same (the other order: 91.7 -> 95 us).
           if (!mbar_wait_warp(w_full0 + 8u * (uint32_t)stage, w_phase, abortp, SB_SITE_MLP_WEIGHTS)) { ok = false; break; }
           if (l > 0) {
-            // K-chunk c of this layer's input = 64-column chunk c of the previous layer's output
+            // K-chunk c of this layer's input = activation chunk c of the previous layer's output
             if (!mbar_wait_warp(chunk0 + 8u * (uint32_t)c, (chunk_phase >> c) & 1u, abortp, SB_SITE_MLP_ACT)) { ok = false; break; }
             chunk_phase ^= 1u << c;
           }
           tc_fence_after_sync();
-          umma_issue<false, false>(d_tmem, a_lo, hi, w_lo, hi, idesc, accumulate, one);
-          umma_issue<false, false>(d_tmem, a_lo + 2u, hi, w_lo + 2u, hi, idesc, 1u, one && steps > 1);   // beyond the layer's inputs both tiles are zero
-          umma_issue<false, false>(d_tmem, a_lo + 4u, hi, w_lo + 4u, hi, idesc, 1u, one && steps > 2);
-          umma_issue<false, false>(d_tmem, a_lo + 6u, hi, w_lo + 6u, hi, idesc, 1u, one && steps > 3);
+          umma_issue<false, TF32>(d_tmem, a_lo, hi, w_lo, hi, idesc, accumulate, one);
+          umma_issue<false, TF32>(d_tmem, a_lo + 2u, hi, w_lo + 2u, hi, idesc, 1u, one && steps > 1);   // beyond the layer's inputs both tiles are zero
+          umma_issue<false, TF32>(d_tmem, a_lo + 4u, hi, w_lo + 4u, hi, idesc, 1u, one && steps > 2);
+          umma_issue<false, TF32>(d_tmem, a_lo + 6u, hi, w_lo + 6u, hi, idesc, 1u, one && steps > 3);
           accumulate = 1u;
           a_lo += FM_CHUNK_BYTES >> 4;
           tc_commit(w_empty0 + 8u * (uint32_t)stage, one);
@@ -398,7 +418,7 @@ mlp_fused_kernel(const __grid_constant__ FusedMaps maps, const __grid_constant__
         }
         if (!ok) break;
         tc_commit(l < L - 1 ? smem_u32(&bar_acc_full[acc]) : smem_u32(&bar_head_full[acc]), one);
-        if (l == 0) tc_commit(smem_u32(&bar_x_empty), one);     // the input tile may be refilled
+        if (l == (p.x_shared ? L - 1 : 0)) tc_commit(smem_u32(&bar_x_empty), one);     // the input tile may be refilled
       }
     }
   } else if (warp == 2) {
@@ -415,7 +435,7 @@ mlp_fused_kernel(const __grid_constant__ FusedMaps maps, const __grid_constant__
             if (!mbar_wait_warp(smem_u32(&bar_chunk[c]), (chunk_phase >> c) & 1u, abortp, SB_SITE_MLP_ACT)) { ok = false; break; }
             chunk_phase ^= 1u << c;
             if (one) {
-              tma_store_2d(&maps.act[l], act_base + (uint32_t)c * FM_CHUNK_BYTES, c * 64, tile * 128);
+              tma_store_2d(&maps.act[l], act_base + (uint32_t)c * FM_CHUNK_BYTES, c * CHUNK, tile * 128);
               bulk_commit_group();
             }
           }
@@ -423,6 +443,7 @@ mlp_fused_kernel(const __grid_constant__ FusedMaps maps, const __grid_constant__
           if (one) {
             bulk_wait_group_read<0>();
             mbar_arrive(smem_u32(&bar_act_free));
+            if (p.x_shared && l == L - 2) mbar_arrive(smem_u32(&bar_x_empty));
           }
         }
       }
@@ -488,7 +509,7 @@ mlp_fused_kernel(const __grid_constant__ FusedMaps maps, const __grid_constant__
           if (!ok) break;
           for (int l = 0; l < L - 1; ++l, ++layer) {
             const uint32_t acc = layer & 1u;
-            ok = fused_hidden<BF16, HIDDEN == FM_HIDDEN_NORM>(t_row + acc * (uint32_t)p.acc_stride, p.n_pad[l], has_bias,
+            ok = fused_hidden<CLS, HIDDEN == FM_HIDDEN_NORM>(t_row + acc * (uint32_t)p.acc_stride, p.n_pad[l], has_bias,
                      bias_smem + p.bias_pos[l], act_base, row_in_tile, half, smem_u32(&bar_chunk[0]), p.bits[l], grow,
                      p.batch, smem_u32(&bar_acc_full[acc]), (acc_phase >> acc) & 1u, act_free, act_phase, abortp);
             acc_phase ^= 1u << acc;
@@ -590,17 +611,20 @@ mlp_fused_kernel(const __grid_constant__ FusedMaps maps, const __grid_constant__
 }  // namespace
 
 // 3-D tensor map over the weights of one layer of every ensemble member: [members, rows, cols] with
-// `member_stride` elements between members, box {64 columns, box_rows, 1 member}, 128-byte swizzle.
+// `member_stride` elements between members, box {128 bytes of columns, box_rows, 1 member}, 128-byte swizzle.
 static int make_tmap_members(CUtensorMap* map, const void* base, int in_dtype, int members, long long member_stride,
                              int rows, int cols, int box_rows) {
   EncodeTiledFn enc = get_encode_tiled();
   if (!enc) return sb_fail(SB_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
-  CUtensorMapDataType dt = in_dtype == SB_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
+  CUtensorMapDataType dt = in_dtype == SB_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16
+                           : in_dtype == SB_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16
+                                                : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
+  const cuuint64_t es = (cuuint64_t)sb_dtype_size(in_dtype);
   cuuint64_t gdim[3] = {(cuuint64_t)cols, (cuuint64_t)rows, (cuuint64_t)members};
-  cuuint64_t gstride[2] = {(cuuint64_t)cols * 2u, (cuuint64_t)member_stride * 2u};
-  cuuint32_t box[3] = {64u, (cuuint32_t)box_rows, 1u};
+  cuuint64_t gstride[2] = {(cuuint64_t)cols * es, (cuuint64_t)member_stride * es};
+  cuuint32_t box[3] = {(cuuint32_t)(128u / es), (cuuint32_t)box_rows, 1u};
   cuuint32_t estr[3] = {1, 1, 1};
-  if (members == 1) gstride[1] = (cuuint64_t)rows * cols * 2u;      // unused dimension: any legal stride
+  if (members == 1) gstride[1] = (cuuint64_t)rows * cols * es;      // unused dimension: any legal stride
   gstride[1] = (gstride[1] + 15u) / 16u * 16u;
   CUresult r = enc(map, dt, 3, const_cast<void*>(base), gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                    CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -608,6 +632,22 @@ static int make_tmap_members(CUtensorMap* map, const void* base, int in_dtype, i
     return sb_fail(SB_ERR_CUDA, "cuTensorMapEncodeTiled (3-D) failed with CUresult %d (members=%d rows=%d cols=%d)",
                    (int)r, members, rows, cols);
   return SB_OK;
+}
+
+// Layer graphs that the fused kernel takes: two layers or more, a TF32 input of up to 256 columns in 16-byte rows, hidden
+// layers of multiples of 64 up to 256, outputs as for any head.  Where the input tile, the activation tile and four weight
+// stages do not fit side by side (32-bit values: from 192 columns on), the input shares the activation tile and three
+// stages do: the next tile's input then waits for this one's last layer.
+static bool fused_graph_separate(int x_chunks, int act_chunks, int max_n) {
+  return (size_t)(x_chunks + act_chunks) * FM_CHUNK_BYTES + (size_t)FM_W_STAGES * max_n * 128u + 1024 <= FM_SMEM_LIMIT;
+}
+static bool fused_graph_ok(int n_layers, const int* sizes, int prefix) {
+  if (n_layers < 2 || n_layers > FM_MAX_LAYERS || !sizes) return false;
+  if (sizes[0] < 4 || sizes[0] > 256 || sizes[0] % 4) return false;
+  for (int i = 1; i < n_layers; ++i)
+    if (sizes[i] < 64 || sizes[i] > 256 || sizes[i] % 64) return false;
+  const int n_out = sizes[n_layers];
+  return n_out >= 1 && prefix <= n_out && (n_out <= 64 || (n_out <= 256 && prefix >= 0 && prefix <= 64));
 }
 
 // What the per-decision tail writes (all null = no tail).
@@ -620,20 +660,25 @@ struct FusedDecide {
 };
 
 // Validates and launches the fused kernel.  `head`: n is set here; argmax_out / sample_out are
-// [members, batch].  `who` names the entry point in error texts.
+// [members, batch].  `who` names the entry point in error texts.  `layer_weights`: a layer graph in TF32 storage, the
+// weights of every layer on their own instead of one parameter vector (the hidden activations then go to `acts_out`).
 static int fused_launch(const char* who, int n_layers, const int* sizes, int batch, int members, int in_dtype,
                         const void* x, const void* w_compute, const float* params, SbRowHead head, int hidden_norm,
                         float* out, const FusedDecide* decide, void* stream, void* const* acts_out = nullptr,
-                        void* const* bits_out = nullptr) {
+                        void* const* bits_out = nullptr, const void* const* layer_weights = nullptr) {
+  const bool graph = layer_weights != nullptr;
   if (members < 1 || members > 1024) return sb_fail(SB_ERR_BAD_ARG, "%s: 1..1024 ensemble members", who);
   if (n_layers < 1 || n_layers > FM_MAX_LAYERS) return sb_fail(SB_ERR_UNSUPPORTED, "%s: 1..%d layers", who, FM_MAX_LAYERS);
   if (!sizes) return sb_fail(SB_ERR_BAD_ARG, "%s: sizes is null", who);
-  if (in_dtype != SB_F16 && in_dtype != SB_BF16)
-    return sb_fail(SB_ERR_UNSUPPORTED, "%s: 16-bit arithmetic classes only (SB_F16, SB_BF16)", who);
+  if (graph ? in_dtype != SB_TF32 : in_dtype != SB_F16 && in_dtype != SB_BF16)
+    return sb_fail(SB_ERR_UNSUPPORTED, graph ? "%s: TF32 storage only" : "%s: 16-bit arithmetic classes only (SB_F16, SB_BF16)", who);
   if (batch < 0) return sb_fail(SB_ERR_BAD_ARG, "%s: negative batch", who);
   if (head.flags & ~(SB_EPI_MASKED_SOFTMAX | SB_EPI_REGRET_MATCHING | SB_EPI_ARGMAX | SB_EPI_SAMPLE))
     return sb_fail(SB_ERR_BAD_ARG, "%s: the head may hold softmax, regret matching, arg-max and sampling", who);
-  if (sizes[0] < 8 || sizes[0] > 512 || sizes[0] % 8) return sb_fail(SB_ERR_UNSUPPORTED, "%s: input width %d (8..512, multiple of 8)", who, sizes[0]);
+  if (graph) {
+    if (!fused_graph_ok(n_layers, sizes, head.prefix))
+      return sb_fail(SB_ERR_UNSUPPORTED, "%s: widths that the fused graph does not take", who);
+  } else if (sizes[0] < 8 || sizes[0] > 512 || sizes[0] % 8) return sb_fail(SB_ERR_UNSUPPORTED, "%s: input width %d (8..512, multiple of 8)", who, sizes[0]);
   for (int i = 1; i < n_layers; ++i)
     if (sizes[i] < 64 || sizes[i] > 256 || sizes[i] % 64)
       return sb_fail(SB_ERR_UNSUPPORTED, "%s: hidden width %d (64..256, multiple of 64)", who, sizes[i]);
@@ -643,7 +688,7 @@ static int fused_launch(const char* who, int n_layers, const int* sizes, int bat
     return sb_fail(SB_ERR_UNSUPPORTED, "%s: output width %d (1..64, or up to 256 under a prefix mask of at most 64 columns)", who, n_out);
   if (hidden_norm && params) return sb_fail(SB_ERR_UNSUPPORTED, "%s: row-normalised hidden layers take no bias (params must be null)", who);
   if (batch == 0) return SB_OK;
-  if (!x || !w_compute || !out) return sb_fail(SB_ERR_BAD_ARG, "%s: null pointer", who);
+  if (!x || (!w_compute && !graph) || !out) return sb_fail(SB_ERR_BAD_ARG, "%s: null pointer", who);
   if ((head.flags & SB_EPI_ARGMAX) && !head.argmax_out) return sb_fail(SB_ERR_BAD_ARG, "%s: SB_EPI_ARGMAX without an actions buffer", who);
   if ((head.flags & SB_EPI_SAMPLE) && !head.sample_out) return sb_fail(SB_ERR_BAD_ARG, "%s: SB_EPI_SAMPLE without an indices buffer", who);
   if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w_compute)) & 15)
@@ -664,20 +709,23 @@ static int fused_launch(const char* who, int n_layers, const int* sizes, int bat
   p.num_items = p.num_tiles * members;
   p.member_stride = off[2 * n_layers];
   p.out_stride = (long long)batch * n_out;
+  const int es = sb_dtype_size(in_dtype), chunk = 128 / es;
   int max_n = 32;
   uint32_t max_act_chunks = 1;
   for (int l = 0; l <= n_layers; ++l) p.width[l] = sizes[l];
   for (int l = 0; l < n_layers; ++l) {
     const bool last = l == n_layers - 1;
     p.n_pad[l] = last ? (head_cols + 15) / 16 * 16 : sizes[l + 1];
-    p.k_chunks[l] = (sizes[l] + 63) / 64;
-    p.k_steps[l] = (sizes[l] + 15) / 16;
+    p.k_chunks[l] = (sizes[l] + chunk - 1) / chunk;
+    p.k_steps[l] = (sizes[l] * es + 31) / 32;
     p.idesc[l] = sb_umma_idesc(in_dtype, 0, 0, 128, p.n_pad[l]);
     p.w_bytes[l] = (uint32_t)p.n_pad[l] * 128u;
     p.bias[l] = params ? params + off[2 * l + 1] : nullptr;
     if (p.n_pad[l] > max_n) max_n = p.n_pad[l];
     if (l > 0 && (uint32_t)p.k_chunks[l] > max_act_chunks) max_act_chunks = (uint32_t)p.k_chunks[l];
-    const void* w = reinterpret_cast<const char*>(w_compute) + off[2 * l] * 2;
+    const void* w = graph ? layer_weights[l] : reinterpret_cast<const char*>(w_compute) + off[2 * l] * 2;
+    if (graph && (!w || (reinterpret_cast<uintptr_t>(w) & 15)))
+      return sb_fail(SB_ERR_MISALIGNED, "%s: weights[%d] is null or not 16-byte aligned", who, l);
     rc = make_tmap_members(&maps.w[l], w, in_dtype, members, p.member_stride, sizes[l + 1], sizes[l], p.n_pad[l]);
     if (rc != SB_OK) return rc;
   }
@@ -687,18 +735,19 @@ static int fused_launch(const char* who, int n_layers, const int* sizes, int bat
     for (int l = 0; l + 1 < n_layers; ++l) {
       if (!acts_out[l] || (reinterpret_cast<uintptr_t>(acts_out[l]) & 15))
         return sb_fail(SB_ERR_BAD_ARG, "%s: activations[%d] is null or not 16-byte aligned", who, l);
-      rc = make_tmap_2d(&maps.act[l], acts_out[l], in_dtype, batch, sizes[l + 1], 128, 64, SWZ_128);
+      rc = make_tmap_2d(&maps.act[l], acts_out[l], in_dtype, batch, sizes[l + 1], 128, chunk, SWZ_128);
       if (rc != SB_OK) return rc;
       p.bits[l] = (bits_out && bits_out[l]) ? reinterpret_cast<uint32_t*>(bits_out[l]) : nullptr;
     }
     p.store_acts = 1;
   }
   for (int l = acts_out ? (n_layers > 1 ? n_layers - 1 : 0) : 0; l < FM_MAX_LAYERS; ++l) maps.act[l] = maps.w[0];
-  rc = make_tmap_2d(&maps.x, x, in_dtype, batch, sizes[0], 128, 64, SWZ_128);
+  rc = make_tmap_2d(&maps.x, x, in_dtype, batch, sizes[0], 128, chunk, SWZ_128);
   if (rc != SB_OK) return rc;
   p.x_chunks = (uint32_t)p.k_chunks[0];
-  p.act_offset = p.x_chunks * FM_CHUNK_BYTES;
-  p.w_offset = p.act_offset + max_act_chunks * FM_CHUNK_BYTES;
+  p.x_shared = graph && !fused_graph_separate((int)p.x_chunks, (int)max_act_chunks, max_n);
+  p.act_offset = p.x_shared ? 0u : p.x_chunks * FM_CHUNK_BYTES;
+  p.w_offset = p.x_shared && p.x_chunks > max_act_chunks ? p.x_chunks * FM_CHUNK_BYTES : p.act_offset + max_act_chunks * FM_CHUNK_BYTES;
   p.acc_stride = 32;
   while (p.acc_stride < max_n) p.acc_stride <<= 1;
   p.tmem_cols = 2 * p.acc_stride;            // two accumulators (at most 2 x 256 columns)
@@ -710,7 +759,7 @@ static int fused_launch(const char* who, int n_layers, const int* sizes, int bat
   }
   p.stage_bytes = ((uint32_t)max_n * 128u + 1023u) / 1024u * 1024u;     // stages stay 1024-byte aligned (swizzle atoms)
   // Which nets are taken depends on the widths alone, not on how few columns the head of a call needs.
-  const uint32_t full_n = (uint32_t)((n_out + 15) / 16 * 16 > max_n ? (n_out + 15) / 16 * 16 : max_n);
+  const uint32_t full_n = p.x_shared ? 0u : graph ? (uint32_t)max_n : (uint32_t)((n_out + 15) / 16 * 16 > max_n ? (n_out + 15) / 16 * 16 : max_n);
   const size_t smem_needed = (size_t)p.w_offset + (size_t)FM_W_STAGES * (full_n * 128u) + 1024;
   if (smem_needed > FM_SMEM_LIMIT)
     return sb_fail(SB_ERR_UNSUPPORTED, "%s: the input tile, the widest hidden tile and the weight ring need %zu bytes of "
@@ -729,15 +778,17 @@ static int fused_launch(const char* who, int n_layers, const int* sizes, int bat
   p.bias_offset = p.w_offset + (uint32_t)p.w_stages * p.stage_bytes;
   const size_t smem = (size_t)p.bias_offset + bias_bytes + 1024;
 
-  static void (*const kernels[2][3])(FusedMaps, FusedParams) = {
-      {mlp_fused_kernel<false, FM_HIDDEN_NONE>, mlp_fused_kernel<false, FM_HIDDEN_RELU>, mlp_fused_kernel<false, FM_HIDDEN_NORM>},
-      {mlp_fused_kernel<true, FM_HIDDEN_NONE>, mlp_fused_kernel<true, FM_HIDDEN_RELU>, mlp_fused_kernel<true, FM_HIDDEN_NORM>}};
+  static void (*const kernels[3][3])(FusedMaps, FusedParams) = {
+      {mlp_fused_kernel<FM_F16, FM_HIDDEN_NONE>, mlp_fused_kernel<FM_F16, FM_HIDDEN_RELU>, mlp_fused_kernel<FM_F16, FM_HIDDEN_NORM>},
+      {mlp_fused_kernel<FM_BF16, FM_HIDDEN_NONE>, mlp_fused_kernel<FM_BF16, FM_HIDDEN_RELU>, mlp_fused_kernel<FM_BF16, FM_HIDDEN_NORM>},
+      {nullptr, mlp_fused_kernel<FM_TF32, FM_HIDDEN_RELU>, mlp_fused_kernel<FM_TF32, FM_HIDDEN_NORM>}};   // a graph has hidden layers
   static std::atomic<bool> attr_set[64];
   int dev = 0;
   SB_CUDA(cudaGetDevice(&dev));
   if (dev >= 0 && dev < 64 && !attr_set[dev].load(std::memory_order_acquire)) {
-    for (int b = 0; b < 2; ++b)
-      for (int k = 0; k < 3; ++k) SB_CUDA(cudaFuncSetAttribute(kernels[b][k], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FM_SMEM_LIMIT));
+    for (int b = 0; b < 3; ++b)
+      for (int k = 0; k < 3; ++k)
+        if (kernels[b][k]) SB_CUDA(cudaFuncSetAttribute(kernels[b][k], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FM_SMEM_LIMIT));
     attr_set[dev].store(true, std::memory_order_release);
   }
   const int sms = sb_sm_count();
@@ -746,7 +797,7 @@ static int fused_launch(const char* who, int n_layers, const int* sizes, int bat
   for (int l = 0; l < n_layers; ++l) flops += 2.0 * batch * (double)sizes[l] * sizes[l + 1] * members;
   sb_prof_before((cudaStream_t)stream);
   const int hidden = n_layers == 1 ? FM_HIDDEN_NONE : hidden_norm ? FM_HIDDEN_NORM : FM_HIDDEN_RELU;
-  SB_CUDA(sb_launch(kernels[in_dtype == SB_BF16][hidden], dim3(grid), dim3(fm_threads(hidden)), smem, (cudaStream_t)stream, 1, maps, p));
+  SB_CUDA(sb_launch(kernels[in_dtype == SB_TF32 ? FM_TF32 : in_dtype == SB_BF16 ? FM_BF16 : FM_F16][hidden], dim3(grid), dim3(fm_threads(hidden)), smem, (cudaStream_t)stream, 1, maps, p));
   sb_prof_after((cudaStream_t)stream, flops);
   SB_COUNT_LAUNCH();
   SB_CUDA(cudaGetLastError());
@@ -821,6 +872,18 @@ extern "C" int sb_policy_decide(const sb_decide_args* a, void* stream) {
   d.prob_selected = a->sampling_prob_selected; d.prob_ensemble = a->sampling_prob_ensemble;
   return fused_launch("sb_policy_decide", a->n_layers, a->sizes, (int)a->rows, a->members, a->in_dtype, a->x, a->w_compute,
                       a->params, h, a->hidden_norm, a->output_probs, &d, stream);
+}
+
+extern "C" int sb_layers_fused_supported(int n_layers, const int* sizes, int prefix) {
+  return fused_graph_ok(n_layers, sizes, prefix < 0 ? -1 : prefix) ? 1 : 0;
+}
+
+extern "C" int sb_layers_forward_fused(int n_layers, const int* sizes, int rows, const float* x, const void* const* weights,
+                                       int hidden_norm, void* const* hidden, const sb_head_spec* head, float* out, void* stream) {
+  if (!head || !weights || !hidden) return sb_fail(SB_ERR_BAD_ARG, "sb_layers_forward_fused: null pointer");
+  if (head->flags & SB_EPI_BINARIZE) return sb_fail(SB_ERR_UNSUPPORTED, "sb_layers_forward_fused: no sign hash in the fused kernel");
+  return fused_launch("sb_layers_forward_fused", n_layers, sizes, rows, 1, SB_TF32, x, nullptr, nullptr, fused_head_from_spec(head),
+                      hidden_norm, out, nullptr, stream, hidden, nullptr, weights);
 }
 
 // True when the fused kernel can run this net (the checks of fused_launch that depend on the shape only).

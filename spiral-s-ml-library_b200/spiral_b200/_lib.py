@@ -130,6 +130,8 @@ SIGNATURES = {
     "sb_mlp_fused_supported": (_I, [_I, _IP, _I]),
     "sb_mlp_forward_fused_train": (_I, [_I, _IP, _I, _I, _P, _P, _P, _PP, _PP, _I, _P, _P, _P, _P]),
     "sb_mlp_forward_fused_head": (_I, [_I, _IP, _I, _I, _I, _P, _P, _P, _I, POINTER(HeadSpec), _P, _P]),
+    "sb_layers_fused_supported": (_I, [_I, _IP, _I]),
+    "sb_layers_forward_fused": (_I, [_I, _IP, _I, _P, _PP, _I, _PP, POINTER(HeadSpec), _P, _P]),
     "sb_policy_decide": (_I, [POINTER(DecideArgs), _P]),
     "sb_mlp_forward_static": (_I, [_I, _IP, _I, _I, _P, _P, _P, _I, _P, _P, _P, _P]),
     "sb_mlp_backward_scratch_bytes": (_I, [_I, _IP, _I, _I, POINTER(c_size_t)]),

@@ -9,9 +9,10 @@ N(0, 0.1) as weight_init :460-463), ``key_extract`` (:321-325) and
 ``graph_run_host`` (:339-344).
 
 Differences by design: the reference emits one device function per node and a
-global-memory pass for every activation and head; here ``graph_run_host`` fuses
-``matmul -> relu`` and ``matmul -> head`` chains into one GEMM launch each, and
-only nodes that cannot be fused run as stand-alone kernels.  Tensors are 3-D in
+global-memory pass for every activation and head; here ``graph_run_host`` runs a
+net of plain dense layers as one launch, fuses ``matmul -> relu`` and ``matmul ->
+head`` chains into one GEMM launch each elsewhere, and only nodes that cannot be
+fused run as stand-alone kernels.  Tensors are 3-D in
 the reference (blocks, rows, features); the leading dimensions are the batch.
 """
 import ctypes
@@ -252,7 +253,8 @@ def graph_run_host(model, stream=None, ensemble=0, seed=None, row_offset=0):
     that every member's run advances (ml/models.spi:47-49); without a seed they use the uniform numbers
     the caller uploaded into ``model.uniforms(node)``.
 
-    Fusion: ``matmul [-> ln_l2] -> relu`` is one GEMM launch, and so is ``matmul -> softmax /
+    Fusion: a net of plain dense layers with a head is one launch (``_Plan._dense_net``); otherwise
+    ``matmul [-> ln_l2] -> relu`` is one GEMM launch, and so is ``matmul -> softmax /
     regret_matching [-> sample] | argmax | binarize`` (a prefix mask is an argument of the head: no mask
     matrix, no allocation, no synchronisation); everything else runs as a stand-alone kernel."""
     plan = model.plan(ensemble, seed is not None)
@@ -276,7 +278,7 @@ class _Plan:
         while i < len(nodes):
             n = nodes[i]
             if n.op == "matmul":
-                i = self._matmul(model, ensemble, draw, i)
+                i = self._dense_net(model, ensemble, draw, i) or self._matmul(model, ensemble, draw, i)
                 continue
             src, out = model.tensor(n.src), model.tensor(n)
             if n.op == "relu":
@@ -315,24 +317,12 @@ class _Plan:
                 _lib.DTYPE_CODES[out.dtype], flags, None, None, None, None)
         self.steps.append(lambda stream, seed, row_offset: _lib.call(*args, stream))
 
-    def _matmul(self, model, ensemble, draw, i):
-        """The launch that starts with the matmul node ``i``; returns the node after the last one it covers."""
-        nodes, n, j = model.nodes, model.nodes[i], i + 1
-        src, w = model.tensor(n.src), model.weight(n, ensemble)
-        # hidden layer: [ln_l2 ->] relu
-        k, epilogue = j, ()
-        if model.in_dtype == "tf32" and k + 1 < len(nodes) and nodes[k].op == "ln_l2" and nodes[k + 1].op == "relu" \
-                and n.cols % 32 == 0 and n.cols <= 256:
-            epilogue, k = ("ln_l2", "relu"), k + 2
-        elif k < len(nodes) and nodes[k].op == "relu":
-            epilogue, k = ("relu",), k + 1
-        if epilogue:
-            feeds_matmul = k < len(nodes) and nodes[k].op == "matmul"
-            self._gemm(model, src, w, model.tensor(nodes[k - 1], rounded=feeds_matmul), epilogue)
-            return k
-        # row head: softmax and regret matching fuse (in that order) when they share one prefix,
-        # then one of sample / argmax; or the sign hash by itself
-        head, size, last, k = [], None, n, j
+    @staticmethod
+    def _head(model, ensemble, draw, k, n):
+        """The row head that follows the matmul node ``n`` from node ``k`` on: softmax and regret matching fuse (in that
+        order) when they share one prefix, then one of sample / argmax; or the sign hash by itself."""
+        nodes = model.nodes
+        head, size, last = [], None, n
         while k < len(nodes) and nodes[k].op in ("softmax", "regret_matching"):
             want = "masked_softmax" if nodes[k].op == "softmax" else "regret_matching"
             if want in head or (want == "masked_softmax" and "regret_matching" in head):
@@ -355,10 +345,68 @@ class _Plan:
             head.append("binarize")
             kw = dict(hash_out=model.tensor(nodes[k]), modulo=nodes[k].attrs["modulo"])
             k += 1
+        return tuple(head), size, last, kw, drawn, k
+
+    def _dense_net(self, model, ensemble, draw, i):
+        """``matmul [-> ln_l2] -> relu -> ... -> matmul -> head`` from the matmul node ``i`` on as one launch, where the
+        fused kernel takes these widths.  Three layers with ln_l2, us with a launch per layer / as one: 64 rows of 64 columns
+        28 / 14, 8192 rows of 128 29.6 / 14.0, of 256 41.6 / 23.6, 65536 rows of 64 56 / 27, of 256 130 / 98 -- faster
+        over the whole range, so the widths alone decide.  Nets of ensemble layers keep a launch per layer: callers that
+        run member after member count on that (``launch_count``).  Returns the node after the last one covered, or None."""
+        nodes, k, hidden, norm = model.nodes, i, [], None
+        if model.in_dtype != "tf32" or nodes[i].rows < 1:
+            return None
+        while k + 2 < len(nodes) and nodes[k].op == "matmul":
+            step = 3 if nodes[k + 1].op == "ln_l2" else 2
+            if nodes[k + step - 1].op != "relu" or (norm is not None and norm != step - 2) or k + step >= len(nodes):
+                break
+            norm = step - 2
+            hidden.append((nodes[k], nodes[k + step - 1]))
+            k += step
+        if not hidden or nodes[k].op != "matmul":
+            return None
+        n = nodes[k]
+        head, size, last, kw, drawn, end = self._head(model, ensemble, draw, k + 1, n)
+        prefix = -1 if size is None else size
+        matmuls = [m for m, _ in hidden] + [n]
+        if any("members" in m.attrs for m in matmuls):
+            return None
+        widths = [nodes[i].src.cols] + [m.cols for m in matmuls]
+        sizes = (ctypes.c_int * len(widths))(*widths)
+        if not head or "binarize" in head or not _lib.load().sb_layers_fused_supported(len(matmuls), sizes, prefix):
+            return None
+        weights = (ctypes.c_void_p * len(matmuls))(*[model.weight(m, ensemble).ptr for m in matmuls])
+        outputs = (ctypes.c_void_p * len(hidden))(*[model.tensor(r).ptr for _, r in hidden])
+        args = ("sb_layers_forward_fused", len(matmuls), sizes, n.rows, model.tensor(nodes[i].src).ptr, weights, norm, outputs)
+        out = model.tensor(last).ptr
+
+        def run(stream, seed, row_offset):         # a head description of its own per run: the seed is in it
+            spec = head_spec(head, prefix=prefix, seed=int(seed) if drawn else 0, row_offset=int(row_offset) if drawn else 0, **kw)
+            _lib.call(*args, ctypes.byref(spec), out, stream)
+
+        self.steps.append(run)
+        return end
+
+    def _matmul(self, model, ensemble, draw, i):
+        """The launch that starts with the matmul node ``i``; returns the node after the last one it covers."""
+        nodes, n, j = model.nodes, model.nodes[i], i + 1
+        src, w = model.tensor(n.src), model.weight(n, ensemble)
+        # hidden layer: [ln_l2 ->] relu
+        k, epilogue = j, ()
+        if model.in_dtype == "tf32" and k + 1 < len(nodes) and nodes[k].op == "ln_l2" and nodes[k + 1].op == "relu" \
+                and n.cols % 32 == 0 and n.cols <= 256:
+            epilogue, k = ("ln_l2", "relu"), k + 2
+        elif k < len(nodes) and nodes[k].op == "relu":
+            epilogue, k = ("relu",), k + 1
+        if epilogue:
+            feeds_matmul = k < len(nodes) and nodes[k].op == "matmul"
+            self._gemm(model, src, w, model.tensor(nodes[k - 1], rounded=feeds_matmul), epilogue)
+            return k
+        head, size, last, kw, drawn, k = self._head(model, ensemble, draw, j, n)
         if not head:
             self._gemm(model, src, w, model.tensor(n))
             return j
-        out, prefix, head = model.tensor(last), -1 if size is None else size, tuple(head)
+        out, prefix = model.tensor(last), -1 if size is None else size
         m, n_cols, depth = _dims(False, True, src, w, out)
         args = ("sb_matmul_head", 0, 1, 1.0, src.ptr, w.ptr, 0.0, out.ptr, m, n_cols, depth,
                 _lib.DTYPE_CODES[model.in_dtype], 0, None)

@@ -408,6 +408,45 @@ def test_layer_graph_sampling_head(gpu):
     np.testing.assert_array_equal(L.graph_run_host(model).numpy(), np.full(512, 4, np.int32))
 
 
+@pytest.mark.parametrize("norm", [True, False])
+@pytest.mark.parametrize("widths,rows", [([4, 64, 3], 1), ([100, 128, 64, 5], 300), ([128, 128, 128, 128], 128 * 149 + 7),
+                                         ([160, 128, 128, 40], 1000), ([64] * 9, 129), ([192, 64, 256], 5000),
+                                         ([256, 256, 256, 64], 128 * 297 + 1), ([192, 192, 192], 20000), ([256, 64, 64, 7], 130),
+                                         ([8, 256, 3], 128 * 300)])
+def test_layer_graph_of_dense_layers_is_one_launch(gpu, widths, rows, norm):
+    """Hidden outputs, probabilities and sampled indices of the one launch equal those of a launch per layer."""
+    L = gpu.layers
+    h = L.input("x", (1, rows, widths[0]))
+    hidden = []
+    for a, b in zip(widths[:-2], widths[1:-1]):
+        h = L.matmul((a, b), h)
+        h = L.relu(L.ln_l2(h) if norm else h)
+        hidden.append(h)
+    sample = L.masked_softmax_and_discrete_sample(min(3, widths[-1]), L.matmul((widths[-2], widths[-1]), h))
+    model = L.create_model(sample)
+    g = so.rng(81)
+    L.key_extract(model, "x").upload(g.normal(size=(rows, widths[0])).astype(np.float32))
+    L.pass_init(model)
+    l0 = gpu.launch_count()
+    L.graph_run_host(model, seed=5, row_offset=11)
+    assert gpu.launch_count() - l0 == 1
+    got = [model.tensor(n).numpy() for n in hidden + [sample.src, sample]]
+    x = model.tensor(model.nodes[0])
+    weights = [model.weight(n) for n in model.nodes if n.op == "matmul"]
+    for n, w, have in zip(hidden, weights, got):
+        y = gpu.DeviceArray((rows, n.cols), "tf32")
+        gpu.matmul(False, True, 1.0, x, w, 0.0, y, in_dtype="tf32", epilogue=("ln_l2", "relu") if norm else ("relu",))
+        np.testing.assert_array_equal(y.numpy(), have)
+        x = y
+    probs = gpu.DeviceArray((rows, widths[-1]), "f32")
+    gpu.matmul(False, True, 1.0, x, weights[-1], 0.0, probs, in_dtype="tf32")
+    gpu.primitives.softmax(probs, probs, prefix=min(3, widths[-1]))
+    assert so.rel_frobenius(got[-2], probs.numpy()) <= 1e-6        # expf and a sum of at most three terms on either side
+    picks = gpu.DeviceArray((rows,), "i32")
+    gpu.primitives.sample_seeded(model.tensor(sample.src), picks, 5, row_offset=11)
+    np.testing.assert_array_equal(picks.numpy(), got[-1].reshape(-1))
+
+
 def test_layer_graph_binarize_head(gpu):
     L = gpu.layers
     g = L.binarize(1000003, L.matmul((32, 24), L.input("input", (1, 300, 32))))
