@@ -220,180 +220,169 @@ colsum_kernel(const DyT* __restrict__ dy, float* __restrict__ db, int rows, int 
   }
 }
 
-// dgrad of a layer with at most 16 outputs (the head): dX[r, n] = gate(r, n) * sum_k dY[r, k] * W[k, n],
-// k < KV.  With so short an inner dimension the tensor-core kernel is all epilogue (it drains a
-// 128 x 256 accumulator in 4.4 us whatever K is); here a thread keeps its 8 columns of W in
-// registers, 8 * KV fused multiply-adds make one 16-byte store, rows are taken eight at a time so
-// that the sign words of a column block (stored [N / 32, rows]) come as two 16-byte loads, and the
-// output leaves in whole rows.  Column sums of the output (the bias gradient of the layer below) are
-// kept per thread over all its rows and added once per block and column.  (A form of this kernel
-// with the multiply-adds on warp-level MMAs, m16n8k16, was built and measured: 4 us faster at
-// 32768 x 1024 with 10 outputs, 28 us slower for a 3-output head -- gating, packing, column sums
-// and stores cost the same either way and the MMA does 16 multiply-adds whatever K is.)
-constexpr int ND_THREADS = 384;
-constexpr int ND_MAX_SLOTS = ND_THREADS / 32;
-template <typename T, int KV>
-__global__ void __launch_bounds__(ND_THREADS, 1)
-narrow_dgrad_kernel(const T* __restrict__ dy, int ldy, const T* __restrict__ w, int n, const uint32_t* __restrict__ bits,
-                    T* __restrict__ dx, float* __restrict__ colsum, int rows) {
-  __shared__ float sums[1024];
-  // The dY rows of the next eight rows of every slot arrive here (cp.async) while this eight are computed.
-  __shared__ __align__(16) uint4 dy_s[2][ND_MAX_SLOTS][8][2];
+// dgrad of a layer with at most 16 outputs (the head): dX[r, n] = gate(r, n) * sum_k dY[r, k] * W[k, n].
+// With so short an inner dimension there is nothing to pipeline: one warp-level MMA (m16n8k16) has all of K for 16 rows
+// and 8 columns, and what bounds the kernel is the output it writes.  A warp keeps the W fragments of NG x 32
+// columns and goes down the rows 16 at a time, the next step's dY and sign words (stored [N / 32, rows]) on their way.
+// The columns of four MMAs are dealt so that a thread ends up with 8 neighbouring ones of a row: column c of MMA j
+// is column 8 (c / 2) + 2 j + c % 2 of the 32, a 16-byte store per row.  Column sums of the output (the bias gradient of
+// the layer below) stay in registers over all the rows of a warp and are added once.
+// The form before this one did the multiply-adds on the CUDA cores: 110 instructions for 8 outputs of 10 terms on twelve
+// warps of an SM, issue-bound at half of the slots.  Here it is some 35 on sixteen.  Training steps with it, us, before and
+// now: 32-256-3, 65536 rows 59 -> 52.7; 512-1024-10, 262144 rows 822 -> 785 (the kernel 183 -> 146), 64-1024-16, 65536 rows
+// 255 -> 189.  Rows leave in 128-byte pieces (NG = 2); with 64-byte ones 800 to 845 us, three blocks to an SM
+// with 80 registers spill (863), two steps of 16 rows at a time are the same (779).
+constexpr int ND_THREADS = 256;
+
+template <typename T>
+__device__ __forceinline__ void mma_16x8x16(float* c, const uint32_t* a, uint32_t b0, uint32_t b1);
+template <>
+__device__ __forceinline__ void mma_16x8x16<__nv_bfloat16>(float* c, const uint32_t* a, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+template <>
+__device__ __forceinline__ void mma_16x8x16<__half>(float* c, const uint32_t* a, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+template <typename T>
+__device__ __forceinline__ uint32_t pack_pair(float lo, float hi);
+template <>
+__device__ __forceinline__ uint32_t pack_pair<__nv_bfloat16>(float lo, float hi) {
+  uint32_t d;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(hi), "f"(lo));
+  return d;
+}
+template <>
+__device__ __forceinline__ uint32_t pack_pair<__half>(float lo, float hi) {
+  uint32_t d;
+  asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(hi), "f"(lo));
+  return d;
+}
+
+// dy [rows, ldy] with ldy 8 or 16 (zero beyond the real outputs), w [.., n] of which k_real rows are read, n a multiple of
+// 32 NG, bits [n / 32, rows].  A block's eight warps: col_warps side by side, the others further down the rows.
+template <typename T, int NG>
+__global__ void __launch_bounds__(ND_THREADS, 2)
+narrow_dgrad_kernel(const T* __restrict__ dy, int ldy, const T* __restrict__ w, int k_real, int n, const uint32_t* __restrict__ bits,
+                    T* __restrict__ dx, float* __restrict__ colsum, int rows, int col_warps) {
   sb_grid_dependency_wait();
   sb_grid_dependents_launch();
-  const int groups = n >> 3;                                    // 16-byte column groups of a row
-  const int tpr = groups < 128 ? ((groups + 31) & ~31) : 128;   // threads per row slot: whole warps
-  const int slots = ND_THREADS / tpr;                           // row slots of a block (3 when n >= 1024)
-  const int slot = (int)threadIdx.x / tpr, t = (int)threadIdx.x % tpr;
-  const long long stride = (long long)gridDim.x * slots * 8;
-  const int iters = (int)((rows + stride - 1) / stride);        // the same for every thread: the loop holds barriers
-  const int halves = ldy >= 16 ? 2 : 1;                         // 16-byte pieces of a dY row that are read
-  for (int cg0 = 0; cg0 < groups; cg0 += 128) {                 // n > 1024: one pass per 1024 columns
-    const int cg = cg0 + t;
-    const bool live = cg < groups && slot < slots;
-    unsigned long long wr[KV][4];            // the thread's 8 columns of W as four fp32 pairs per k
+  const int warp = (int)threadIdx.x >> 5, lane = (int)threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int row_warps = (ND_THREADS / 32) / col_warps;
+  const int group = (int)blockIdx.x * col_warps + warp % col_warps, row_warp = warp / col_warps;
+  const int col0 = group * 32 * NG;
+  if (row_warp >= row_warps || col0 >= n) return;
+  uint32_t b[NG][4][2];
 #pragma unroll
-    for (int k = 0; k < KV; ++k) {
-      uint4 raw = make_uint4(0u, 0u, 0u, 0u);
-      if (live) raw = *reinterpret_cast<const uint4*>(w + (long long)k * n + cg * 8);
-      const T* e = reinterpret_cast<const T*>(&raw);
+  for (int h = 0; h < NG; ++h)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) wr[k][j] = pack_f32x2((float)e[2 * j], (float)e[2 * j + 1]);
-    }
-    float cs[8];
+    for (int j = 0; j < 4; ++j) {
+      const int col = col0 + 32 * h + 8 * (g >> 1) + 2 * j + (g & 1);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) cs[j] = 0.f;
-    const int shift = (cg & 3) * 8;                // this thread's 8 bits inside its 32-column sign word
-    const long long first = ((long long)blockIdx.x * slots + slot) * 8;
-
-    // Thread t < 16 of a slot fetches piece (t & 1) of row (t >> 1) of the slot's eight rows.
-    auto fetch_dy = [&](int it) {
-      if (slot < slots && t < 16) {
-        const long long r = first + (long long)it * stride + (t >> 1);
-        if (r < rows && (t & 1) < halves)
-          cp_async_16(smem_u32(&dy_s[it & 1][slot][t >> 1][t & 1]), dy + r * ldy + (t & 1) * 8);
+      for (int p = 0; p < 2; ++p) {
+        const int k = 2 * t + 8 * p;
+        const uint16_t lo = k < k_real ? *reinterpret_cast<const uint16_t*>(w + (long long)k * n + col) : (uint16_t)0;
+        const uint16_t hi = k + 1 < k_real ? *reinterpret_cast<const uint16_t*>(w + (long long)(k + 1) * n + col) : (uint16_t)0;
+        b[h][j][p] = (uint32_t)lo | (uint32_t)hi << 16;
       }
-      cp_async_commit();
-    };
-    auto fetch_gate = [&](int it, uint32_t* gate) {
-      const long long r0 = first + (long long)it * stride;
-      if (!live || r0 >= rows) return;
-      if (bits) {
-        const uint32_t* g = bits + (long long)(cg >> 2) * rows + r0;
-        if (r0 + 8 <= rows && ((reinterpret_cast<uintptr_t>(g) & 15) == 0)) {
-          const uint4 a = __ldg(reinterpret_cast<const uint4*>(g)), b = __ldg(reinterpret_cast<const uint4*>(g) + 1);
-          gate[0] = a.x; gate[1] = a.y; gate[2] = a.z; gate[3] = a.w;
-          gate[4] = b.x; gate[5] = b.y; gate[6] = b.z; gate[7] = b.w;
-        } else {
+    }
+  float cs[NG][8];
 #pragma unroll
-          for (int i = 0; i < 8; ++i) gate[i] = r0 + i < rows ? __ldg(g + i) : 0u;
+  for (int h = 0; h < NG; ++h)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) cs[h][j] = 0.f;
+  const uint32_t* words = bits + (long long)(col0 >> 5) * rows;
+  // Row r of the step (g, g + 8): this thread's pieces of the dY row and the sign words of its columns.
+  auto fetch = [&](long long r0, uint32_t* a, uint32_t* gate) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const long long r = r0 + g + 8 * i;
+      const bool ok = r < rows;
+      a[i] = ok ? __ldg(reinterpret_cast<const uint32_t*>(dy + r * ldy + 2 * t)) : 0u;
+      a[2 + i] = ok && ldy > 8 ? __ldg(reinterpret_cast<const uint32_t*>(dy + r * ldy + 2 * t + 8)) : 0u;
+#pragma unroll
+      for (int h = 0; h < NG; ++h) gate[2 * h + i] = ok ? __ldg(words + (long long)h * rows + r) : 0u;
+    }
+  };
+  const long long stride = 16LL * gridDim.y * row_warps;
+  long long r0 = 16LL * ((long long)blockIdx.y * row_warps + row_warp);
+  uint32_t a[4], gate[2 * NG], a_next[4], gate_next[2 * NG];
+  fetch(r0, a, gate);
+  for (; r0 < rows; r0 += stride) {
+    fetch(r0 + stride, a_next, gate_next);
+#pragma unroll
+    for (int h = 0; h < NG; ++h) {
+      float c[4][4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        c[j][0] = c[j][1] = c[j][2] = c[j][3] = 0.f;
+        mma_16x8x16<T>(c[j], a, b[h][j][0], b[h][j][1]);
+      }
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {              // rows g and g + 8
+        const uint32_t mine = gate[2 * h + i] >> (8 * t);
+        float v[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          v[j] = (mine >> j) & 1u ? c[j >> 1][2 * i + (j & 1)] : 0.f;
+          cs[h][j] += v[j];
         }
-      } else {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) gate[i] = 0xffffffffu;
+        if (r0 + g + 8 * i < rows)
+          *reinterpret_cast<uint4*>(dx + (r0 + g + 8 * i) * n + col0 + 32 * h + 8 * t) =
+              make_uint4(pack_pair<T>(v[0], v[1]), pack_pair<T>(v[2], v[3]), pack_pair<T>(v[4], v[5]), pack_pair<T>(v[6], v[7]));
       }
-    };
-
-    uint32_t gate[8], gate_next[8];
-    fetch_dy(0);
-    fetch_gate(0, gate);
-    for (int it = 0; it < iters; ++it) {
-      cp_async_wait_all();
-      __syncthreads();                       // this iteration's dY rows are in; the other buffer is free
-      if (it + 1 < iters) {
-        fetch_dy(it + 1);
-        fetch_gate(it + 1, gate_next);
-      }
-      const long long r0 = first + (long long)it * stride;
-      if (live && r0 < rows) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const long long r = r0 + i;
-          if (r < rows) {
-            float d[KV];
-#pragma unroll
-            for (int k8 = 0; k8 < KV; k8 += 8) {
-              const uint4 raw = dy_s[it & 1][slot][i][k8 >> 3];      // the same address for the whole warp
-              const T* e = reinterpret_cast<const T*>(&raw);
-#pragma unroll
-              for (int j = 0; j < 8; ++j)
-                if (k8 + j < KV) d[k8 + j] = (float)e[j];
-            }
-            unsigned long long acc2[4] = {0ull, 0ull, 0ull, 0ull};
-#pragma unroll
-            for (int k = 0; k < KV; ++k) {
-              const unsigned long long dd = pack_f32x2(d[k], d[k]);
-#pragma unroll
-              for (int j = 0; j < 4; ++j) fma_f32x2(acc2[j], dd, wr[k][j]);
-            }
-            float acc[8];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) unpack_f32x2(acc2[j], acc[2 * j], acc[2 * j + 1]);
-            const uint32_t gb = gate[i] >> shift;
-            uint4 out;
-            T* o = reinterpret_cast<T*>(&out);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              const float v = ((gb >> j) & 1u) ? acc[j] : 0.f;
-              cs[j] += v;
-              o[j] = (T)v;
-            }
-            *reinterpret_cast<uint4*>(dx + r * n + cg * 8) = out;
-          }
-        }
-      }
-#pragma unroll
-      for (int i = 0; i < 8; ++i) gate[i] = gate_next[i];
     }
-    __syncthreads();
-    if (colsum) {
-      // One addition per block and column: the row slots fold in shared memory first.
-      for (int c = (int)threadIdx.x; c < tpr * 8; c += ND_THREADS) sums[c] = 0.f;
-      __syncthreads();
-      if (live) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) atomicAdd(&sums[t * 8 + j], cs[j]);
-      }
-      __syncthreads();
-      for (int c = (int)threadIdx.x; c < tpr * 8; c += ND_THREADS) {
-        const int col = cg0 * 8 + c;
-        const float v = sums[c];
-        if (col < n && v != 0.f) atomicAdd(colsum + col, v);
-      }
-      __syncthreads();
+    for (int i = 0; i < 4; ++i) a[i] = a_next[i];
+#pragma unroll
+    for (int i = 0; i < 2 * NG; ++i) gate[i] = gate_next[i];
+  }
+  if (!colsum) return;
+  // The eight row slots g fold together; lane (g, t) then adds column 8 t + g of each 32.
+#pragma unroll
+  for (int h = 0; h < NG; ++h) {
+    float sum = 0.f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      float v = cs[h][j];
+      v += __shfl_xor_sync(0xffffffffu, v, 4);
+      v += __shfl_xor_sync(0xffffffffu, v, 8);
+      v += __shfl_xor_sync(0xffffffffu, v, 16);
+      if (g == j) sum = v;
     }
+    atomicAdd(colsum + col0 + 32 * h + 8 * t + g, sum);
   }
 }
 
 // Whether the narrow dgrad kernel serves a layer: a 16-bit storage type, at most 16 (real) outputs,
-// rows of whole 16-byte groups.
+// whole sign words per row.
 bool narrow_dgrad_ok(int fan_out_real, int fan_in, int in_dtype) {
   static int off = -1;
   if (off < 0) {
     const char* e = getenv("SB_NARROW_DGRAD");          // SB_NARROW_DGRAD=0: the tensor-core kernel for every layer
     off = (e && e[0] == '0') ? 1 : 0;
   }
-  return !off && (in_dtype == SB_BF16 || in_dtype == SB_F16) && fan_out_real >= 1 && fan_out_real <= 16 && fan_in % 8 == 0;
+  return !off && (in_dtype == SB_BF16 || in_dtype == SB_F16) && fan_out_real >= 1 && fan_out_real <= 16 && fan_in % 32 == 0;
 }
 
 template <typename T>
 int narrow_dgrad_launch(const void* dy, int ldy, const void* w, int fan_out_real, int n, const uint32_t* bits, void* dx,
                         float* colsum, int rows, cudaStream_t s) {
-  const int groups = n / 8;
-  const int tpr = groups < 128 ? ((groups + 31) & ~31) : 128;
-  const int slots = ND_THREADS / tpr;
-  long long want = ((long long)rows + slots * 8 - 1) / (slots * 8);
-  const int grid = (int)(want < sb_sm_count() ? (want < 1 ? 1 : want) : sb_sm_count());
+  const int ng = n % 64 == 0 ? 2 : 1, groups = n / (32 * ng);
+  const int col_warps = groups < ND_THREADS / 32 ? groups : ND_THREADS / 32, row_warps = (ND_THREADS / 32) / col_warps;
+  const int strips = (groups + col_warps - 1) / col_warps;
+  // Two blocks to an SM, each with at least four steps of 16 rows to pay for its W fragments and column sums.
+  long long want = ((long long)rows + 64LL * row_warps - 1) / (64LL * row_warps);
+  long long most = (2LL * sb_sm_count() + strips - 1) / strips;
+  if (most > 65535) most = 65535;
+  const dim3 grid((unsigned)strips, (unsigned)(want < 1 ? 1 : want < most ? want : most));
   const T* dyp = reinterpret_cast<const T*>(dy);
   const T* wp = reinterpret_cast<const T*>(w);
   T* dxp = reinterpret_cast<T*>(dx);
-#define SB_ND(KV) SB_CUDA(sb_launch(narrow_dgrad_kernel<T, KV>, dim3(grid), dim3(ND_THREADS), 0, s, 1, dyp, ldy, wp, n, bits, dxp, colsum, rows))
-  if (fan_out_real <= 4) SB_ND(4);
-  else if (fan_out_real <= 8) SB_ND(8);
-  else if (fan_out_real <= 10) SB_ND(10);
-  else if (fan_out_real <= 12) SB_ND(12);
-  else SB_ND(16);
-#undef SB_ND
+  if (ng == 2) SB_CUDA(sb_launch(narrow_dgrad_kernel<T, 2>, grid, dim3(ND_THREADS), 0, s, 1, dyp, ldy, wp, fan_out_real, n, bits, dxp, colsum, rows, col_warps));
+  else SB_CUDA(sb_launch(narrow_dgrad_kernel<T, 1>, grid, dim3(ND_THREADS), 0, s, 1, dyp, ldy, wp, fan_out_real, n, bits, dxp, colsum, rows, col_warps));
   SB_COUNT_LAUNCH();
   SB_CUDA(cudaGetLastError());
   return SB_OK;

@@ -118,6 +118,14 @@ def test_backward_gradients_head_widths(gpu, in_dtype, sizes, batch):
         assert so.rel_frobenius(gb, wb) <= 5e-3, "db of layer %d" % i
 
 
+@pytest.mark.parametrize("in_dtype", ["bf16", "f16"])
+@pytest.mark.parametrize("sizes,batch", [([16, 32, 1], 5), ([16, 32, 16], 17), ([16, 64, 9], 300), ([16, 224, 10], 1003),
+                                         ([16, 1056, 3], 40), ([16, 2112, 16], 129)])
+def test_head_dgrad_on_warp_mmas_at_its_edges(gpu, in_dtype, sizes, batch):
+    """One group of 32 columns to several strips of eight warps, odd numbers of groups, fewer rows than a step of 16."""
+    test_backward_gradients_head_widths(gpu, in_dtype, sizes, batch)
+
+
 def test_train_step_updates_master_and_compute_weights(gpu):
     sizes, batch, lr = [32, 256, 256, 256, 3], 4096, 1e-3
     net, ws, bs = build(gpu, sizes, batch, "bf16", 6, training=True)
