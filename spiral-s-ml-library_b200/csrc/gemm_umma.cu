@@ -1360,7 +1360,8 @@ int cached_sm_count() { return sb_sm_count(); }
 // Chooses block_n / stages / grid for a problem; `sms` = SM count to plan for.
 // `allow_pair`: CTA pairs may be used (needs at least two 128-row blocks and a
 // tile at least 64 columns wide; row heads stay on single CTAs).
-void plan_umma(UmmaGemmParams& p, int in_dtype, int sms, bool allow_pair, bool chunks32 = false) {
+// `items_per_tile`: the split-K factor; 0: a tile has to span the row.
+void plan_umma(UmmaGemmParams& p, int in_dtype, int sms, bool allow_pair, bool chunks32 = false, int items_per_tile = 1) {
   const int es = sb_dtype_size(in_dtype);
   p.mn_box_elems = 128 / es;
   p.pair = (allow_pair && p.M > UG_BLOCK_M && p.N >= 64 && sms >= 2) ? 1 : 0;
@@ -1393,6 +1394,14 @@ void plan_umma(UmmaGemmParams& p, int in_dtype, int sms, bool allow_pair, bool c
       }
     }
   }
+  // Few tiles: narrower ones as long as the launch stays a single wave of items.  An item's time falls with its width
+  // (operand bytes, MMAs and the chunks that an epilogue warp drains one after the other), and SMs without one have
+  // nothing else to do.  us, with tiles of up to 256 columns / these: 128 x 4096 x 2048 TF32 30.0 / 14.2, 3080 x 212 x 1062
+  // TF32 18.6 / 12.4, 324 x 216 x 3936 fp16 28.1 / 21.0, 682 x 856 x 540 TF32 13.1 / 10.1, 512^3 in the fp32 class 12.5 / 11.3,
+  // 2048 x 1024 x 1024 with bias, ReLU and sign words 11.0 / 9.2; of 58 shapes none slower.
+  if (allow_pair && items_per_tile > 0)
+    for (int bn = 192; bn >= (p.pair ? 64 : 32); bn -= bn > 64 ? 64 : 32)
+      if (bn % gran == 0 && bn < best_bn && (long long)p.tiles_m * ((p.N + bn - 1) / bn) * items_per_tile <= workers) best_bn = bn;
   // Pipeline bytes.  The three products of the fp32 class keep both parts of a K range in one stage and need two
   // stages: on a single CTA a tile is no wider than what a reserve leaves room for (without one 256 columns fit).
   const int budget = UG_SMEM_LIMIT - 2048 - UG_EPI_STAGING - g_gemm_smem_reserve.load(std::memory_order_relaxed);
@@ -1517,7 +1526,8 @@ int sb_umma_gemm_launch(int a_trans, int b_trans, float alpha, const void* A, co
   // Whole 32-column chunks per tile where every chunk must leave as a box: sign words, column sums, and
   // tiles that are added to C (split-K accumulation, peer copies).
   plan_umma(p, in_dtype, cached_sm_count(), !(epi & EPI_HEAD_MASK) && sb_pair_mode_enabled(),
-            (epi & (EPI_GATE_MASK | SB_EPI_COLSUM_OUT)) != 0 || (split_partials && splits > 1) || to_peers);
+            (epi & (EPI_GATE_MASK | SB_EPI_COLSUM_OUT)) != 0 || (split_partials && splits > 1) || to_peers,
+            (epi & SB_EPI_LN_L2) ? 0 : splits > 1 ? splits : 1);
   p.N = N;
   p.alpha = alpha; p.beta = beta;
   p.C = C; p.ldc = N; p.out_dtype = out_dtype;

@@ -63,6 +63,21 @@ def test_ragged_4000x3000x1000(gpu, at, bt, in_dtype):
     assert so.rel_frobenius(got, so.matmul(at, bt, 1.0, a, b, 0.0, None)) <= TIGHT
 
 
+@pytest.mark.parametrize("in_dtype,out_dtype", [("bf16", "f32"), ("f16", "f16"), ("tf32", "f32")])
+@pytest.mark.parametrize("at,bt", LAYOUTS[:3])
+@pytest.mark.parametrize("m,n", [(104, 3000), (128, 8968), (304, 520), (704, 2480), (1000, 3400)])
+def test_narrow_tiles_of_a_single_wave(gpu, at, bt, m, n, in_dtype, out_dtype):
+    """Few tiles: 32 to 192 columns wide, single CTAs and pairs, with ragged edges, bias and ReLU."""
+    k = 264
+    a, b, c = operands(63, at, bt, m, n, k, in_dtype)
+    bias = so.rng(64).normal(size=n).astype(np.float32)
+    plan = gpu.matmul_plan(at, bt, m, n, k, in_dtype)
+    assert (plan["block_n"] < 256 or n == 3400) and plan["grid"] <= gpu.sm_count()     # 192 columns are no whole boxes of a 16-bit MN-major B
+    got = run(gpu, at, bt, 1.0, a, b, 0.0, c, in_dtype, out_dtype, epilogue=("bias", "relu"), bias=gpu.DeviceArray.from_numpy(bias))
+    want = so.relu(so.matmul(at, bt, 1.0, a, b, 0.0, None) + bias)
+    assert so.rel_frobenius(got, want) <= (TIGHT if out_dtype == "f32" else TOL)
+
+
 @pytest.mark.parametrize("in_dtype,out_dtype", [("bf16", "f32"), ("f16", "bf16"), ("tf32", "f32")])
 @pytest.mark.parametrize("at,bt", LAYOUTS[:3])
 def test_last_wave_of_half_width_tiles(gpu, at, bt, in_dtype, out_dtype):
