@@ -695,9 +695,7 @@ __device__ __forceinline__ uint32_t wide_prepare(float* v, float bias_lane, uint
 // box while this pair is computed.  One store (one proxy fence) serves the pair.
 //
 // `held` (modes with column sums, a single column tile): the sums of this warp's four chunks over all its tiles, for one
-// reduction per kernel instead of one per tile.  A 65536 x 256 dgrad sends 16384 reductions to eight 128-byte lines:
-// 28.1 us, 20.7 without any, 24.7 held back; the Leduc training step 191 -> 187.5 us.  With one tile per worker it
-// costs more than it saves (11.9 -> 13.6 us for 18944 rows): p.hold_colsum says where the line lies.
+// reduction per CTA and column at the end of the kernel instead of one per warp and tile.
 template <typename OutT, int MODE>
 __device__ __noinline__ bool epilogue_tile_wide(uint32_t t_row, int row0_warp, int n0, int block_n, int split,
                                                 uint32_t bar_full, uint32_t parity, float4* held) {
@@ -1237,12 +1235,29 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
       acc ^= 1;
       if (acc == 0) acc_phase ^= 1u;
     }
-    if (held) {
-      const int col0 = 64 * half;
-      add_colsum(held_sums.x, col0, lane);
-      add_colsum(held_sums.y, col0 + 32, lane);
-      add_colsum(held_sums.z, col0 + 128, lane);
-      add_colsum(held_sums.w, col0 + 160, lane);
+    if (EW == 8 && held) {
+      // The four warps of a half add up in the staging boxes first: one reduction per CTA and column.  (One per warp sent
+      // 592 to each of 256 addresses at the end of the launch, 4 us.  K = N = 256, 1 / 2 / 3 / 12 tiles per worker: added per
+      // tile 12.3 / 18.8 / 25.1 / 86.6 us, held per warp 13.6 / 17.7 / 22.1 / 63.2, this 10.8 / 14.6 / 19.1 / 62.0.)  Every epilogue warp comes here, also after
+      // an expired wait.
+      if (lane == 0) bulk_wait_group_read<0>();
+      __syncwarp();
+      const uint32_t mine = g_epi.box_base + (uint32_t)(warp - 2) * 4096u + 4u * (uint32_t)lane;
+      const float part[4] = {held_sums.x, held_sums.y, held_sums.z, held_sums.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) asm volatile("st.shared.f32 [%0], %1;" ::"r"(mine + 128u * (uint32_t)i), "f"(part[i]) : "memory");
+      asm volatile("bar.sync 1, 256;" ::: "memory");
+      // Column c is in chunk slot 2 (c / 128) + c / 32 % 2 of half c / 64 % 2.
+      const uint32_t c = (uint32_t)(warp - 2) * 32u + (uint32_t)lane;
+      const uint32_t at = g_epi.box_base + ((c >> 6) & 1u) * 16384u + (((c >> 7) & 1u) * 2u + ((c >> 5) & 1u)) * 128u + 4u * (c & 31u);
+      float sum = 0.f;
+#pragma unroll
+      for (uint32_t q = 0; q < 4; ++q) {
+        float v;
+        asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(at + 4096u * q) : "memory");
+        sum += v;
+      }
+      add_colsum(sum, (int)(c & ~31u), lane);
     }
   }
 
@@ -1639,12 +1654,8 @@ int sb_umma_gemm_launch(int a_trans, int b_trans, float alpha, const void* A, co
     }
   }
   // One column tile, all of whose items are whole tiles or the 128-column halves of a 256-column one.  (The right half of
-  // a 128-column tile gives columns 64 and 96 to the warps that hold 0 and 32 of a whole one.)  And enough tiles per
-  // worker: adding at the end costs 4 us (in local memory, and nothing left to hide it) and saves 2.4 (256 columns) or
-  // 1.4 (128) a tile.
-  const int sum_workers = p.pair ? cached_sm_count() / 2 : cached_sm_count();
-  p.hold_colsum = p.wide && p.tiles_n == 1 && (p.tail_first == p.num_work || p.block_n == 256) &&
-                  2LL * p.num_tiles > (p.block_n >= 192 ? 3LL : 4LL) * sum_workers ? 1 : 0;
+  // a 128-column tile gives columns 64 and 96 to the warps that hold 0 and 32 of a whole one.)
+  p.hold_colsum = p.wide && p.tiles_n == 1 && (p.tail_first == p.num_work || p.block_n == 256) ? 1 : 0;
   if (p.reduce_add && !p.tma_store)
     return sb_fail(SB_ERR_UNSUPPORTED, "internal: split-K accumulation was chosen for a C that cannot take TMA stores");
   const size_t smem = umma_dyn_smem(p);
