@@ -6,7 +6,7 @@
 #include "common.cuh"
 #include "row_head.cuh"
 
-int sb_umma_plan(int a_trans, int b_trans, int M, int N, int K, int in_dtype, int sms, int* plan5);
+int sb_umma_plan(int a_trans, int b_trans, int M, int N, int K, int in_dtype, int epi, int sms, int* plan5);
 int sb_scale_launch(void* C, long long total, float beta, int out_dtype, cudaStream_t stream);
 int sb_sgemm_launch(int a_trans, int b_trans, float alpha, const float* A, const float* B, float beta,
                     float* C, int M, int N, int K, int epi, const float* bias, cudaStream_t stream);
@@ -341,12 +341,12 @@ int sb_matmul_tf32(int a_trans, int b_trans, float alpha, const float* A, const 
 
 int sb_matmul_plan(int a_trans, int b_trans, int M, int N, int K, int in_dtype, int epilogue,
                    int* plan5) {
-  (void)epilogue;
   if (!plan5) return sb_fail(SB_ERR_BAD_ARG, "sb_matmul_plan: null output");
   if (M <= 0 || N <= 0 || K <= 0) return sb_fail(SB_ERR_BAD_ARG, "sb_matmul_plan: dimensions must be positive");
   if (in_dtype != SB_TF32 && in_dtype != SB_BF16 && in_dtype != SB_F16)
     return sb_fail(SB_ERR_BAD_ARG, "sb_matmul_plan: tensor-core input classes only");
-  return sb_umma_plan(a_trans, b_trans, M, N, K, in_dtype, sb_sm_count(), plan5);
+  if (!sb_umma_head_fits(N, -1)) epilogue &= ~SPEC_HEAD_FLAGS;      // such a head is a kernel of its own behind the product
+  return sb_umma_plan(a_trans, b_trans, M, N, K, in_dtype, epilogue, sb_sm_count(), plan5);
 }
 
 }  // extern "C"

@@ -1475,6 +1475,14 @@ void plan_umma(UmmaGemmParams& p, int in_dtype, int sms, bool allow_pair, bool c
   p.idesc = sb_umma_idesc(in_dtype, p.a_mn, p.b_mn, tile_m, p.block_n);
 }
 
+// The plan of a launch with epilogue `epi`, of which there are `splits` items per tile.  `boxes`: its tiles are added to C
+// (split-K accumulation, peer copies), so that every 32-column chunk has to leave as a box, as with sign words and
+// column sums.
+void plan_for_epilogue(UmmaGemmParams& p, int in_dtype, int sms, int epi, int splits, bool boxes) {
+  plan_umma(p, in_dtype, sms, !(epi & EPI_HEAD_MASK) && sb_pair_mode_enabled(),
+            (epi & (EPI_GATE_MASK | SB_EPI_COLSUM_OUT)) != 0 || boxes, (epi & SB_EPI_LN_L2) ? 0 : splits > 1 ? splits : 1);
+}
+
 size_t umma_dyn_smem(const UmmaGemmParams& p) {
   return (size_t)p.stages * (p.a_stage_bytes + p.b_stage_bytes) + UG_EPI_STAGING + 1024;
 }
@@ -1538,11 +1546,7 @@ int sb_umma_gemm_launch(int a_trans, int b_trans, float alpha, const void* A, co
     // Columns that the head turns into zeros are not multiplied: the tile spans those that it holds in registers.
     p.N = sb_row_head_columns(p.head) < N ? sb_row_head_columns(p.head) : N;
   }
-  // Whole 32-column chunks per tile where every chunk must leave as a box: sign words, column sums, and
-  // tiles that are added to C (split-K accumulation, peer copies).
-  plan_umma(p, in_dtype, cached_sm_count(), !(epi & EPI_HEAD_MASK) && sb_pair_mode_enabled(),
-            (epi & (EPI_GATE_MASK | SB_EPI_COLSUM_OUT)) != 0 || (split_partials && splits > 1) || to_peers,
-            (epi & SB_EPI_LN_L2) ? 0 : splits > 1 ? splits : 1);
+  plan_for_epilogue(p, in_dtype, cached_sm_count(), epi, splits, (split_partials && splits > 1) || to_peers);
   p.N = N;
   p.alpha = alpha; p.beta = beta;
   p.C = C; p.ldc = N; p.out_dtype = out_dtype;
@@ -1694,13 +1698,13 @@ extern "C" int sb_gemm_reserve_smem(int bytes) {
   return SB_OK;
 }
 
-int sb_umma_plan(int a_trans, int b_trans, int M, int N, int K, int in_dtype, int sms, int* plan5) {
+int sb_umma_plan(int a_trans, int b_trans, int M, int N, int K, int in_dtype, int epi, int sms, int* plan5) {
   UmmaGemmParams p;
   memset(&p, 0, sizeof(p));
   p.M = M; p.N = N; p.K = K;
   p.a_mn = a_trans ? 1 : 0;
   p.b_mn = b_trans ? 0 : 1;
-  plan_umma(p, in_dtype, sms, sb_pair_mode_enabled());
+  plan_for_epilogue(p, in_dtype, sms, epi, 1, false);
   plan5[0] = p.pair ? 2 * UG_BLOCK_M : UG_BLOCK_M;
   plan5[1] = p.block_n;
   plan5[2] = p.block_k;

@@ -143,13 +143,17 @@ def matmul_tf32(a_trans, b_trans, alpha, a, b, beta, c, stream=None):
     return c
 
 
-def matmul_plan(a_trans, b_trans, m, n, k, in_dtype="tf32"):
-    """Tile plan of the tensor-core path: dict(block_m, block_n, block_k, stages, grid).
+def matmul_plan(a_trans, b_trans, m, n, k, in_dtype="tf32", epilogue=()):
+    """Tile plan of the tensor-core path for a product with ``epilogue`` (names as for ``matmul``):
+    dict(block_m, block_n, block_k, stages, grid).
 
     Counterpart of matmul_config_tf32 (ml/matmul/run.spi:8-19); unlike it, no
     divisibility of m, n, k by the tile is demanded (ragged edges are zero-filled).
     """
     plan = (ctypes.c_int * 5)()
+    epi = 0
+    for name in epilogue:
+        epi |= EPILOGUE_FLAGS[name]
     _lib.call("sb_matmul_plan", int(bool(a_trans)), int(bool(b_trans)), int(m), int(n), int(k),
-              _lib.DTYPE_CODES[in_dtype], 0, plan)
+              _lib.DTYPE_CODES[in_dtype], epi, plan)
     return dict(zip(("block_m", "block_n", "block_k", "stages", "grid"), list(plan)))

@@ -44,6 +44,19 @@ def test_plan_needs_no_device(sb):
     assert small["block_n"] == 16 and small["grid"] == 128 and small["block_m"] == 128
 
 
+@pytest.mark.parametrize("epilogue,m,n,k,in_dtype,want", [
+    (("ln_l2", "relu"), 512, 256, 128, "tf32", (256, 256, 4)),              # the tile spans the row, however few there are
+    (("ln_l2",), 300, 256, 128, "bf16", (256, 256, 4)),
+    (("masked_softmax", "argmax"), 512, 64, 128, "bf16", (128, 64, 4)),     # a row head: single CTAs, whole rows
+    (("regret_matching",), 512, 256, 128, "bf16", (256, 64, 16)),           # a head beyond 64 columns runs behind a plain product
+    (("bias", "relu"), 512, 256, 128, "bf16", (256, 64, 16)),
+    (("bias", "relu", "relu_mask_out"), 128, 96, 128, "bf16", (128, 32, 3)),
+    ((), 512, 256, 128, "tf32", (256, 64, 16))])
+def test_plan_is_that_of_the_launch_with_its_epilogue(sb, epilogue, m, n, k, in_dtype, want):
+    plan = sb.matmul_plan(False, True, m, n, k, in_dtype, epilogue=epilogue)
+    assert (plan["block_m"], plan["block_n"], plan["grid"]) == want
+
+
 def test_bad_arguments_are_rejected_before_any_launch(sb):
     from spiral_b200 import _lib
     with pytest.raises(sb.SpiralError) as e:
