@@ -1659,7 +1659,13 @@ int sb_umma_gemm_launch(int a_trans, int b_trans, float alpha, const void* A, co
   }
   // One column tile, all of whose items are whole tiles or the 128-column halves of a 256-column one.  (The right half of
   // a 128-column tile gives columns 64 and 96 to the warps that hold 0 and 32 of a whole one.)
-  p.hold_colsum = p.wide && p.tiles_n == 1 && (p.tail_first == p.num_work || p.block_n == 256) ? 1 : 0;
+  // The meeting at the end takes 0.3 us: a warp with a single tile of at most 128 columns adds its one or two chunks at
+  // once.  us, gated, K = 256, added per tile / held: 4736 rows of 64 columns 5.9 / 6.3, of 128 6.5 / 6.75, of 256 6.8 / 6.7; 14208
+  // rows (three tiles for four workers) 7.15 / 7.0, 7.45 / 7.6, 10.2 / 9.4; 18944 (one each) 7.6 / 7.5, 8.1 / 8.1, 11.1 / 10.0, and with
+  // K = 1024 9.5 / 9.8, 10.0 / 10.3, 15.1 / 14.0; 23680 9.9 / 9.5, 11.1 / 10.3, 13.7 / 11.9.
+  const int sum_workers = p.pair ? cached_sm_count() / 2 : cached_sm_count();
+  p.hold_colsum = p.wide && p.tiles_n == 1 && (p.tail_first == p.num_work || p.block_n == 256) &&
+                  (p.block_n > 128 || p.num_tiles > sum_workers) ? 1 : 0;
   if (p.reduce_add && !p.tma_store)
     return sb_fail(SB_ERR_UNSUPPORTED, "internal: split-K accumulation was chosen for a C that cannot take TMA stores");
   const size_t smem = umma_dyn_smem(p);

@@ -281,6 +281,15 @@ def test_column_sums_over_many_tiles(gpu, n, k, in_dtype, bt, waves, tiles, rows
         np.testing.assert_allclose(sums.numpy(), want, rtol=rtol)
 
 
+@pytest.mark.parametrize("n", [32, 64, 128, 192])
+@pytest.mark.parametrize("bt", [False, True])
+@pytest.mark.parametrize("waves,tiles,rows", [(0, 2, -200), (0, 37, 3), (1, 0, 0), (2, 0, 0), (2, 0, 1)])
+def test_column_sums_up_to_one_tile_per_worker(gpu, n, bt, waves, tiles, rows):
+    """The line between sums added per tile and sums held over the launch: at most one tile per worker (CTA pair, single CTA
+    with 32 columns), and one more."""
+    test_column_sums_over_many_tiles(gpu, n, 128, "bf16", bt, waves, tiles, rows)
+
+
 def test_column_sums_rejects_unsupported_combinations(gpu):
     a, b, c = operands(44, False, True, 64, 64, 64, "bf16")
     sums = gpu.DeviceArray.zeros((64,), "f32")
