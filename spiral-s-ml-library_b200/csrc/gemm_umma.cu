@@ -1413,10 +1413,26 @@ void plan_umma(UmmaGemmParams& p, int in_dtype, int sms, bool allow_pair, bool c
   // (operand bytes, MMAs and the chunks that an epilogue warp drains one after the other), and SMs without one have
   // nothing else to do.  us, with tiles of up to 256 columns / these: 128 x 4096 x 2048 TF32 30.0 / 14.2, 3080 x 212 x 1062
   // TF32 18.6 / 12.4, 324 x 216 x 3936 fp16 28.1 / 21.0, 682 x 856 x 540 TF32 13.1 / 10.1, 512^3 in the fp32 class 12.5 / 11.3,
-  // 2048 x 1024 x 1024 with bias, ReLU and sign words 11.0 / 9.2; of 58 shapes none slower.
-  if (allow_pair && items_per_tile > 0)
-    for (int bn = 192; bn >= (p.pair ? 64 : 32); bn -= bn > 64 ? 64 : 32)
-      if (bn % gran == 0 && bn < best_bn && (long long)p.tiles_m * ((p.N + bn - 1) / bn) * items_per_tile <= workers) best_bn = bn;
+  // 2048 x 1024 x 1024 with bias, ReLU and sign words 11.0 / 9.2.
+  // Not where the whole tiles have little to give and the narrow ones read A again for a busy chip: tiles of 64, 96 or 128
+  // columns stay whole from three (128: four) tenths of the workers on.  us, whole / narrow: 9472 x 96 x 1024 bf16 with bias,
+  // ReLU and sign words 6.95 / 8.07, 9472 x 128 x 1024 gated with column sums 8.4 / 9.0, TF32 10.6 / 10.9; 6144 x 96 x 1024 7.2 / 8.0 -- but
+  // 4608 x 128 x 1024 8.1 / 7.4 (18 tiles), 9472 x 256 x 1024 12.2 / 10.2, a tile of 48 columns always (6144 x 48 x 256 bf16 4.6 / 3.4).
+  // And with less than 1 KB of K not where more than a quarter of the columns would be padding, if that fills more than half of the
+  // workers or every chunk has to be a whole box: 9472 x 160 x 256 bf16 with sign words 6.4 / 6.9.
+  if (allow_pair && items_per_tile > 0) {
+    const int whole_n = best_bn, whole_tiles = (p.N + best_bn - 1) / best_bn;
+    const long long whole_items = (long long)p.tiles_m * whole_tiles * items_per_tile;
+    const bool boxes = whole_n % 32 == 0;        // of whole 32-column chunks; a tail of 16 columns is slower than what follows
+    const bool stay = boxes && whole_n <= 128 && 10 * whole_items >= (whole_n == 128 ? 4LL : 3LL) * workers;
+    for (int bn = 192; !stay && bn >= (p.pair ? 64 : 32); bn -= bn > 64 ? 64 : 32) {
+      const int tiles_n = (p.N + bn - 1) / bn;
+      const long long items = (long long)p.tiles_m * tiles_n * items_per_tile;
+      const bool padded = boxes && 4LL * tiles_n * bn > 5LL * whole_tiles * whole_n && (long long)p.K * es < 1024 &&
+                          (chunks32 || 2 * items > workers);
+      if (bn % gran == 0 && bn < best_bn && items <= workers && !padded) best_bn = bn;
+    }
+  }
   // Pipeline bytes.  The three products of the fp32 class keep both parts of a K range in one stage and need two
   // stages: on a single CTA a tile is no wider than what a reserve leaves room for (without one 256 columns fit).
   const int budget = UG_SMEM_LIMIT - 2048 - UG_EPI_STAGING - g_gemm_smem_reserve.load(std::memory_order_relaxed);
@@ -1478,9 +1494,11 @@ void plan_umma(UmmaGemmParams& p, int in_dtype, int sms, bool allow_pair, bool c
 // The plan of a launch with epilogue `epi`, of which there are `splits` items per tile.  `boxes`: its tiles are added to C
 // (split-K accumulation, peer copies), so that every 32-column chunk has to leave as a box, as with sign words and
 // column sums.
-void plan_for_epilogue(UmmaGemmParams& p, int in_dtype, int sms, int epi, int splits, bool boxes) {
+void plan_for_epilogue(UmmaGemmParams& p, int in_dtype, int sms, int epi, float beta, int splits, bool boxes) {
+  // A C of less than 64 columns that is read, too, keeps one tile: 468 x 56 x 64 with beta = 1, bf16 6.1 us, 7.0 with two.
+  const bool whole = (epi & SB_EPI_LN_L2) || (beta != 0.0f && p.N < 64);
   plan_umma(p, in_dtype, sms, !(epi & EPI_HEAD_MASK) && sb_pair_mode_enabled(),
-            (epi & (EPI_GATE_MASK | SB_EPI_COLSUM_OUT)) != 0 || boxes, (epi & SB_EPI_LN_L2) ? 0 : splits > 1 ? splits : 1);
+            (epi & (EPI_GATE_MASK | SB_EPI_COLSUM_OUT)) != 0 || boxes, whole ? 0 : splits > 1 ? splits : 1);
 }
 
 size_t umma_dyn_smem(const UmmaGemmParams& p) {
@@ -1546,7 +1564,7 @@ int sb_umma_gemm_launch(int a_trans, int b_trans, float alpha, const void* A, co
     // Columns that the head turns into zeros are not multiplied: the tile spans those that it holds in registers.
     p.N = sb_row_head_columns(p.head) < N ? sb_row_head_columns(p.head) : N;
   }
-  plan_for_epilogue(p, in_dtype, cached_sm_count(), epi, splits, (split_partials && splits > 1) || to_peers);
+  plan_for_epilogue(p, in_dtype, cached_sm_count(), epi, beta, splits, (split_partials && splits > 1) || to_peers);
   p.N = N;
   p.alpha = alpha; p.beta = beta;
   p.C = C; p.ldc = N; p.out_dtype = out_dtype;
@@ -1710,7 +1728,7 @@ int sb_umma_plan(int a_trans, int b_trans, int M, int N, int K, int in_dtype, in
   p.M = M; p.N = N; p.K = K;
   p.a_mn = a_trans ? 1 : 0;
   p.b_mn = b_trans ? 0 : 1;
-  plan_for_epilogue(p, in_dtype, sms, epi, 1, false);
+  plan_for_epilogue(p, in_dtype, sms, epi, 0.0f, 1, false);
   plan5[0] = p.pair ? 2 * UG_BLOCK_M : UG_BLOCK_M;
   plan5[1] = p.block_n;
   plan5[2] = p.block_k;

@@ -57,6 +57,16 @@ def test_plan_is_that_of_the_launch_with_its_epilogue(sb, epilogue, m, n, k, in_
     assert (plan["block_m"], plan["block_n"], plan["grid"]) == want
 
 
+@pytest.mark.parametrize("in_dtype,m,n,k,block_n", [
+    ("bf16", 9472, 96, 1024, 96), ("bf16", 9472, 128, 1024, 128), ("tf32", 6144, 96, 1024, 96), ("bf16", 6400, 64, 64, 64),
+    ("bf16", 7424, 128, 1024, 64), ("bf16", 7680, 128, 1024, 128),        # 29 and 30 of 74 pairs
+    ("bf16", 5632, 96, 1024, 64), ("bf16", 5888, 96, 1024, 96),           # 22 and 23
+    ("bf16", 9472, 256, 1024, 128), ("bf16", 9472, 160, 256, 160), ("bf16", 9472, 192, 1024, 128), ("bf16", 1280, 160, 256, 64),
+    ("bf16", 6144, 48, 256, 32), ("bf16", 18944, 256, 1024, 256)])
+def test_tiles_that_occupy_the_chip_stay_whole(sb, in_dtype, m, n, k, block_n):
+    assert sb.matmul_plan(False, True, m, n, k, in_dtype)["block_n"] == block_n
+
+
 def test_bad_arguments_are_rejected_before_any_launch(sb):
     from spiral_b200 import _lib
     with pytest.raises(sb.SpiralError) as e:
