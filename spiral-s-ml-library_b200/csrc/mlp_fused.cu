@@ -451,7 +451,8 @@ mlp_fused_kernel(const __grid_constant__ FusedMaps maps, const __grid_constant__
     }
   } else if (warp == 3) {
     // Biases: a member's go to shared memory as a whole, once for a single net, and per item (two buffers that take turns)
-    // for an ensemble.
+    // for an ensemble.  All copies of an item are on their way at once, since a first tile waits for them: through registers,
+    // one layer's round trip after the other, a single tile of 64-128-128-3 took 6.56 us, this way 5.35 (5.1 without biases).
     if (p.bias_bytes) {
       int n = 0;
       for (int item = blockIdx.x; item < p.num_items; item += gridDim.x, ++n) {
@@ -463,12 +464,9 @@ mlp_fused_kernel(const __grid_constant__ FusedMaps maps, const __grid_constant__
           const float* src = p.bias[l] + pofs;
           const uint32_t dst = bias_base + buf * p.bias_bytes + p.bias_pos[l];
           const int live = p.width[l + 1], n_pad = l < L - 1 ? live : FM_HEAD_BIAS;
-#pragma unroll 8
-          for (int j = lane; j < n_pad; j += 32) {
-            const float b = j < live ? __ldg(src + j) : 0.f;
-            asm volatile("st.shared.f32 [%0], %1;" ::"r"(dst + 4u * (uint32_t)j), "f"(b) : "memory");
-          }
+          for (int j = lane; j < n_pad; j += 32) cp_async_4(dst + 4u * (uint32_t)j, j < live ? src + j : src, j < live);
         }
+        cp_async_wait_all();
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&bar_bias_full[buf]));
       }

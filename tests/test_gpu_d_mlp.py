@@ -249,6 +249,13 @@ def test_fused_forward_over_many_tiles_per_cta(gpu, sizes, with_bias):
     assert so.rel_frobenius(got[rows], want) <= TOL
 
 
+@pytest.mark.parametrize("sizes", [[16] + [256] * 7 + [5], [512, 128, 128, 3], [320, 192, 3], [64, 64, 64, 64, 64]])
+def test_fused_forward_with_the_biases_of_deep_and_wide_nets(gpu, sizes):
+    """Up to 59 bias values per lane, all asked for at once; with biases the weight ring of the second and third net has
+    three stages."""
+    test_fused_forward_over_many_tiles_per_cta(gpu, sizes, True)
+
+
 def test_fused_forward_other_shapes_and_limits(gpu):
     from spiral_b200 import SpiralError
     sizes, batch = [64, 128, 64, 10], 777
