@@ -19,6 +19,7 @@
 #include "common.cuh"
 
 #include <mutex>
+#include <type_traits>
 
 namespace {
 
@@ -221,31 +222,66 @@ colsum_kernel(const DyT* __restrict__ dy, float* __restrict__ db, int rows, int 
 }
 
 // dgrad of a layer with at most 16 outputs (the head): dX[r, n] = gate(r, n) * sum_k dY[r, k] * W[k, n].
-// With so short an inner dimension there is nothing to pipeline: one warp-level MMA (m16n8k16) has all of K for 16 rows
+// With so short an inner dimension there is nothing to pipeline: warp-level MMAs have all of K for 16 rows
 // and 8 columns, and what bounds the kernel is the output it writes.  A warp keeps the W fragments of NG x 32
 // columns and goes down the rows 16 at a time, the next step's dY and sign words (stored [N / 32, rows]) on their way.
 // The columns of four MMAs are dealt so that a thread ends up with 8 neighbouring ones of a row: column c of MMA j
 // is column 8 (c / 2) + 2 j + c % 2 of the 32, a 16-byte store per row.  Column sums of the output (the bias gradient of
-// the layer below) stay in registers over all the rows of a warp and are added once.
+// the layer below) stay in registers over all the rows of a warp, fold over the row warps of a block and are added once.
 // The form before this one did the multiply-adds on the CUDA cores: 110 instructions for 8 outputs of 10 terms on twelve
-// warps of an SM, issue-bound at half of the slots.  Here it is some 35 on sixteen.  Training steps with it, us, before and
-// now: 32-256-3, 65536 rows 59 -> 52.7; 512-1024-10, 262144 rows 822 -> 785 (the kernel 183 -> 146), 64-1024-16, 65536 rows
-// 255 -> 189.  Rows leave in 128-byte pieces (NG = 2); with 64-byte ones 800 to 845 us, three blocks to an SM
-// with 80 registers spill (863), two steps of 16 rows at a time are the same (779).
-constexpr int ND_THREADS = 256;
+// warps of an SM, issue-bound at half of the slots.  Here it is some 35 on sixteen.  ce_grad, the head's wgrad and this, us, then
+// and now: 32 columns, 3 outputs, 65536 rows 24.8 / 18.4; 64 columns 22.7 / 16.3; 256 columns 26.9 / 22.9, 2048 rows 15.1 / 10.9; 1024
+// columns, 10 outputs, 65536 rows 92.6 / 74.4.  Rows leave in 128-byte pieces (NG = 2): with 64-byte ones 15 % more (fp16 with more than
+// 8 outputs, whose fragments take twice the registers, has them: 512 columns, 10 outputs, 262144 rows 174 / 169); three blocks to
+// an SM with 80 registers spill, two steps of 16 rows at a time are the same.
 
-template <typename T>
-__device__ __forceinline__ void mma_16x8x16(float* c, const uint32_t* a, uint32_t b0, uint32_t b1);
-template <>
-__device__ __forceinline__ void mma_16x8x16<__nv_bfloat16>(float* c, const uint32_t* a, uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-template <>
-__device__ __forceinline__ void mma_16x8x16<__half>(float* c, const uint32_t* a, uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
+// The products of 16 rows and 8 columns.  KP: registers that hold a thread's part of W per MMA.  bf16: one m16n8k16 on the
+// values as they are.  fp16: its subnormals (gradients of a large batch) would be summed with the exponent of the smallest
+// normal value, bits of the sum below it lost; as TF32 every fp16 value is a normal one, exactly.  One m16n8k8 has eight k's,
+// slot t the even and slot t + 4 the odd one of a thread's pair.
+template <typename T, int KP>
+struct NarrowMma;
+template <int KP>
+struct NarrowMma<__nv_bfloat16, KP> {
+  static_assert(KP == 2, "all of K in one product");
+  uint32_t a[4];
+  __device__ __forceinline__ void load(const uint32_t* words) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) a[i] = words[i];
+  }
+  __device__ __forceinline__ static void weights(uint32_t* b, const uint32_t* words) { b[0] = words[0]; b[1] = words[1]; }
+  __device__ __forceinline__ void run(float* c, const uint32_t* b) const {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+  }
+};
+template <int KP>
+struct NarrowMma<__half, KP> {
+  static_assert(KP == 2 || KP == 4, "eight or sixteen k's");
+  uint32_t a[2 * KP];
+  __device__ __forceinline__ static void unpack(uint32_t word, uint32_t& even, uint32_t& odd) {
+    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&word));
+    even = __float_as_uint(f.x);
+    odd = __float_as_uint(f.y);
+  }
+  __device__ __forceinline__ void load(const uint32_t* words) {
+#pragma unroll
+    for (int p = 0; p < KP / 2; ++p)
+#pragma unroll
+      for (int i = 0; i < 2; ++i) unpack(words[2 * p + i], a[4 * p + i], a[4 * p + 2 + i]);
+  }
+  __device__ __forceinline__ static void weights(uint32_t* b, const uint32_t* words) {
+#pragma unroll
+    for (int p = 0; p < KP / 2; ++p) unpack(words[p], b[2 * p], b[2 * p + 1]);
+  }
+  __device__ __forceinline__ void run(float* c, const uint32_t* b) const {
+#pragma unroll
+    for (int p = 0; p < KP / 2; ++p)
+      asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                   : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                   : "r"(a[4 * p]), "r"(a[4 * p + 1]), "r"(a[4 * p + 2]), "r"(a[4 * p + 3]), "r"(b[2 * p]), "r"(b[2 * p + 1]));
+  }
+};
 template <typename T>
 __device__ __forceinline__ uint32_t pack_pair(float lo, float hi);
 template <>
@@ -262,31 +298,35 @@ __device__ __forceinline__ uint32_t pack_pair<__half>(float lo, float hi) {
 }
 
 // dy [rows, ldy] with ldy 8 or 16 (zero beyond the real outputs), w [.., n] of which k_real rows are read, n a multiple of
-// 32 NG, bits [n / 32, rows].  A block's eight warps: col_warps side by side, the others further down the rows.
-template <typename T, int NG>
-__global__ void __launch_bounds__(ND_THREADS, 2)
+// 32 NG, bits [n / 32, rows].  A block's warps: col_warps side by side, the others further down the rows.  FOLD: a single strip
+// of blocks, which add once per column; otherwise every row warp does.
+template <typename T, int NG, int KP, int THREADS, bool FOLD>
+__global__ void __launch_bounds__(THREADS, 512 / THREADS)
 narrow_dgrad_kernel(const T* __restrict__ dy, int ldy, const T* __restrict__ w, int k_real, int n, const uint32_t* __restrict__ bits,
                     T* __restrict__ dx, float* __restrict__ colsum, int rows, int col_warps) {
   sb_grid_dependency_wait();
   sb_grid_dependents_launch();
   const int warp = (int)threadIdx.x >> 5, lane = (int)threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  const int row_warps = (ND_THREADS / 32) / col_warps;
+  const int row_warps = (THREADS / 32) / col_warps;
   const int group = (int)blockIdx.x * col_warps + warp % col_warps, row_warp = warp / col_warps;
   const int col0 = group * 32 * NG;
-  if (row_warp >= row_warps || col0 >= n) return;
-  uint32_t b[NG][4][2];
+  const bool active = row_warp < row_warps && col0 < n;
+  if (!FOLD && !active) return;
+  uint32_t b[NG][4][KP];
 #pragma unroll
   for (int h = 0; h < NG; ++h)
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const int col = col0 + 32 * h + 8 * (g >> 1) + 2 * j + (g & 1);
+      uint32_t words[2];
 #pragma unroll
       for (int p = 0; p < 2; ++p) {
         const int k = 2 * t + 8 * p;
         const uint16_t lo = k < k_real ? *reinterpret_cast<const uint16_t*>(w + (long long)k * n + col) : (uint16_t)0;
         const uint16_t hi = k + 1 < k_real ? *reinterpret_cast<const uint16_t*>(w + (long long)(k + 1) * n + col) : (uint16_t)0;
-        b[h][j][p] = (uint32_t)lo | (uint32_t)hi << 16;
+        words[p] = (uint32_t)lo | (uint32_t)hi << 16;
       }
+      NarrowMma<T, KP>::weights(b[h][j], words);
     }
   float cs[NG][8];
 #pragma unroll
@@ -309,16 +349,19 @@ narrow_dgrad_kernel(const T* __restrict__ dy, int ldy, const T* __restrict__ w, 
   const long long stride = 16LL * gridDim.y * row_warps;
   long long r0 = 16LL * ((long long)blockIdx.y * row_warps + row_warp);
   uint32_t a[4], gate[2 * NG], a_next[4], gate_next[2 * NG];
+  if (FOLD && !active) r0 = rows;
   fetch(r0, a, gate);
   for (; r0 < rows; r0 += stride) {
     fetch(r0 + stride, a_next, gate_next);
+    NarrowMma<T, KP> mma;
+    mma.load(a);
 #pragma unroll
     for (int h = 0; h < NG; ++h) {
       float c[4][4];
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         c[j][0] = c[j][1] = c[j][2] = c[j][3] = 0.f;
-        mma_16x8x16<T>(c[j], a, b[h][j][0], b[h][j][1]);
+        mma.run(c[j], b[h][j]);
       }
 #pragma unroll
       for (int i = 0; i < 2; ++i) {              // rows g and g + 8
@@ -340,7 +383,9 @@ narrow_dgrad_kernel(const T* __restrict__ dy, int ldy, const T* __restrict__ w, 
     for (int i = 0; i < 2 * NG; ++i) gate[i] = gate_next[i];
   }
   if (!colsum) return;
-  // The eight row slots g fold together; lane (g, t) then adds column 8 t + g of each 32.
+  // The eight row slots g fold together; lane (g, t) then has column 8 t + g of each 32.  The row warps of a block add up
+  // before they add to memory.
+  __shared__ float part[FOLD ? THREADS / 32 : 1][32 * NG];
 #pragma unroll
   for (int h = 0; h < NG; ++h) {
     float sum = 0.f;
@@ -352,7 +397,16 @@ narrow_dgrad_kernel(const T* __restrict__ dy, int ldy, const T* __restrict__ w, 
       v += __shfl_xor_sync(0xffffffffu, v, 16);
       if (g == j) sum = v;
     }
-    atomicAdd(colsum + col0 + 32 * h + 8 * t + g, sum);
+    if (!FOLD) atomicAdd(colsum + col0 + 32 * h + 8 * t + g, sum);
+    else part[warp][32 * h + 8 * t + g] = sum;
+  }
+  if (!FOLD) return;
+  __syncthreads();
+  for (int c = (int)threadIdx.x; c < n; c += THREADS) {
+    float sum = 0.f;
+#pragma unroll 4
+    for (int w = c / (32 * NG); w < row_warps * col_warps; w += col_warps) sum += part[w][c % (32 * NG)];
+    atomicAdd(colsum + c, sum);
   }
 }
 
@@ -370,19 +424,38 @@ bool narrow_dgrad_ok(int fan_out_real, int fan_in, int in_dtype) {
 template <typename T>
 int narrow_dgrad_launch(const void* dy, int ldy, const void* w, int fan_out_real, int n, const uint32_t* bits, void* dx,
                         float* colsum, int rows, cudaStream_t s) {
-  const int ng = n % 64 == 0 ? 2 : 1, groups = n / (32 * ng);
-  const int col_warps = groups < ND_THREADS / 32 ? groups : ND_THREADS / 32, row_warps = (ND_THREADS / 32) / col_warps;
+  constexpr bool HALF = std::is_same<T, __half>::value;
+  const bool long_k = HALF && fan_out_real > 8;
+  const int ng = n % 64 == 0 && !long_k ? 2 : 1, groups = n / (32 * ng);
+  // A column gets an addition to memory per row warp (`direct`), or one per block of sixteen warps.  Up to 512 columns a row
+  // warp is one of two to sixteen of its block: their additions at the end of a launch, up to 2368 to an address, cost up to 4 us
+  // (64 columns, 65536 rows: 20.5, folded 16.3) and the accuracy of the sum (relative error 5.0e-7, folded 1.6e-7; 262144 rows
+  // 6.8e-7 and 1.7e-7).  Wider ones have a row warp per block, 148 additions at most.  Few rows are done sooner without the
+  // meeting: 64 rows of 256 columns 8.3 / 9.0, 256 rows of 32 10.4 / 12.1, but 1024 of 256 10.7 / 10.6, 4096 of 256 11.6 / 11.1.
+  const bool direct = groups > 8 || rows <= 512;
+  const int threads = direct ? 256 : 512, warps = threads / 32;
+  const int col_warps = groups < 8 ? groups : 8, row_warps = warps / col_warps;
   const int strips = (groups + col_warps - 1) / col_warps;
-  // Two blocks to an SM, each with at least four steps of 16 rows to pay for its W fragments and column sums.
-  long long want = ((long long)rows + 64LL * row_warps - 1) / (64LL * row_warps);
-  long long most = (2LL * sb_sm_count() + strips - 1) / strips;
+  const int least = direct ? 64 : 16;             // rows of a warp, to pay for its W fragments and its additions
+  long long want = ((long long)rows + (long long)least * row_warps - 1) / ((long long)least * row_warps);
+  long long most = ((direct ? 2LL : 1LL) * sb_sm_count() + strips - 1) / strips;
   if (most > 65535) most = 65535;
   const dim3 grid((unsigned)strips, (unsigned)(want < 1 ? 1 : want < most ? want : most));
   const T* dyp = reinterpret_cast<const T*>(dy);
   const T* wp = reinterpret_cast<const T*>(w);
   T* dxp = reinterpret_cast<T*>(dx);
-  if (ng == 2) SB_CUDA(sb_launch(narrow_dgrad_kernel<T, 2>, grid, dim3(ND_THREADS), 0, s, 1, dyp, ldy, wp, fan_out_real, n, bits, dxp, colsum, rows, col_warps));
-  else SB_CUDA(sb_launch(narrow_dgrad_kernel<T, 1>, grid, dim3(ND_THREADS), 0, s, 1, dyp, ldy, wp, fan_out_real, n, bits, dxp, colsum, rows, col_warps));
+#define SB_ND_LAUNCH(NG, KP, THREADS, FOLD) \
+  SB_CUDA(sb_launch(narrow_dgrad_kernel<T, NG, KP, THREADS, FOLD>, grid, dim3(THREADS), 0, s, 1, dyp, ldy, wp, fan_out_real, n, bits, dxp, colsum, rows, col_warps))
+#define SB_ND_BY_FOLD(NG, KP)                       \
+  do {                                              \
+    if (direct) SB_ND_LAUNCH(NG, KP, 256, false);   \
+    else SB_ND_LAUNCH(NG, KP, 512, true);           \
+  } while (0)
+  if (long_k) SB_ND_BY_FOLD(1, HALF ? 4 : 2);
+  else if (ng == 2) SB_ND_BY_FOLD(2, 2);
+  else SB_ND_BY_FOLD(1, 2);
+#undef SB_ND_BY_FOLD
+#undef SB_ND_LAUNCH
   SB_COUNT_LAUNCH();
   SB_CUDA(cudaGetLastError());
   return SB_OK;
@@ -853,7 +926,7 @@ static int backward_impl(int n_layers, const int* sizes, int batch, float inv_gl
       const bool sum_cols = bits && with_bias;
       float* db_below = grads + off[2 * (i - 1) + 1];
       if (bits && narrow_dgrad_ok(sizes[i + 1], fan_in, in_dtype) && st == in_dtype) {
-        // A head layer: the inner dimension is at most 16, nothing for the tensor cores to do.
+        // A head layer: the inner dimension is at most 16, a single warp-level product.
         const uint32_t* gate = reinterpret_cast<const uint32_t*>(relu_bits[i - 1]);
         rc = in_dtype == SB_BF16
                  ? narrow_dgrad_launch<__nv_bfloat16>(dy_cur, fan_out, w, sizes[i + 1], fan_in, gate, dy_next, sum_cols ? db_below : nullptr, batch, s)

@@ -126,6 +126,35 @@ def test_head_dgrad_on_warp_mmas_at_its_edges(gpu, in_dtype, sizes, batch):
     test_backward_gradients_head_widths(gpu, in_dtype, sizes, batch)
 
 
+@pytest.mark.parametrize("in_dtype", ["bf16", "f16"])
+@pytest.mark.parametrize("sizes,batch", [([16, 32, 8], 512), ([16, 512, 9], 513), ([16, 256, 8], 513), ([16, 288, 16], 700), ([16, 576, 2], 530),
+                                         ([16, 32, 3], 128 * 149 + 7)])
+def test_head_dgrad_sums_per_row_warp_and_per_block(gpu, in_dtype, sizes, batch):
+    """Both sides of the lines between one addition per row warp and one per block: 512 rows, eight column warps."""
+    test_backward_gradients_head_widths(gpu, in_dtype, sizes, batch)
+
+
+@pytest.mark.parametrize("in_dtype,sizes,batch", [("bf16", [32, 64, 3], 262144), ("bf16", [32, 256, 3], 65536), ("f16", [64, 64, 16], 262144),
+                                                  ("f16", [64, 64, 7], 65536), ("bf16", [64, 64, 16], 2048)])
+def test_head_dgrad_bias_gradients_against_float64(gpu, in_dtype, sizes, batch):
+    """Column sums of the head dgrad against the same sums in float64.  A column's sum is at most one addition to memory
+    per SM, each off by half a last place of the sum or less, to either side: sqrt(additions) * 2^-25.  The fp16 case
+    has dY in the subnormal range, as a large batch has without a loss scale."""
+    g = so.rng(17)
+    net, ws, _ = build(gpu, sizes, batch, in_dtype, 18, training=True)
+    mask = gpu.DeviceArray.from_numpy(np.ones((batch, sizes[-1]), np.uint8))
+    target = g.random((batch, sizes[-1]), dtype=np.float32)
+    dx = gpu.to_storage(g.random((batch, sizes[0]), dtype=np.float32), in_dtype)
+    net.forward(dx, mask, head_flags=8)
+    net.backward(dx, mask, gpu.DeviceArray.from_numpy(target / target.sum(1, keepdims=True)))
+    got = net.split_flat(net.grads.numpy())[0][1]
+    dy = net.layer_dy(1).numpy().astype(np.float64)[:, :sizes[-1]]
+    words = net.relu_bits[0].numpy().view(np.uint32).reshape(sizes[1] // 32, batch)
+    gate = ((words.T[:, :, None] >> np.arange(32, dtype=np.uint32)) & 1).reshape(batch, sizes[1]).astype(bool)
+    want = np.where(gate, dy @ so.round_input(ws[1], in_dtype).astype(np.float64), 0).sum(axis=0)
+    assert so.rel_frobenius(got, want) <= gpu.sm_count() ** 0.5 * 2.0 ** -25
+
+
 def test_train_step_updates_master_and_compute_weights(gpu):
     sizes, batch, lr = [32, 256, 256, 256, 3], 4096, 1e-3
     net, ws, bs = build(gpu, sizes, batch, "bf16", 6, training=True)
