@@ -166,6 +166,18 @@ def test_fp32_class_stays_inside_the_workspace_that_it_asks_for(gpu, m, n, k, sh
 
 
 @pytest.mark.parametrize("at,bt", [(False, True), (False, False), (True, False)])
+@pytest.mark.parametrize("m,n,k,beta", [(100, 56, 64, 1.0), (468, 56, 144, 1.0), (468, 56, 144, 0.0), (64, 1000, 300, 0.5), (300, 256, 1000, 0.0),
+                                        (1000, 520, 160, -0.5)])
+def test_fp32_class_on_narrow_tiles(gpu, at, bt, m, n, k, beta):
+    """Few tiles in the fp32 class: narrow ones with one chain of K or several, and a C of less than 64 columns that is
+    read, which keeps one tile."""
+    a, b, c = _operands(80 + m + n, at, bt, m, n, k, "normal")
+    dc = gpu.DeviceArray.from_numpy(c)
+    gpu.matmul(at, bt, 1.0, gpu.DeviceArray.from_numpy(a), gpu.DeviceArray.from_numpy(b), beta, dc, in_dtype="f32")
+    assert so.rel_frobenius(dc.numpy(), so.matmul(at, bt, 1.0, a, b, beta, c)) <= TOL_F32
+
+
+@pytest.mark.parametrize("at,bt", [(False, True), (False, False), (True, False)])
 @pytest.mark.parametrize("m,n,k", [(100, 252, 300), (128, 256, 64), (64, 1000, 512), (300, 256, 300)])
 def test_fp32_class_beside_a_shared_memory_reserve(gpu, at, bt, m, n, k):
     """Two stages of a single CTA's 256-column tile take all of the pipeline's memory: with 64 KB reserved its tiles are

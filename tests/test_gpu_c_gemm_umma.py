@@ -65,17 +65,61 @@ def test_ragged_4000x3000x1000(gpu, at, bt, in_dtype):
 
 @pytest.mark.parametrize("in_dtype,out_dtype", [("bf16", "f32"), ("f16", "f16"), ("tf32", "f32")])
 @pytest.mark.parametrize("at,bt", LAYOUTS[:3])
-@pytest.mark.parametrize("m,n", [(104, 3000), (128, 8968), (304, 520), (704, 2480), (1000, 3400)])
-def test_narrow_tiles_of_a_single_wave(gpu, at, bt, m, n, in_dtype, out_dtype):
-    """Few tiles: 32 to 192 columns wide, single CTAs and pairs, with ragged edges, bias and ReLU."""
+@pytest.mark.parametrize("m,n,width,width_of_boxes", [(104, 3000, 32, 64), (128, 8968, 64, 64), (304, 520, 64, 128), (704, 2480, 128, 128),
+                                                      (1000, 3400, 192, 256)])
+def test_narrow_tiles_of_a_single_wave(gpu, at, bt, m, n, width, width_of_boxes, in_dtype, out_dtype):
+    """Few tiles: 32 to 192 columns wide, single CTAs and pairs, with ragged edges, bias and ReLU.  The narrowest width at which
+    the tiles fit into one wave of 148 SMs; a 16-bit MN-major B comes in boxes of 64 columns per CTA."""
     k = 264
     a, b, c = operands(63, at, bt, m, n, k, in_dtype)
     bias = so.rng(64).normal(size=n).astype(np.float32)
     plan = gpu.matmul_plan(at, bt, m, n, k, in_dtype)
-    assert (plan["block_n"] < 256 or n == 3400) and plan["grid"] <= gpu.sm_count()     # 192 columns are no whole boxes of a 16-bit MN-major B
+    assert plan["grid"] <= gpu.sm_count()
+    if gpu.sm_count() == 148:
+        assert plan["block_n"] == (width_of_boxes if in_dtype != "tf32" and not bt else width)
     got = run(gpu, at, bt, 1.0, a, b, 0.0, c, in_dtype, out_dtype, epilogue=("bias", "relu"), bias=gpu.DeviceArray.from_numpy(bias))
     want = so.relu(so.matmul(at, bt, 1.0, a, b, 0.0, None) + bias)
     assert so.rel_frobenius(got, want) <= (TIGHT if out_dtype == "f32" else TOL)
+
+
+@pytest.mark.parametrize("bt", [False, True])
+@pytest.mark.parametrize("m,n", [(100, 32), (128, 352), (300, 96), (300, 512), (2000, 192), (4608, 128), (9472, 96), (9472, 160)])
+def test_narrow_tiles_with_sign_words_and_column_sums(gpu, bt, m, n):
+    """Tiles of one wave whose chunks have to leave as whole boxes: sign words out, and a gated product with column
+    sums, narrowed or kept whole; both against the plain product of the same operands."""
+    k = 128
+    a, b, c = operands(65 + m, False, bt, m, n, k, "bf16")
+    bits = gpu.DeviceArray.zeros((n // 32, m), "i32")
+    got = run(gpu, False, bt, 1.0, a, b, 0.0, c, "bf16", out_dtype="bf16", epilogue=("relu", "relu_mask_out"), aux_out=bits)
+    prod = so.matmul(False, bt, 1.0, a, b, 0.0, None)
+    assert so.rel_frobenius(got, so.round_bf16(so.relu(prod))) <= 3e-3
+    np.testing.assert_array_equal(bits_to_bool(bits.numpy(), m, n), got > 0)
+    gate = so.rng(66).integers(0, 2 ** 32, size=(n // 32, m), dtype=np.uint64).astype(np.uint32)
+    sums = gpu.DeviceArray.zeros((n,), "f32")
+    got = run(gpu, False, bt, 1.0, a, b, 0.0, c, "bf16", out_dtype="bf16", epilogue=("relu_grad_mask", "colsum_out"),
+              aux_in=gpu.DeviceArray.from_numpy(gate.view(np.int32), "i32"), aux_out=sums)
+    want = np.where(bits_to_bool(gate, m, n), prod, 0)
+    assert so.rel_frobenius(got, so.round_bf16(want.astype(np.float32))) <= 3e-3
+    np.testing.assert_allclose(sums.numpy(), want.sum(axis=0, dtype=np.float64), rtol=0, atol=2e-4 * np.sqrt(m * k))
+
+
+@pytest.mark.parametrize("out,fan_in,batch", [(64, 96, 700), (200, 72, 1500), (256, 520, 1200), (520, 264, 900)])
+def test_narrow_tiles_added_to_a_weight_gradient(gpu, out, fan_in, batch):
+    """Split-K weight gradients of a small batch, whose narrow tiles are added to the output as boxes: a backward pass
+    of one layer against the oracle."""
+    g = so.rng(67)
+    net = gpu.PolicyMLP([fan_in, out], batch, in_dtype="bf16", training=True)
+    ws, bs = so.mlp_weights(68, [fan_in, out])
+    net.load_weights(ws, bs)
+    x = g.random((batch, fan_in), dtype=np.float32)
+    mask = np.ones((batch, out), np.uint8)
+    target = so.random_target(69, mask)
+    dx, dm = gpu.to_storage(x, "bf16"), gpu.DeviceArray.from_numpy(mask)
+    net.forward(dx, dm, head_flags=8)
+    net.backward(dx, dm, gpu.DeviceArray.from_numpy(target))
+    got = net.split_flat(net.grads.numpy())
+    _, _, _, want = so.mlp_train_step(x, [so.round_input(w, "bf16") for w in ws], bs, mask, target, 0.0, in_dtype="bf16", act_dtype="bf16")
+    assert so.rel_frobenius(got[0][0], want[0][0]) <= TOL
 
 
 @pytest.mark.parametrize("in_dtype,out_dtype", [("bf16", "f32"), ("f16", "bf16"), ("tf32", "f32")])

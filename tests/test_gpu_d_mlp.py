@@ -89,16 +89,16 @@ def test_backward_gradients(gpu, in_dtype, sizes, batch):
 
 
 @pytest.mark.parametrize("in_dtype,sizes,batch", [
-    ("bf16", [64, 1088, 7], 1001),       # 1088 columns: two passes of the head dgrad; odd batch: unaligned sign words
-    ("f16", [64, 96, 12], 777),          # 12 outputs, a row of three warps' worth of 16-byte groups
-    ("bf16", [32, 160, 16], 520),        # 16 outputs: the widest head the CUDA-core dgrad takes
+    ("bf16", [64, 1088, 7], 1001),       # 1088 columns: strips of blocks; odd batch: unaligned sign words
+    ("f16", [64, 96, 12], 777),          # 12 outputs: two products of eight k's; an odd number of 32-column groups
+    ("bf16", [32, 160, 16], 520),        # 16 outputs: the widest head that the warp-level dgrad takes
     ("bf16", [32, 128, 8], 4096),
     ("bf16", [32, 128, 256, 3], 65536),  # and the tensor-core dgrad of a layer with 128 inputs over more tiles than workers
     ("bf16", [64, 96, 256, 10], 65536),
 ])
 def test_backward_gradients_head_widths(gpu, in_dtype, sizes, batch):
-    """The dgrad of a head with at most 16 outputs runs on the CUDA cores (one instance per width class,
-    sign words read 8 rows at a time, column sums per block): gradients against the oracle for the
+    """The dgrad of a head with at most 16 outputs runs on warp-level MMAs (32 or 64 columns to a warp, rows 16 at a
+    time, column sums per row warp or per block): gradients against the oracle for the
     widths, row lengths and batch sizes that take its different paths."""
     net, ws, bs = build(gpu, sizes, batch, in_dtype, 14, training=True, bias_scale=0.05)
     g = so.rng(15)
