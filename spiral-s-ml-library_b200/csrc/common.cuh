@@ -277,11 +277,6 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst_smem, const CUtensorMap
       ::"r"(dst_smem), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(x), "r"(y), "r"(bar), "r"((uint32_t)issue)
       : "memory");
 }
-// Four bytes from global to shared memory without passing through registers (cp.async); zeros where `real` is false.
-__device__ __forceinline__ void cp_async_4(uint32_t dst_smem, const void* src, bool real) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst_smem), "l"(src), "r"(real ? 4u : 0u) : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 // The same as tma_load_2d for a 3-D tensor (x innermost).
 __device__ __forceinline__ void tma_load_3d(uint32_t dst_smem, const CUtensorMap* tmap, int x, int y, int z,
                                             uint32_t bar, bool issue) {

@@ -280,8 +280,8 @@ def test_fused_forward_over_many_tiles_per_cta(gpu, sizes, with_bias):
 
 @pytest.mark.parametrize("sizes", [[16] + [256] * 7 + [5], [512, 128, 128, 3], [320, 192, 3], [64, 64, 64, 64, 64]])
 def test_fused_forward_with_the_biases_of_deep_and_wide_nets(gpu, sizes):
-    """Up to 59 bias values per lane, all asked for at once; with biases the weight ring of the second and third net has
-    three stages."""
+    """Odd and even numbers of layers, up to 59 bias values per lane; with biases the weight ring of the second and third
+    net has three stages."""
     test_fused_forward_over_many_tiles_per_cta(gpu, sizes, True)
 
 
