@@ -1375,8 +1375,9 @@ int cached_sm_count() { return sb_sm_count(); }
 // Chooses block_n / stages / grid for a problem; `sms` = SM count to plan for.
 // `allow_pair`: CTA pairs may be used (needs at least two 128-row blocks and a
 // tile at least 64 columns wide; row heads stay on single CTAs).
-// `items_per_tile`: the split-K factor; 0: a tile has to span the row.
-void plan_umma(UmmaGemmParams& p, int in_dtype, int sms, bool allow_pair, bool chunks32 = false, int items_per_tile = 1) {
+// `chunks32`: whole 32-column chunks per tile.  `items_per_tile`: the split-K factor; 0: a tile has to span the row.
+// `sums`: with column sums.
+void plan_umma(UmmaGemmParams& p, int in_dtype, int sms, bool allow_pair, bool chunks32, int items_per_tile, bool sums) {
   const int es = sb_dtype_size(in_dtype);
   p.mn_box_elems = 128 / es;
   p.pair = (allow_pair && p.M > UG_BLOCK_M && p.N >= 64 && sms >= 2) ? 1 : 0;
@@ -1419,7 +1420,8 @@ void plan_umma(UmmaGemmParams& p, int in_dtype, int sms, bool allow_pair, bool c
   // ReLU and sign words 6.95 / 8.07, 9472 x 128 x 1024 gated with column sums 8.4 / 9.0, TF32 10.6 / 10.9; 6144 x 96 x 1024 7.2 / 8.0 -- but
   // 4608 x 128 x 1024 8.1 / 7.4 (18 tiles), 9472 x 256 x 1024 12.2 / 10.2, a tile of 48 columns always (6144 x 48 x 256 bf16 4.6 / 3.4).
   // And with less than 1 KB of K not where more than a quarter of the columns would be padding, if that fills more than half of the
-  // workers or every chunk has to be a whole box: 9472 x 160 x 256 bf16 with sign words 6.4 / 6.9.
+  // workers (9472 x 160 x 256 bf16 with sign words 6.4 / 6.9) or there are column sums, whose wide epilogue wants 64 columns (3072 x
+  // 96 x 256 5.75 / 6.0; with sign words 5.5 / 5.25).
   if (allow_pair && items_per_tile > 0) {
     const int whole_n = best_bn, whole_tiles = (p.N + best_bn - 1) / best_bn;
     const long long whole_items = (long long)p.tiles_m * whole_tiles * items_per_tile;
@@ -1429,7 +1431,7 @@ void plan_umma(UmmaGemmParams& p, int in_dtype, int sms, bool allow_pair, bool c
       const int tiles_n = (p.N + bn - 1) / bn;
       const long long items = (long long)p.tiles_m * tiles_n * items_per_tile;
       const bool padded = boxes && 4LL * tiles_n * bn > 5LL * whole_tiles * whole_n && (long long)p.K * es < 1024 &&
-                          (chunks32 || 2 * items > workers);
+                          (sums || 2 * items > workers);
       if (bn % gran == 0 && bn < best_bn && items <= workers && !padded) best_bn = bn;
     }
   }
@@ -1498,7 +1500,7 @@ void plan_for_epilogue(UmmaGemmParams& p, int in_dtype, int sms, int epi, float 
   // A C of less than 64 columns that is read, too, keeps one tile: 468 x 56 x 64 with beta = 1, bf16 6.1 us, 7.0 with two.
   const bool whole = (epi & SB_EPI_LN_L2) || (beta != 0.0f && p.N < 64);
   plan_umma(p, in_dtype, sms, !(epi & EPI_HEAD_MASK) && sb_pair_mode_enabled(),
-            (epi & (EPI_GATE_MASK | SB_EPI_COLSUM_OUT)) != 0 || boxes, whole ? 0 : splits > 1 ? splits : 1);
+            (epi & (EPI_GATE_MASK | SB_EPI_COLSUM_OUT)) != 0 || boxes, whole ? 0 : splits > 1 ? splits : 1, (epi & SB_EPI_COLSUM_OUT) != 0);
 }
 
 size_t umma_dyn_smem(const UmmaGemmParams& p) {

@@ -67,6 +67,11 @@ def test_tiles_that_occupy_the_chip_stay_whole(sb, in_dtype, m, n, k, block_n):
     assert sb.matmul_plan(False, True, m, n, k, in_dtype)["block_n"] == block_n
 
 
+def test_padded_narrow_tiles_with_column_sums(sb):
+    for epilogue, block_n in ((("relu", "relu_mask_out"), 64), (("relu_grad_mask",), 64), (("relu_grad_mask", "colsum_out"), 96)):
+        assert sb.matmul_plan(False, True, 3072, 96, 256, "bf16", epilogue=epilogue)["block_n"] == block_n
+
+
 def test_bad_arguments_are_rejected_before_any_launch(sb):
     from spiral_b200 import _lib
     with pytest.raises(sb.SpiralError) as e:
