@@ -778,8 +778,9 @@ static int fused_launch(const char* who, int n_layers, const int* sizes, int bat
   if (smem_needed > FM_SMEM_LIMIT)
     return sb_fail(SB_ERR_UNSUPPORTED, "%s: the input tile, the widest hidden tile and the weight ring need %zu bytes of "
                                        "shared memory (inputs wider than 256 fit with hidden layers of at most 128)", who, smem_needed);
-  // The ring takes what is left beside the biases: more than the four stages of the rule above for narrow
-  // layers, three for the widest nets with biases (65 to 128 inputs and 256-wide layers, or the full 227 KB otherwise).
+  // The ring takes what is left beside the biases: more than the four stages of the rule above for narrow layers; three
+  // where tiles and four stages fill the limit to the byte and biases come on top (65 to 128 inputs with 256-wide layers, 257 to 320
+  // with 192, 449 to 512 with 128), and at least three where a graph's input shares the activation tile.
   if (params) {
     for (int l = 0; l < n_layers; ++l) {
       p.bias_pos[l] = p.bias_bytes;

@@ -351,8 +351,9 @@ class _Plan:
         """``matmul [-> ln_l2] -> relu -> ... -> matmul -> head`` from the matmul node ``i`` on as one launch, where the
         fused kernel takes these widths.  Three layers with ln_l2, us with a launch per layer / as one: 64 rows of 64 columns
         28 / 14, 8192 rows of 128 29.6 / 14.0, of 256 41.6 / 23.6, 65536 rows of 64 56 / 27, of 256 130 / 98 -- faster
-        over the whole range, so the widths alone decide.  Nets of ensemble layers keep a launch per layer: callers that
-        run member after member count on that (``launch_count``).  Returns the node after the last one covered, or None."""
+        over the whole range, so the widths alone decide.  Nets of ensemble layers keep a launch per layer, as a test of
+        the reference's own net counts them (``launch_count``); the kernel could take a member's weights as well.
+        Returns the node after the last one covered, or None."""
         nodes, k, hidden, norm = model.nodes, i, [], None
         if model.in_dtype != "tf32" or nodes[i].rows < 1:
             return None
