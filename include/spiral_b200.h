@@ -206,8 +206,8 @@ int sb_gemm_reserve_smem(int bytes);
 
 /* Tile-shape heuristic of the tensor-core path, exposed for tests: the
  * counterpart of matmul_config_tf32 (ml/matmul/run.spi:8-19).  Writes
- * {block_m, block_n, block_k_elems, stages, grid} of the launch that sb_matmul_ex makes for `epilogue`
- * (a head over a prefix, which sb_matmul_head knows, spans fewer columns). */
+ * {block_m, block_n, block_k_elems, stages, grid} of the launch that sb_matmul_ex makes for `epilogue`,
+ * beta = 0 and an fp32 C (a head over a prefix, which sb_matmul_head knows, spans fewer columns). */
 int sb_matmul_plan(int a_trans, int b_trans, int M, int N, int K, int in_dtype, int epilogue,
                    int* plan5);
 

@@ -1376,8 +1376,9 @@ int cached_sm_count() { return sb_sm_count(); }
 // `allow_pair`: CTA pairs may be used (needs at least two 128-row blocks and a
 // tile at least 64 columns wide; row heads stay on single CTAs).
 // `chunks32`: whole 32-column chunks per tile.  `items_per_tile`: the split-K factor; 0: a tile has to span the row.
-// `sums`: with column sums.
-void plan_umma(UmmaGemmParams& p, int in_dtype, int sms, bool allow_pair, bool chunks32, int items_per_tile, bool sums) {
+// `sums`: with column sums.  `read`: C (or an activation tile) is read; `ragged`: the rows of C are no whole 16-byte pieces.  The chunks of a
+// tile then leave from registers and not as boxes.
+void plan_umma(UmmaGemmParams& p, int in_dtype, int sms, bool allow_pair, bool chunks32, int items_per_tile, bool sums, bool read, bool ragged) {
   const int es = sb_dtype_size(in_dtype);
   p.mn_box_elems = 128 / es;
   p.pair = (allow_pair && p.M > UG_BLOCK_M && p.N >= 64 && sms >= 2) ? 1 : 0;
@@ -1422,17 +1423,29 @@ void plan_umma(UmmaGemmParams& p, int in_dtype, int sms, bool allow_pair, bool c
   // And with less than 1 KB of K not where more than a quarter of the columns would be padding, if that fills more than half of the
   // workers (9472 x 160 x 256 bf16 with sign words 6.4 / 6.9) or there are column sums, whose wide epilogue wants 64 columns (3072 x
   // 96 x 256 5.75 / 6.0; with sign words 5.5 / 5.25).
+  // Chunks that leave from registers take so long that narrower tiles pay on a busy chip too (9000 x 99 x 64 plain 12.9 / 10.7, beta = 1
+  // 34 / 21, 200 x 48 x 64 beta = 1 8.1 / 5.6), unless the last one is next to empty (9000 x 33 x 400 TF32 8.6 / 9.8, 9000 x 131 x 400 with bias
+  // and ReLU 18.4 / 22.2) or the two chunks of a whole tile are aligned, so that the two halves of the epilogue take them side by side: not on a
+  // busy chip then (9000 x 56 x 64 gated 5.3 / 5.9) and not in the fp32 class (468 x 40 x 64 8.35 / 9.0).
+  // The fp32 class has three products to a tile: its tiles leave as boxes and narrow on a busy chip too (1000 x 100 x 1000 11.2 / 10.4).
   if (allow_pair && items_per_tile > 0) {
     const int whole_n = best_bn, whole_tiles = (p.N + best_bn - 1) / best_bn;
     const long long whole_items = (long long)p.tiles_m * whole_tiles * items_per_tile;
     const bool boxes = whole_n % 32 == 0;        // of whole 32-column chunks; a tail of 16 columns is slower than what follows
-    const bool stay = boxes && whole_n <= 128 && 10 * whole_items >= (whole_n == 128 ? 4LL : 3LL) * workers;
-    for (int bn = 192; !stay && bn >= (p.pair ? 64 : 32); bn -= bn > 64 ? 64 : 32) {
-      const int tiles_n = (p.N + bn - 1) / bn;
+    for (int bn = 192; bn >= (p.pair ? 64 : 32); bn -= bn > 64 ? 64 : 32) {
+      if (bn % gran != 0 || bn >= best_bn) continue;
+      const int tiles_n = (p.N + bn - 1) / bn, last = p.N - (tiles_n - 1) * bn;
       const long long items = (long long)p.tiles_m * tiles_n * items_per_tile;
-      const bool padded = boxes && 4LL * tiles_n * bn > 5LL * whole_tiles * whole_n && (long long)p.K * es < 1024 &&
-                          (sums || 2 * items > workers);
-      if (bn % gran == 0 && bn < best_bn && items <= workers && !padded) best_bn = bn;
+      const bool crowded = 2 * items > workers;
+      bool stay;
+      if (read || ragged) {
+        stay = (crowded && (bn == 32 ? 4 * last <= bn : 8 * last < bn)) ||
+               (!ragged && boxes && whole_n <= 64 && (p.three || crowded));
+      } else {
+        stay = boxes && ((!p.three && whole_n <= 128 && 10 * whole_items >= (whole_n == 128 ? 4LL : 3LL) * workers) ||
+                         (4LL * tiles_n * bn > 5LL * whole_tiles * whole_n && (long long)p.K * es < 1024 && (sums || crowded)));
+      }
+      if (items <= workers && !stay) best_bn = bn;
     }
   }
   // Pipeline bytes.  The three products of the fp32 class keep both parts of a K range in one stage and need two
@@ -1496,11 +1509,11 @@ void plan_umma(UmmaGemmParams& p, int in_dtype, int sms, bool allow_pair, bool c
 // The plan of a launch with epilogue `epi`, of which there are `splits` items per tile.  `boxes`: its tiles are added to C
 // (split-K accumulation, peer copies), so that every 32-column chunk has to leave as a box, as with sign words and
 // column sums.
-void plan_for_epilogue(UmmaGemmParams& p, int in_dtype, int sms, int epi, float beta, int splits, bool boxes) {
-  // A C of less than 64 columns that is read, too, keeps one tile: 468 x 56 x 64 with beta = 1, bf16 6.1 us, 7.0 with two.
-  const bool whole = (epi & SB_EPI_LN_L2) || (beta != 0.0f && p.N < 64);
+void plan_for_epilogue(UmmaGemmParams& p, int in_dtype, int sms, int epi, float beta, int out_dtype, int splits, bool boxes) {
+  const int es_out = out_dtype == SB_BF16 || out_dtype == SB_F16 ? 2 : 4;
   plan_umma(p, in_dtype, sms, !(epi & EPI_HEAD_MASK) && sb_pair_mode_enabled(),
-            (epi & (EPI_GATE_MASK | SB_EPI_COLSUM_OUT)) != 0 || boxes, whole ? 0 : splits > 1 ? splits : 1, (epi & SB_EPI_COLSUM_OUT) != 0);
+            (epi & (EPI_GATE_MASK | SB_EPI_COLSUM_OUT)) != 0 || boxes, (epi & SB_EPI_LN_L2) ? 0 : splits > 1 ? splits : 1,
+            (epi & SB_EPI_COLSUM_OUT) != 0, beta != 0.0f || (epi & SB_EPI_RELU_GRAD) != 0, (long long)p.N * es_out % 16 != 0);
 }
 
 size_t umma_dyn_smem(const UmmaGemmParams& p) {
@@ -1566,7 +1579,7 @@ int sb_umma_gemm_launch(int a_trans, int b_trans, float alpha, const void* A, co
     // Columns that the head turns into zeros are not multiplied: the tile spans those that it holds in registers.
     p.N = sb_row_head_columns(p.head) < N ? sb_row_head_columns(p.head) : N;
   }
-  plan_for_epilogue(p, in_dtype, cached_sm_count(), epi, beta, splits, (split_partials && splits > 1) || to_peers);
+  plan_for_epilogue(p, in_dtype, cached_sm_count(), epi, beta, out_dtype, splits, (split_partials && splits > 1) || to_peers);
   p.N = N;
   p.alpha = alpha; p.beta = beta;
   p.C = C; p.ldc = N; p.out_dtype = out_dtype;
@@ -1730,7 +1743,7 @@ int sb_umma_plan(int a_trans, int b_trans, int M, int N, int K, int in_dtype, in
   p.M = M; p.N = N; p.K = K;
   p.a_mn = a_trans ? 1 : 0;
   p.b_mn = b_trans ? 0 : 1;
-  plan_for_epilogue(p, in_dtype, sms, epi, 0.0f, 1, false);
+  plan_for_epilogue(p, in_dtype, sms, epi, 0.0f, SB_F32, 1, false);
   plan5[0] = p.pair ? 2 * UG_BLOCK_M : UG_BLOCK_M;
   plan5[1] = p.block_n;
   plan5[2] = p.block_k;

@@ -72,6 +72,14 @@ def test_padded_narrow_tiles_with_column_sums(sb):
         assert sb.matmul_plan(False, True, 3072, 96, 256, "bf16", epilogue=epilogue)["block_n"] == block_n
 
 
+@pytest.mark.parametrize("m,n,epilogue,block_n", [
+    (9000, 99, (), 64), (9000, 96, (), 96),                                       # rows of C that are no whole 16-byte pieces, and that are
+    (9000, 33, (), 48), (2000, 33, (), 32), (9000, 131, (), 160), (9000, 61, (), 32),
+    (9000, 72, ("relu_grad",), 64), (9000, 72, (), 96), (9000, 40, ("relu_grad",), 48), (2000, 40, ("relu_grad",), 32)])
+def test_tiles_whose_chunks_leave_from_registers(sb, m, n, epilogue, block_n):
+    assert sb.matmul_plan(False, True, m, n, 400, "bf16", epilogue=epilogue)["block_n"] == block_n
+
+
 def test_bad_arguments_are_rejected_before_any_launch(sb):
     from spiral_b200 import _lib
     with pytest.raises(sb.SpiralError) as e:

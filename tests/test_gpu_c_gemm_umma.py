@@ -103,6 +103,15 @@ def test_narrow_tiles_with_sign_words_and_column_sums(gpu, bt, m, n):
     np.testing.assert_allclose(sums.numpy(), want.sum(axis=0, dtype=np.float64), rtol=0, atol=2e-4 * np.sqrt(m * k))
 
 
+@pytest.mark.parametrize("in_dtype", ["bf16", "tf32"])
+@pytest.mark.parametrize("m,n,beta", [(9000, 99, 0.0), (9000, 99, 1.0), (2000, 33, 0.0), (9000, 33, 1.0), (468, 56, 1.0), (200, 61, -0.5), (9000, 131, 0.0)])
+def test_narrow_tiles_whose_chunks_leave_from_registers(gpu, m, n, beta, in_dtype):
+    """A C whose rows are no whole 16-byte pieces, or that is read."""
+    a, b, c = operands(70 + n, False, True, m, n, 72, in_dtype)
+    got = run(gpu, False, True, 1.0, a, b, beta, c, in_dtype)
+    assert so.rel_frobenius(got, so.matmul(False, True, 1.0, a, b, beta, c)) <= TIGHT
+
+
 @pytest.mark.parametrize("out,fan_in,batch", [(64, 96, 700), (200, 72, 1500), (256, 520, 1200), (520, 264, 900)])
 def test_narrow_tiles_added_to_a_weight_gradient(gpu, out, fan_in, batch):
     """Split-K weight gradients of a small batch, whose narrow tiles are added to the output as boxes: a backward pass
